@@ -356,6 +356,350 @@ __global__ void latent_combine_kernel(const float* __restrict__ part_acc, const 
     }
 }
 
+// ---------------------------------------------------------------------------------
+// Single tokens over a bfloat16 cache, on the tensor cores (mma.sync m16n8k16).  All heads read the same cached rows, so 16
+// heads are the 16 rows of a tile: S = Q K^T over the whole row (L + R values), O += P V with V the same row's first L
+// values, both from one copy of the row in shared memory.  The queries and the probabilities stay 32-bit: each is cut into
+// three bfloat16 numbers whose sum it is (8 + 8 + 8 bits), and each part is multiplied exactly with the bfloat16 row and
+// summed in 32-bit, three products for one.
+// Block = 16 warps, one an SM, one run of keys of one sequence, tiles of 32 keys in four buffers (cp.async, three tiles
+// ahead).  For the scores the warps share the row's steps of 16 values (a warp keeps its KW steps of Q in registers; the
+// partial scores meet in shared memory); for the softmax each takes one of the 16 rows; for the output each takes NW tiles of
+// 8 of the latent's columns.  The next tile's scores are formed beside this tile's values, so that a round of products has
+// work for every warp, and the softmax between two rounds is short.  Bound by mma.sync's rate (a tile is 816 products, the
+// tensor pipe active half of the time and more) and, in small steps, by two launches and one tile's chain.  16 heads, latent
+// 512 + 64, a whole step with its merge, replayed from a graph, before (latent_attn_kernel, plain FMA) and now: 8 sequences of
+// about 4,000 keys 160.6 -> 31.4 us (35 MB), 32 of 2,000 319 -> 73 us, one of 16,384 161.6 -> 28.9 us, one of 64 35.4 -> 10.5 us.
+// With 8 warps, two blocks an SM and the phases one after the other the first was 33 us, the third 38 us.
+// ---------------------------------------------------------------------------------
+#define LD_KEYS 32
+#define LD_MIN_TILES 2                  // tiles a run has at least (where the sequence has them)
+#define LD_WARPS 16
+#define LD_STAGES 4
+#define LD_ROW 40                       // values between rows of the partial scores and of P: accesses without bank conflicts
+
+// A sequence's visible keys in runs of whole tiles of 32, by its own length and window only: from tile `first`, `per` tiles a
+// run, `count` runs (at most `target`).
+struct LatentRuns { int first, per, count; };
+__host__ __device__ __forceinline__ LatentRuns latent_runs(int len, int window, int target) {
+    const int k_lo = window > 0 && len > window ? len - window : 0;
+    const int first = k_lo / LD_KEYS, tiles = (len - 1) / LD_KEYS - first + 1;
+    int per = (tiles + target - 1) / target;
+    if (per < LD_MIN_TILES) per = LD_MIN_TILES;
+    return {first, per, (tiles + per - 1) / per};
+}
+
+__device__ __forceinline__ uint32_t ld_pack(float lo, float hi) {
+    __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);
+    return *reinterpret_cast<uint32_t*>(&v);
+}
+// (x, y) as three packed pairs of bfloat16 whose sums are x and y to 24 bits
+__device__ __forceinline__ void ld_split3(float x, float y, uint32_t* out) {
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+        out[i] = ld_pack(x, y);
+        x -= __uint_as_float(out[i] << 16);
+        y -= __uint_as_float(out[i] & 0xffff0000u);
+    }
+}
+__device__ __forceinline__ void ld_mma(float* d, const uint32_t* a, uint32_t b0, uint32_t b1) {
+    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+                 : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+__device__ __forceinline__ void ld_ldsm(uint32_t* r, const bf16* p) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"((uint32_t)__cvta_generic_to_shared(p)));
+}
+__device__ __forceinline__ void ld_ldsm_trans(uint32_t* r, const bf16* p) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"((uint32_t)__cvta_generic_to_shared(p)));
+}
+
+// 256 KW >= L + R, 128 NW >= L; L and R multiples of 8, pool 16-byte aligned, page_size a multiple of 32.
+template <int KW, int NW>
+__global__ void __launch_bounds__(32 * LD_WARPS, 1)
+latent_decode_mma_kernel(const float* __restrict__ q_abs, const float* __restrict__ q_rot, const bf16* __restrict__ pool,
+                         const int* __restrict__ page_table, const int* __restrict__ pos0, const float* __restrict__ sink,
+                         bf16* __restrict__ out, int n_tok, int H, int L, int R, int page_size, int table_width, float scale,
+                         int window, int target, int max_runs, float* __restrict__ part_acc, float* __restrict__ part_ml) {
+    pdl_wait();
+    pdl_launch_dependents();
+    const int dk = L + R, steps = (dk + 15) / 16, ldk = steps * 16 + 8;     // 16 bytes more than whole steps between rows
+    extern __shared__ __align__(16) unsigned char ld_smem[];
+    float* Sp = reinterpret_cast<float*>(ld_smem);                  // [LD_WARPS][16][LD_ROW]
+    bf16* Pb = reinterpret_cast<bf16*>(Sp + LD_WARPS * 16 * LD_ROW);        // [3][16][LD_ROW]
+    float* rescale = reinterpret_cast<float*>(Pb + 3 * 16 * LD_ROW);        // [16]
+    bf16* Ks = reinterpret_cast<bf16*>(rescale + 16);               // [LD_STAGES][LD_KEYS][ldk]
+    const int b = blockIdx.z, h0 = blockIdx.y * 16;
+    const int len = pos0[b] + 1;
+    const LatentRuns runs = latent_runs(len, window, target);
+    if ((int)blockIdx.x >= runs.count) return;
+    const int tile0 = runs.first + (int)blockIdx.x * runs.per;
+    const int key_first = max(tile0 * LD_KEYS, window > 0 ? len - window : 0), key_end = min((tile0 + runs.per) * LD_KEYS, len);
+    const int kt0 = tile0 * LD_KEYS, n_tiles = (key_end - kt0 + LD_KEYS - 1) / LD_KEYS;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t2 = (lane & 3) * 2;
+    const int* pages = page_table + (size_t)b * table_width;
+
+    auto copy_tile = [&](int t) {                                   // a warp copies two rows; one commit group a tile, also beyond the last
+        const int kt = kt0 + t * LD_KEYS;
+        if (t < n_tiles) {
+            const bf16* src = pool + ((size_t)pages[kt / page_size] * page_size + kt % page_size) * dk;
+            bf16* dst = Ks + (t % LD_STAGES) * LD_KEYS * ldk;
+#pragma unroll
+            for (int r = warp; r < LD_KEYS; r += LD_WARPS) {
+                const bool in = kt + r < key_end;                   // rows beyond the run: zeros
+                const bf16* from = src + (in ? (size_t)r * dk : 0);
+                const uint32_t to = (uint32_t)__cvta_generic_to_shared(dst + r * ldk);
+                for (int c = lane * 8; c < dk; c += 256)
+                    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(to + 2 * c), "l"(from + c), "r"(in ? 16 : 0));
+            }
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    for (int t = 0; t < LD_STAGES - 1; ++t) copy_tile(t);
+    if (dk < steps * 16 && threadIdx.x < LD_STAGES * LD_KEYS)       // the last step's values beyond the row: zeros
+        *reinterpret_cast<uint4*>(Ks + threadIdx.x * ldk + dk) = make_uint4(0, 0, 0, 0);
+
+    // this warp's steps of Q (warp, warp + 16, ...), rows g and g + 8: all asked for, then cut
+    float2 qv[KW][4];
+#pragma unroll
+    for (int k = 0; k < KW; ++k)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            const int h = h0 + g + (e & 1) * 8, d = (warp + LD_WARPS * k) * 16 + t2 + (e >> 1) * 8;
+            const float* from = d < L ? q_abs + ((size_t)h * n_tok + b) * L + d : q_rot + ((size_t)b * H + h) * R + (d - L);
+            qv[k][e] = h < H && d < dk ? *reinterpret_cast<const float2*>(from) : make_float2(0.f, 0.f);
+        }
+    uint32_t qa[KW][3][4];
+#pragma unroll
+    for (int k = 0; k < KW; ++k)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            uint32_t three[3];
+            ld_split3(qv[k][e].x * scale, qv[k][e].y * scale, three);
+            qa[k][0][e] = three[0]; qa[k][1][e] = three[1]; qa[k][2][e] = three[2];
+        }
+    float o[NW][4];
+#pragma unroll
+    for (int j = 0; j < NW; ++j) o[j][0] = o[j][1] = o[j][2] = o[j][3] = 0.f;
+    float m = -INFINITY, l = 0.f;                                   // of row `warp`
+
+    auto scores = [&](int t) {                                      // this warp's part of tile t's scores
+        const bf16* Kt = Ks + (t % LD_STAGES) * LD_KEYS * ldk;
+        float s[4][4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) s[j][0] = s[j][1] = s[j][2] = s[j][3] = 0.f;
+#pragma unroll
+        for (int k = 0; k < KW; ++k) {
+            if (warp + LD_WARPS * k >= steps) continue;
+            const int d = (warp + LD_WARPS * k) * 16 + ((lane >> 3) & 1) * 8;
+            uint32_t kb[2][4];
+#pragma unroll
+            for (int j = 0; j < 2; ++j) ld_ldsm(kb[j], Kt + (j * 16 + (lane & 7) + (lane >> 4) * 8) * ldk + d);
+#pragma unroll
+            for (int i = 0; i < 3; ++i)
+#pragma unroll
+                for (int j = 0; j < 2; ++j) {
+                    ld_mma(s[2 * j], qa[k][i], kb[j][0], kb[j][1]);
+                    ld_mma(s[2 * j + 1], qa[k][i], kb[j][2], kb[j][3]);
+                }
+        }
+        float* mine = Sp + warp * 16 * LD_ROW;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            *reinterpret_cast<float2*>(mine + g * LD_ROW + j * 8 + t2) = make_float2(s[j][0], s[j][1]);
+            *reinterpret_cast<float2*>(mine + (g + 8) * LD_ROW + j * 8 + t2) = make_float2(s[j][2], s[j][3]);
+        }
+    };
+    const int parts = min(LD_WARPS, steps);                         // warps that hold a part of the scores
+    auto softmax = [&](int t) {                                     // row `warp`, a key a lane
+        const int key = kt0 + t * LD_KEYS + lane;
+        const bool seen = key >= key_first && key < key_end;
+        float sum = 0.f;
+#pragma unroll
+        for (int w = 0; w < LD_WARPS; ++w)                          // the warps' parts, in their order
+            if (w < parts) sum += Sp[(w * 16 + warp) * LD_ROW + lane];
+        const float top = fmaxf(m, warp_max(seen ? sum : -INFINITY));       // every tile holds a visible key
+        const float alpha = expf(m - top);
+        float p = seen ? expf(sum - top) : 0.f;
+        l = l * alpha + warp_sum(p);
+        m = top;
+#pragma unroll
+        for (int i = 0; i < 3; ++i) {
+            const bf16 part = __float2bfloat16_rn(p);
+            Pb[(i * 16 + warp) * LD_ROW + lane] = part;
+            p -= __bfloat162float(part);
+        }
+        if (lane == 0) rescale[warp] = alpha;
+    };
+    asm volatile("cp.async.wait_group %0;" ::"n"(LD_STAGES - 2) : "memory");
+    __syncthreads();
+    scores(0);
+    __syncthreads();
+    softmax(0);
+    for (int t = 0; t < n_tiles; ++t) {
+        asm volatile("cp.async.wait_group %0;" ::"n"(LD_STAGES - 3) : "memory");
+        __syncthreads();                                            // tile t + 1 and tile t's P are there; tile t - 1 is read
+        copy_tile(t + LD_STAGES - 1);
+        if (t + 1 < n_tiles) scores(t + 1);
+        const bf16* Kt = Ks + (t % LD_STAGES) * LD_KEYS * ldk;
+        if (t > 0) {
+            const float a0 = rescale[g], a1 = rescale[g + 8];
+#pragma unroll
+            for (int j = 0; j < NW; ++j) { o[j][0] *= a0; o[j][1] *= a0; o[j][2] *= a1; o[j][3] *= a1; }
+        }
+#pragma unroll
+        for (int k = 0; k < 2; ++k) {                               // 16 keys a step
+            uint32_t pa[3][4], vb[(NW + 1) / 2][4];
+#pragma unroll
+            for (int i = 0; i < 3; ++i) ld_ldsm(pa[i], Pb + (i * 16 + (lane & 7) + ((lane >> 3) & 1) * 8) * LD_ROW + k * 16 + (lane >> 4) * 8);
+            const int kr = (k * 16 + (lane & 7) + ((lane >> 3) & 1) * 8) * ldk + (lane >> 4) * 8;
+#pragma unroll
+            for (int j = 0; j < NW; j += 2)
+                if ((warp * NW + j) * 8 < L) ld_ldsm_trans(vb[j / 2], Kt + kr + (warp * NW + j) * 8);
+#pragma unroll
+            for (int i = 0; i < 3; ++i)
+#pragma unroll
+                for (int j = 0; j < NW; j += 2)
+                    if ((warp * NW + j) * 8 < L) {
+                        ld_mma(o[j], pa[i], vb[j / 2][0], vb[j / 2][1]);
+                        ld_mma(o[j + 1], pa[i], vb[j / 2][2], vb[j / 2][3]);
+                    }
+        }
+        __syncthreads();
+        if (t + 1 < n_tiles) softmax(t + 1);
+    }
+    const int row_h = h0 + warp;
+    if (max_runs > 1) {                                             // left for latent_merge_kernel
+        if (lane == 0 && row_h < H) {
+            const size_t at = ((size_t)b * H + row_h) * max_runs + blockIdx.x;
+            part_ml[2 * at] = m; part_ml[2 * at + 1] = l;
+        }
+    } else {                                                        // the rows' factors, for every warp
+        if (lane == 0) {
+            float li = l, f = 1.f;
+            if (sink && row_h < H) {                                // one more term in the denominator, with no value
+                const float top = fmaxf(m, sink[row_h]);
+                f = expf(m - top);
+                li = li * f + expf(sink[row_h] - top);
+            }
+            rescale[warp] = f / li;
+        }
+        __syncthreads();
+    }
+#pragma unroll
+    for (int r = 0; r < 2; ++r) {
+        const int h = h0 + g + 8 * r;
+        if (h >= H) continue;
+        float* acc = part_acc + (((size_t)b * H + h) * max_runs + blockIdx.x) * L;
+        const float f = max_runs > 1 ? 1.f : rescale[g + 8 * r];
+#pragma unroll
+        for (int j = 0; j < NW; ++j) {
+            const int d = (warp * NW + j) * 8 + t2;
+            if (d >= L) continue;
+            if (max_runs > 1) *reinterpret_cast<float2*>(acc + d) = make_float2(o[j][2 * r], o[j][2 * r + 1]);
+            else *reinterpret_cast<uint32_t*>(out + ((size_t)h * n_tok + b) * L + d) = ld_pack(o[j][2 * r] * f, o[j][2 * r + 1] * f);
+        }
+    }
+}
+
+// The runs of one (sequence, head) merged, 128 columns a block: as latent_combine_kernel, with the runs that
+// latent_decode_mma_kernel made.  grid (H, B, ceil(L / 128)).
+#define LD_MAX_RUNS 128
+__global__ void __launch_bounds__(128)
+latent_merge_kernel(const float* __restrict__ part_acc, const float* __restrict__ part_ml, const int* __restrict__ pos0,
+                    const float* __restrict__ sink, bf16* __restrict__ out, int n_tok, int H, int L, int window, int target, int max_runs) {
+    pdl_wait();
+    pdl_launch_dependents();
+    __shared__ float wts[LD_MAX_RUNS], red[2];
+    const int h = blockIdx.x, b = blockIdx.y, tid = threadIdx.x, d = blockIdx.z * 128 + tid;
+    const int count = latent_runs(pos0[b] + 1, window, target).count;
+    const size_t base = ((size_t)b * H + h) * max_runs;
+    float v[16];                                                    // the first runs' values are asked for before the weights are made
+#pragma unroll
+    for (int i = 0; i < 16; ++i) v[i] = i < count && d < L ? part_acc[(base + i) * L + d] : 0.f;
+    const float mine = tid < count ? part_ml[2 * (base + tid)] : -INFINITY, sum = tid < count ? part_ml[2 * (base + tid) + 1] : 0.f;
+    wts[tid] = mine;
+    __syncthreads();
+    if (tid < 32) {
+        float mx = fmaxf(fmaxf(wts[tid], wts[tid + 32]), fmaxf(wts[tid + 64], wts[tid + 96]));
+        mx = warp_max(mx);
+        if (tid == 0) red[0] = sink ? fmaxf(mx, sink[h]) : mx;
+    }
+    __syncthreads();
+    const float M = red[0], f = mine == -INFINITY ? 0.f : expf(mine - M);
+    wts[tid] = sum * f;
+    __syncthreads();
+    if (tid < 32) {
+        const float all = warp_sum(wts[tid] + wts[tid + 32] + wts[tid + 64] + wts[tid + 96]);
+        if (tid == 0) red[1] = 1.f / (all + (sink ? expf(sink[h] - M) : 0.f));
+    }
+    __syncthreads();
+    wts[tid] = f;
+    __syncthreads();
+    if (d >= L) return;
+    float acc = 0.f;
+#pragma unroll
+    for (int i = 0; i < 16; ++i) acc += v[i] * wts[i];
+    for (int r = 16; r < count; r += 16) {
+#pragma unroll
+        for (int i = 0; i < 16; ++i) v[i] = r + i < count ? part_acc[(base + r + i) * L + d] : 0.f;
+#pragma unroll
+        for (int i = 0; i < 16; ++i) acc += v[i] * wts[(r + i) & (LD_MAX_RUNS - 1)];
+    }
+    out[((size_t)h * n_tok + b) * L + d] = from_f32<bf16>(acc * red[1]);
+}
+
+// The most runs of a sequence.  8 sequences of 4,096 keys / one of 16,384 / 32 of 2,048, us: 16 runs 31.7 / 79.8 / 55.5,
+// 32 runs 29.2 / 45.0 / 64.0, 64 runs 31.7 / 28.9 / 73.4, 128 runs 38.5 / 22.1 / 72.5 (more runs: more blocks for one long
+// sequence, more partial results to write and merge for many).
+#define QWB_LATENT_MMA_RUNS 64
+#define QWB_LATENT_MMA_MAX_ROW 640
+
+// Runs a sequence of up to max_len keys has at most; 0: latent_decode_mma does not take these sizes.
+extern "C" int qwb_latent_decode_mma_runs(int dtype, int L, int R, int page_size, int max_len, int window) {
+    if (dtype != QWB_DT_BF16 || L <= 0 || R < 0 || L % 8 || R % 8 || L > 512 || L + R > QWB_LATENT_MMA_MAX_ROW || page_size <= 0 || page_size % LD_KEYS ||
+        max_len <= 0)
+        return 0;
+    int tiles = (max_len + LD_KEYS - 1) / LD_KEYS;
+    if (window > 0) { const int seen = (window + LD_KEYS - 2) / LD_KEYS + 1; tiles = tiles < seen ? tiles : seen; }
+    const int runs = (tiles + LD_MIN_TILES - 1) / LD_MIN_TILES;
+    return runs < QWB_LATENT_MMA_RUNS ? runs : QWB_LATENT_MMA_RUNS;
+}
+
+// One token per sequence; max_runs from qwb_latent_decode_mma_runs (of the bound on the lengths); scratch: max_runs * B * H *
+// (L + 2) floats if max_runs > 1.
+extern "C" int qwb_latent_decode_mma(const float* q_abs, const float* q_rot, const void* pool, const int* page_table, const int* pos0,
+                                     const float* sink, void* out, int B, int H, int L, int R, int page_size, int table_width, float scale,
+                                     int window, int max_runs, float* scratch, cudaStream_t stream) {
+    if (B <= 0) return 0;
+    if (H <= 0 || max_runs < 1 || max_runs > QWB_LATENT_MMA_RUNS || table_width <= 0 || (max_runs > 1 && !scratch) || (uintptr_t)pool % 16 ||
+        (uintptr_t)q_abs % 8 || (uintptr_t)q_rot % 8 || !qwb_latent_decode_mma_runs(QWB_DT_BF16, L, R, page_size, 1, window))
+        return qwb_fail(QWB_ERR_ARG, "latent_decode_mma: %d heads, latent %d + rotated %d, pages of %d, %d runs", H, L, R, page_size, max_runs);
+    if (B > 65535 || H > 65535) return qwb_fail(QWB_ERR_ARG, "latent_decode_mma: batch %d or heads %d are too many", B, H);
+    const int dk = L + R;
+    float* part_acc = scratch;
+    float* part_ml = max_runs > 1 ? scratch + (size_t)max_runs * B * H * L : nullptr;
+#define QWB_LATENT_MMA(KW, NW)                                                                                                     \
+    do {                                                                                                                           \
+        const size_t smem = (size_t)LD_STAGES * LD_KEYS * ((dk + 15) / 16 * 16 + 8) * sizeof(bf16) + 16 * LD_ROW * (LD_WARPS * sizeof(float) + 3 * sizeof(bf16)) + 64; \
+        cudaError_t e = cudaFuncSetAttribute(latent_decode_mma_kernel<KW, NW>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); \
+        if (e != cudaSuccess) return qwb_fail(QWB_ERR_CUDA, "latent_decode_mma: %s", cudaGetErrorString(e));                       \
+        qwb_launch(latent_decode_mma_kernel<KW, NW>, dim3(max_runs, (H + 15) / 16, B), 32 * LD_WARPS, smem, stream, q_abs, q_rot, (const bf16*)pool, \
+                   page_table, pos0, sink, (bf16*)out, B, H, L, R, page_size, table_width, scale, window, QWB_LATENT_MMA_RUNS, max_runs, part_acc, part_ml); \
+    } while (0)
+    if (dk <= 512 && L <= 256) QWB_LATENT_MMA(2, 2);
+    else QWB_LATENT_MMA(3, 4);
+#undef QWB_LATENT_MMA
+    if (int rc = qwb_check_launch("latent_decode_mma")) return rc;
+    if (max_runs > 1) {
+        qwb_launch(latent_merge_kernel, dim3(H, B, (L + 127) / 128), 128, 0, stream, (const float*)part_acc, (const float*)part_ml, pos0, sink,
+                   (bf16*)out, B, H, L, window, QWB_LATENT_MMA_RUNS, max_runs);
+        return qwb_check_launch("latent_merge");
+    }
+    return 0;
+}
+
 #define QWB_LATENT_RUN_KEYS 64
 
 template <typename T>

@@ -1639,6 +1639,17 @@ def latent_attention(q_abs: torch.Tensor, q_rot: torch.Tensor, pool: torch.Tenso
             raise KernelError(f"latent_attention: {sink.numel()} sinks for {H} heads")
     out = torch.empty((H, T, L), dtype=pool.dtype, device=q_abs.device)
     max_runs, scratch = 0, None
+    if ctx.single_token and T == ctx.n_seqs and not (pool.data_ptr() % 16 or q_abs.data_ptr() % 8 or q_rot.data_ptr() % 8):
+        # bfloat16 rows in sizes that the tensor-core kernel takes: runs by each sequence's own length, then a merge
+        max_runs = _lookup("attention_latent", "qwb_latent_decode_mma_runs")[1](_i(_dt(pool.dtype)), _i(L), _i(R), _i(pool.shape[2]),
+                                                                                 _i(ctx.max_len), _i(window))
+    if max_runs:
+        if max_runs > 1:
+            scratch = torch.empty((max_runs * T * H * (L + 2),), dtype=torch.float32, device=q_abs.device)
+        _call("attention_latent", "qwb_latent_decode_mma", _ptr(q_abs), _ptr(q_rot), _ptr(pool), _ptr(page_table), _ptr(ctx.pos0),
+              _ptr(sink), _ptr(out), _i(T), _i(H), _i(L), _i(R), _i(pool.shape[2]), _i(page_table.shape[1]), _f(scale), _i(window),
+              _i(max_runs), _ptr(scratch), _stream(), kernels=2 if max_runs > 1 else 1)
+        return out
     if ctx.single_token and ctx.max_len > LATENT_RUN_KEYS:
         # one token per sequence over more than one run of keys: a block a run (cut by the key's index, so a sequence's
         # result does not depend on the batch), then a merge; ctx.max_len bounds every sequence's length
