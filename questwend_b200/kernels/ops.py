@@ -1321,6 +1321,12 @@ def maps_prefill_mma_fits(dtype: torch.dtype, maps: int, dim: int, vdim: int) ->
     return bool(_lookup("attention_maps", "qwb_maps_prefill_mma_fits")[1](_i(DT_BF16), _i(maps), _i(dim), _i(vdim)))
 
 
+def maps_prefill_tc_fits(dtype: torch.dtype, maps: int, dim: int, vdim: int, group: int) -> bool:
+    """Whether prompts with two maps take the tcgen05 kernel: bfloat16, key and value sizes in multiples of 8 up to 128."""
+    return (MAPS_PREFILL_MMA and dtype == torch.bfloat16 and maps == 2 and 1 <= group <= 64
+            and all(0 < n <= PART_ATTN_MAX_DIM and n % 8 == 0 for n in (dim, vdim)))
+
+
 def maps_attention(q: torch.Tensor, k_pool, v_pool, page_table, ctx, maps: int, scale: float, softcap: float = 0.0,
                    chunk: int = 0, lam: float = 0.0, norm_out: bool = False, eps: float = 0.0, out_scale: float = 1.0,
                    impl: str = "auto", window: int = 0, gate: torch.Tensor | None = None, gate_col0: int = 0) -> torch.Tensor:
@@ -1333,8 +1339,9 @@ def maps_attention(q: torch.Tensor, k_pool, v_pool, page_table, ctx, maps: int, 
     One uncapped map in bfloat16 with keys and values of up to 128 (multiples of 8) is plain grouped-query attention and
     takes its kernels (``impl`` "auto" or "tc"): in steps of one token per sequence the tensor-core decode kernel (all keys
     visible), in others the tcgen05 one.  Else steps of one token per sequence take the kernel for maps that cuts the keys
-    into runs (sizes that are multiples of 8), and other steps the tensor-core kernel for maps where it fits ("mma":
-    mma.sync), else the plain one ("plain")."""
+    into runs (sizes that are multiples of 8); other steps with two maps the tcgen05 kernel with a stream a map where it
+    fits (``impl`` "auto" or "tc"), else the tensor-core kernel for maps where that fits ("mma": mma.sync), else the plain
+    one ("plain")."""
     _need(q, "q", k_pool.dtype, 3)
     T, H, kdim = q.shape
     G, vdim = k_pool.shape[1], v_pool.shape[3]
@@ -1363,6 +1370,13 @@ def maps_attention(q: torch.Tensor, k_pool, v_pool, page_table, ctx, maps: int, 
     if one_map and ctx.max_new * (H // G) >= 64:
         return attn_prefill(q, k_pool, v_pool, page_table, ctx.cu_seqlens, ctx.pos0, ctx.max_new, scale, window=window, impl="tc",
                             chunk=chunk)
+    if (impl in ("auto", "tc") and scale > 0.0 and ctx.max_new * (H // G) >= 64 and maps_prefill_tc_fits(q.dtype, maps, dim, vdim, H // G)
+            and not any(t.data_ptr() % 16 for t in (q, k_pool, v_pool))):
+        _call("attention_streams", "qwb_maps_prefill_tc", _ptr(q), _ptr(k_pool), _ptr(v_pool), _ptr(page_table), _ptr(ctx.cu_seqlens),
+              _ptr(ctx.pos0), _ptr(out), _i(ctx.n_seqs), _i(T), _i(ctx.max_new), _i(k_pool.shape[0]), _i(H), _i(G), _i(dim), _i(vdim), _i(width),
+              _f(scale), _f(softcap), _i(chunk), _i(window), _f(lam), _i(1 if norm_out else 0), _f(eps), _f(out_scale), *gate_args,
+              _ptr(gemm_tc_error_word(q.device)), _stream())
+        return out
     if impl == "mma" or (impl == "auto" and maps_prefill_mma_fits(q.dtype, maps, dim, vdim)):
         _call("attention_maps", "qwb_maps_prefill_mma", _ptr(q), _ptr(k_pool), _ptr(v_pool), _ptr(page_table), _ptr(ctx.cu_seqlens),
               _ptr(ctx.pos0), _ptr(out), _i(ctx.n_seqs), _i(ctx.max_new), _i(H), _i(G), _i(maps), _i(dim), _i(vdim), _i(width),
@@ -1583,6 +1597,15 @@ def latent_prefill_fits(dtype: torch.dtype, dim: int, rot_dim: int, vdim: int, r
             and vdim <= 256 and rank % 8 == 0 and tiles <= 220 * 1024)
 
 
+LATENT_PREFILL_TC = True    # prompts take the tcgen05 kernel where it fits; False: always the mma.sync one
+
+
+def latent_prefill_tc_fits(dim: int, rot_dim: int, vdim: int) -> bool:
+    """Whether the tcgen05 prompt kernel takes these head sizes: up to three pieces of 64 query values, values of up to 128."""
+    return (LATENT_PREFILL_TC and dim > 0 and rot_dim >= 0 and 0 < vdim <= 128 and not (dim % 8 or rot_dim % 8 or vdim % 8)
+            and -(-dim // 64) + -(-rot_dim // 64) <= 3)
+
+
 def latent_prefill(q: torch.Tensor, k_plain: torch.Tensor, rows: torch.Tensor, v: torch.Tensor, ctx, sink, scale: float,
                    window: int, heads: int, dim: int, rot_dim: int, vdim: int, gate: torch.Tensor | None = None,
                    gate_col0: int = 0) -> torch.Tensor:
@@ -1601,6 +1624,12 @@ def latent_prefill(q: torch.Tensor, k_plain: torch.Tensor, rows: torch.Tensor, v
         _need(sink, "sink", torch.float32, 1)
     out = torch.empty((T, heads * vdim), dtype=torch.bfloat16, device=q.device)
     ld = rows.shape[1]
+    if scale > 0.0 and ld % 8 == 0 and latent_prefill_tc_fits(dim, rot_dim, vdim):
+        _call("attention_streams", "qwb_latent_prefill_tc", _ptr(q), _ptr(k_plain),
+              ctypes.c_void_p(rows.data_ptr() + 2 * (ld - rot_dim)), _i(ld), _ptr(v), _ptr(ctx.cu_seqlens), _ptr(sink), _ptr(out),
+              _i(ctx.n_seqs), _i(T), _i(ctx.max_new), _i(heads), _i(dim), _i(rot_dim), _i(vdim), _f(scale), _i(window),
+              *_column_gate("latent_prefill", gate, gate_col0, T, heads), _ptr(gemm_tc_error_word(q.device)), _stream())
+        return out
     _call("attention_latent_mma", "qwb_latent_prefill_mma", _ptr(q), _ptr(k_plain),
           ctypes.c_void_p(rows.data_ptr() + 2 * (ld - rot_dim)), _i(ld), _ptr(v), _ptr(ctx.cu_seqlens), _ptr(sink), _ptr(out),
           _i(ctx.n_seqs), _i(ctx.max_new), _i(heads), _i(dim), _i(rot_dim), _i(vdim), _f(scale), _i(window),

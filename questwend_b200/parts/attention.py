@@ -337,6 +337,8 @@ class ScoreMapsAttention(Mixer):
             mods.append("attention_tc")         # prompts of one uncapped map ...
             if self.chunk == 0:
                 mods.append("attention_mma")    # ... and its single tokens over all keys or a window
+        if ops.maps_prefill_tc_fits(self.runtime.dtype, self.maps, self.head_dim, self.value_dim, self.n_heads // self.n_kv_heads):
+            mods.append("attention_streams")    # prompts of two maps
         return tuple(mods)
 
     def kv_spec(self):

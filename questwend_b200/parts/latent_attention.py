@@ -98,6 +98,8 @@ class LatentAttention(Mixer):
         mods = ["attention_latent", "elementwise", "rope_kv", *linear_modules(self.runtime.dtype)]
         if ops.latent_prefill_fits(self.runtime.dtype, self.dim, self.rot_dim, self.vdim, self.kv_rank):
             mods.append("attention_latent_mma")
+            if ops.latent_prefill_tc_fits(self.dim, self.rot_dim, self.vdim):
+                mods.append("attention_streams")
         return tuple(mods)
 
     def kv_spec(self):

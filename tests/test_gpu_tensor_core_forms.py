@@ -73,3 +73,97 @@ def test_latent_single_tokens_on_the_tensor_cores(H, L, R, window):
             assert (err <= 2.0 ** -8 * ref.abs() + 2e-5).all(), (lens[b], err.max())
     for i, b in enumerate([1, 9, 10]):                      # a sequence's result does not depend on the batch
         assert torch.equal(alone[0][:, b], alone[i + 1][:, 0])
+
+
+# ----------------------------------------------------------------------------- prompts with two softmax streams a block (tcgen05)
+def prompt_step(lens, before=None):
+    before = before or [0] * len(lens)
+    cu = [0]
+    for n in lens:
+        cu.append(cu[-1] + n)
+    return SimpleNamespace(single_token=False, n_seqs=len(lens), max_new=max(lens), max_len=max(n + p for n, p in zip(lens, before)),
+                           cu_seqlens=torch.tensor(cu, device=DEV).int(), pos0=torch.tensor(before, device=DEV).int())
+
+
+def bf16_close(got, ref, spread):
+    """Probabilities and results are bfloat16 (half a unit in the last of 8 bits each): a result's error is at most 2^-8 of
+    itself and 2^-8 of what its probabilities weigh, of which ``spread``, the largest |value|, is a bound that a row's
+    average of rounding errors stays well below."""
+    err = (got.double() - ref).abs()
+    assert torch.isfinite(got).all() and (err <= 2.0 ** -8 * ref.abs() + 2.0 ** -9 * spread).all(), err.max()
+    assert err.square().mean().sqrt() <= 2.0 ** -8 * ref.square().mean().sqrt()
+
+
+@pytest.mark.parametrize("dim, rot, vdim", [(128, 64, 128), (64, 0, 64), (32, 16, 72), (8, 8, 8), (128, 0, 120), (72, 24, 128)])
+@pytest.mark.parametrize("window", [0, 1, 64, 200])
+def test_latent_prompts_with_two_streams(dim, rot, vdim, window):
+    """Prompts at the edges of 64-key tiles, of 128-row streams and of 256-row blocks; a value that is infinite in one
+    sequence stays there."""
+    torch.manual_seed(dim + rot + window)
+    lens, H = [1, 63, 64, 65, 128, 129, 256, 257, 511], 3
+    T = sum(lens)
+    q, k, rows_, v = (torch.randn(s, device=DEV).to(BF) for s in ((T, H, dim + rot), (T, H * dim), (T, 16 + rot), (T, H * vdim)))
+    sink = torch.randn(H, device=DEV) if window != 64 else None
+    gate = torch.randn(T, H, device=DEV) if window else None
+    scale = (dim + rot) ** -0.5
+    for copies in (1, 8):                                   # 8: enough blocks that one takes 256 rows
+        pick = lens * copies
+        step = prompt_step(pick)
+        rep = lambda t: t.repeat(copies, *([1] * (t.dim() - 1)))
+        vv = rep(v)
+        at = sum(lens[:4])                                  # the first token of the fifth sequence
+        vv[at] = math.inf
+        got = ops.latent_prefill(rep(q), rep(k), rep(rows_), vv, step, sink, scale, window, H, dim, rot, vdim,
+                                 gate=None if gate is None else rep(gate)).view(copies, T, H, vdim)
+        start = 0
+        for i, n in enumerate(lens):
+            pos = torch.arange(n, device=DEV)
+            part = slice(start, start + n)
+            for h in range(H):
+                keys = torch.cat([k[part].view(n, H, dim)[:, h], rows_[part, 16:]], 1).double()
+                ref = softmax(q[part, h].double(), keys, v[part].view(n, H, vdim)[:, h].double(), scale, pos, window,
+                              sink=None if sink is None else sink[h].double())
+                ref = ref if gate is None else ref * torch.sigmoid(gate[part, h:h + 1].double())
+                for c in range(copies):
+                    if i != 4 or c:
+                        bf16_close(got[c, part, h], ref, 4.0)
+            start += n
+        ops.gemm_tc_check(DEV)
+
+
+@pytest.mark.parametrize("H, G, dim, vdim", [(16, 4, 64, 128), (2, 2, 8, 8), (6, 2, 40, 72), (4, 1, 128, 128), (3, 1, 72, 64)])
+@pytest.mark.parametrize("softcap, window, chunk, gated", [(0.0, 0, 0, False), (50.0, 0, 0, True), (3.0, 100, 0, False), (0.0, 65, 128, True), (20.0, 0, 96, False)])
+def test_two_map_prompts_with_a_stream_a_map(H, G, dim, vdim, softcap, window, chunk, gated):
+    """Whole prompts and portions behind cached tokens; caps far above the scores (the series) and among them (ex2 and rcp)."""
+    torch.manual_seed(H + dim + window + chunk)
+    lens, before = [1, 63, 64, 130, 300, 33, 64], [0, 0, 0, 0, 0, 70, 191]
+    T = sum(lens)
+    table, (k_pool, v_pool) = paged([n + b for n, b in zip(lens, before)], lambda s: torch.randn(s, device=DEV).to(BF), [(G, 2 * dim), (G, vdim)])
+    q = (2.0 * torch.randn(T, H, 2 * dim, device=DEV)).to(BF)
+    gate = torch.randn(T, H + 3, device=DEV) if gated else None
+    kw = dict(softcap=softcap, window=window, chunk=chunk, lam=0.4, norm_out=True, eps=1e-5, out_scale=0.3, gate=gate, gate_col0=2 if gated else 0)
+    got = ops.maps_attention(q, k_pool, v_pool, table, prompt_step(lens, before), 2, dim ** -0.5, impl="tc", **kw).view(T, H, vdim)
+    start = 0
+    for b, (n, p) in enumerate(zip(lens, before)):
+        ks, vs = rows(k_pool, table[b], n + p), rows(v_pool, table[b], n + p)
+        pos = p + torch.arange(n, device=DEV)
+        for h in range(H):
+            part, g = slice(start, start + n), h // (H // G)
+            a = []
+            for m in (0, 1):
+                ref = torch.empty(n, vdim, dtype=F64, device=DEV)
+                qs, kk = q[part, h, m * dim:(m + 1) * dim].double(), ks[g, :, m * dim:(m + 1) * dim]
+                for c in (range(0, n + p, chunk) if chunk else [0]):      # chunk by chunk
+                    mine = (pos >= c) & (pos < c + chunk) if chunk else torch.ones_like(pos, dtype=torch.bool)
+                    if mine.any():
+                        ref[mine] = softmax(qs[mine], kk[c:], vs[g][c:], dim ** -0.5, pos[mine] - c, window, softcap)
+                a.append(ref)
+            ref = a[0] - 0.4 * a[1]
+            size = ref.square().mean(1, keepdim=True).add(1e-5).rsqrt()
+            ref = ref * size * 0.3
+            size = size * 0.3 * (1.4 * 4.0)
+            if gated:
+                ref, size = ref * torch.sigmoid(gate[part, h + 2:h + 3].double()), size * torch.sigmoid(gate[part, h + 2:h + 3].double())
+            bf16_close(got[part, h], ref, size)
+        start += n
+    ops.gemm_tc_check(DEV)
