@@ -43,6 +43,73 @@ __global__ void short_conv_kernel(const float* __restrict__ x, int ld, const flo
     out[(size_t)t * C + c] = from_f32<TOut>(act == 1 ? silu_f(acc) : (act == 2 ? acc + v : acc));
 }
 
+// The same for 2 to 4 taps and channels in fours (aligned): a thread takes four channels of eight tokens, whose inputs it asks
+// for together and keeps, so that an input is read once and not once a tap.  The sums run in the same order.  One prompt of
+// 2,048 tokens, 6,144 channels, 4 taps: 29 us in ncu (100 MB), about 90 with a channel and a token a thread.
+#define QWB_CONV_TOKENS 8
+__device__ __forceinline__ void conv_store4(float* p, const float* v) { *reinterpret_cast<float4*>(p) = make_float4(v[0], v[1], v[2], v[3]); }
+__device__ __forceinline__ void conv_store4(bf16* p, const float* v) {
+    __nv_bfloat162 a = __floats2bfloat162_rn(v[0], v[1]), b = __floats2bfloat162_rn(v[2], v[3]);
+    *reinterpret_cast<uint2*>(p) = make_uint2(*reinterpret_cast<uint32_t*>(&a), *reinterpret_cast<uint32_t*>(&b));
+}
+template <typename TOut, int TAPS>
+__global__ void __launch_bounds__(128)
+short_conv4_kernel(const float* __restrict__ x, int ld, const float* __restrict__ w, const float* __restrict__ bias, const float* __restrict__ in_bias,
+                   const float* tail, const int* __restrict__ tok_seq, const int* __restrict__ cu_seqlens, const int* __restrict__ slots,
+                   TOut* __restrict__ out, int T, int C, int act) {
+    pdl_wait();
+    pdl_launch_dependents();
+    const int c = (blockIdx.y * 128 + threadIdx.x) * 4, t_first = blockIdx.x * QWB_CONV_TOKENS;
+    if (c >= C) return;
+    const int n = min(QWB_CONV_TOKENS, T - t_first);
+    auto four = [](const float* p, float* v) { const float4 q = *reinterpret_cast<const float4*>(p); v[0] = q.x; v[1] = q.y; v[2] = q.z; v[3] = q.w; };
+    float in[QWB_CONV_TOKENS][4];
+#pragma unroll
+    for (int k = 0; k < QWB_CONV_TOKENS; ++k) four(x + (size_t)(t_first + min(k, n - 1)) * ld + c, in[k]);
+    float wv[4 * TAPS], b4[4] = {0.f, 0.f, 0.f, 0.f}, ib[4] = {0.f, 0.f, 0.f, 0.f}, before[TAPS - 1][4];
+#pragma unroll
+    for (int k = 0; k < TAPS; ++k) four(w + (size_t)c * TAPS + 4 * k, wv + 4 * k);      // [channel][tap]
+    if (bias) four(bias + c, b4);
+    if (in_bias) four(in_bias + c, ib);
+    int b = -1, start = 0;
+#pragma unroll
+    for (int k = 0; k < QWB_CONV_TOKENS; ++k) {
+        if (k >= n) break;
+        const int t = t_first + k;
+        if (b < 0 || t == start) {                                  // the block's first token, or a sequence's: what came before it
+            b = tok_seq[t];
+            const int i = t - cu_seqlens[b];
+            start = cu_seqlens[b + 1];
+            const float* tl = tail + (size_t)slots[b] * (TAPS - 1) * C + c;
+#pragma unroll
+            for (int r = 0; r < TAPS - 1; ++r) {
+                const int src = i - (TAPS - 1) + r;
+                if (src >= 0) {
+                    four(x + (size_t)(t - (TAPS - 1) + r) * ld + c, before[r]);
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) before[r][e] += ib[e];
+                } else {
+                    four(tl + (size_t)(TAPS - 1 + src) * C, before[r]);
+                }
+            }
+        }
+        float v[4];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            const float cur = in[k][e] + ib[e];
+            float acc = b4[e];
+#pragma unroll
+            for (int r = 0; r < TAPS - 1; ++r) acc += wv[e * TAPS + r] * before[r][e];
+            acc += wv[e * TAPS + TAPS - 1] * cur;
+            v[e] = act == 1 ? silu_f(acc) : (act == 2 ? acc + cur : acc);
+#pragma unroll
+            for (int r = 0; r < TAPS - 2; ++r) before[r][e] = before[r + 1][e];
+            before[TAPS - 2][e] = cur;
+        }
+        conv_store4(out + (size_t)t * C + c, v);
+    }
+}
+
 // The tail after the step: the last taps - 1 inputs of each sequence (new ones, then what is left of the old tail).
 __global__ void conv_tail_kernel(const float* __restrict__ x, int ld, const float* __restrict__ in_bias, float* tail,
                                  const int* __restrict__ cu_seqlens, const int* __restrict__ slots, int B, int C, int taps) {
@@ -94,7 +161,14 @@ static int launch_short_conv(const float* x, int ld, const float* w, const float
         qwb_launch(short_conv_step_kernel<TOut>, dim3(B, (C + block - 1) / block), block, 0, stream, x, ld, w, bias, in_bias, tail, slots, out, B, C, taps, act, update_tail);
         return qwb_check_launch("short_conv_step");
     }
-    qwb_launch(short_conv_kernel<TOut>, dim3(T, (C + block - 1) / block), block, 0, stream, x, ld, w, bias, in_bias, (const float*)tail, tok_seq, cu_seqlens, slots, out, T, C, taps, act);
+    bool fours = taps >= 2 && taps <= 4 && C % 4 == 0 && ld % 4 == 0 && (uintptr_t)out % (4 * sizeof(TOut)) == 0;
+    for (const void* p : {(const void*)x, (const void*)w, (const void*)bias, (const void*)in_bias, (const void*)tail}) fours = fours && (uintptr_t)p % 16 == 0;
+    if (fours) {
+        auto kernel = taps == 2 ? short_conv4_kernel<TOut, 2> : (taps == 3 ? short_conv4_kernel<TOut, 3> : short_conv4_kernel<TOut, 4>);
+        qwb_launch(kernel, dim3((T + QWB_CONV_TOKENS - 1) / QWB_CONV_TOKENS, (C / 4 + 127) / 128), 128, 0, stream, x, ld, w, bias, in_bias, (const float*)tail, tok_seq, cu_seqlens, slots, out, T, C, act);
+    } else {
+        qwb_launch(short_conv_kernel<TOut>, dim3(T, (C + block - 1) / block), block, 0, stream, x, ld, w, bias, in_bias, (const float*)tail, tok_seq, cu_seqlens, slots, out, T, C, taps, act);
+    }
     if (int rc = qwb_check_launch("short_conv")) return rc;
     if (update_tail && taps > 1) {
         qwb_launch(conv_tail_kernel, dim3((C + block - 1) / block, B), block, 0, stream, x, ld, in_bias, tail, cu_seqlens, slots, B, C, taps);

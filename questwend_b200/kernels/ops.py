@@ -889,11 +889,19 @@ def short_conv(x: torch.Tensor, col0: int, channels: int, weight: torch.Tensor, 
     return out
 
 
+# Tokens of a step's longest sequence from which the recurrence runs in chunks (csrc/recurrent_chunks.cu).  With its
+# convolution, 64 heads of 64 x 128, us, scan / chunks: 64 tokens 33 / 42, 100 tokens 48 / 48, three sequences of 67 80 / 64,
+# 400 tokens 179 / 74.
+SSM_CHUNKED_FROM = 96
+CHUNK_SCRATCH_MAX = 1 << 30     # floats of scratch memory that a chunked form may take; a longer prompt runs as a scan
+
+
 def ssm_scan(xbc: torch.Tensor, dt: torch.Tensor, dt_col0: int, dt_bias, a_log, d_skip, state: torch.Tensor, ctx,
              heads: int, vdim: int, n_state: int, groups: int, write_state: bool = True) -> torch.Tensor:
     """The Mamba-2 recurrence over a step's tokens.  ``xbc`` float32 [T, heads * vdim + 2 * groups * n_state] (x | B | C,
     after convolution and SiLU); the raw step sizes are columns ``dt_col0 ..`` of float32 ``dt`` [T, ld]; ``state``
-    float32 [slots, heads, vdim, n_state] (column by column) is read and written back.  Returns y float32 [T, heads * vdim]."""
+    float32 [slots, heads, vdim, n_state] (column by column) is read and written back.  Steps with a sequence of at least
+    ``SSM_CHUNKED_FROM`` tokens run in chunks of 128.  Returns y float32 [T, heads * vdim]."""
     _need(xbc, "xbc", torch.float32, 2)
     _need(dt, "dt", torch.float32, 2)
     _need(state, "state", torch.float32, 4)
@@ -906,6 +914,17 @@ def ssm_scan(xbc: torch.Tensor, dt: torch.Tensor, dt_col0: int, dt_bias, a_log, 
         if t.numel() != heads:
             raise KernelError(f"ssm_scan: {name} has {t.numel()} entries for {heads} heads")
     y = torch.empty((T, heads * vdim), dtype=torch.float32, device=xbc.device)
+    if ctx.max_new >= SSM_CHUNKED_FROM and xbc.shape[1] % 4 == 0 and not (xbc.data_ptr() % 16 or state.data_ptr() % 16):
+        lib, size = _lookup("recurrent_chunks", "qwb_ssm_chunked_scratch")
+        size.restype = ctypes.c_longlong
+        floats = size(_i(T), _i(ctx.n_seqs), _i(heads), _i(vdim), _i(n_state), _i(groups))
+        if 0 < floats <= CHUNK_SCRATCH_MAX:
+            scratch = torch.empty((floats,), dtype=torch.float32, device=xbc.device)
+            _call("recurrent_chunks", "qwb_ssm_chunked", _ptr(xbc), _i(xbc.shape[1]), ctypes.c_void_p(dt.data_ptr() + 4 * dt_col0),
+                  _i(dt.shape[1]), _ptr(dt_bias), _ptr(a_log), _ptr(d_skip), _ptr(state), _ptr(ctx.cu_seqlens), _ptr(ctx.slots), _ptr(y),
+                  _ptr(scratch), _i(T), _i(ctx.n_seqs), _i(ctx.max_new), _i(heads), _i(vdim), _i(n_state), _i(groups),
+                  _i(1 if write_state else 0), _stream(), kernels=3)
+            return y
     _call("recurrent", "qwb_ssm_scan", _ptr(xbc), _i(xbc.shape[1]), ctypes.c_void_p(dt.data_ptr() + 4 * dt_col0),
           _i(dt.shape[1]), _ptr(dt_bias), _ptr(a_log), _ptr(d_skip), _ptr(state), _ptr(ctx.cu_seqlens), _ptr(ctx.slots),
           _ptr(y), _i(ctx.n_seqs), _i(heads), _i(vdim), _i(n_state), _i(groups), _i(1 if write_state else 0), _stream())

@@ -70,7 +70,7 @@ class Mamba2Mixer(Mixer):
         self.norm_w = _f32(weights, px + n["norm"])
 
     def kernel_modules(self):
-        return ("recurrent", *linear_modules(self.runtime.dtype))
+        return ("recurrent", "recurrent_chunks", *linear_modules(self.runtime.dtype))
 
     def state_spec(self):
         return (StateSpec((self.taps - 1, self.channels), torch.float32),

@@ -167,3 +167,79 @@ def test_two_map_prompts_with_a_stream_a_map(H, G, dim, vdim, softcap, window, c
             bf16_close(got[part, h], ref, size)
         start += n
     ops.gemm_tc_check(DEV)
+
+
+# ----------------------------------------------------------------------------- recurrences in chunks
+class Steps(SimpleNamespace):
+    """What a recurrence reads of a step: sequences with these numbers of tokens, in these slots."""
+
+    def __init__(self, counts, slots):
+        cu = [0]
+        for n in counts:
+            cu.append(cu[-1] + n)
+        seq = [b for b, n in enumerate(counts) for _ in range(n)]
+        super().__init__(cu_seqlens=torch.tensor(cu, device=DEV).int(), slots=torch.tensor(slots, device=DEV).int(), n_seqs=len(counts),
+                         max_new=max(counts), single_token=all(n == 1 for n in counts), tok_seq=torch.tensor(seq, device=DEV).int())
+
+
+def sums_close(got, ref, terms=2 ** -15):
+    """32-bit sums of a few hundred terms of either sign: far below 2^-15 of the largest."""
+    err = (got.double() - ref).abs().max()
+    assert torch.isfinite(got).all() and err <= terms * ref.abs().max(), err / ref.abs().max()
+
+
+@pytest.mark.parametrize("H, P, N, G", [(2, 64, 128, 1), (4, 4, 4, 2), (3, 68, 132, 3), (8, 32, 64, 2), (2, 128, 256, 1)])
+@pytest.mark.parametrize("pace", [0.01, 1.0, 40.0])
+def test_mamba2_in_chunks(H, P, N, G, pace):
+    """Sequences at the edges of the chunks of 128, from a state, with slow, usual and immediate decays; the scan, which takes
+    shorter steps, gives the same; slots of others stay as they are."""
+    torch.manual_seed(H + P + N)
+    lens, slots = [1, 64, 127, 128, 129, 300], [4, 2, 7, 1, 5, 3]       # the longest one sends the step into chunks
+    T, inner = sum(lens), H * P
+    step = Steps(lens, slots)
+    xbc, dt = torch.randn(T, inner + 2 * G * N, device=DEV), torch.randn(T, H + 5, device=DEV)
+    bias, a_log, d = torch.randn(H, device=DEV), torch.log(pace * (1 + torch.rand(H, device=DEV))), torch.randn(H, device=DEV)
+    start = torch.randn(9, H, P, N, device=DEV)
+    state, again = start.clone(), start.clone()
+    y = ops.ssm_scan(xbc, dt, 3, bias, a_log, d, state, step, H, P, N, G)
+    step.max_new = 1                                        # taken for a short step: the scan
+    y_scan = ops.ssm_scan(xbc, dt, 3, bias, a_log, d, again, step, H, P, N, G)
+    t = 0
+    for n, slot in zip(lens, slots):
+        S = start[slot].double()
+        ref = torch.empty(n, inner, dtype=F64, device=DEV)
+        for i in range(n):
+            row = xbc[t + i].double()
+            x, (b, c) = row[:inner].view(H, P), (row[inner + k * G * N:inner + (k + 1) * G * N].view(G, N).repeat_interleave(H // G, 0) for k in (0, 1))
+            s = torch.nn.functional.softplus(dt[t + i, 3:3 + H].double() + bias.double(), threshold=100.0)
+            S = torch.exp(-torch.exp(a_log.double()) * s)[:, None, None] * S + (s[:, None] * x)[:, :, None] * b[:, None, :]
+            ref[i] = ((S @ c[:, :, None])[..., 0] + d.double()[:, None] * x).reshape(-1)
+        for got, st in ((y, state), (y_scan, again)):
+            sums_close(got[t:t + n], ref)
+            sums_close(st[slot], S)
+        t += n
+    assert torch.equal(state[[0, 6, 8]], start[[0, 6, 8]])
+    step.max_new, before = max(lens), state.clone()
+    ops.ssm_scan(xbc, dt, 3, bias, a_log, d, state, step, H, P, N, G, write_state=False)
+    assert torch.equal(state, before)
+
+
+@pytest.mark.parametrize("taps, C", [(2, 4), (3, 20), (4, 516), (4, 24)])
+@pytest.mark.parametrize("mode", ["silu", "plain", "plus", "bf16"])
+def test_convolutions_of_four_channels_a_thread(taps, C, mode):
+    """Sequences that begin and end inside a block of eight tokens, against the kernel of one channel a thread (a row that is
+    shifted by one float takes it): the same bits."""
+    torch.manual_seed(taps + C)
+    lens, slots = [3, 1, 9, 8, 40, 2], [1, 0, 5, 3, 2, 6]
+    step, T = Steps(lens, slots), sum(lens)
+    wide = torch.randn(T, C + 8, device=DEV)
+    shifted = torch.zeros(T, C + 8, device=DEV)
+    shifted[:, 1:] = wide[:, :-1]
+    w, bias, in_bias = torch.randn(C, taps, device=DEV), torch.randn(C, device=DEV), torch.randn(C, device=DEV)
+    tail = torch.randn(7, taps - 1, C, device=DEV)
+    kw = dict(activation=mode == "silu", plus_input=mode == "plus", out_dtype=BF if mode == "bf16" else torch.float32,
+              in_bias=in_bias if mode != "silu" else None)
+    a, b = tail.clone(), tail.clone()
+    got = ops.short_conv(wide, 4, C, w, bias if mode != "plain" else None, a, step, **kw)
+    one = ops.short_conv(shifted, 5, C, w, bias if mode != "plain" else None, b, step, **kw)
+    assert torch.equal(got, one) and torch.equal(a, b)
