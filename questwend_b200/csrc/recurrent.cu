@@ -425,6 +425,7 @@ __global__ void delta_prep_kernel(float* qkv, int ld, float* __restrict__ kq, co
         if (lane == 0) kq[(size_t)t * Hk + kh] = dot;
     }
     for (int i = threadIdx.x; i < H; i += blockDim.x) beta[(size_t)t * H + i] = sigmoid_f(b_raw[(size_t)t * ld_b + i]);
+    if (!decay) return;                                             // the chunked form makes its own from the raw ones
     for (int i = threadIdx.x; i < H * decay_k; i += blockDim.x)
         decay[(size_t)t * H * decay_k + i] = expf(-expf(A_log[i / decay_k]) * softplus_f(a_raw[(size_t)t * ld_a + i] + dt_bias[i]));
 }

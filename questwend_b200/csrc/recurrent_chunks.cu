@@ -408,3 +408,512 @@ extern "C" int qwb_ssm_chunked(const float* xbc, int ldx, const float* dt_raw, i
     qwb_launch(ssm_chunk_out_kernel, dim3(chunks, H * ptiles, B), 128, 0, stream, a, ptiles);
     return qwb_check_launch("ssm_chunk_out");
 }
+
+// ---------------------------------------------------------------------------------
+// The gated delta rule in chunks of 64 tokens.  Per head, S (K x P), with l_t the log decays of token t per key channel and
+// e_ij = exp(sum of l over the tokens behind j up to i) per channel,
+//     u_i = beta_i (v_i - S0^T (k_i e_i0) - sum_{j < i} A_ij u_j),    A_ij = k_i . (k_j e_ij)
+//     o_i = S0^T (q_i e_i0) + sum_{j <= i} Q_ij u_j,                  Q_ij = q_i . (k_j e_ij)
+//     S_end = e_end,0 S0 + sum_j (k_j e_end,j) u_j^T
+// (S0: the state at the chunk's start, e_i0: the decays of its tokens up to i).  The equations of a chunk's u are triangular;
+// solved for the right-hand sides beta v and beta k e_i0 instead of what depends on S0 they give u = U - W S0.  Three kernels:
+//   delta_chunk_prep   every chunk by itself: A, Q, U and W by forward substitution, k e_end,j and q e_i0
+//   delta_chunk_walk   a sequence's chunks in order: u = U - W S0, then the next S0; 16 value columns of a head a block
+//   delta_chunk_out    every chunk by itself: o
+// A decay per channel does not factor into a number of i and a number of j that are both small, so the tokens are taken in
+// sub-blocks of 16: inside one, every pair and channel has an exponential of its own; between two, what decays behind j up to
+// its sub-block's end, what decays in the sub-blocks between, and what decays from the start of i's sub-block to i are three
+// factors of at most 1.  Sums of logarithms (base 2) span what they decay and nothing else.
+// Chunk c of sequence b is place cu_seqlens[b] / 64 + b + c of the scratch memory, which T / 64 + B places hold.
+// 16 heads of 128 x 128 with a decay per channel, the convolution before it, the scan and now: 2,048 tokens 955 -> 323 us (prep 121,
+// walk 131, out 49 in ncu), three sequences of 2,900 in all 1,194 -> 472 us; a decay per head, four of 4,096 in all, 1,198 -> 588 us.
+// Bound by what shared memory hands to registers (128 bytes a cycle), the walk more than the others.
+// Scratch of a place and head:
+//     W [64][K] | k e_end [64][K] | q e_0 [64][K] | Q [64 (j)][64 (i)] | U, then u [64][P] | decay of the chunk [K] | S0 [K][P]
+// ---------------------------------------------------------------------------------
+#define DC_TOKENS 64
+#define DC_SUB 16
+#define DC_MAX_K 128
+#define DC_WALK_P 16
+
+struct DcArgs {
+    const float *qkv, *beta, *a_raw, *dt_bias, *A_log;
+    const int *cu_seqlens, *slots;
+    float *state, *o, *scratch;
+    int ld, ld_a, H, Hk, K, P, decay_k, write_state;
+};
+struct DcPlace { float *w, *k_end, *q0, *q_pairs, *u, *decay, *start; };
+__host__ __device__ __forceinline__ size_t dc_floats(int K, int P) {      // of one place and head: a multiple of 4
+    return (size_t)3 * K * DC_TOKENS + DC_TOKENS * DC_TOKENS + (size_t)DC_TOKENS * P + K + (size_t)K * P;
+}
+__device__ __forceinline__ DcPlace dc_place(const DcArgs& a, int b, int c, int h) {
+    const size_t place = (size_t)(a.cu_seqlens[b] / DC_TOKENS + b + c);
+    DcPlace p;
+    p.w = a.scratch + (place * a.H + h) * dc_floats(a.K, a.P);
+    p.k_end = p.w + a.K * DC_TOKENS;
+    p.q0 = p.k_end + a.K * DC_TOKENS;
+    p.q_pairs = p.q0 + a.K * DC_TOKENS;
+    p.u = p.q_pairs + DC_TOKENS * DC_TOKENS;
+    p.decay = p.u + DC_TOKENS * a.P;
+    p.start = p.decay + a.K;
+    return p;
+}
+__device__ __forceinline__ float dc_exp2(float x) {
+    float y;
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+}
+// Place of channel k of token `row` in a tile of 64 x 128: odd rows have their 16-byte pieces four apart exchanged, so that two
+// threads' groups of four that read neighbouring rows at the same channels meet in no bank.
+__device__ __forceinline__ int dc_at(int row, int k) { return row * DC_MAX_K + (k ^ ((row & 1) << 4)); }
+// beta_i A_ij, token j by token j: behind each other the 16 rows of a sub-block's tokens, a row holding i from the sub-block's
+// first token to 63 (64, 48, 32 or 16 values)
+#define DC_A_FLOATS 2560
+__device__ __forceinline__ int dc_row(int j) { const int s = j / DC_SUB; return 16 * (64 * s - 8 * s * (s - 1)) + (j % DC_SUB) * (64 - 16 * s) - 16 * s; }
+__device__ __forceinline__ float dc_quad_sum(float v) {
+    v += __shfl_xor_sync(0xffffffffu, v, 1);
+    return v + __shfl_xor_sync(0xffffffffu, v, 2);
+}
+
+// grid (chunks, H, B), 256 threads; dynamic shared memory: 3 x [64][128], A, totals [4][128], beta [64] (two blocks an SM)
+__global__ void __launch_bounds__(256, 2)
+delta_chunk_prep_kernel(const DcArgs a) {
+    pdl_wait();
+    pdl_launch_dependents();
+    extern __shared__ __align__(16) float dc_smem[];
+    float* ks = dc_smem;                                            // k; then k times what decays behind it
+    float* qs = ks + DC_TOKENS * DC_MAX_K;                             // q; then q times what decays from its sub-block's start on
+    float* gs = qs + DC_TOKENS * DC_MAX_K;                             // sums of logarithms in the sub-block; then k as q
+    float* As = gs + DC_TOKENS * DC_MAX_K;                             // beta_i A_ij
+    float* totals = As + DC_A_FLOATS;                               // [4][128]
+    float* beta = totals + 4 * DC_MAX_K;
+    const int c = blockIdx.x, h = blockIdx.y, b = blockIdx.z, tid = threadIdx.x, K = a.K, P = a.P;
+    const int t0 = a.cu_seqlens[b] + c * DC_TOKENS, n = min(DC_TOKENS, a.cu_seqlens[b + 1] - t0);
+    if (n <= 0) return;
+    const DcPlace at = dc_place(a, b, c, h);
+    const int kh = h / (a.H / a.Hk);
+    const float rate = -expf(a.A_log[h]) * 1.4426950408889634f;
+    if (tid < DC_TOKENS) beta[tid] = tid < n ? a.beta[(size_t)(t0 + tid) * a.H + h] : 0.f;
+    const int warp = tid >> 5, e_lane = (tid & 31) * 4;             // a warp takes every eighth token, a lane four channels
+    if (e_lane < K) {
+        float bias[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) bias[i] = a.dt_bias[a.decay_k == 1 ? h : h * K + e_lane + i];
+#pragma unroll
+        for (int half = 0; half < 2; ++half) {                      // four tokens' loads at a time
+            float4 q[4], k[4];
+            float raw[4][4];
+#pragma unroll
+            for (int r = 0; r < 4; ++r) {
+                const int j = warp + 8 * (4 * half + r);
+                const float* row = a.qkv + (size_t)(t0 + (j < n ? j : 0)) * a.ld + kh * K + e_lane;
+                q[r] = rc_load4(row, j < n);
+                k[r] = rc_load4(row + a.Hk * K, j < n);
+                const float* decays = a.a_raw + (size_t)(t0 + (j < n ? j : 0)) * a.ld_a + (a.decay_k == 1 ? h : h * K + e_lane);
+#pragma unroll
+                for (int i = 0; i < 4; ++i) raw[r][i] = decays[a.decay_k == 1 ? 0 : i];
+            }
+#pragma unroll
+            for (int r = 0; r < 4; ++r) {
+                const int j = warp + 8 * (4 * half + r);
+                float g[4];
+                g[0] = rate * rc_softplus(raw[r][0] + bias[0]);
+#pragma unroll
+                for (int i = 1; i < 4; ++i) g[i] = a.decay_k == 1 ? g[0] : rate * rc_softplus(raw[r][i] + bias[i]);
+                *reinterpret_cast<float4*>(qs + dc_at(j, e_lane)) = q[r];
+                *reinterpret_cast<float4*>(ks + dc_at(j, e_lane)) = k[r];
+                *reinterpret_cast<float4*>(gs + dc_at(j, e_lane)) = j < n ? make_float4(g[0], g[1], g[2], g[3]) : make_float4(0.f, 0.f, 0.f, 0.f);
+            }
+        }
+    }
+    __syncthreads();
+    for (int idx = tid; idx < 4 * DC_MAX_K; idx += 256) {           // sums in the sub-blocks
+        const int s = idx / DC_MAX_K, k = idx - s * DC_MAX_K;
+        if (k >= K) continue;
+        float sum = 0.f;
+#pragma unroll
+        for (int j = 0; j < DC_SUB; ++j) {
+            sum += gs[dc_at(s * DC_SUB + j, k)];
+            gs[dc_at(s * DC_SUB + j, k)] = sum;
+        }
+        totals[idx] = sum;
+    }
+    __syncthreads();
+    // pairs of one sub-block, four threads a pair: 136 with j <= i of each
+    const int lane4 = (tid & 3) * 4;
+    for (int task = tid >> 2; task < 4 * 136; task += 64) {         // 544 = 8.5 rounds of 64: the last one half full, by whole warps
+        const int s = task / 136, t = task - s * 136;
+        int i = (int)((sqrtf(8.f * (float)t + 1.f) - 1.f) * 0.5f);
+        while ((i + 1) * (i + 2) / 2 <= t) ++i;
+        while (i * (i + 1) / 2 > t) --i;
+        const int j = t - i * (i + 1) / 2, ri = s * DC_SUB + i, rj = s * DC_SUB + j;
+        float sa = 0.f, sq = 0.f;
+#pragma unroll 4
+        for (int k = lane4; k < K; k += 16) {
+            const int pi = dc_at(ri, k), pj = dc_at(rj, k);
+            const float4 gi = *reinterpret_cast<const float4*>(gs + pi), gj = *reinterpret_cast<const float4*>(gs + pj);
+            const float4 ki = *reinterpret_cast<const float4*>(ks + pi), kj = *reinterpret_cast<const float4*>(ks + pj);
+            const float4 qi = *reinterpret_cast<const float4*>(qs + pi);
+            const float x = kj.x * dc_exp2(gi.x - gj.x), y = kj.y * dc_exp2(gi.y - gj.y), z = kj.z * dc_exp2(gi.z - gj.z), w = kj.w * dc_exp2(gi.w - gj.w);
+            sa += ki.x * x + ki.y * y + ki.z * z + ki.w * w;
+            sq += qi.x * x + qi.y * y + qi.z * z + qi.w * w;
+        }
+        sa = dc_quad_sum(sa);
+        sq = dc_quad_sum(sq);
+        if (lane4 == 0) {
+            const int gi_ = s * DC_SUB + i, gj_ = s * DC_SUB + j;
+            if (j < i) As[dc_row(gj_) + gi_] = beta[gi_] * sa;
+            at.q_pairs[gj_ * DC_TOKENS + gi_] = sq;
+            if (j < i) at.q_pairs[gi_ * DC_TOKENS + gj_] = 0.f;
+        }
+    }
+    __syncthreads();
+    // q and k by what decays from their sub-block's start on (k's into gs), k by what decays behind it in the sub-block
+#pragma unroll 4
+    for (int j = warp; j < DC_TOKENS && e_lane < K; j += 8) {
+        const int e = e_lane, s = j / DC_SUB;
+        float4* gp = reinterpret_cast<float4*>(gs + dc_at(j, e));
+        float4* kp = reinterpret_cast<float4*>(ks + dc_at(j, e));
+        float4* qp = reinterpret_cast<float4*>(qs + dc_at(j, e));
+        const float4 g = *gp, k = *kp, q = *qp, tot = *reinterpret_cast<const float4*>(totals + s * DC_MAX_K + e);
+        const float4 f = make_float4(dc_exp2(g.x), dc_exp2(g.y), dc_exp2(g.z), dc_exp2(g.w));
+        *gp = make_float4(k.x * f.x, k.y * f.y, k.z * f.z, k.w * f.w);
+        *qp = make_float4(q.x * f.x, q.y * f.y, q.z * f.z, q.w * f.w);
+        *kp = make_float4(k.x * dc_exp2(tot.x - g.x), k.y * dc_exp2(tot.y - g.y), k.z * dc_exp2(tot.z - g.z), k.w * dc_exp2(tot.w - g.w));
+    }
+    // pairs of two sub-blocks: rows of sub-block s with all before it, 2 x 2 pairs to four threads
+    for (int s = 1; s < 4; ++s) {
+        __syncthreads();
+        if (s > 1) {                                                // the sub-block between has decayed too
+            for (int j = warp; j < (s - 1) * DC_SUB && e_lane < K; j += 8) {
+                const int e = e_lane;
+                float4* kp = reinterpret_cast<float4*>(ks + dc_at(j, e));
+                const float4 k = *kp, tot = *reinterpret_cast<const float4*>(totals + (s - 1) * DC_MAX_K + e);
+                *kp = make_float4(k.x * dc_exp2(tot.x), k.y * dc_exp2(tot.y), k.z * dc_exp2(tot.z), k.w * dc_exp2(tot.w));
+            }
+            __syncthreads();
+        }
+        for (int round = 0; round < s; ++round) {                   // sub-block `round` against sub-block s: 64 tiles of 2 x 2
+            const int task = tid >> 2, i = task >> 3, j = task & 7;
+            const int i0 = s * DC_SUB + i, j0 = round * DC_SUB + j;
+            float sa[2][2] = {{0.f, 0.f}, {0.f, 0.f}}, sq[2][2] = {{0.f, 0.f}, {0.f, 0.f}};
+#pragma unroll 2
+            for (int k = lane4; k < K; k += 16) {
+                float4 l[2], q[2], r[2];
+#pragma unroll
+                for (int e = 0; e < 2; ++e) {
+                    l[e] = *reinterpret_cast<const float4*>(gs + dc_at(i0 + 8 * e, k));
+                    q[e] = *reinterpret_cast<const float4*>(qs + dc_at(i0 + 8 * e, k));
+                    r[e] = *reinterpret_cast<const float4*>(ks + dc_at(j0 + 8 * e, k));
+                }
+#pragma unroll
+                for (int x = 0; x < 2; ++x)
+#pragma unroll
+                    for (int y = 0; y < 2; ++y) {
+                        sa[x][y] += l[x].x * r[y].x + l[x].y * r[y].y + l[x].z * r[y].z + l[x].w * r[y].w;
+                        sq[x][y] += q[x].x * r[y].x + q[x].y * r[y].y + q[x].z * r[y].z + q[x].w * r[y].w;
+                    }
+            }
+#pragma unroll
+            for (int x = 0; x < 2; ++x)
+#pragma unroll
+                for (int y = 0; y < 2; ++y) {
+                    const float va = dc_quad_sum(sa[x][y]), vq = dc_quad_sum(sq[x][y]);
+                    if (lane4 == 4 * (2 * x + y)) {                 // one of the four threads each
+                        const int ii = i0 + 8 * x, jj = j0 + 8 * y;
+                        As[dc_row(jj) + ii] = beta[ii] * va;
+                        at.q_pairs[jj * DC_TOKENS + ii] = vq;
+                        at.q_pairs[ii * DC_TOKENS + jj] = 0.f;
+                    }
+                }
+        }
+    }
+    __syncthreads();
+    // k e_end: one more sub-block behind all but the last; q and k by what decays before their sub-block; the chunk's decay
+    if (e_lane < K) {
+        float4 before[4], sum = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+        for (int s = 0; s < 4; ++s) {
+            before[s] = make_float4(dc_exp2(sum.x), dc_exp2(sum.y), dc_exp2(sum.z), dc_exp2(sum.w));
+            const float4 tot = *reinterpret_cast<const float4*>(totals + s * DC_MAX_K + e_lane);
+            sum = make_float4(sum.x + tot.x, sum.y + tot.y, sum.z + tot.z, sum.w + tot.w);
+        }
+        if (warp == 0) *reinterpret_cast<float4*>(at.decay + e_lane) = make_float4(dc_exp2(sum.x), dc_exp2(sum.y), dc_exp2(sum.z), dc_exp2(sum.w));
+        const float4 last = *reinterpret_cast<const float4*>(totals + 3 * DC_MAX_K + e_lane);
+        const float4 behind = make_float4(dc_exp2(last.x), dc_exp2(last.y), dc_exp2(last.z), dc_exp2(last.w));
+#pragma unroll
+        for (int r = 0; r < 8; ++r) {
+            const int j = warp + 8 * r, s = r / 2;                  // 16 tokens a sub-block
+            float4 k = *reinterpret_cast<const float4*>(ks + dc_at(j, e_lane));
+            if (s < 3) k = make_float4(k.x * behind.x, k.y * behind.y, k.z * behind.z, k.w * behind.w);
+            *reinterpret_cast<float4*>(at.k_end + j * K + e_lane) = k;
+            const float4 q = *reinterpret_cast<const float4*>(qs + dc_at(j, e_lane)), f = before[s];
+            *reinterpret_cast<float4*>(at.q0 + j * K + e_lane) = make_float4(f.x * q.x, f.y * q.y, f.z * q.z, f.w * q.w);
+            const float4 l = *reinterpret_cast<const float4*>(gs + dc_at(j, e_lane));
+            const float w = beta[j];
+            *reinterpret_cast<float4*>(gs + dc_at(j, e_lane)) = make_float4(w * f.x * l.x, w * f.y * l.y, w * f.z * l.z, w * f.w * l.w);
+        }
+    }
+    // forward substitution of K + P columns, a column a thread: 128 at a time by each half of the block, in place in gs
+    // (the columns of k) and, 128 at a time, in ks (those of v)
+    const int half = tid >> 7, lane_col = tid & 127;
+    for (int v0 = 0; v0 == 0 || v0 < P; v0 += 128) {
+        __syncthreads();                                            // gs is whole, ks is read
+        const bool key = half == 0;
+        if (key ? (v0 > 0 || lane_col >= K) : v0 + lane_col >= P) continue;
+        float* X = key ? gs : ks;
+        if (!key) {
+            const float* v = a.qkv + (size_t)t0 * a.ld + 2 * a.Hk * K + h * P + v0 + lane_col;
+#pragma unroll 16
+            for (int i = 0; i < DC_TOKENS; ++i) X[dc_at(i, lane_col)] = beta[i] * (i < n ? v[(size_t)i * a.ld] : 0.f);
+        }
+        float* out = key ? at.w + lane_col : at.u + v0 + lane_col;
+        const int stride = key ? K : P;
+#pragma unroll 1
+        for (int s = 0; s < 4; ++s) {
+            float x[DC_SUB];
+#pragma unroll
+            for (int i = 0; i < DC_SUB; ++i) x[i] = X[dc_at(s * DC_SUB + i, lane_col)];
+#pragma unroll 4
+            for (int j = 0; j < s * DC_SUB; ++j) {                  // the sub-blocks before
+                const float xj = X[dc_at(j, lane_col)];
+                const float4* m = reinterpret_cast<const float4*>(As + dc_row(j) + s * DC_SUB);
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    const float4 f = m[i];
+                    x[4 * i] -= f.x * xj; x[4 * i + 1] -= f.y * xj; x[4 * i + 2] -= f.z * xj; x[4 * i + 3] -= f.w * xj;
+                }
+            }
+#pragma unroll
+            for (int j = 0; j < DC_SUB; ++j) {                      // its own tokens, one after the other
+                const float* m = As + dc_row(s * DC_SUB + j) + s * DC_SUB;
+#pragma unroll
+                for (int i = j / 4; i < 4; ++i) {
+                    const float4 f = *reinterpret_cast<const float4*>(m + 4 * i);
+                    if (4 * i > j) x[4 * i] -= f.x * x[j];
+                    if (4 * i + 1 > j) x[4 * i + 1] -= f.y * x[j];
+                    if (4 * i + 2 > j) x[4 * i + 2] -= f.z * x[j];
+                    if (4 * i + 3 > j) x[4 * i + 3] -= f.w * x[j];
+                }
+            }
+#pragma unroll
+            for (int i = 0; i < DC_SUB; ++i) {
+                X[dc_at(s * DC_SUB + i, lane_col)] = x[i];
+                out[(s * DC_SUB + i) * stride] = x[i];
+            }
+        }
+    }
+}
+
+// grid (ceil(P / 16), H, B), 256 threads; dynamic shared memory: W [64][K + 4], k e_end 2 x [64][K], S^T [16][K + 4], u [64][20].
+// For u a thread sums 4 tokens x 1 value over all channels, four channels a load; the state lives in registers, 4 channels x 2
+// values a thread, and in shared memory for u.  A chunk is two products in a chain, with two barriers.
+__global__ void __launch_bounds__(256)
+delta_chunk_walk_kernel(const DcArgs a) {
+    pdl_wait();
+    pdl_launch_dependents();
+    extern __shared__ __align__(16) float dc_smem[];
+    constexpr int LU = DC_WALK_P + 4;
+    const int h = blockIdx.y, b = blockIdx.z, tid = threadIdx.x, K = a.K, P = a.P, p0 = blockIdx.x * DC_WALK_P, ldw = K + 4;
+    float* Ws = dc_smem;
+    float* Ke = Ws + ldw * DC_TOKENS;
+    float* Ss = Ke + 2 * K * DC_TOKENS;                             // [16][ldw]
+    float* Us = Ss + DC_WALK_P * ldw;                               // [64][LU]
+    const int t0 = a.cu_seqlens[b], n_tok = a.cu_seqlens[b + 1] - t0;
+    if (n_tok <= 0) return;
+    const int chunks = (n_tok + DC_TOKENS - 1) / DC_TOKENS;
+    float* state = a.state + ((size_t)a.slots[b] * a.H + h) * P * K;
+    const int warp = tid >> 5, lane4 = (tid & 31) * 4;
+    auto copy = [&](float* dst, int ld, const float* src, bool wanted) {        // 64 rows of K, one commit group
+        if (wanted && lane4 < K) {
+#pragma unroll
+            for (int i = 0; i < DC_TOKENS / 8; ++i) rc_copy16(dst + (warp + 8 * i) * ld + lane4, src + (warp + 8 * i) * K + lane4, true);
+        }
+        rc_commit();
+    };
+    DcPlace at = dc_place(a, b, 0, h);
+    const size_t step = a.H * dc_floats(K, P);
+    copy(Ws, ldw, at.w, true);
+    copy(Ke, K, at.k_end, true);
+    const int p = (tid & 3) + 4 * (warp & 3), ig = ((tid >> 2) & 7) + 8 * (warp >> 2);      // u: value p, tokens ig, ig + 16, ig + 32, ig + 48
+    const int ps = (tid & 7) * 2, kg = (tid >> 3) * 4;              // state: values ps, ps + 1, channels kg ..
+    const bool p_ok = p0 + p < P, s_ok = p0 + ps < P && kg < K;
+    float S[2][4];
+#pragma unroll
+    for (int e = 0; e < 2; ++e) {
+        const float4 v = rc_load4(state + (size_t)(p0 + ps + e) * K + kg, s_ok);
+        S[e][0] = v.x; S[e][1] = v.y; S[e][2] = v.z; S[e][3] = v.w;
+        if (kg < K) *reinterpret_cast<float4*>(Ss + (ps + e) * ldw + kg) = v;
+    }
+    for (int c = 0; c < chunks; ++c) {
+        float own[4];                                               // U, asked for early
+#pragma unroll
+        for (int i = 0; i < 4; ++i) own[i] = p_ok ? at.u[(size_t)(ig + 16 * i) * P + p0 + p] : 0.f;
+        const float4 fade = rc_load4(at.decay + kg, kg < K);
+        rc_wait<0>();                                               // W and k e_end
+        __syncthreads();                                            // and S is whole; the last chunk's k e_end is read
+        copy(Ke + ((c + 1) & 1) * K * DC_TOKENS, K, at.k_end + step, c + 1 < chunks);
+        if (s_ok) {                                                 // left for the outputs
+#pragma unroll
+            for (int k = 0; k < 4; ++k) *reinterpret_cast<float2*>(at.start + (size_t)(kg + k) * P + p0 + ps) = make_float2(S[0][k], S[1][k]);
+        }
+        const float *w = Ws + ig * ldw, *s = Ss + p * ldw;
+        float part[4][2] = {{0.f, 0.f}, {0.f, 0.f}, {0.f, 0.f}, {0.f, 0.f}};
+#pragma unroll 8
+        for (int k = 0; k < K; k += 4) {
+            const float4 y = *reinterpret_cast<const float4*>(s + k);
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const float4 x = *reinterpret_cast<const float4*>(w + 16 * i * ldw + k);
+                part[i][0] += x.x * y.x; part[i][1] += x.y * y.y;
+                part[i][0] += x.z * y.z; part[i][1] += x.w * y.w;
+            }
+        }
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const float u = own[i] - (part[i][0] + part[i][1]);
+            Us[(ig + 16 * i) * LU + p] = u;
+            if (p_ok) at.u[(size_t)(ig + 16 * i) * P + p0 + p] = u;
+        }
+        __syncthreads();                                            // u is whole; W is read
+        copy(Ws, ldw, at.w + step, c + 1 < chunks);
+#pragma unroll
+        for (int e = 0; e < 2; ++e) { S[e][0] *= fade.x; S[e][1] *= fade.y; S[e][2] *= fade.z; S[e][3] *= fade.w; }
+        if (kg < K) {
+            const float* ke = Ke + (c & 1) * K * DC_TOKENS + kg;
+#pragma unroll 16
+            for (int j = 0; j < DC_TOKENS; ++j) {
+                const float4 x = *reinterpret_cast<const float4*>(ke + j * K);
+                const float2 y = *reinterpret_cast<const float2*>(Us + j * LU + ps);
+                S[0][0] += x.x * y.x; S[0][1] += x.y * y.x; S[0][2] += x.z * y.x; S[0][3] += x.w * y.x;
+                S[1][0] += x.x * y.y; S[1][1] += x.y * y.y; S[1][2] += x.z * y.y; S[1][3] += x.w * y.y;
+            }
+#pragma unroll
+            for (int e = 0; e < 2; ++e) *reinterpret_cast<float4*>(Ss + (ps + e) * ldw + kg) = make_float4(S[e][0], S[e][1], S[e][2], S[e][3]);
+        }
+        at.w += step; at.k_end += step; at.u += step; at.decay += step; at.start += step;
+    }
+    if (a.write_state && s_ok) {
+#pragma unroll
+        for (int e = 0; e < 2; ++e) *reinterpret_cast<float4*>(state + (size_t)(p0 + ps + e) * K + kg) = make_float4(S[e][0], S[e][1], S[e][2], S[e][3]);
+    }
+}
+
+// grid (chunks, H * ptiles, B), 128 threads: a chunk's 64 tokens x 128 values, from S0 and then from the chunk's own u
+__global__ void __launch_bounds__(128, 3)
+delta_chunk_out_kernel(const DcArgs a, int ptiles) {
+    pdl_wait();
+    pdl_launch_dependents();
+    // a tile: 16 channels or tokens x 128 values, and q of 64 tokens x 16 channels or their pairs with 16 tokens, 16 x 64
+    constexpr int ROWS = 16, LDV = 132, LDQ = ROWS + 4, LDP = 68;
+    __shared__ __align__(16) float values[3][ROWS * LDV], lefts[3][DC_TOKENS * LDQ];
+    const int c = blockIdx.x, h = blockIdx.y / ptiles, p0 = (blockIdx.y - h * ptiles) * 128, b = blockIdx.z, tid = threadIdx.x, K = a.K, P = a.P;
+    const int t0 = a.cu_seqlens[b] + c * DC_TOKENS, n = min(DC_TOKENS, a.cu_seqlens[b + 1] - t0);
+    if (n <= 0) return;
+    const DcPlace at = dc_place(a, b, c, h);
+    const int state_tiles = (K + ROWS - 1) / ROWS, n_tiles = state_tiles + (n + ROWS - 1) / ROWS;
+    auto copy = [&](int t) {                                        // one commit group a tile, also beyond the last
+        if (t < n_tiles) {
+            const bool from_state = t < state_tiles;
+            const int row0 = (from_state ? t : t - state_tiles) * ROWS, limit = from_state ? K : n;
+            const float* right = from_state ? at.start : at.u;
+#pragma unroll
+            for (int i = 0; i < 2; ++i) {
+                if (from_state) {
+                    const int r = (tid >> 2) + 32 * i, e = (tid & 3) * 4;
+                    const bool ok = row0 + e < K;
+                    rc_copy16(&lefts[t % 3][r * LDQ + e], at.q0 + (ok ? r * K + row0 + e : 0), ok);
+                } else {
+                    const int r = (tid >> 4) + 8 * i, e = (tid & 15) * 4;
+                    const bool ok = row0 + r < n;
+                    rc_copy16(&lefts[t % 3][r * LDP + e], at.q_pairs + (ok ? (row0 + r) * DC_TOKENS + e : 0), ok);
+                }
+            }
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const int r = (tid >> 5) + 4 * i, e = (tid & 31) * 4;
+                const bool ok = row0 + r < limit && p0 + e < P;
+                rc_copy16(&values[t % 3][r * LDV + e], right + (ok ? (size_t)(row0 + r) * P + p0 + e : 0), ok);
+            }
+        }
+        rc_commit();
+    };
+    copy(0);
+    copy(1);
+    const int ig = (tid >> 4) * 4, pg = (tid & 15) * 4;             // tokens ig .., 32 + ig ..; values pg .., 64 + pg ..
+    float acc[8][8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+#pragma unroll
+        for (int j = 0; j < 8; ++j) acc[i][j] = 0.f;
+    for (int t = 0; t < n_tiles; ++t) {
+        rc_wait<1>();
+        __syncthreads();
+        copy(t + 2);
+        const float *left = lefts[t % 3], *right = values[t % 3];
+        if (t >= state_tiles) {
+            rc_outer<ROWS>(acc, left, LDP, ig, 32 + ig, right, LDV, pg, 64 + pg);
+        } else {
+#pragma unroll
+            for (int k = 0; k < ROWS; k += 4) {                     // q four channels a load
+                float4 q[8];
+#pragma unroll
+                for (int i = 0; i < 8; ++i) q[i] = *reinterpret_cast<const float4*>(left + ((i >> 2) * 32 + ig + (i & 3)) * LDQ + k);
+#pragma unroll
+                for (int r = 0; r < 4; ++r) {
+                    const float4 y0 = *reinterpret_cast<const float4*>(right + (k + r) * LDV + pg), y1 = *reinterpret_cast<const float4*>(right + (k + r) * LDV + 64 + pg);
+                    const float y[8] = {y0.x, y0.y, y0.z, y0.w, y1.x, y1.y, y1.z, y1.w};
+#pragma unroll
+                    for (int i = 0; i < 8; ++i) {
+                        const float x = r == 0 ? q[i].x : (r == 1 ? q[i].y : (r == 2 ? q[i].z : q[i].w));
+#pragma unroll
+                        for (int j = 0; j < 8; ++j) acc[i][j] += x * y[j];
+                    }
+                }
+            }
+        }
+    }
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+        const int t = (i >> 2) * 32 + ig + (i & 3);
+        if (t >= n) continue;
+        float* out = a.o + (size_t)(t0 + t) * a.H * P + h * P + p0;
+#pragma unroll
+        for (int half = 0; half < 2; ++half) {
+            const int p = 64 * half + pg;
+            if (p0 + p < P) *reinterpret_cast<float4*>(out + p) = make_float4(acc[i][4 * half], acc[i][4 * half + 1], acc[i][4 * half + 2], acc[i][4 * half + 3]);
+        }
+    }
+}
+
+// Floats of scratch that qwb_delta_chunked needs; 0: these sizes are not taken.
+extern "C" long long qwb_delta_chunked_scratch(int T, int B, int H, int K, int P) {
+    if (T <= 0 || B <= 0 || H <= 0 || K <= 0 || P <= 0 || K % 4 || P % 4 || K > DC_MAX_K) return 0;
+    return ((long long)T / DC_TOKENS + B) * H * (long long)dc_floats(K, P);
+}
+
+// The same step as qwb_delta_prep and qwb_delta_scan with beta, after qwb_delta_prep made q and k unit vectors and beta; the raw
+// decays come as qwb_delta_prep takes them.  16-byte aligned tensors, rows of a multiple of 4 floats.
+extern "C" int qwb_delta_chunked(const float* qkv, int ld, const float* beta, const float* a_raw, int ld_a, const float* dt_bias, const float* A_log,
+                                 float* state, const int* cu_seqlens, const int* slots, float* o, float* scratch, int T, int B, int max_new, int H,
+                                 int Hk, int K, int P, int decay_k, int write_state, cudaStream_t stream) {
+    if (T <= 0 || B <= 0 || max_new <= 0) return 0;
+    if (!qwb_delta_chunked_scratch(T, B, H, K, P) || Hk <= 0 || H % Hk || ld % 4 || ld < 2 * Hk * K + H * P || (decay_k != K && decay_k != 1) || ld_a < H * decay_k)
+        return qwb_fail(QWB_ERR_ARG, "delta_chunked: %d heads, %d key heads, state %d x %d in rows of %d, %d decays a head", H, Hk, K, P, ld, decay_k);
+    for (const void* p : {(const void*)qkv, (const void*)state, (const void*)o, (const void*)scratch})
+        if (!p || !rc_aligned16(p)) return qwb_fail(QWB_ERR_ARG, "delta_chunked: a tensor is not 16-byte aligned");
+    const int chunks = (max_new + DC_TOKENS - 1) / DC_TOKENS, ptiles = (P + 127) / 128;
+    if (B > 65535 || (long long)H * ptiles > 65535) return qwb_fail(QWB_ERR_ARG, "delta_chunked: %d sequences or %d heads are too many", B, H);
+    const DcArgs a = {qkv, beta, a_raw, dt_bias, A_log, cu_seqlens, slots, state, o, scratch, ld, ld_a, H, Hk, K, P, decay_k, write_state};
+    const size_t smem1 = (3 * DC_TOKENS * DC_MAX_K + DC_A_FLOATS + 4 * DC_MAX_K + DC_TOKENS) * sizeof(float);
+    const size_t smem2 = ((3 * K + 4) * DC_TOKENS + DC_WALK_P * (K + 4) + DC_TOKENS * (DC_WALK_P + 4)) * sizeof(float);
+    cudaError_t e = cudaFuncSetAttribute(delta_chunk_prep_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem1);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(delta_chunk_walk_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem2);
+    if (e != cudaSuccess) return qwb_fail(QWB_ERR_CUDA, "delta_chunked: %s", cudaGetErrorString(e));
+    qwb_launch(delta_chunk_prep_kernel, dim3(chunks, H, B), 256, smem1, stream, a);
+    if (int rc = qwb_check_launch("delta_chunk_prep")) return rc;
+    qwb_launch(delta_chunk_walk_kernel, dim3((P + DC_WALK_P - 1) / DC_WALK_P, H, B), 256, smem2, stream, a);
+    if (int rc = qwb_check_launch("delta_chunk_walk")) return rc;
+    qwb_launch(delta_chunk_out_kernel, dim3(chunks, H * ptiles, B), 128, 0, stream, a, ptiles);
+    return qwb_check_launch("delta_chunk_out");
+}

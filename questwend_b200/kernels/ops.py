@@ -931,6 +931,12 @@ def ssm_scan(xbc: torch.Tensor, dt: torch.Tensor, dt_col0: int, dt_bias, a_log, 
     return y
 
 
+# Tokens of a step's longest sequence from which the delta rule runs in chunks (csrc/recurrent_chunks.cu).  With its
+# convolution, 16 heads of 128 x 128, us, scan / chunks: 64 tokens 44 / 68, 100 tokens (a decay per head) 43 / 68, three sequences
+# of 67 94 / 84, 400 tokens 194 / 94.
+DELTA_CHUNKED_FROM = 144
+
+
 def delta_rule(qkv: torch.Tensor, b_raw: torch.Tensor, b_col0: int, a_raw: torch.Tensor, dt_bias, a_log,
                state: torch.Tensor, ctx, heads: int, key_heads: int, key_dim: int, vdim: int, unit_eps: float,
                q_scale: float, write_state: bool = True, per_head: bool = False, a_col0: int = 0) -> torch.Tensor:
@@ -939,7 +945,8 @@ def delta_rule(qkv: torch.Tensor, b_raw: torch.Tensor, b_col0: int, a_raw: torch
     in place, q times ``q_scale``); columns ``b_col0 .. b_col0 + heads`` of ``b_raw`` [T, ld] and ``a_raw``
     [T, heads * key_dim] are the raw write strengths and decays; ``state`` float32 [slots, heads, vdim, key_dim] (column by column).  Returns o float32 [T, heads * vdim].
     ``per_head``: one decay per head instead: the raw decays are columns ``a_col0 .. a_col0 + heads`` of ``a_raw`` [T, ld],
-    ``dt_bias`` has ``heads`` entries."""
+    ``dt_bias`` has ``heads`` entries.  Steps with a sequence of at least ``DELTA_CHUNKED_FROM`` tokens run in chunks of 64 (keys
+    of up to 128, sizes in multiples of 4)."""
     _need(qkv, "qkv", torch.float32, 2)
     _need(b_raw, "b_raw", torch.float32, 2)
     _need(a_raw, "a_raw", torch.float32, 2)
@@ -957,12 +964,24 @@ def delta_rule(qkv: torch.Tensor, b_raw: torch.Tensor, b_col0: int, a_raw: torch
     dev = qkv.device
     kq = torch.empty((T, key_heads), dtype=torch.float32, device=dev)
     beta = torch.empty((T, heads), dtype=torch.float32, device=dev)
-    decay = torch.empty((T, heads * decay_k), dtype=torch.float32, device=dev)
+    raw_decays = (ctypes.c_void_p(a_raw.data_ptr() + 4 * a_col0), _i(a_raw.shape[1]), _ptr(dt_bias), _ptr(a_log))
+    floats = 0
+    if ctx.max_new >= DELTA_CHUNKED_FROM and qkv.shape[1] % 4 == 0 and not (qkv.data_ptr() % 16 or state.data_ptr() % 16):
+        size = _lookup("recurrent_chunks", "qwb_delta_chunked_scratch")[1]
+        size.restype = ctypes.c_longlong
+        floats = size(_i(T), _i(ctx.n_seqs), _i(heads), _i(key_dim), _i(vdim))
+    chunked = 0 < floats <= CHUNK_SCRATCH_MAX
+    decay = None if chunked else torch.empty((T, heads * decay_k), dtype=torch.float32, device=dev)
     _call("recurrent", "qwb_delta_prep", _ptr(qkv), _i(qkv.shape[1]), _ptr(kq), ctypes.c_void_p(b_raw.data_ptr() + 4 * b_col0),
-          _i(b_raw.shape[1]), _ptr(beta), ctypes.c_void_p(a_raw.data_ptr() + 4 * a_col0), _i(a_raw.shape[1]),
-          _ptr(dt_bias), _ptr(a_log), _ptr(decay), _i(T), _i(heads), _i(key_heads), _i(key_dim), _i(decay_k), _f(unit_eps),
+          _i(b_raw.shape[1]), _ptr(beta), *raw_decays, _ptr(decay), _i(T), _i(heads), _i(key_heads), _i(key_dim), _i(decay_k), _f(unit_eps),
           _f(q_scale), _stream())
     o = torch.empty((T, heads * vdim), dtype=torch.float32, device=dev)
+    if chunked:
+        scratch = torch.empty((floats,), dtype=torch.float32, device=dev)
+        _call("recurrent_chunks", "qwb_delta_chunked", _ptr(qkv), _i(qkv.shape[1]), _ptr(beta), *raw_decays, _ptr(state), _ptr(ctx.cu_seqlens),
+              _ptr(ctx.slots), _ptr(o), _ptr(scratch), _i(T), _i(ctx.n_seqs), _i(ctx.max_new), _i(heads), _i(key_heads), _i(key_dim), _i(vdim),
+              _i(decay_k), _i(1 if write_state else 0), _stream(), kernels=3)
+        return o
     _call("recurrent", "qwb_delta_scan", _ptr(qkv), _i(qkv.shape[1]), _ptr(kq), _ptr(beta), _ptr(decay), _ptr(state),
           _ptr(ctx.cu_seqlens), _ptr(ctx.slots), _ptr(o), _i(ctx.n_seqs), _i(heads), _i(key_heads), _i(key_dim), _i(vdim),
           _i(1 if write_state else 0), _i(heads * decay_k), _i(decay_k), _stream())

@@ -146,7 +146,7 @@ class GatedDeltaMixer(Mixer):
         self.a_log, self.dt_bias, self.norm_w = (_f32(weights, px + n[k]) for k in ("A_log", "dt_bias", "norm"))
 
     def kernel_modules(self):
-        return ("recurrent", "elementwise", *linear_modules(self.runtime.dtype))
+        return ("recurrent", "recurrent_chunks", "elementwise", *linear_modules(self.runtime.dtype))
 
     def state_spec(self):
         return (StateSpec((self.taps - 1, self.channels), torch.float32),
@@ -347,7 +347,7 @@ class GatedDeltaHeadMixer(Mixer):
         self.a_log, self.dt_bias, self.norm_w = (_f32(weights, px + n[k]) for k in ("A_log", "dt_bias", "norm"))
 
     def kernel_modules(self):
-        return ("recurrent", "elementwise", *linear_modules(self.runtime.dtype))
+        return ("recurrent", "recurrent_chunks", "elementwise", *linear_modules(self.runtime.dtype))
 
     def state_spec(self):
         state = StateSpec((self.heads, self.vdim, self.key_dim), torch.float32)       # column by column

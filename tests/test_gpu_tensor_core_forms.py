@@ -243,3 +243,47 @@ def test_convolutions_of_four_channels_a_thread(taps, C, mode):
     got = ops.short_conv(wide, 4, C, w, bias if mode != "plain" else None, a, step, **kw)
     one = ops.short_conv(shifted, 5, C, w, bias if mode != "plain" else None, b, step, **kw)
     assert torch.equal(got, one) and torch.equal(a, b)
+
+
+@pytest.mark.parametrize("H, Hk, K, P, per_head", [(2, 2, 128, 128, False), (4, 1, 128, 128, True), (2, 1, 4, 4, False), (3, 3, 36, 20, False), (2, 2, 100, 260, True)])
+@pytest.mark.parametrize("pace", [0.01, 1.0, 60.0])
+def test_delta_rule_in_chunks(H, Hk, K, P, per_head, pace):
+    """Sequences at the edges of the chunks of 64 and their sub-blocks of 16, from a state, with slow, usual and immediate
+    decays; the scan gives the same; slots of others stay as they are."""
+    torch.manual_seed(H + K + P)
+    lens, slots = [1, 15, 16, 17, 63, 64, 65, 200], [4, 2, 7, 1, 5, 3, 8, 9]
+    T, n_decay = sum(lens), H if per_head else H * K
+    step = Steps(lens, slots)
+    C = 2 * Hk * K + H * P
+    qkv, b_raw, a_raw = torch.randn(T, C, device=DEV), torch.randn(T, H + 3, device=DEV), torch.randn(T, n_decay + (5 if per_head else 0), device=DEV)
+    bias, a_log = torch.randn(n_decay, device=DEV), torch.log(pace * (1 + torch.rand(H, device=DEV)))
+    start = 0.3 * torch.randn(11, H, P, K, device=DEV)
+    col, scale = 2 if per_head else 0, K ** -0.5
+
+    def run(state, **kw):
+        return ops.delta_rule(qkv.clone(), b_raw, 1, a_raw, bias, a_log, state, step, H, Hk, K, P, 1e-6, scale, per_head=per_head, a_col0=col, **kw)
+
+    state, again = start.clone(), start.clone()
+    o = run(state)
+    step.max_new = 1                                        # taken for a short step: the scan
+    o_scan = run(again)
+    t = 0
+    for n, slot in zip(lens, slots):
+        S = start[slot].double()
+        ref = torch.empty(n, H * P, dtype=F64, device=DEV)
+        for i in range(n):
+            row = qkv[t + i].double()
+            q, k = (x / torch.sqrt((x * x).sum(-1, keepdim=True) + 1e-6) for x in (row[m * Hk * K:(m + 1) * Hk * K].view(Hk, K).repeat_interleave(H // Hk, 0) for m in (0, 1)))
+            raw = torch.nn.functional.softplus(a_raw[t + i, col:col + n_decay].double() + bias.double(), threshold=100.0).view(H, -1)
+            S = S * torch.exp(-torch.exp(a_log.double())[:, None] * raw)[:, None, :]
+            u = torch.sigmoid(b_raw[t + i, 1:1 + H].double())[:, None] * (row[2 * Hk * K:].view(H, P) - (S @ k[:, :, None])[..., 0])
+            S = S + u[:, :, None] * k[:, None, :]
+            ref[i] = (S @ (q * scale)[:, :, None]).reshape(-1)
+        for got, st in ((o, state), (o_scan, again)):
+            sums_close(got[t:t + n], ref)
+            sums_close(st[slot], S)
+        t += n
+    assert torch.equal(state[[0, 6, 10]], start[[0, 6, 10]])
+    step.max_new, before = max(lens), state.clone()
+    run(state, write_state=False)
+    assert torch.equal(state, before)
