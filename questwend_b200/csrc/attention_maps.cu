@@ -1010,10 +1010,10 @@ extern "C" int qwb_maps_prefill_mma(const void* q, const void* k_pool, const voi
 // block: a page's K and V tiles go to shared memory; thread (key, half of the rows) forms the scores; a warp per row
 // updates maximum and sum; thread d accumulates p v for all rows.
 // ---------------------------------------------------------------------------------
-__device__ __host__ __forceinline__ int maps_run_pages(int first_key, int len) {
+__device__ __host__ __forceinline__ int maps_run_pages(int first_key, int len, int max_runs) {
     const int span = (len - 1) / QWB_MAPS_PAGE - first_key / QWB_MAPS_PAGE + 1;
     int rp = QWB_MAPS_RUN_PAGES;
-    while (span > rp * QWB_MAPS_MAX_RUNS) rp *= 2;
+    while (span > rp * max_runs) rp *= 2;
     return rp;
 }
 
@@ -1033,7 +1033,7 @@ __global__ void maps_decode_kernel(const T* __restrict__ q, const T* __restrict_
     const int b = blockIdx.z, run = blockIdx.x;
     const int len = seq_len[b];
     const int first = maps_first_key(len - 1, mask);
-    const int rp = maps_run_pages(first, len);
+    const int rp = maps_run_pages(first, len, QWB_MAPS_MAX_RUNS);
     const int page_lo = first / PG;
     const int row_first = max(first, (page_lo + run * rp) * PG);
     const int row_end = min(len, (page_lo + (run + 1) * rp) * PG);
@@ -1186,76 +1186,287 @@ __global__ void maps_decode_kernel(const T* __restrict__ q, const T* __restrict_
     }
 }
 
-// Per (query head, sequence): each map's a = sum_r acc_r e^(m_r - M) / sum_r l_r e^(m_r - M), M = max_r m_r, over the
-// sequence's runs in index order; then the difference of the maps, the norm and the factor.  grid (H, B), 128 threads:
-// warp m first makes map m's weights e^(m_r - M) / L once for all columns, then thread d sums its column.
-template <typename T>
-__global__ void maps_merge_kernel(const float* __restrict__ part_acc, const float* __restrict__ part_m, const float* __restrict__ part_l,
-                                  const int* __restrict__ seq_len, T* __restrict__ out, int H, int maps, int vdim, MapsMask mask, int n_runs,
-                                  float lambda, int norm_out, float eps, float out_scale, MapsGate gate) {
+// ---------------------------------------------------------------------------------
+// The same step over a bfloat16 cache on the tensor cores (mma.sync m16n8k16), keys of up to 256 values in all and values of up
+// to 128: rows, slices and runs as above (up to MD_MAX_RUNS runs).  A block is four warps that share nothing but their run until
+// its end: warp w takes the run's keys w * 16 .., w * 16 + 64 .., sixteen at a time through stages of its own (cp.async; a
+// group's keys lie one after the other in the cache and are copied as they lie).  The order of a key's values in the sum is free,
+// so lane t of a key's four takes values 32 s + 8 t .. for steps 2 s and 2 s + 1 (q in the same order); the order of the output's
+// columns is free, so lane group g takes values 8 g .. of four keys and tile j holds columns 8 g + j: operands are 16-byte loads
+// and no ldmatrix.  q is zero outside a row's own map, so that one product over a whole key row gives every row its map's score.
+// Probabilities stay 32-bit: each is cut into three bfloat16 numbers whose sum it is; the tile's other eight rows take the second
+// one, a product of its own the third.  What a lane holds of the scores is what it needs of the probabilities.
+// Bound by the chain of a group (about 700 instructions a warp, twelve warps an SM): a third stage, which leaves room for eight,
+// is slower.  16 heads of 2 x 64 over 4 key/value heads, values of 128, with the merge, replayed from a graph, before
+// (maps_decode_kernel, plain FMA) and now: 8 sequences of about 8,000 keys 74.4 -> 43.9 us (123 MB), 32 of 300 23.9 -> 16.3 us, one of
+// 16,384 (cap 50) 53.9 -> 33.1 us, one of 64 14.0 -> 10.4 us.
+// ---------------------------------------------------------------------------------
+#define MD_WARPS 4
+#define MD_STAGES 2
+#define MD_KEYS 16
+// The most runs of a sequence.  With three stages, 8 sequences of 8,192 keys / one of 16,384, us: 16 runs 50.0 / 57.0, 32 runs
+// 49.8 / 33.4, 64 runs 61.7 / 25.7.
+#define MD_MAX_RUNS 32
+
+static bool maps_decode_mma_fits(int dtype, int maps, int dim, int vdim) { return dtype == QWB_DT_BF16 && maps * dim <= 256 && vdim <= 128; }
+static size_t maps_decode_mma_smem(int kdim, int vdim) {
+    const size_t stages = (size_t)MD_WARPS * MD_STAGES * MD_KEYS * (kdim + vdim) * sizeof(bf16);
+    const size_t sums = (size_t)MD_WARPS * QWB_MAPS_ROWS * (vdim + 2) * sizeof(float);      // over the stages, once they are read
+    return stages > sums ? stages : sums;
+}
+
+template <int KC>           // pieces of 32 key values there is room for
+__global__ void __launch_bounds__(32 * MD_WARPS, KC <= 4 ? 3 : 2)
+maps_decode_mma_kernel(const bf16* __restrict__ q, const bf16* __restrict__ k_pool, const bf16* __restrict__ v_pool,
+                       const int* __restrict__ page_table, const int* __restrict__ seq_len, float* __restrict__ part_acc,
+                       float* __restrict__ part_m, float* __restrict__ part_l, int H, int G, int maps, int dim, int vdim,
+                       int table_width, float scale, float softcap, MapsMask mask, int n_runs) {
     pdl_wait();
     pdl_launch_dependents();
+    constexpr int RT = QWB_MAPS_ROWS, PG = QWB_MAPS_PAGE, NV = 16;
+    const int b = blockIdx.z, run = blockIdx.x, len = seq_len[b];
+    const int first = maps_first_key(len - 1, mask);
+    const int rp = maps_run_pages(first, len, MD_MAX_RUNS);
+    const int row_lo = (first / PG + run * rp) * PG, row_first = max(first, row_lo), row_end = min(len, row_lo + rp * PG);
+    if (row_first >= row_end) return;
+    const int rows_g = (H / G) * maps, slices = (rows_g + RT - 1) / RT;
+    const int g = blockIdx.y / slices, r0 = (blockIdx.y % slices) * RT, rcount = min(RT, rows_g - r0);
+    const int kdim = maps * dim;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, row = lane >> 2, t = lane & 3;
+    const int* pages = page_table + (size_t)b * table_width;
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    const int stage_size = MD_KEYS * (kdim + vdim);                 // 16 keys, then their values
+    bf16* mine = reinterpret_cast<bf16*>(smem_raw) + (size_t)warp * MD_STAGES * stage_size;
+
+    const int key0 = row_first / MD_KEYS * MD_KEYS;                 // the run's first group of 16 keys; this warp's group i: ...
+    const int n_groups = (row_end - key0 + MD_KEYS - 1) / MD_KEYS, n_mine = n_groups > warp ? (n_groups - warp + MD_WARPS - 1) / MD_WARPS : 0;
+    auto copy = [&](int i) {                                        // ... keys key0 + 16 (warp + 4 i) ..; one commit group, also beyond the last
+        if (i < n_mine) {
+            const int key = key0 + MD_KEYS * (warp + MD_WARPS * i), n = min(MD_KEYS, row_end - key);   // rows behind the run: zeros
+            const size_t at = ((size_t)pages[key / PG] * G + g) * PG + key % PG;
+            bf16* dst = mine + (size_t)(i % MD_STAGES) * stage_size;
+            auto rows = [&](const bf16* src, int size, bf16* to) {
+#pragma unroll 4
+                for (int e = lane * 8; e < MD_KEYS * size; e += 256) mm_cp16(to + e, src + (e < n * size ? e : 0), e < n * size ? 16 : 0);
+            };
+            rows(k_pool + at * kdim, kdim, dst);
+            rows(v_pool + at * vdim, vdim, dst + MD_KEYS * kdim);
+        }
+        mm_commit();
+    };
+    for (int i = 0; i < MD_STAGES - 1; ++i) copy(i);
+
+    // this lane's values of q: row `row` of the slice, piece c's values 8 t .., zero outside the row's map
+    uint4 qa[KC];
+    const int my_map = (r0 + row) % maps;
+    const bf16* q_row = q + ((size_t)b * H + (size_t)g * (H / G) + (r0 + row) / maps) * kdim;
+#pragma unroll
+    for (int c = 0; c < KC; ++c) {
+        const int d = 32 * c + 8 * t;
+        qa[c] = row < rcount && d >= my_map * dim && d < (my_map + 1) * dim ? *reinterpret_cast<const uint4*>(q_row + d) : make_uint4(0, 0, 0, 0);
+    }
+    const float inv_cap = softcap > 0.f ? 1.f / softcap : 0.f;
+    float o[NV][4];
+#pragma unroll
+    for (int j = 0; j < NV; ++j) o[j][0] = o[j][1] = o[j][2] = o[j][3] = 0.f;
+    float m = -INFINITY, l = 0.f;
+
+    for (int i = 0; i < n_mine; ++i) {
+        mm_wait<MD_STAGES - 2>();
+        __syncwarp();                                               // group i is there for every lane, group i - 1 is read
+        copy(i + MD_STAGES - 1);
+        const bf16* Kt = mine + (size_t)(i % MD_STAGES) * stage_size;
+        const bf16* Vt = Kt + MD_KEYS * kdim;
+        float s[2][2][4];                                           // two chains a tile of eight keys
+#pragma unroll
+        for (int n = 0; n < 2; ++n)
+#pragma unroll
+            for (int c = 0; c < 2; ++c) s[n][c][0] = s[n][c][1] = s[n][c][2] = s[n][c][3] = 0.f;
+#pragma unroll
+        for (int c = 0; c < KC; ++c) {
+            if (32 * c >= kdim) continue;
+#pragma unroll
+            for (int n = 0; n < 2; ++n) {
+                uint4 k = make_uint4(0, 0, 0, 0);
+                if (32 * c + 8 * t < kdim) k = *reinterpret_cast<const uint4*>(Kt + (n * 8 + row) * kdim + 32 * c + 8 * t);
+                mm_mma(s[n][0], qa[c].x, 0u, qa[c].y, 0u, k.x, k.y);
+                mm_mma(s[n][1], qa[c].z, 0u, qa[c].w, 0u, k.z, k.w);
+            }
+        }
+        const int key = key0 + MD_KEYS * (warp + MD_WARPS * i) + 2 * t;
+        float sc[4], mx = m;
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            const int at = key + (e >> 1) * 8 + (e & 1);
+            const float raw = s[e >> 1][0][e & 1] + s[e >> 1][1][e & 1];
+            sc[e] = at >= row_first && at < row_end ? maps_cap(raw * scale, softcap, inv_cap) : -INFINITY;
+            mx = fmaxf(mx, sc[e]);
+        }
+        mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 1));
+        mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 2));
+        const float base = mx == -INFINITY ? 0.f : mx;              // a group before the first visible key
+        if (__any_sync(0xffffffffu, mx != m)) {
+            const float alpha = expf(m - base);
+            l *= alpha;
+#pragma unroll
+            for (int j = 0; j < NV; ++j) { o[j][0] *= alpha; o[j][1] *= alpha; o[j][2] *= alpha; o[j][3] *= alpha; }
+        }
+        m = mx;
+        float p[4];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) { p[e] = expf(sc[e] - base); l += p[e]; }       // this lane's keys: the row's four lanes are added at the end
+        uint32_t part[3][2];                                        // p in three numbers of 8 bits
+#pragma unroll
+        for (int k = 0; k < 3; ++k)
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+                part[k][e] = mm_pack(p[2 * e], p[2 * e + 1]);
+                p[2 * e] -= __uint_as_float(part[k][e] << 16);
+                p[2 * e + 1] -= __uint_as_float(part[k][e] & 0xffff0000u);
+            }
+#pragma unroll
+        for (int half = 0; half < 2; ++half) {
+            if (64 * half >= vdim) continue;
+            uint32_t v[4][4];                                       // keys 2 t, 2 t + 1, 2 t + 8, 2 t + 9: values 64 half + 8 g ..
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                uint4 x = make_uint4(0, 0, 0, 0);
+                if (64 * half + 8 * row < vdim) x = *reinterpret_cast<const uint4*>(Vt + (2 * t + (e & 1) + (e >> 1) * 8) * vdim + 64 * half + 8 * row);
+                v[e][0] = x.x; v[e][1] = x.y; v[e][2] = x.z; v[e][3] = x.w;
+            }
+#pragma unroll
+            for (int k = 0; k < 2; ++k)                             // the first two parts, then the third: eight chains side by side
+#pragma unroll
+                for (int w = 0; w < 4; ++w)
+#pragma unroll
+                    for (int e = 0; e < 2; ++e) {                   // tile 2 w + e: the low or high halves of word w
+                        const uint32_t b0 = __byte_perm(v[0][w], v[1][w], e ? 0x7632 : 0x5410), b1 = __byte_perm(v[2][w], v[3][w], e ? 0x7632 : 0x5410);
+                        if (k == 0) mm_mma(o[8 * half + 2 * w + e], part[0][0], part[1][0], part[0][1], part[1][1], b0, b1);
+                        else mm_mma(o[8 * half + 2 * w + e], part[2][0], 0u, part[2][1], 0u, b0, b1);
+                    }
+        }
+    }
+    l += __shfl_xor_sync(0xffffffffu, l, 1);
+    l += __shfl_xor_sync(0xffffffffu, l, 2);
+    // the warps' results side by side (over the stages), then merged
+    mm_wait<0>();
+    __syncthreads();
+    float* all = reinterpret_cast<float*>(smem_raw);                // [warps][rows][vdim], maxima [warps][rows], sums [warps][rows]
+    float *all_m = all + MD_WARPS * RT * vdim, *all_l = all_m + MD_WARPS * RT;
+#pragma unroll
+    for (int j = 0; j < NV; ++j) {
+        const int d = 64 * (j >> 3) + 16 * t + (j & 7);             // columns 2 t and 2 t + 1 of tile j
+        float* dst = all + (warp * RT + row) * vdim + d;
+        if (d < vdim) dst[0] = o[j][0] + o[j][2];
+        if (d + 8 < vdim) dst[8] = o[j][1] + o[j][3];
+    }
+    if (t == 0) { all_m[warp * RT + row] = m; all_l[warp * RT + row] = l; }
+    __syncthreads();
+    const size_t row_base = ((size_t)b * G + g) * rows_g + r0;
+    for (int r = warp; r < rcount; r += MD_WARPS) {                 // a row a warp
+        float top = all_m[r], f[MD_WARPS], total = 0.f;
+#pragma unroll
+        for (int w = 1; w < MD_WARPS; ++w) top = fmaxf(top, all_m[w * RT + r]);
+#pragma unroll
+        for (int w = 0; w < MD_WARPS; ++w) {
+            f[w] = all_m[w * RT + r] == -INFINITY ? 0.f : expf(all_m[w * RT + r] - top);
+            total += f[w] * all_l[w * RT + r];
+        }
+        const size_t at = (row_base + r) * n_runs + run;
+        for (int d = lane; d < vdim; d += 32) {
+            float sum = 0.f;
+#pragma unroll
+            for (int w = 0; w < MD_WARPS; ++w) sum += f[w] * all[(w * RT + r) * vdim + d];
+            part_acc[at * vdim + d] = sum;
+        }
+        if (lane == 0) { part_m[at] = top; part_l[at] = total; }
+    }
+}
+
+// Per (query head, sequence): each map's a = sum_r acc_r e^(m_r - M) / sum_r l_r e^(m_r - M), M = max_r m_r, over the
+// sequence's runs in index order; then the difference of the maps, the norm and the factor.  grid (H, B), 128 threads a map:
+// a map's first warp makes its weights e^(m_r - M) / L once for all columns, while the first runs' values are on their way.
+template <typename T>
+__global__ void __launch_bounds__(128 * QWB_MAPS_MAX)
+maps_merge_kernel(const float* __restrict__ part_acc, const float* __restrict__ part_m, const float* __restrict__ part_l,
+                  const int* __restrict__ seq_len, T* __restrict__ out, int H, int maps, int vdim, MapsMask mask, int n_runs, int max_runs,
+                  float lambda, int norm_out, float eps, float out_scale, MapsGate gate) {
+    pdl_wait();
+    pdl_launch_dependents();
+    constexpr int AHEAD = 16;
     __shared__ float red[32];
-    __shared__ float wts[QWB_MAPS_MAX][QWB_MAPS_MAX_RUNS];
-    const int h = blockIdx.x, b = blockIdx.y, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    __shared__ float wts[QWB_MAPS_MAX][QWB_MAPS_MAX_RUNS], second[2 * 128];
+    const int h = blockIdx.x, b = blockIdx.y, mp = threadIdx.x >> 7, tid = threadIdx.x & 127, lane = tid & 31;
     const int len = seq_len[b];
     const int first = maps_first_key(len - 1, mask);
-    const int rp = maps_run_pages(first, len);
+    const int rp = maps_run_pages(first, len, max_runs);
     const int runs = min(n_runs, ((len - 1) / QWB_MAPS_PAGE - first / QWB_MAPS_PAGE) / rp + 1);
-    if (warp < maps) {
-        const size_t row = ((size_t)b * H + h) * maps + warp;
+    const size_t row = ((size_t)b * H + h) * maps + mp;
+    const float* acc = part_acc + row * n_runs * vdim;
+    float v[2][AHEAD];
+#pragma unroll
+    for (int c = 0; c < 2; ++c)
+#pragma unroll
+        for (int r = 0; r < AHEAD; ++r) v[c][r] = r < runs && tid + c * 128 < vdim ? acc[(size_t)r * vdim + tid + c * 128] : 0.f;
+    const float g = maps_gate(gate, b, h);
+    if (tid < 32) {
         float M = -INFINITY;
         for (int r = lane; r < runs; r += 32) M = fmaxf(M, part_m[row * n_runs + r]);
         M = warp_max(M);
         float L = 0.f;
-        for (int r = lane; r < runs; r += 32) {
-            const float e = M == -INFINITY ? 0.f : expf(part_m[row * n_runs + r] - M);
-            wts[warp][r] = e;
-            L += part_l[row * n_runs + r] * e;
+        for (int r = lane; r < QWB_MAPS_MAX_RUNS; r += 32) {
+            const float e = M == -INFINITY || r >= runs ? 0.f : expf(part_m[row * n_runs + r] - M);
+            wts[mp][r] = e;
+            if (r < runs) L += part_l[row * n_runs + r] * e;
         }
         L = warp_sum(L);
         const float inv = L > 0.f ? 1.f / L : 0.f;
-        for (int r = lane; r < runs; r += 32) wts[warp][r] *= inv;
+        for (int r = lane; r < QWB_MAPS_MAX_RUNS; r += 32) wts[mp][r] *= inv;
     }
     __syncthreads();
     float res[2] = {0.f, 0.f};
-    for (int mp = 0; mp < maps; ++mp) {
-        const size_t row = ((size_t)b * H + h) * maps + mp;
 #pragma unroll
-        for (int c = 0; c < 2; ++c) {
-            const int d = tid + c * 128;
-            if (d >= vdim) continue;
-            const float* col = part_acc + row * n_runs * vdim + d;
-            float a = 0.f;
-#pragma unroll 8
-            for (int r = 0; r < runs; ++r) a += col[(size_t)r * vdim] * wts[mp][r];
-            res[c] = mp == 0 ? a : res[c] - lambda * a;
-        }
+    for (int c = 0; c < 2; ++c) {
+        const int d = tid + c * 128;
+        if (d >= vdim) continue;
+        float a = 0.f;
+#pragma unroll
+        for (int r = 0; r < AHEAD; ++r) a += v[c][r] * wts[mp][r];
+#pragma unroll 16
+        for (int r = AHEAD; r < runs; ++r) a += acc[(size_t)r * vdim + d] * wts[mp][r];
+        res[c] = a;
+        if (mp == 1) second[d] = a;
+    }
+    if (maps == 2) {
+        __syncthreads();
+#pragma unroll
+        for (int c = 0; c < 2; ++c) if (tid + c * 128 < vdim) res[c] -= lambda * second[tid + c * 128];
     }
     float mul = 1.f;
     if (norm_out) {
         float ss = 0.f;
 #pragma unroll
-        for (int c = 0; c < 2; ++c) if (tid + c * 128 < vdim) ss += res[c] * res[c];
+        for (int c = 0; c < 2; ++c) if (mp == 0 && tid + c * 128 < vdim) ss += res[c] * res[c];
         mul = rsqrtf(block_sum(ss, red) / (float)vdim + eps) * out_scale;
     }
-    mul *= maps_gate(gate, b, h);
+    mul *= g;
 #pragma unroll
     for (int c = 0; c < 2; ++c) {
         const int d = tid + c * 128;
-        if (d < vdim) out[((size_t)b * H + h) * vdim + d] = from_f32<T>(res[c] * mul);
+        if (mp == 0 && d < vdim) out[((size_t)b * H + h) * vdim + d] = from_f32<T>(res[c] * mul);
     }
 }
 
 // runs of the grid for sequences of up to max_len tokens
-extern "C" int qwb_maps_decode_runs(int max_len, int chunk, int window) {
+extern "C" int qwb_maps_decode_runs(int dtype, int maps, int dim, int vdim, int max_len, int chunk, int window) {
     if (max_len <= 0) return 1;
     // the most pages a sequence's visible keys touch: a chunk or a window may begin anywhere in its first page
     const int pages_all = (max_len + QWB_MAPS_PAGE - 1) / QWB_MAPS_PAGE;
     const int most = chunk > 0 && window > 0 ? min(chunk, window) : max(chunk, window);
     const int pages = most > 0 ? min(pages_all, (most + QWB_MAPS_PAGE - 2) / QWB_MAPS_PAGE + 1) : pages_all;
     const int runs = (pages + QWB_MAPS_RUN_PAGES - 1) / QWB_MAPS_RUN_PAGES;
-    return runs < QWB_MAPS_MAX_RUNS ? runs : QWB_MAPS_MAX_RUNS;
+    const int max_runs = maps_decode_mma_fits(dtype, maps, dim, vdim) ? MD_MAX_RUNS : QWB_MAPS_MAX_RUNS;
+    return runs < max_runs ? runs : max_runs;
 }
 
 extern "C" long long qwb_maps_decode_scratch_floats(int B, int H, int maps, int vdim, int n_runs) {
@@ -1273,18 +1484,33 @@ static int launch_maps_decode(const void* q, const void* k_pool, const void* v_p
     float* part_acc = scratch;
     float* part_m = part_acc + rows * n_runs * vdim;
     float* part_l = part_m + rows * n_runs;
-    const size_t smem = ((size_t)QWB_MAPS_PAGE * (kdim + VEC) + (size_t)QWB_MAPS_PAGE * vdim) * sizeof(T) +
-                        ((size_t)QWB_MAPS_ROWS * dim + QWB_MAPS_ROWS * QWB_MAPS_PAGE + 3 * QWB_MAPS_ROWS) * sizeof(float);
-    if (smem > 48 * 1024) {
-        cudaError_t e = cudaFuncSetAttribute(maps_decode_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e != cudaSuccess) return qwb_fail(QWB_ERR_CUDA, "maps_decode: %s", cudaGetErrorString(e));
-    }
     const int rows_g = (H / G) * maps, slices = (rows_g + QWB_MAPS_ROWS - 1) / QWB_MAPS_ROWS;
-    qwb_launch(maps_decode_kernel<T>, dim3(n_runs, G * slices, B), 128, smem, stream, (const T*)q, (const T*)k_pool, (const T*)v_pool,
-               page_table, seq_len, part_acc, part_m, part_l, H, G, maps, dim, vdim, table_width, scale, softcap, mask, n_runs);
+    const bool mma = std::is_same<T, bf16>::value && maps_decode_mma_fits(QWB_DT_BF16, maps, dim, vdim);
+    const size_t smem = mma ? maps_decode_mma_smem(kdim, vdim)
+                            : ((size_t)QWB_MAPS_PAGE * (kdim + VEC) + (size_t)QWB_MAPS_PAGE * vdim) * sizeof(T) +
+                                  ((size_t)QWB_MAPS_ROWS * dim + QWB_MAPS_ROWS * QWB_MAPS_PAGE + 3 * QWB_MAPS_ROWS) * sizeof(float);
+    const dim3 grid(n_runs, G * slices, B);
+    auto room = [&](const void* kernel) -> int {
+        if (smem <= 48 * 1024) return 0;
+        cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        return e == cudaSuccess ? 0 : qwb_fail(QWB_ERR_CUDA, "maps_decode: %s", cudaGetErrorString(e));
+    };
+    if constexpr (std::is_same<T, bf16>::value) {
+        if (mma) {
+            auto kernel = kdim <= 128 ? maps_decode_mma_kernel<4> : maps_decode_mma_kernel<8>;
+            if (int rc = room((const void*)kernel)) return rc;
+            qwb_launch(kernel, grid, 32 * MD_WARPS, smem, stream, (const bf16*)q, (const bf16*)k_pool, (const bf16*)v_pool, page_table, seq_len, part_acc, part_m,
+                       part_l, H, G, maps, dim, vdim, table_width, scale, softcap, mask, n_runs);
+        }
+    }
+    if (!mma) {
+        if (int rc = room((const void*)maps_decode_kernel<T>)) return rc;
+        qwb_launch(maps_decode_kernel<T>, grid, 128, smem, stream, (const T*)q, (const T*)k_pool, (const T*)v_pool, page_table, seq_len, part_acc, part_m, part_l,
+                   H, G, maps, dim, vdim, table_width, scale, softcap, mask, n_runs);
+    }
     if (int rc = qwb_check_launch("maps_decode")) return rc;
-    qwb_launch(maps_merge_kernel<T>, dim3(H, B), 128, 0, stream, (const float*)part_acc, (const float*)part_m, (const float*)part_l,
-               seq_len, (T*)out, H, maps, vdim, mask, n_runs, lambda, norm_out, eps, out_scale, gate);
+    qwb_launch(maps_merge_kernel<T>, dim3(H, B), 128 * maps, 0, stream, (const float*)part_acc, (const float*)part_m, (const float*)part_l,
+               seq_len, (T*)out, H, maps, vdim, mask, n_runs, mma ? MD_MAX_RUNS : QWB_MAPS_MAX_RUNS, lambda, norm_out, eps, out_scale, gate);
     return qwb_check_launch("maps_merge");
 }
 

@@ -287,3 +287,46 @@ def test_delta_rule_in_chunks(H, Hk, K, P, per_head, pace):
     step.max_new, before = max(lens), state.clone()
     run(state, write_state=False)
     assert torch.equal(state, before)
+
+
+# ----------------------------------------------------------------------------- score maps, single tokens
+@pytest.mark.parametrize("maps, H, G, dim, vdim", [(2, 16, 4, 64, 128), (2, 2, 2, 8, 8), (2, 15, 3, 40, 72), (1, 10, 1, 128, 128), (2, 4, 1, 128, 120), (1, 3, 3, 24, 16)])
+@pytest.mark.parametrize("softcap, window, chunk, gated", [(0.0, 0, 0, False), (5.0, 0, 0, True), (3.0, 100, 0, False), (2.0, 1, 0, True), (20.0, 0, 96, False)])
+def test_score_maps_of_single_tokens_on_the_tensor_cores(maps, H, G, dim, vdim, softcap, window, chunk, gated):
+    """Scores are exact products, probabilities 32-bit, so what is left is the rounding of the bfloat16 results (and of sums of
+    32-bit products, which the norm of a small difference enlarges)."""
+    if maps == 1 and not softcap and not gated and not chunk:
+        return                                              # plain grouped-query attention: its own kernel
+    torch.manual_seed(H + dim + window + chunk)
+    lens = [1, 15, 16, 17, 63, 64, 65, 130, 1000, 2049, 4500]
+    B = len(lens)
+    table, (k_pool, v_pool) = paged(lens, lambda s: torch.randn(s, device=DEV).to(BF), [(G, maps * dim), (G, vdim)])
+    q = (2.0 * torch.randn(B, H, maps * dim, device=DEV)).to(BF)
+    gate = torch.randn(B, H + 3, device=DEV) if gated else None
+    alone = []
+    for pick in (list(range(B)), [1], [9], [10]):
+        ctx = SimpleNamespace(single_token=True, n_seqs=len(pick), max_new=1, max_len=max(lens[b] for b in pick),
+                              seq_len=torch.tensor([lens[b] for b in pick], device=DEV).int())
+        out = ops.maps_attention(q[pick].contiguous(), k_pool, v_pool, table[pick].contiguous(), ctx, maps, dim ** -0.5, softcap=softcap, window=window,
+                                 chunk=chunk, lam=0.4, norm_out=maps == 2, eps=1e-5, out_scale=0.3, gate=None if gate is None else gate[pick].contiguous(),
+                                 gate_col0=2 if gated else 0).view(len(pick), H, vdim)
+        alone.append(out)
+        for i, b in enumerate(pick):
+            n = lens[b]
+            ks, vs = rows(k_pool, table[b], n), rows(v_pool, table[b], n)
+            c = (n - 1) // chunk * chunk if chunk else 0
+            pos = torch.tensor([n - 1 - c], device=DEV)
+            for h in range(H):
+                g = h // (H // G)
+                a = [softmax(q[b, h:h + 1, m * dim:(m + 1) * dim].double(), ks[g, c:, m * dim:(m + 1) * dim], vs[g, c:], dim ** -0.5, pos, window, softcap)[0] for m in range(maps)]
+                ref, grown = a[0], 1.0
+                if maps == 2:
+                    ref = a[0] - 0.4 * a[1]
+                    grown = 0.3 * float(ref.square().mean().add(1e-5).rsqrt())
+                    ref = ref * grown
+                if gated:
+                    ref = ref * torch.sigmoid(gate[b, h + 2].double())
+                err = (out[i, h].double() - ref).abs()
+                assert (err <= 2.0 ** -8 * ref.abs() + 2e-5 * max(1.0, grown)).all(), (n, h, err.max())
+    for i, b in enumerate([1, 9, 10]):                      # a sequence's result does not depend on the batch
+        assert torch.equal(alone[0][b], alone[i + 1][0])
