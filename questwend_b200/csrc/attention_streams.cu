@@ -8,27 +8,36 @@
 //                       streams are the two maps of the same 128 (token, head of the group) rows; a tile's key rows hold both
 //                       maps, its values serve both, and the difference, its norm and the gate are taken at the end.
 //
-// Per stream and tile, as in attention_tc.cu: S = Q K^T into tensor memory (64 columns, two buffers), P = softmax by four
-// warps, a thread a row, written to shared memory as bfloat16, O += P V in tensor memory (VD columns), the row's reference
-// maximum moved only when a tile exceeds it by more than 2^8.  With two streams in one block the tensor cores work on one
-// while the other is in its softmax, what two blocks an SM give attention_tc.cu, but the Q, K and V tiles of 192-value keys
-// would not leave room for a second block (2 x 48 KB of Q, K and V in two stages: 208 KB), and K and V cross L2 once for 256
-// rows.  Warp 0 loads, warp 1 issues the products, warps 2-5 and 6-9 are the streams' softmax warps.  Every wait is bounded.
+// Per stream and tile: S = Q K^T into tensor memory (64 columns, two buffers), P = softmax by four warps, a thread a row, left as
+// bfloat16 in tensor memory over the scores it came from, O += P V with P read from there, O in tensor memory (VD columns), the
+// row's reference maximum moved only when a tile exceeds it by more than 2^8.  A stream waits for its product only when it
+// rescales O; otherwise it may be two tiles ahead.  With two streams in one block the tensor cores work on one while the other is
+// in its softmax, what two blocks an SM give attention_tc.cu, but the Q, K and V tiles of 192-value keys would not leave room for
+// a second block (2 x 48 KB of Q, K and V in three stages: 216 KB), and K and V cross L2 once for 256 rows.  Warp 0 loads, warp 1
+// issues the products, warps 2-5 and 6-9 are the streams' softmax warps.  Every wait is bounded.
 //
 // Sizes that are no multiples of 64 are filled up by the TMA loads with zeros.  In the last tile, rows of V behind the last
 // key that the block sees are overwritten with zeros before the product: they can belong to another sequence, and what stands
 // there, infinite or not a number, must not meet a probability of 0.
 //
-// Bound by the softmax warps' chain (wait for S, tensor-memory loads, maximum, 64 exponentials a row, P to shared memory): an
-// ncu capture shows the special-function unit at 35 %, issue slots at 30 %, the tensor pipe at 38 %.  16 heads, replayed from
-// a graph, with the mma.sync kernels and now: latent 128 + 64 / 128, one prompt of 4,096: 816 -> 155 us, of 600: 55 -> 19 us, of
-// 64: 8.2 -> 5.6 us; two maps of 64 over 4 key/value heads, values of 128, 8,192 tokens: 2,447 -> 707 us (cap 50: 3,261 -> 795),
-// 1,000 tokens: 79 -> 31 us, 64 tokens: 9.8 -> 8.2 us.
+// Bound by the tensor cores' products of 64 keys (clocks in a block: the issuing warp is busy all of the time, a softmax warp two
+// thirds of a tile's waiting for scores).  16 heads, replayed from a graph, with the mma.sync kernels, with P in shared memory, and
+// now: latent 128 + 64 / 128, one prompt of 4,096: 816 -> 155 -> 108 us, of 600: 55 -> 19 -> 14.5 us; two maps of 64 over 4
+// key/value heads, values of 128, 8,192 tokens: 2,447 -> 707 -> 529 us (cap 50: 3,261 -> 795 -> 607), 2,048 tokens with a window of
+// 1,024: 170 -> 52 -> 41 us.  Of the last step P in tensor memory and the third and fourth stage gave 5 to 10 %, the elected lane
+// in place of `lane == 0` the rest.
 #include "attention_tc.cuh"
 
 #define AS_THREADS 320
-#define AS_STAGES 2
+#define AS_MAX_STAGES 4
+#define AS_SMEM (227 * 1024)
 
+// A from tensor memory: a row a lane, two bfloat16 a column
+__device__ __forceinline__ void as_mma_ts(uint32_t tmem_d, uint32_t tmem_a, uint64_t desc_b, uint32_t idesc, uint32_t accumulate) {
+    asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+                 "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, {%5, %5, %5, %5}, p;\n\t}"
+                 ::"r"(tmem_d), "r"(tmem_a), "l"(desc_b), "r"(idesc), "r"(accumulate), "r"(0u) : "memory");
+}
 __device__ __forceinline__ uint64_t as_two(float lo, float hi) {
     uint64_t v;
     asm("mov.b64 %0, {%1, %2};" : "=l"(v) : "f"(lo), "f"(hi));
@@ -70,9 +79,12 @@ struct AsSmem {
     static constexpr size_t Q_BYTES = (size_t)2 * KA * AT_ROWS * 128;                       // stream by stream, [128 rows][128 bytes] a piece
     static constexpr size_t K_BYTES = (size_t)(MAPS ? 2 : 1) * KA * AT_KEYS * 128;          // (map by map,) [64 keys][128 bytes] a piece
     static constexpr size_t V_BYTES = (size_t)VA * AT_KEYS * 128;
-    static constexpr size_t P_BYTES = (size_t)AT_ROWS * 128;
-    static constexpr size_t TILES = Q_BYTES + AS_STAGES * (K_BYTES + V_BYTES) + 2 * P_BYTES;
-    static constexpr size_t BYTES = TILES + 256 + (MAPS ? 4 * AT_ROWS * sizeof(float) : 0);
+    static constexpr size_t MORE = 512 + (MAPS ? 4 * AT_ROWS * sizeof(float) : 0);          // barriers; what the maps' streams exchange
+    static constexpr int FIT = (int)((AS_SMEM - MORE - Q_BYTES) / (K_BYTES + V_BYTES));
+    static constexpr int STAGES = FIT < AS_MAX_STAGES ? FIT : AS_MAX_STAGES;
+    static constexpr size_t TILES = Q_BYTES + STAGES * (K_BYTES + V_BYTES);
+    static constexpr size_t BYTES = TILES + MORE;
+    static_assert(STAGES >= 2, "the tiles do not fit");
 };
 
 struct AsArgs {
@@ -90,7 +102,7 @@ __global__ void __launch_bounds__(AS_THREADS, 1)
 attn_streams_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_q2, const __grid_constant__ CUtensorMap map_k,
                     const __grid_constant__ CUtensorMap map_k2, const __grid_constant__ CUtensorMap map_v, const AsArgs p) {
     using Smem = AsSmem<KA, VA, MAPS>;
-    constexpr int VD = 64 * VA;
+    constexpr int VD = 64 * VA, STAGES = Smem::STAGES;
     constexpr uint32_t K_BYTES = Smem::K_BYTES, V_BYTES = Smem::V_BYTES;
     extern __shared__ __align__(1024) unsigned char smem_raw[];
     if (at_smem(smem_raw) & 1023u) {                    // never seen; refuse rather than compute with a wrong layout
@@ -99,19 +111,18 @@ attn_streams_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
     }
     unsigned char* q_tile = smem_raw;
     unsigned char* k_tiles = q_tile + Smem::Q_BYTES;
-    unsigned char* v_tiles = k_tiles + AS_STAGES * K_BYTES;
-    unsigned char* p_tiles = v_tiles + AS_STAGES * V_BYTES;
+    unsigned char* v_tiles = k_tiles + STAGES * K_BYTES;
     uint64_t* q_full = reinterpret_cast<uint64_t*>(smem_raw + Smem::TILES);
     uint64_t* k_full = q_full + 1;
-    uint64_t* k_empty = k_full + AS_STAGES;
-    uint64_t* v_full = k_empty + AS_STAGES;
-    uint64_t* v_empty = v_full + AS_STAGES;
-    uint64_t* s_full = v_empty + AS_STAGES;             // [stream][2]
-    uint64_t* s_empty = s_full + 4;                     // [stream][2]
-    uint64_t* p_full = s_empty + 4;                     // [stream]
-    uint64_t* o_full = p_full + 2;                      // [stream]
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(o_full + 2);
-    float* swap = reinterpret_cast<float*>(smem_raw + Smem::TILES + 256);       // MAPS: [2][128] factors, [2][128] sums of squares
+    uint64_t* k_empty = k_full + STAGES;
+    uint64_t* v_full = k_empty + STAGES;
+    uint64_t* v_empty = v_full + STAGES;
+    // [stream][tile & 1] each: a stream may be up to two tiles ahead of the tensor cores, and a barrier tells two phases apart
+    uint64_t* s_full = v_empty + STAGES;
+    uint64_t* p_full = s_full + 4;
+    uint64_t* o_full = p_full + 4;
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(o_full + 4);
+    float* swap = reinterpret_cast<float*>(smem_raw + Smem::TILES + 512);       // MAPS: [2][128] factors, [2][128] sums of squares
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int b = blockIdx.z;
@@ -141,12 +152,11 @@ attn_streams_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
 
     if (threadIdx.x == 0) {
         at_bar_init(q_full, 1);
-        for (int s = 0; s < AS_STAGES; ++s) {
+        for (int s = 0; s < STAGES; ++s) {
             at_bar_init(&k_full[s], 1); at_bar_init(&k_empty[s], 1);
             at_bar_init(&v_full[s], 1); at_bar_init(&v_empty[s], 1);
         }
-        for (int i = 0; i < 4; ++i) { at_bar_init(&s_full[i], 1); at_bar_init(&s_empty[i], 4); }
-        for (int i = 0; i < 2; ++i) { at_bar_init(&p_full[i], 4); at_bar_init(&o_full[i], 1); }
+        for (int i = 0; i < 4; ++i) { at_bar_init(&s_full[i], 1); at_bar_init(&p_full[i], 4); at_bar_init(&o_full[i], 1); }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == 1) {
@@ -183,10 +193,10 @@ attn_streams_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
             bool ok = true;
             int k_issued = 0, v_issued = 0;
             auto load = [&](int j, bool is_k) -> bool {
-                const int s = j % AS_STAGES;
+                const int s = j % STAGES;
                 uint64_t* empty = is_k ? &k_empty[s] : &v_empty[s];
                 uint64_t* full = is_k ? &k_full[s] : &v_full[s];
-                if (j >= AS_STAGES && !at_wait(empty, ((j / AS_STAGES) - 1) & 1)) return false;
+                if (j >= STAGES && !at_wait(empty, ((j / STAGES) - 1) & 1)) return false;
                 const uint32_t bytes = is_k ? K_BYTES : V_BYTES;
                 unsigned char* dst = (is_k ? k_tiles : v_tiles) + (size_t)s * bytes;
                 at_expect_tx(full, bytes);
@@ -221,21 +231,20 @@ attn_streams_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
                 atomicExch(p.error, 1);
                 // copies already issued still write shared memory: wait for them (bounded) before the block ends
                 at_wait(q_full, 0);
-                for (int j = max(0, k_issued - AS_STAGES); j < k_issued; ++j) at_wait(&k_full[j % AS_STAGES], (j / AS_STAGES) & 1);
-                for (int j = max(0, v_issued - AS_STAGES); j < v_issued; ++j) at_wait(&v_full[j % AS_STAGES], (j / AS_STAGES) & 1);
+                for (int j = max(0, k_issued - STAGES); j < k_issued; ++j) at_wait(&k_full[j % STAGES], (j / STAGES) & 1);
+                for (int j = max(0, v_issued - STAGES); j < v_issued; ++j) at_wait(&v_full[j % STAGES], (j / STAGES) & 1);
             }
         }
-    } else if (warp == 1) {                             // all lanes wait, lane 0 issues
+    } else if (warp == 1) {                             // all lanes wait, one issues
         constexpr uint32_t idesc_s = at_idesc(AT_ROWS, AT_KEYS, false), idesc_o = at_idesc(AT_ROWS, VD, true);
         auto all = [](bool ok) -> bool { return __all_sync(0xffffffffu, ok); };
         bool ok = all(at_wait(q_full, 0));
         auto issue_s = [&](int x, int j) -> bool {      // S of stream x for tile j, two tiles ahead of its product with V
-            const int i = j - from(x), s = j % AS_STAGES;
-            bool good = at_wait(&k_full[s], (j / AS_STAGES) & 1);
-            if (i >= 2) good = good && at_wait(&s_empty[2 * x + (i & 1)], ((i >> 1) - 1) & 1);
-            if (!all(good)) return false;
+            const int i = j - from(x), s = j % STAGES;
+            bool good = at_wait(&k_full[s], (j / STAGES) & 1);
+            if (!all(good)) return false;               // the buffer's last scores were read, and its P used by a product issued before
             at_fence_after();
-            if (lane == 0) {
+            if (at_elect()) {
                 const unsigned char* qt = q_tile + (size_t)x * KA * AT_ROWS * 128;
                 const unsigned char* kt = k_tiles + (size_t)s * K_BYTES + (MAPS ? (size_t)x * KA * AT_KEYS * 128 : 0);
 #pragma unroll
@@ -254,12 +263,12 @@ attn_streams_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
 #pragma unroll
             for (int x = 0; x < 2 && ok; ++x)
                 if (active(x, j)) ok = issue_s(x, j);
-            if (ok && lane == 0) at_commit(&k_empty[j % AS_STAGES]);
+            if (ok && at_elect()) at_commit(&k_empty[j % STAGES]);
         }
         for (int j = 0; j < n_tiles && ok; ++j) {
-            const int s = j % AS_STAGES;
+            const int s = j % STAGES;
             unsigned char* vt = v_tiles + (size_t)s * V_BYTES;
-            ok = all(at_wait(&v_full[s], (j / AS_STAGES) & 1));
+            ok = all(at_wait(&v_full[s], (j / STAGES) & 1));
             if (!ok) break;
             const int kept = k_last + 1 - (first_tile + j) * AT_KEYS;
             if (kept < AT_KEYS) {                       // the last tile: rows behind the last key
@@ -274,31 +283,29 @@ attn_streams_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
             for (int x = 0; x < 2 && ok; ++x) {
                 if (active(x, j)) {
                     const int i = j - from(x);
-                    ok = all(at_wait(&p_full[x], i & 1));
+                    ok = all(at_wait(&p_full[2 * x + (i & 1)], (i >> 1) & 1));
                     if (!ok) break;
                     at_fence_after();
-                    if (lane == 0) {
+                    if (at_elect()) {
 #pragma unroll
                         for (int k = 0; k < AT_KEYS / 16; ++k) {
-                            const uint64_t da = at_desc_kmajor(p_tiles + (size_t)x * Smem::P_BYTES) + 2 * k;
                             const uint64_t db = at_desc_mnmajor(vt + (size_t)k * 16 * 128, AT_KEYS * 128);
-                            at_mma(tmem + 256 + 128 * x, da, db, idesc_o, (i > 0 || k > 0) ? 1u : 0u);
+                            as_mma_ts(tmem + 256 + 128 * x, tmem + 128 * x + 64 * (i & 1) + 8 * k, db, idesc_o, (i > 0 || k > 0) ? 1u : 0u);
                         }
-                        at_commit(&o_full[x]);
+                        at_commit(&o_full[2 * x + (i & 1)]);
                     }
                     __syncwarp();
                 }
                 if (j + 2 < n_tiles && active(x, j + 2)) ok = issue_s(x, j + 2);
             }
-            if (ok && lane == 0) {
+            if (ok && at_elect()) {
                 at_commit(&v_empty[s]);
-                if (j + 2 < n_tiles) at_commit(&k_empty[j % AS_STAGES]);        // tile j + 2 sits in the same stage
+                if (j + 2 < n_tiles) at_commit(&k_empty[(j + 2) % STAGES]);
             }
         }
-        if (!ok && lane == 0) {
+        if (!ok && at_elect()) {
             atomicExch(p.error, 2);
-            for (int i = 0; i < 4; ++i) at_commit(&s_full[i]);
-            for (int i = 0; i < 2; ++i) at_commit(&o_full[i]);
+            for (int i = 0; i < 4; ++i) { at_commit(&s_full[i]); at_commit(&o_full[i]); }
         }
     } else {
         const int x = (warp - 2) >> 2, lane_group = warp & 3;
@@ -316,14 +323,13 @@ attn_streams_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
         // series to t^9 (the next term is below 2^-24 of the value at 0.3), on raw scores as v (c0 + v^2 (c1 + ..)): packed
         // multiply-adds, where the form by ex2 and rcp keeps the special-function unit, which the probabilities need too,
         // busy for three turns a score.  One sequence of 8,192 tokens, 16 heads of 2 x 64, cap 50:
-        // 795 us, 1,063 by ex2 and rcp alone.
+        // 795 us with it (P still in shared memory), 1,063 by ex2 and rcp alone.
         const float poly_up_to = CAP ? 0.3f / fabsf(to_t) : 0.f, tt = to_t * to_t;
         const float c0 = cap2 * to_t, c1 = c0 * tt * (-1.f / 3.f), c2 = c0 * tt * tt * (2.f / 15.f), c3 = c0 * tt * tt * tt * (-17.f / 315.f),
                     c4 = c0 * tt * tt * tt * tt * (62.f / 2835.f);
         int own = p.window > 0 ? max(0, qp - p.window + 1) : 0;                         // the first key that the row sees
         if (MAPS && p.chunk > 0 && qp >= 0) own = max(own, (qp / p.chunk) * p.chunk);
         float m_ref = -INFINITY, l = 0.f;
-        uint4* p_row = reinterpret_cast<uint4*>(p_tiles + (size_t)x * Smem::P_BYTES + (size_t)r * 128);
         bool ok = true;
         const int n_mine = to(x) - from(x);
         for (int i = 0; i < n_mine; ++i) {
@@ -334,9 +340,6 @@ attn_streams_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
             uint32_t sv[2][32];
             at_ld32(tmem_s + (i & 1) * 64 + lane_off, sv[0]);
             at_ld32(tmem_s + (i & 1) * 64 + lane_off + 32, sv[1]);
-            at_fence_before();                                                          // this S buffer may be filled again
-            __syncwarp();
-            if (lane == 0) at_arrive(&s_empty[2 * x + (i & 1)]);
             const bool all_visible = key0 + AT_KEYS - 1 <= qp && key0 >= own;           // no mask needed
             float mx = -INFINITY;
             bool series = false;
@@ -382,7 +385,7 @@ attn_streams_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
             const float alpha = rescale ? at_exp2((m_ref - m_new) * sl2) : 1.f;        // m_ref = -inf gives 0
             const float base = m_new == -INFINITY ? 0.f : m_new * sl2;
             m_ref = m_new;
-            uint32_t pk[2][16];
+            uint32_t pk[32];                                                            // two keys' probabilities each
             float sum[4] = {l * alpha, 0.f, 0.f, 0.f};
             auto probabilities = [&](auto argument) {
 #pragma unroll
@@ -394,7 +397,7 @@ attn_streams_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
                         const float p0v = at_exp2(a0), p1v = at_exp2(a1);
                         sum[(c / 2) & 3] += p0v + p1v;
                         __nv_bfloat162 v = __floats2bfloat162_rn(p0v, p1v);
-                        pk[h][c / 2] = *reinterpret_cast<uint32_t*>(&v);
+                        pk[16 * h + c / 2] = *reinterpret_cast<uint32_t*>(&v);
                     }
             };
             if (CAP && series) {
@@ -411,33 +414,26 @@ attn_streams_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
                 });
             }
             l = (sum[0] + sum[1]) + (sum[2] + sum[3]);
-            if (i > 0) {                                                               // the product before this one has read P and written O
-                ok = at_wait(&o_full[x], (i - 1) & 1);
+            if (i > 0 && __any_sync(0xffffffffu, rescale)) {                            // a row of this warp moves its reference: rescale O,
+                ok = at_wait(&o_full[2 * x + ((i - 1) & 1)], ((i - 1) >> 1) & 1);       // which the product before this one has written
                 at_fence_after();
                 if (!ok) { if (lane == 0) atomicExch(p.error, 4); break; }
-                if (__any_sync(0xffffffffu, rescale)) {
 #pragma unroll 1
-                    for (int c = 0; c < VD; c += 32) {
-                        uint32_t ov[32];
-                        at_ld32(tmem_o + lane_off + c, ov);
+                for (int c = 0; c < VD; c += 32) {
+                    uint32_t ov[32];
+                    at_ld32(tmem_o + lane_off + c, ov);
 #pragma unroll
-                        for (int e = 0; e < 32; ++e) ov[e] = __float_as_uint(__uint_as_float(ov[e]) * alpha);
-                        at_st32(tmem_o + lane_off + c, ov);
-                    }
+                    for (int e = 0; e < 32; ++e) ov[e] = __float_as_uint(__uint_as_float(ov[e]) * alpha);
+                    at_st32(tmem_o + lane_off + c, ov);
                 }
             }
-#pragma unroll
-            for (int h = 0; h < 2; ++h)
-#pragma unroll
-                for (int c = 0; c < 4; ++c)
-                    p_row[(h * 4 + c) ^ (r & 7)] = make_uint4(pk[h][4 * c], pk[h][4 * c + 1], pk[h][4 * c + 2], pk[h][4 * c + 3]);
-            at_fence_before();                                                          // O is rescaled (if at all); P is written
-            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+            at_st32(tmem_s + (i & 1) * 64 + lane_off, pk);                              // P over the scores it came from
+            at_fence_before();
             __syncwarp();
-            if (lane == 0) at_arrive(&p_full[x]);
+            if (lane == 0) at_arrive(&p_full[2 * x + (i & 1)]);
         }
         if (ok && n_mine > 0) {
-            ok = at_wait(&o_full[x], (n_mine - 1) & 1);
+            ok = at_wait(&o_full[2 * x + ((n_mine - 1) & 1)], ((n_mine - 1) >> 1) & 1);
             at_fence_after();
             if (!ok && lane == 0) atomicExch(p.error, 5);
         }
@@ -526,7 +522,6 @@ static int as_map(const char* what, CUtensorMap* map, const void* base, int rank
 template <int KA, int VA, bool MAPS, bool CAP>
 static int as_launch(const char* what, dim3 grid, const CUtensorMap* maps, const AsArgs& args, cudaStream_t stream) {
     constexpr size_t smem = AsSmem<KA, VA, MAPS>::BYTES;
-    static_assert(smem <= 227 * 1024, "the tiles do not fit");
     auto kernel = attn_streams_kernel<KA, VA, MAPS, CAP>;
     cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return qwb_fail(QWB_ERR_CUDA, "%s: %s", what, cudaGetErrorString(e));

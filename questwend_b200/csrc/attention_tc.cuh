@@ -30,6 +30,14 @@ __device__ __forceinline__ bool at_wait(uint64_t* bar, uint32_t parity) {
     }
     return false;
 }
+// One lane of a converged warp, the same one every time.  tcgen05.mma takes its operands from registers that a warp shares;
+// issued under `lane == 0`, which the compiler cannot tell from any other condition, a product took about 100 cycles of the
+// issuing warp, whatever its size.  Under this it does not.
+__device__ __forceinline__ bool at_elect() {
+    uint32_t one;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(one));
+    return one;
+}
 __device__ __forceinline__ void at_tma_2d(void* dst, const CUtensorMap* map, uint64_t* bar, int c0, int c1) {
     asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
                  ::"r"(at_smem(dst)), "l"(map), "r"(at_smem(bar)), "r"(c0), "r"(c1) : "memory");
