@@ -32,21 +32,36 @@ __device__ __forceinline__ void mlstm_log_gates(MlstmRows rows, MlstmGates g, in
 }
 
 // ---------------------------------------------------------------------------------
-// Gates of a step that brings several tokens.  grid (H, B), 256 threads.  A token is the map m -> max(m + f, i); maps compose
-// into maps of the same form, so the running maxima are a scan over the tokens (in 64-bit, 256 at a time).  With the rounded
-// maxima, log_decay = m + f - m' telescopes exactly.  Outputs [T, H].
+// Gates of a step that brings several tokens.  grid (H, B), up to 1,024 threads, a token each.  A token is the map
+// m -> max(m + f, i); maps compose into maps of the same form, so the running maxima are a scan over the tokens (in 64-bit),
+// over a warp's tokens and then over the warps.  With the rounded maxima, log_decay = m + f - m' telescopes exactly.
+// Outputs [T, H].  What it costs is a sequence's chain of passes, each its loads, its logarithms and its scans one after the
+// other: 256 tokens a pass took 4,096 tokens through 16 passes (4 heads of 64 x 64 in chunks, 59.6 us in all), 1,024 take
+// them through four (51.7).  Short steps are as fast as they were: a block has no more warps than the step fills.
 // ---------------------------------------------------------------------------------
-__global__ void __launch_bounds__(256)
+#define QWB_MLSTM_GATE_THREADS 1024
+
+// an inclusive scan over the warp's lanes, the earlier map first: (F1, X1), then (F, X)
+__device__ __forceinline__ void mlstm_scan_maps(double& F, double& X) {
+    const int lane = threadIdx.x & 31;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const double F1 = __shfl_up_sync(0xffffffffu, F, o), X1 = __shfl_up_sync(0xffffffffu, X, o);
+        if (lane >= o) { X = fmax(X1 + F, X); F += F1; }
+    }
+}
+
+__global__ void __launch_bounds__(QWB_MLSTM_GATE_THREADS)
 mlstm_gates_kernel(MlstmRows rows, MlstmGates gates, const float* __restrict__ m_state, const int* __restrict__ cu_seqlens,
                    const int* __restrict__ slots, float* __restrict__ log_decay, float* __restrict__ write, float* __restrict__ m_run, int H, int P) {
     pdl_wait();
     pdl_launch_dependents();
-    __shared__ double tot_f[8], tot_x[8];
-    __shared__ float last_m[8];
-    const int h = blockIdx.x, b = blockIdx.y, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    __shared__ double tot_f[32], tot_x[32];
+    __shared__ float last_m[32];
+    const int h = blockIdx.x, b = blockIdx.y, warp = threadIdx.x >> 5, lane = threadIdx.x & 31, warps = blockDim.x >> 5;
     const int t0 = cu_seqlens[b], t1 = cu_seqlens[b + 1];
     double carry = (double)m_state[((size_t)slots[b] * H + h) * (P + 1)];
-    for (int base = t0; base < t1; base += 256) {
+    for (int base = t0; base < t1; base += blockDim.x) {
         const int t = base + threadIdx.x;
         float i = 0.f, f = 0.f;
         double F = 0.0, X = -INFINITY;                              // beyond the end: the map that changes nothing
@@ -54,18 +69,12 @@ mlstm_gates_kernel(MlstmRows rows, MlstmGates gates, const float* __restrict__ m
             mlstm_log_gates(rows, gates, t, h, i, f);
             F = (double)f; X = (double)i;
         }
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {                          // earlier map first: (F1, X1), then (F, X)
-            const double F1 = __shfl_up_sync(0xffffffffu, F, o), X1 = __shfl_up_sync(0xffffffffu, X, o);
-            if (lane >= o) { X = fmax(X1 + F, X); F += F1; }
-        }
+        mlstm_scan_maps(F, X);
         if (lane == 31) { tot_f[warp] = F; tot_x[warp] = X; }
         __syncthreads();
-        double start = carry, end = carry;                          // m before this warp's tokens, and after all 256
-        for (int w = 0; w < 8; ++w) {
-            if (w == warp) start = end;
-            end = fmax(end + tot_f[w], tot_x[w]);
-        }
+        double Fw = lane < warp ? tot_f[lane] : 0.0, Xw = lane < warp ? tot_x[lane] : -INFINITY;        // the warps before this one
+        if (warp > 0) mlstm_scan_maps(Fw, Xw);
+        const double start = fmax(carry + __shfl_sync(0xffffffffu, Fw, 31), __shfl_sync(0xffffffffu, Xw, 31));
         const float m = (float)fmax(start + F, X);
         if (lane == 31) last_m[warp] = m;
         __syncthreads();
@@ -77,10 +86,11 @@ mlstm_gates_kernel(MlstmRows rows, MlstmGates gates, const float* __restrict__ m
             write[at] = expf(i - m);
             m_run[at] = m;
         }
-        carry = (double)last_m[7];                                  // the rounded maximum goes on
+        carry = (double)last_m[warps - 1];                          // the rounded maximum goes on
         __syncthreads();
     }
 }
+static int mlstm_gate_threads(int T) { return T < QWB_MLSTM_GATE_THREADS ? (T + 31) / 32 * 32 : QWB_MLSTM_GATE_THREADS; }
 
 // ---------------------------------------------------------------------------------
 // The recurrence.  Warp = CW columns of one head of one sequence; lane l keeps rows l * PER .. l * PER + PER - 1 of each.
@@ -553,7 +563,7 @@ extern "C" int qwb_mlstm_scan(const float* x, int ld, int i_col, int f_col, cons
     if (!(cap > 0.f) || (single && T != B) || (!single && !gate_rows)) return qwb_fail(QWB_ERR_ARG, "mlstm_scan: cap %g, %d tokens of %d sequences", (double)cap, T, B);
     float *log_decay = gate_rows, *write = gate_rows + (size_t)T * H, *m_run = gate_rows + 2 * (size_t)T * H;
     if (!single) {
-        qwb_launch(mlstm_gates_kernel, dim3(H, B), 256, 0, stream, rows, gates, (const float*)m_state, cu_seqlens, slots, log_decay, write, m_run, H, P);
+        qwb_launch(mlstm_gates_kernel, dim3(H, B), mlstm_gate_threads(T), 0, stream, rows, gates, (const float*)m_state, cu_seqlens, slots, log_decay, write, m_run, H, P);
         if (int rc = qwb_check_launch("mlstm_gates")) return rc;
     }
     int per = 1;
@@ -597,7 +607,7 @@ extern "C" int qwb_mlstm_chunked(const float* x, int ld, int i_col, int f_col, c
     float *log_decay = gate_rows, *write = gate_rows + (size_t)T * H, *m_run = gate_rows + 2 * (size_t)T * H;
     float* totals = scratch + (size_t)B * n_chunks * H * (P + 1) * K;
     const bool vec = K % 4 == 0 && P % 4 == 0 && ld % 4 == 0 && mlstm_aligned(x) && mlstm_aligned(scratch) && mlstm_aligned(raw) && mlstm_aligned(state);
-    qwb_launch(mlstm_gates_kernel, dim3(H, B), 256, 0, stream, rows, gates, (const float*)m_state, cu_seqlens, slots, log_decay, write, m_run, H, P);
+    qwb_launch(mlstm_gates_kernel, dim3(H, B), mlstm_gate_threads(T), 0, stream, rows, gates, (const float*)m_state, cu_seqlens, slots, log_decay, write, m_run, H, P);
     if (int rc = qwb_check_launch("mlstm_gates")) return rc;
     const size_t smem1 = (size_t)QWB_MLSTM_CHUNK * (64 + pt) * sizeof(float);
     auto state_kernel = pt == 128 ? (vec ? mlstm_chunk_state_kernel<128, true> : mlstm_chunk_state_kernel<128, false>)

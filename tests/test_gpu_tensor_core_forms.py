@@ -224,6 +224,45 @@ def test_mamba2_in_chunks(H, P, N, G, pace):
     assert torch.equal(state, before)
 
 
+def matrix_memory(row, at, H, K, P, i_b, f_b, cap, S, top):
+    """The mLSTM in 64 bits over one sequence's rows from a memory [H, P + 1, K] and its maxima [H]: (read-outs, divisors, both after it)."""
+    row, n, n_qkv, S, top = row.double(), len(row), H * (2 * K + P), S.double().transpose(1, 2), top.double()
+    q, k, v = (row[:, a:b].reshape(n, H, -1) for a, b in ((0, H * K), (H * K, 2 * H * K), (2 * H * K, n_qkv)))
+    v = torch.cat([v, torch.ones(n, H, 1, dtype=F64, device=DEV)], 2)
+    li, lf = (cap * torch.tanh((row[:, c:c + H] + b.double()) / cap) for c, b in ((at, i_b), (at + H, f_b)))
+    lf = torch.nn.functional.logsigmoid(lf)
+    raw, div = torch.empty(n, H * P, dtype=F64, device=DEV), torch.empty(n, H, dtype=F64, device=DEV)
+    for i in range(n):
+        new = torch.maximum(top + lf[i], li[i])
+        S = torch.exp(top + lf[i] - new)[:, None, None] * S + torch.exp(li[i] - new)[:, None, None] * k[i][:, :, None] * v[i][:, None, :]
+        top = new
+        read = torch.einsum("hk,hkp->hp", q[i], S) * K ** -0.5
+        raw[i], div[i] = read[:, :P].reshape(-1), torch.maximum(read[:, P].abs(), torch.exp(-top)) + 1e-6
+    return raw, div, S.transpose(1, 2), top
+
+
+@pytest.mark.parametrize("lens", [[1025, 31, 1], [2100, 1024, 33], [3, 1, 20]])
+@pytest.mark.parametrize("forget", [2.0, 9.0])
+def test_exponential_gates_over_several_passes(lens, forget):
+    """Running maxima, decays and write strengths of sequences at the edges of a warp and of a pass of 1,024 tokens."""
+    torch.manual_seed(sum(lens))
+    H, K, P, cap = 2, 4, 4, 15.0
+    T, at, step = sum(lens), H * (2 * K + P), Steps(lens, [2, 0, 1])
+    proj = torch.randn(T, at + 2 * H, device=DEV)
+    proj[:, at + H:] += forget
+    i_b, f_b = 0.3 * torch.randn(H, device=DEV), 0.3 * torch.randn(H, device=DEV)
+    start, m_start = 0.5 * torch.randn(3, H, P + 1, K, device=DEV), (2 * torch.rand(3, H, 1, device=DEV)).repeat(1, 1, P + 1)
+    for chunked in (False, True):
+        st, m, t = start.clone(), m_start.clone(), 0
+        raw, div = ops.mlstm_scan(proj, at, at + H, i_b, f_b, cap, st, m, step, H, K, P, K ** -0.5, 1e-6, chunked=chunked)
+        for n, slot in zip(lens, [2, 0, 1]):
+            ref, div_ref, S, top = matrix_memory(proj[t:t + n], at, H, K, P, i_b, f_b, cap, start[slot], m_start[slot, :, 0])
+            for got, want in ((raw[t:t + n], ref), (div[t:t + n], div_ref), (st[slot], S)):
+                sums_close(got, want)
+            assert (m[slot].double() - top[:, None]).abs().max() <= 2 ** -20 * (1 + top.abs().max())
+            t += n
+
+
 @pytest.mark.parametrize("taps, C", [(2, 4), (3, 20), (4, 516), (4, 24)])
 @pytest.mark.parametrize("mode", ["silu", "plain", "plus", "bf16"])
 def test_convolutions_of_four_channels_a_thread(taps, C, mode):
