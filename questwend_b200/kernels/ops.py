@@ -1105,6 +1105,12 @@ def gated_part_norm(y: torch.Tensor, gate: torch.Tensor, gate_col0: int, weight:
 
 # ----------------------------------------------------------------------------- matrix memory with exponential gates
 MLSTM_CHUNKED_FROM = 64         # steps whose longest sequence brings at least this many tokens take the chunked form
+# Its chunks of 128 tokens (csrc/mlstm.cu: mlstm_tile_*), for sizes and rows in multiples of 4: keys of at least MLSTM_TILES_KEYS, whose
+# tiles are what hides the copies, and at least MLSTM_TILES_BLOCKS blocks of 128 tokens x 64 values, three an SM.  us, 64 / 128
+# tokens a chunk: 4 heads of 256 x 512, 1,000 tokens (249 blocks) 113 / 113, 2,048 233 / 194, 4,096 437 / 374, 4 x 1,024 438 / 367; 4 of
+# 256 x 256, 2,048 tokens (256) 118 / 133, 4,096 240 / 227; 8 of 512 x 256, 1,000 tokens 218 / 233, 2,048 433 / 392; 16 of
+# 128 x 128, 4,096 tokens (1,024) 289 / 295; 4 of 64 x 64, 4,096 tokens 51 / 69.
+MLSTM_TILES_KEYS, MLSTM_TILES_BLOCKS = 256, 512
 
 
 def mlstm_scan(proj: torch.Tensor, i_col: int, f_col: int, i_bias: torch.Tensor, f_bias: torch.Tensor, gate_cap: float,
@@ -1139,12 +1145,22 @@ def mlstm_scan(proj: torch.Tensor, i_col: int, f_col: int, i_bias: torch.Tensor,
     inputs = (_ptr(proj), _i(ld), _i(i_col), _i(f_col), _ptr(i_bias), _ptr(f_bias), _f(gate_cap), _ptr(state), _ptr(m_state),
               _ptr(ctx.cu_seqlens), _ptr(ctx.slots), _ptr(gate_rows))
     if chunked and not single:
+        sizes = (_i(T), _i(ctx.n_seqs), _i(ctx.max_new), _i(heads), _i(key_dim), _i(vdim))
+        if key_dim >= MLSTM_TILES_KEYS and T * heads * vdim >= MLSTM_TILES_BLOCKS * 128 * 64 and ld % 4 == 0 and proj.data_ptr() % 16 == 0:
+            lib, size = _lookup("mlstm", "qwb_mlstm_tiles_scratch")
+            size.restype = ctypes.c_longlong
+            floats = size(_i(T), _i(ctx.n_seqs), _i(heads), _i(key_dim), _i(vdim))
+            if 0 < floats <= CHUNK_SCRATCH_MAX:
+                scratch = torch.empty((floats,), dtype=torch.float32, device=dev)
+                _call("mlstm", "qwb_mlstm_tiles", *inputs, _ptr(scratch), _ptr(raw), _ptr(divisor), *sizes, _f(q_scale), _f(tiny),
+                      _i(1 if write_state else 0), _stream(), kernels=4)
+                return raw, divisor
         lib = _lookup("mlstm", "qwb_mlstm_scratch_floats")[0]
         lib.qwb_mlstm_scratch_floats.restype = ctypes.c_longlong
         scratch = torch.empty((lib.qwb_mlstm_scratch_floats(_i(ctx.n_seqs), _i(ctx.max_new), _i(heads), _i(key_dim), _i(vdim)),),
                               dtype=torch.float32, device=dev)
-        _call("mlstm", "qwb_mlstm_chunked", *inputs, _ptr(scratch), _ptr(raw), _ptr(divisor), _i(T), _i(ctx.n_seqs), _i(ctx.max_new),
-              _i(heads), _i(key_dim), _i(vdim), _f(q_scale), _f(tiny), _i(1 if write_state else 0), _stream(), kernels=4)
+        _call("mlstm", "qwb_mlstm_chunked", *inputs, _ptr(scratch), _ptr(raw), _ptr(divisor), *sizes, _f(q_scale), _f(tiny),
+              _i(1 if write_state else 0), _stream(), kernels=4)
     else:
         _call("mlstm", "qwb_mlstm_scan", *inputs, _ptr(raw), _ptr(divisor), _i(T), _i(ctx.n_seqs), _i(heads), _i(key_dim), _i(vdim),
               _f(q_scale), _f(tiny), _i(1 if single else 0), _i(1 if write_state else 0), _stream(), kernels=1 if single else 2)

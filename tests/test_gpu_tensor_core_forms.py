@@ -263,6 +263,45 @@ def test_exponential_gates_over_several_passes(lens, forget):
             t += n
 
 
+@pytest.mark.parametrize("H, K, P", [(1, 4, 4), (2, 64, 128), (3, 20, 68), (2, 132, 60), (2, 256, 512)])
+@pytest.mark.parametrize("forget", [-4.0, 2.0, 9.0])
+def test_matrix_memory_in_chunks_of_128(H, K, P, forget, monkeypatch):
+    """Sequences at the edges of the chunks of 128, from a memory, that fade, last and mix; rows shifted by one float take the
+    general form, which gives the same; slots of others stay as they are."""
+    torch.manual_seed(H + K + P)
+    monkeypatch.setattr(ops, "MLSTM_TILES_KEYS", 4)
+    monkeypatch.setattr(ops, "MLSTM_TILES_BLOCKS", 0)
+    lens, slots, cap = [1, 64, 127, 128, 129, 300], [4, 2, 7, 1, 5, 3], 15.0
+    T, n_qkv, step = sum(lens), H * (2 * K + P), Steps(lens, slots)
+    wide = torch.randn(T, -(-(n_qkv + 2 * H) // 4) * 4 + 4, device=DEV)
+    at, ld = n_qkv, wide.shape[1]
+    wide[:, at + H:at + 2 * H] += forget
+    flat = torch.empty(T * ld + 1, device=DEV)
+    shifted = flat[1:].view(T, ld)
+    shifted.copy_(wide)
+    i_b, f_b = 0.3 * torch.randn(H, device=DEV), 0.3 * torch.randn(H, device=DEV)
+    start, m_start = 0.5 * torch.randn(9, H, P + 1, K, device=DEV), (2 * torch.rand(9, H, 1, device=DEV)).repeat(1, 1, P + 1)
+    forms = []
+    for proj in (wide, shifted):
+        st, m = start.clone(), m_start.clone()
+        raw, div = ops.mlstm_scan(proj, at, at + H, i_b, f_b, cap, st, m, step, H, K, P, K ** -0.5, 1e-6)
+        forms.append((raw, div, st, m))
+    t = 0
+    for n, slot in zip(lens, slots):
+        ref, div_ref, S, top = matrix_memory(wide[t:t + n], at, H, K, P, i_b, f_b, cap, start[slot], m_start[slot, :, 0])
+        for raw, div, st, m in forms:
+            sums_close(raw[t:t + n], ref)
+            sums_close(div[t:t + n], div_ref)
+            sums_close(st[slot], S)
+            assert (m[slot].double() - top[:, None]).abs().max() <= 2 ** -20 * (1 + top.abs().max())
+        t += n
+    raw, div, st, m = forms[0]
+    assert torch.equal(st[[0, 6, 8]], start[[0, 6, 8]]) and torch.equal(m[[0, 6, 8]], m_start[[0, 6, 8]])
+    before, m_before = st.clone(), m.clone()
+    ops.mlstm_scan(wide, at, at + H, i_b, f_b, cap, st, m, step, H, K, P, K ** -0.5, 1e-6, write_state=False)
+    assert torch.equal(st, before) and torch.equal(m, m_before)
+
+
 @pytest.mark.parametrize("taps, C", [(2, 4), (3, 20), (4, 516), (4, 24)])
 @pytest.mark.parametrize("mode", ["silu", "plain", "plus", "bf16"])
 def test_convolutions_of_four_channels_a_thread(taps, C, mode):
