@@ -456,7 +456,7 @@ delta_chunk_prep_kernel(const DcArgs a) {
     extern __shared__ __align__(16) float dc_smem[];
     float* ks = dc_smem;                                            // k; then k times what decays behind it
     float* qs = ks + DC_TOKENS * DC_MAX_K;                             // q; then q times what decays from its sub-block's start on
-    float* gs = qs + DC_TOKENS * DC_MAX_K;                             // sums of logarithms in the sub-block; then k as q
+    float* gs = qs + DC_TOKENS * DC_MAX_K;                             // logarithms of the decays; then k as q
     float* As = gs + DC_TOKENS * DC_MAX_K;                             // beta_i A_ij
     float* totals = As + DC_A_FLOATS;                               // [4][128]
     float* beta = totals + 4 * DC_MAX_K;
@@ -500,59 +500,68 @@ delta_chunk_prep_kernel(const DcArgs a) {
         }
     }
     __syncthreads();
-    for (int idx = tid; idx < 4 * DC_MAX_K; idx += 256) {           // sums in the sub-blocks
-        const int s = idx / DC_MAX_K, k = idx - s * DC_MAX_K;
-        if (k >= K) continue;
-        float sum = 0.f;
-#pragma unroll
-        for (int j = 0; j < DC_SUB; ++j) {
-            sum += gs[dc_at(s * DC_SUB + j, k)];
-            gs[dc_at(s * DC_SUB + j, k)] = sum;
-        }
-        totals[idx] = sum;
-    }
-    __syncthreads();
-    // pairs of one sub-block, four threads a pair: 136 with j <= i of each
+    // pairs of one sub-block, four threads a token j: i goes down the tokens from j on, and what decays on the way is summed from j
+    // on, never taken as the difference of two sums from the sub-block's start (after a token that forgets, the difference has
+    // lost the digits of those that keep, and after a logarithm of -infinity it is no number)
     const int lane4 = (tid & 3) * 4;
-    for (int task = tid >> 2; task < 4 * 136; task += 64) {         // 544 = 8.5 rounds of 64: the last one half full, by whole warps
-        const int s = task / 136, t = task - s * 136;
-        int i = (int)((sqrtf(8.f * (float)t + 1.f) - 1.f) * 0.5f);
-        while ((i + 1) * (i + 2) / 2 <= t) ++i;
-        while (i * (i + 1) / 2 > t) --i;
-        const int j = t - i * (i + 1) / 2, ri = s * DC_SUB + i, rj = s * DC_SUB + j;
-        float sa = 0.f, sq = 0.f;
-#pragma unroll 4
-        for (int k = lane4; k < K; k += 16) {
-            const int pi = dc_at(ri, k), pj = dc_at(rj, k);
-            const float4 gi = *reinterpret_cast<const float4*>(gs + pi), gj = *reinterpret_cast<const float4*>(gs + pj);
-            const float4 ki = *reinterpret_cast<const float4*>(ks + pi), kj = *reinterpret_cast<const float4*>(ks + pj);
-            const float4 qi = *reinterpret_cast<const float4*>(qs + pi);
-            const float x = kj.x * dc_exp2(gi.x - gj.x), y = kj.y * dc_exp2(gi.y - gj.y), z = kj.z * dc_exp2(gi.z - gj.z), w = kj.w * dc_exp2(gi.w - gj.w);
-            sa += ki.x * x + ki.y * y + ki.z * z + ki.w * w;
-            sq += qi.x * x + qi.y * y + qi.z * z + qi.w * w;
+    {
+        const int j = tid >> 2, end = (j / DC_SUB + 1) * DC_SUB;
+        float4 kj[DC_MAX_K / 16], sum[DC_MAX_K / 16];
+#pragma unroll
+        for (int c = 0; c < DC_MAX_K / 16; ++c) {
+            kj[c] = lane4 + 16 * c < K ? *reinterpret_cast<const float4*>(ks + dc_at(j, lane4 + 16 * c)) : make_float4(0.f, 0.f, 0.f, 0.f);
+            sum[c] = make_float4(0.f, 0.f, 0.f, 0.f);
         }
-        sa = dc_quad_sum(sa);
-        sq = dc_quad_sum(sq);
-        if (lane4 == 0) {
-            const int gi_ = s * DC_SUB + i, gj_ = s * DC_SUB + j;
-            if (j < i) As[dc_row(gj_) + gi_] = beta[gi_] * sa;
-            at.q_pairs[gj_ * DC_TOKENS + gi_] = sq;
-            if (j < i) at.q_pairs[gi_ * DC_TOKENS + gj_] = 0.f;
+#pragma unroll 1
+        for (int i = 8 * warp; i < end; ++i) {                      // from the first of the warp's eight tokens on
+            float sa = 0.f, sq = 0.f;
+#pragma unroll
+            for (int c = 0; c < DC_MAX_K / 16; ++c) {
+                if (lane4 + 16 * c >= K) continue;
+                const int pi = dc_at(i, lane4 + 16 * c);
+                const float4 l = *reinterpret_cast<const float4*>(gs + pi), ki = *reinterpret_cast<const float4*>(ks + pi), qi = *reinterpret_cast<const float4*>(qs + pi);
+                if (i > j) sum[c] = make_float4(sum[c].x + l.x, sum[c].y + l.y, sum[c].z + l.z, sum[c].w + l.w);
+                const float x = kj[c].x * dc_exp2(sum[c].x), y = kj[c].y * dc_exp2(sum[c].y), z = kj[c].z * dc_exp2(sum[c].z), w = kj[c].w * dc_exp2(sum[c].w);
+                sa += ki.x * x + ki.y * y + ki.z * z + ki.w * w;
+                sq += qi.x * x + qi.y * y + qi.z * z + qi.w * w;
+            }
+            sa = dc_quad_sum(sa);
+            sq = dc_quad_sum(sq);
+            if (lane4 == 0 && i >= j) {
+                if (i > j) As[dc_row(j) + i] = beta[i] * sa;
+                at.q_pairs[j * DC_TOKENS + i] = sq;
+                if (i > j) at.q_pairs[i * DC_TOKENS + j] = 0.f;
+            }
         }
     }
     __syncthreads();
-    // q and k by what decays from their sub-block's start on (k's into gs), k by what decays behind it in the sub-block
-#pragma unroll 4
-    for (int j = warp; j < DC_TOKENS && e_lane < K; j += 8) {
-        const int e = e_lane, s = j / DC_SUB;
-        float4* gp = reinterpret_cast<float4*>(gs + dc_at(j, e));
-        float4* kp = reinterpret_cast<float4*>(ks + dc_at(j, e));
-        float4* qp = reinterpret_cast<float4*>(qs + dc_at(j, e));
-        const float4 g = *gp, k = *kp, q = *qp, tot = *reinterpret_cast<const float4*>(totals + s * DC_MAX_K + e);
-        const float4 f = make_float4(dc_exp2(g.x), dc_exp2(g.y), dc_exp2(g.z), dc_exp2(g.w));
-        *gp = make_float4(k.x * f.x, k.y * f.y, k.z * f.z, k.w * f.w);
-        *qp = make_float4(q.x * f.x, q.y * f.y, q.z * f.z, q.w * f.w);
-        *kp = make_float4(k.x * dc_exp2(tot.x - g.x), k.y * dc_exp2(tot.y - g.y), k.z * dc_exp2(tot.z - g.z), k.w * dc_exp2(tot.w - g.w));
+    // q and k by what decays from their sub-block's start on (k's into gs), k by what decays behind it in the sub-block, each
+    // from a sum of its own; two channels of a sub-block's tokens a thread
+    {
+        const int s = tid >> 6, e = (tid & 63) * 2;
+        if (e < K) {
+            float2 l[DC_SUB];
+            float x = 0.f, y = 0.f;
+#pragma unroll
+            for (int j = 0; j < DC_SUB; ++j) l[j] = *reinterpret_cast<const float2*>(gs + dc_at(s * DC_SUB + j, e));
+#pragma unroll
+            for (int j = 0; j < DC_SUB; ++j) {
+                const int p = dc_at(s * DC_SUB + j, e);
+                x += l[j].x; y += l[j].y;
+                const float fx = dc_exp2(x), fy = dc_exp2(y);
+                const float2 k = *reinterpret_cast<const float2*>(ks + p), q = *reinterpret_cast<const float2*>(qs + p);
+                *reinterpret_cast<float2*>(gs + p) = make_float2(k.x * fx, k.y * fy);
+                *reinterpret_cast<float2*>(qs + p) = make_float2(q.x * fx, q.y * fy);
+            }
+            *reinterpret_cast<float2*>(totals + s * DC_MAX_K + e) = make_float2(x, y);
+            x = y = 0.f;
+#pragma unroll
+            for (int j = DC_SUB - 1; j >= 0; --j) {
+                float2* kp = reinterpret_cast<float2*>(ks + dc_at(s * DC_SUB + j, e));
+                *kp = make_float2(kp->x * dc_exp2(x), kp->y * dc_exp2(y));
+                x += l[j].x; y += l[j].y;
+            }
+        }
     }
     // pairs of two sub-blocks: rows of sub-block s with all before it, 2 x 2 pairs to four threads
     for (int s = 1; s < 4; ++s) {

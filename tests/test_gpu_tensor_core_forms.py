@@ -367,6 +367,41 @@ def test_delta_rule_in_chunks(H, Hk, K, P, per_head, pace):
     assert torch.equal(state, before)
 
 
+@pytest.mark.parametrize("per_head", [False, True])
+@pytest.mark.parametrize("rate, forget", [(16.0, 10.0), (1.0, 1000.0), (1.0, 1e5), (2.0, math.inf)])
+def test_delta_rule_in_chunks_with_tokens_that_forget(per_head, rate, forget):
+    """Tokens that clear most of the memory among tokens that keep it.  The scan multiplies by a token's own decay, an error of a
+    rounding or two a token whatever came before; the chunks' error is of that size."""
+    torch.manual_seed(int(rate))
+    H, Hk, K, P, T = 2, 2, 128, 64, 400
+    n_decay, C, col = H if per_head else H * K, 2 * Hk * K + H * P, 3 if per_head else 0
+    step = Steps([T], [1])
+    qkv, b_raw, a_raw = torch.randn(T, C, device=DEV), torch.randn(T, H, device=DEV), torch.randn(T, n_decay + col, device=DEV) - 8.0
+    bias, a_log = torch.zeros(n_decay, device=DEV), torch.full((H,), math.log(rate), device=DEV)
+    if per_head:
+        a_raw[3::8, col:] = forget
+    else:
+        a_raw[3::8, torch.rand(n_decay, device=DEV) < 0.7] = forget
+    start = 0.3 * torch.randn(2, H, P, K, device=DEV)
+    S, ref = start[1].double(), torch.empty(T, H * P, dtype=F64, device=DEV)
+    for i in range(T):
+        row = qkv[i].double()
+        q, k = (x / torch.sqrt((x * x).sum(-1, keepdim=True) + 1e-6) for x in (row[m * Hk * K:(m + 1) * Hk * K].view(Hk, K).repeat_interleave(H // Hk, 0) for m in (0, 1)))
+        raw = torch.nn.functional.softplus(a_raw[i, col:].double(), threshold=100.0).view(H, -1)
+        S = S * torch.exp(-torch.exp(a_log.double())[:, None] * raw)[:, None, :]
+        u = torch.sigmoid(b_raw[i].double())[:, None] * (row[2 * Hk * K:].view(H, P) - (S @ k[:, :, None])[..., 0])
+        S = S + u[:, :, None] * k[:, None, :]
+        ref[i] = (S @ (q * K ** -0.5)[:, :, None]).reshape(-1)
+    errors = []
+    for longest in (T, 1):                                  # the chunks, the scan
+        step.max_new, state = longest, start.clone()
+        o = ops.delta_rule(qkv.clone(), b_raw, 0, a_raw, bias, a_log, state, step, H, Hk, K, P, 1e-6, K ** -0.5, per_head=per_head, a_col0=col)
+        assert torch.isfinite(o).all() and torch.isfinite(state).all()
+        errors.append([float((got.double() - want).norm() / want.norm()) for got, want in ((o, ref), (state[1], S))])
+    for chunks, scan in zip(*errors):
+        assert chunks <= 2 * scan + 2.0 ** -23, errors
+
+
 # ----------------------------------------------------------------------------- score maps, single tokens
 @pytest.mark.parametrize("maps, H, G, dim, vdim", [(2, 16, 4, 64, 128), (2, 2, 2, 8, 8), (2, 15, 3, 40, 72), (1, 10, 1, 128, 128), (2, 4, 1, 128, 120), (1, 3, 3, 24, 16)])
 @pytest.mark.parametrize("softcap, window, chunk, gated", [(0.0, 0, 0, False), (5.0, 0, 0, True), (3.0, 100, 0, False), (2.0, 1, 0, True), (20.0, 0, 96, False)])
