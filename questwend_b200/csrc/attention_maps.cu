@@ -1208,7 +1208,10 @@ __global__ void maps_decode_kernel(const T* __restrict__ q, const T* __restrict_
 // 49.8 / 33.4, 64 runs 61.7 / 25.7.
 #define MD_MAX_RUNS 32
 
-static bool maps_decode_mma_fits(int dtype, int maps, int dim, int vdim) { return dtype == QWB_DT_BF16 && maps * dim <= 256 && vdim <= 128; }
+// q is read in pieces of 16 bytes, which maps_decode_kernel does not do: from another address it takes that one.
+static bool maps_decode_mma_fits(int dtype, int maps, int dim, int vdim, const void* q) {
+    return dtype == QWB_DT_BF16 && maps * dim <= 256 && vdim <= 128 && (uintptr_t)q % 16 == 0;
+}
 static size_t maps_decode_mma_smem(int kdim, int vdim) {
     const size_t stages = (size_t)MD_WARPS * MD_STAGES * MD_KEYS * (kdim + vdim) * sizeof(bf16);
     const size_t sums = (size_t)MD_WARPS * QWB_MAPS_ROWS * (vdim + 2) * sizeof(float);      // over the stages, once they are read
@@ -1457,15 +1460,15 @@ maps_merge_kernel(const float* __restrict__ part_acc, const float* __restrict__ 
     }
 }
 
-// runs of the grid for sequences of up to max_len tokens
-extern "C" int qwb_maps_decode_runs(int dtype, int maps, int dim, int vdim, int max_len, int chunk, int window) {
+// runs of the grid for sequences of up to max_len tokens; q: what qwb_maps_decode will be given (which of the two forms runs follows from it)
+extern "C" int qwb_maps_decode_runs(const void* q, int dtype, int maps, int dim, int vdim, int max_len, int chunk, int window) {
     if (max_len <= 0) return 1;
     // the most pages a sequence's visible keys touch: a chunk or a window may begin anywhere in its first page
     const int pages_all = (max_len + QWB_MAPS_PAGE - 1) / QWB_MAPS_PAGE;
     const int most = chunk > 0 && window > 0 ? min(chunk, window) : max(chunk, window);
     const int pages = most > 0 ? min(pages_all, (most + QWB_MAPS_PAGE - 2) / QWB_MAPS_PAGE + 1) : pages_all;
     const int runs = (pages + QWB_MAPS_RUN_PAGES - 1) / QWB_MAPS_RUN_PAGES;
-    const int max_runs = maps_decode_mma_fits(dtype, maps, dim, vdim) ? MD_MAX_RUNS : QWB_MAPS_MAX_RUNS;
+    const int max_runs = maps_decode_mma_fits(dtype, maps, dim, vdim, q) ? MD_MAX_RUNS : QWB_MAPS_MAX_RUNS;
     return runs < max_runs ? runs : max_runs;
 }
 
@@ -1485,7 +1488,7 @@ static int launch_maps_decode(const void* q, const void* k_pool, const void* v_p
     float* part_m = part_acc + rows * n_runs * vdim;
     float* part_l = part_m + rows * n_runs;
     const int rows_g = (H / G) * maps, slices = (rows_g + QWB_MAPS_ROWS - 1) / QWB_MAPS_ROWS;
-    const bool mma = std::is_same<T, bf16>::value && maps_decode_mma_fits(QWB_DT_BF16, maps, dim, vdim);
+    const bool mma = std::is_same<T, bf16>::value && maps_decode_mma_fits(QWB_DT_BF16, maps, dim, vdim, q);
     const size_t smem = mma ? maps_decode_mma_smem(kdim, vdim)
                             : ((size_t)QWB_MAPS_PAGE * (kdim + VEC) + (size_t)QWB_MAPS_PAGE * vdim) * sizeof(T) +
                                   ((size_t)QWB_MAPS_ROWS * dim + QWB_MAPS_ROWS * QWB_MAPS_PAGE + 3 * QWB_MAPS_ROWS) * sizeof(float);

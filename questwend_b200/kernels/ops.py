@@ -1411,7 +1411,7 @@ def maps_attention(q: torch.Tensor, k_pool, v_pool, page_table, ctx, maps: int, 
         return attn_decode(q, k_pool, v_pool, page_table, ctx.seq_len, scale, ctx.max_len, window=window, impl="mma")
     if ctx.single_token and dim % MAPS_FAST_STEP == 0 and vdim % MAPS_FAST_STEP == 0:
         lib = _lookup("attention_maps", "qwb_maps_decode_runs")[0]
-        n_runs = lib.qwb_maps_decode_runs(_i(_dt(q.dtype)), _i(maps), _i(dim), _i(vdim), _i(ctx.max_len), _i(chunk), _i(window))
+        n_runs = lib.qwb_maps_decode_runs(_ptr(q), _i(_dt(q.dtype)), _i(maps), _i(dim), _i(vdim), _i(ctx.max_len), _i(chunk), _i(window))
         lib.qwb_maps_decode_scratch_floats.restype = ctypes.c_longlong
         scratch = torch.empty((lib.qwb_maps_decode_scratch_floats(_i(T), _i(H), _i(maps), _i(vdim), _i(n_runs)),),
                               dtype=torch.float32, device=q.device)

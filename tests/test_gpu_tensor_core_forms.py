@@ -443,3 +443,18 @@ def test_score_maps_of_single_tokens_on_the_tensor_cores(maps, H, G, dim, vdim, 
                 assert (err <= 2.0 ** -8 * ref.abs() + 2e-5 * max(1.0, grown)).all(), (n, h, err.max())
     for i, b in enumerate([1, 9, 10]):                      # a sequence's result does not depend on the batch
         assert torch.equal(alone[0][b], alone[i + 1][0])
+
+
+@pytest.mark.parametrize("maps, H, G, dim, vdim", [(2, 16, 4, 64, 128), (2, 6, 3, 40, 72)])
+def test_score_maps_of_single_tokens_from_any_address(maps, H, G, dim, vdim):
+    """Queries that do not lie at a multiple of 16 bytes take the form that reads them one by one, with runs of its own."""
+    torch.manual_seed(H + dim)
+    lens = [1, 65, 300, 6000]
+    table, (k_pool, v_pool) = paged(lens, lambda s: torch.randn(s, device=DEV).to(BF), [(G, maps * dim), (G, vdim)])
+    q = torch.randn(len(lens), H, maps * dim, device=DEV).to(BF)
+    flat = torch.empty(q.numel() + 1, dtype=BF, device=DEV)
+    shifted = flat[1:].view(q.shape)
+    shifted.copy_(q)
+    ctx = SimpleNamespace(single_token=True, n_seqs=len(lens), max_new=1, max_len=max(lens), seq_len=torch.tensor(lens, device=DEV).int())
+    a, b = (ops.maps_attention(x, k_pool, v_pool, table, ctx, maps, dim ** -0.5, lam=0.4) for x in (q, shifted))
+    assert ((a.double() - b.double()).abs() <= 2.0 ** -7 * a.double().abs() + 2e-5).all()      # two roundings of nearly the same numbers
