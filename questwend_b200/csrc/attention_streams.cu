@@ -343,7 +343,19 @@ attn_streams_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
             const bool all_visible = key0 + AT_KEYS - 1 <= qp && key0 >= own;           // no mask needed
             float mx = -INFINITY;
             bool series = false;
+            // in tiles that are not wholly visible the row sees the keys [lo, lo + span): one subtraction and one comparison a key
+            const int lo = max(own - key0, 0), span = max(min(qp - key0 + 1, AT_KEYS) - lo, 0);
+            auto mask = [&](uint32_t with) {
+#pragma unroll
+                for (int h = 0; h < 2; ++h)
+#pragma unroll
+                    for (int c = 0; c < 32; ++c)
+                        if ((unsigned)(32 * h + c - lo) >= (unsigned)span) sv[h][c] = with;
+            };
             if (CAP) {
+                // which form the scores take follows from visible keys alone: behind them stand later tokens, and what an earlier
+                // user of the page left there
+                if (!all_visible) mask(0u);
                 const float most = as_max<true>(sv);
                 if (all_visible && most <= poly_up_to) {        // the series below, formed together with the exponent's argument
                     series = true;
@@ -369,16 +381,7 @@ attn_streams_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
                         }
                 }
             }
-            if (!all_visible) {
-                // the row sees the tile's keys [lo, end): one subtraction and one unsigned comparison a key
-                const int end = min(qp - key0 + 1, AT_KEYS), lo = max(own - key0, 0);
-                const unsigned span = end > lo ? (unsigned)(end - lo) : 0u;
-#pragma unroll
-                for (int h = 0; h < 2; ++h)
-#pragma unroll
-                    for (int c = 0; c < 32; ++c)
-                        if ((unsigned)(32 * h + c - lo) >= span) sv[h][c] = 0xff800000u;       // -inf
-            }
+            if (!all_visible) mask(0xff800000u);                                       // -inf
             if (!series) mx = as_max<false>(sv);
             const bool rescale = mx > m_ref + AT_RESCALE_LOG2 / sl2;                    // else keep the old reference
             const float m_new = rescale ? mx : m_ref;

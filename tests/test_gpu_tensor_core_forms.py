@@ -13,9 +13,9 @@ DEV = torch.device("cuda:0")
 BF, F64 = torch.bfloat16, torch.float64
 
 
-def paged(lens, rows_of, width):
+def paged(lens, rows_of, width, behind=math.nan):
     """Sequences of these lengths in pages of 64 dealt out in reverse order: (page table, pools filled by ``rows_of(shape)``
-    for each of ``width``).  The rows behind a sequence's end hold large numbers: nothing may read them."""
+    for each of ``width``).  The rows behind a sequence's end hold no numbers (or ``behind``): nothing of them may reach a result."""
     pages = [-(-n // 64) for n in lens]
     order = list(range(sum(pages)))[::-1]
     table = torch.zeros(len(lens), max(pages), dtype=torch.int32, device=DEV)
@@ -24,7 +24,7 @@ def paged(lens, rows_of, width):
         mine, order = order[:p], order[p:]
         table[b, :p] = torch.tensor(mine, dtype=torch.int32)
         for pool in pools:
-            pool[mine[-1], :, n - 64 * (p - 1):] = 1e4
+            pool[mine[-1], :, n - 64 * (p - 1):] = behind
     return table, pools
 
 
@@ -166,6 +166,27 @@ def test_two_map_prompts_with_a_stream_a_map(H, G, dim, vdim, softcap, window, c
                 ref, size = ref * torch.sigmoid(gate[part, h + 2:h + 3].double()), size * torch.sigmoid(gate[part, h + 2:h + 3].double())
             bf16_close(got[part, h], ref, size)
         start += n
+    ops.gemm_tc_check(DEV)
+
+
+@pytest.mark.parametrize("softcap", [0.0, 3.0, 50.0])
+def test_two_map_prompts_see_nothing_behind_a_row(softcap):
+    """The same bits whatever stands behind the sequence's end in its last page, and whatever tokens follow."""
+    H, G, dim, vdim, lens = 16, 4, 64, 128, [1, 33, 70, 130, 300]
+    results = []
+    for behind, later in ((math.nan, 0), (1e4, 0), (0.0, 0), (0.0, 100)):
+        torch.manual_seed(1)                                # the first tokens of a sequence are the same, however many there are
+        ks, vs, qs = ([torch.randn(400, *size, device=DEV).to(BF) for _ in lens] for size in ((G, 2 * dim), (G, vdim), (H, 2 * dim)))
+        counts = [n + later for n in lens]
+        table, pools = paged(counts, lambda s: torch.zeros(s, dtype=BF, device=DEV), [(G, 2 * dim), (G, vdim)], behind)
+        for b, n in enumerate(counts):
+            at = torch.arange(n, device=DEV)
+            for pool, seq in zip(pools, (ks, vs)):
+                pool[table[b, (at // 64).long()].long(), :, (at % 64).long()] = seq[b][:n]
+        q = torch.cat([x[:n] for x, n in zip(qs, counts)])
+        out = ops.maps_attention(q, *pools, table, prompt_step(counts), 2, dim ** -0.5, softcap=softcap, lam=0.4, impl="tc")
+        results.append(torch.cat([x[:n] for x, n in zip(out.split(counts), lens)]))
+    assert torch.isfinite(results[0]).all() and all(torch.equal(results[0], r) for r in results[1:])
     ops.gemm_tc_check(DEV)
 
 
