@@ -9,22 +9,26 @@
 //                       maps, its values serve both, and the difference, its norm and the gate are taken at the end.
 //
 // Per stream and tile: S = Q K^T into tensor memory (64 columns, two buffers), P = softmax by four warps, a thread a row, left as
-// bfloat16 in tensor memory over the scores it came from, O += P V with P read from there, O in tensor memory (VD columns), the
-// row's reference maximum moved only when a tile exceeds it by more than 2^8.  A stream waits for its product only when it
-// rescales O; otherwise it may be two tiles ahead.  With two streams in one block the tensor cores work on one while the other is
+// bfloat16 in tensor memory over the scores it came from, O += P V with P read from there, O in tensor memory (VD columns).  P is
+// relative to the row's largest score so far, as with the mma.sync kernels: the largest probability is 1 and exact in bfloat16.  A
+// reference that is moved only past 2^8 is faster (8,192 tokens 529 us where this takes 577, one latent prompt the same) but rounds
+// the largest probability too: errors of 0.00213 and 0.00260 of the results in place of 0.00207 and 0.00252, more where few keys weigh.
+// A stream waits for its product only when a row of a warp moves its reference; otherwise it may be two tiles ahead.  With two streams in one block the tensor cores work on one while the other is
 // in its softmax, what two blocks an SM give attention_tc.cu, but the Q, K and V tiles of 192-value keys would not leave room for
 // a second block (2 x 48 KB of Q, K and V in three stages: 216 KB), and K and V cross L2 once for 256 rows.  Warp 0 loads, warp 1
 // issues the products, warps 2-5 and 6-9 are the streams' softmax warps.  Every wait is bounded.
 //
 // Sizes that are no multiples of 64 are filled up by the TMA loads with zeros.  In the last tile, rows of V behind the last
 // key that the block sees are overwritten with zeros before the product: they can belong to another sequence, and what stands
-// there, infinite or not a number, must not meet a probability of 0.
+// there, infinite or not a number, must not meet a probability of 0.  Inside a sequence a value that is not finite does meet
+// the zeros of the rows before it: up to 127 earlier tokens of a latent prompt (64-row tiles: 63) and 128 / (heads a group) - 1 of
+// one with two maps.
 //
 // Bound by the tensor cores' products of 64 keys (clocks in a block: the issuing warp is busy all of the time, a softmax warp two
 // thirds of a tile's waiting for scores).  16 heads, replayed from a graph, with the mma.sync kernels, with P in shared memory, and
-// now: latent 128 + 64 / 128, one prompt of 4,096: 816 -> 155 -> 108 us, of 600: 55 -> 19 -> 14.5 us; two maps of 64 over 4
-// key/value heads, values of 128, 8,192 tokens: 2,447 -> 707 -> 529 us (cap 50: 3,261 -> 795 -> 607), 2,048 tokens with a window of
-// 1,024: 170 -> 52 -> 41 us.  Of the last step P in tensor memory and the third and fourth stage gave 5 to 10 %, the elected lane
+// now: latent 128 + 64 / 128, one prompt of 4,096: 816 -> 155 -> 108 us, of 600: 55 -> 19 -> 16 us; two maps of 64 over 4
+// key/value heads, values of 128, 8,192 tokens: 2,447 -> 707 -> 577 us (cap 50: 3,261 -> 795 -> 693), 2,048 tokens with a window of
+// 1,024: 170 -> 52 -> 48 us.  Of the last step P in tensor memory and the third and fourth stage gave 5 to 10 %, the elected lane
 // in place of `lane == 0` the rest.
 #include "attention_tc.cuh"
 
@@ -383,7 +387,7 @@ attn_streams_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
             }
             if (!all_visible) mask(0xff800000u);                                       // -inf
             if (!series) mx = as_max<false>(sv);
-            const bool rescale = mx > m_ref + AT_RESCALE_LOG2 / sl2;                    // else keep the old reference
+            const bool rescale = mx > m_ref;
             const float m_new = rescale ? mx : m_ref;
             const float alpha = rescale ? at_exp2((m_ref - m_new) * sl2) : 1.f;        // m_ref = -inf gives 0
             const float base = m_new == -INFINITY ? 0.f : m_new * sl2;

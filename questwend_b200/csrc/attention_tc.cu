@@ -27,6 +27,7 @@
 
 #define AT_THREADS 192
 #define AT_KV_STAGES 2
+#define AT_RESCALE_LOG2 8.f
 
 template <int HD, int VD>
 struct AtSmem {

@@ -9,7 +9,6 @@
 #define AT_ROWS 128
 #define AT_KEYS 64
 #define AT_SPIN_LIMIT (1u << 22)
-#define AT_RESCALE_LOG2 8.f
 
 __device__ __forceinline__ uint32_t at_smem(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 __device__ __forceinline__ void at_bar_init(uint64_t* bar, uint32_t count) {

@@ -169,6 +169,41 @@ def test_two_map_prompts_with_a_stream_a_map(H, G, dim, vdim, softcap, window, c
     ops.gemm_tc_check(DEV)
 
 
+def rounded_by_running_maxima(q, k, v, scale):
+    """Causal attention as the tensor cores are given it: tiles of 64 keys, probabilities relative to the largest score so far (which
+    is 1 then, and exact) in bfloat16, all else in 64 bits; the result in bfloat16."""
+    n = len(q)
+    m, l, o = torch.full((n, 1), -math.inf, dtype=F64, device=DEV), 0.0, 0.0
+    for at in range(0, n, 64):
+        s = (q @ k[at:at + 64].T * scale).masked_fill(torch.arange(n, device=DEV)[:, None] < at + torch.arange(len(k[at:at + 64]), device=DEV)[None, :], -math.inf)
+        top = torch.maximum(m, s.amax(1, keepdim=True))
+        p, fade = torch.exp(s - top), torch.exp(m - top)
+        l, o, m = l * fade + p.sum(1, keepdim=True), o * fade + p.float().to(BF).double() @ v[at:at + 64], top
+    return (o / l).float().to(BF).double()
+
+
+@pytest.mark.parametrize("sharp", [1.0, 2.0, 4.0])
+def test_probabilities_of_two_streams_are_relative_to_the_largest(sharp):
+    """A row's largest probability is 1, which costs no rounding: errors are those of the running maximum, also where few keys weigh."""
+    torch.manual_seed(int(sharp))
+    T, H, dim = 600, 4, 64
+    q, k, v = (torch.randn(T, H, n, device=DEV) for n in (dim, dim, 128))
+    q = (sharp * q).to(BF)
+    k, v = k.to(BF), v.to(BF)
+    got = ops.latent_prefill(q, k.view(T, -1), torch.zeros(T, 16, dtype=BF, device=DEV), v.view(T, -1), prompt_step([T]), None, dim ** -0.5, 0, H, dim, 0, 128).view(T, H, 128)
+    table, (k_pool, v_pool) = paged([T], lambda s: torch.randn(s, device=DEV).to(BF), [(H, 2 * dim), (H, 128)])
+    at = torch.arange(T, device=DEV)
+    k_pool[table[0, at // 64].long(), :, at % 64] = torch.cat([k, k], 2)
+    v_pool[table[0, at // 64].long(), :, at % 64] = v
+    two = ops.maps_attention(torch.cat([q, q], 2), k_pool, v_pool, table, prompt_step([T]), 2, dim ** -0.5, lam=0.0, impl="tc").view(T, H, 128)
+    exact, same = (torch.stack([f(q[:, h].double(), k[:, h].double(), v[:, h].double()) for h in range(H)], 1) for f in (
+        lambda a, b, c: softmax(a, b, c, dim ** -0.5, at), lambda a, b, c: rounded_by_running_maxima(a, b, c, dim ** -0.5)))
+    allowed = 1.02 * float((same - exact).norm())           # what 32-bit sums and exponentials move across a rounding is far less
+    for out in (got, two):
+        assert float((out.double() - exact).norm()) <= allowed
+    ops.gemm_tc_check(DEV)
+
+
 @pytest.mark.parametrize("softcap", [0.0, 3.0, 50.0])
 def test_two_map_prompts_see_nothing_behind_a_row(softcap):
     """The same bits whatever stands behind the sequence's end in its last page, and whatever tokens follow."""
