@@ -14,6 +14,25 @@ __device__ __forceinline__ void rc_copy16(float* dst, const float* src, bool ok)
 __device__ __forceinline__ void rc_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 template <int N> __device__ __forceinline__ void rc_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
 
+// Which sequences a chunked form takes: those that bring at least `from` tokens (0: all).  A grid has a plane for each that there can
+// be, `rc_planes`; plane z is the z-th of them, found by every warp for itself.  -1: there are no so many.
+static int rc_planes(int T, int B, int from) { return from > 0 && T / from < B ? T / from : B; }
+__device__ __forceinline__ int rc_sequence(const int* __restrict__ cu_seqlens, int B, int from, int z) {
+    if (from <= 0) return z;
+    const int lane = threadIdx.x & 31;
+    for (int first = 0; first < B; first += 32) {
+        const int b = first + lane;
+        unsigned mine = __ballot_sync(0xffffffffu, b < B && cu_seqlens[b + 1] - cu_seqlens[b] >= from);
+        const int n = __popc(mine);
+        if (z < n) {
+            for (; z > 0; --z) mine &= mine - 1;
+            return first + __ffs(mine) - 1;
+        }
+        z -= n;
+    }
+    return -1;
+}
+
 // acc[8][8] += a[8] x b[8] for `STEPS` rows of two tiles in shared memory: row r of the first at A + r * lda, whose values
 // a0 .. a0 + 3 and a1 .. a1 + 3 are this thread's, and the same for B.
 template <int STEPS>

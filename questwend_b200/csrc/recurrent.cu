@@ -254,7 +254,7 @@ __global__ void __launch_bounds__(32 * QWB_SCAN_WARPS)
 ssm_scan_kernel(const float* __restrict__ xbc, int ldx, const float* __restrict__ dt_raw, int ld_dt,
                 const float* __restrict__ dt_bias, const float* __restrict__ A_log, const float* __restrict__ Dskip,
                 float* __restrict__ state, const int* __restrict__ cu_seqlens, const int* __restrict__ slots,
-                float* __restrict__ y, int H, int P, int N, int G, int write_state) {
+                float* __restrict__ y, int H, int P, int N, int G, int write_state, int below) {
     pdl_wait();
     pdl_launch_dependents();
     const int lane = threadIdx.x & 31;
@@ -262,6 +262,7 @@ ssm_scan_kernel(const float* __restrict__ xbc, int ldx, const float* __restrict_
     if (p0 >= P) return;                                            // P is a multiple of CW: a warp's columns all exist
     const int g = h / (H / G);
     const int t0 = cu_seqlens[b], t1 = cu_seqlens[b + 1];
+    if (below > 0 && t1 - t0 >= below) return;                      // the chunked form's
     const int n0 = lane * PER;
     float* S = state + (((size_t)slots[b] * H + h) * P + p0) * N;
     float s[CW][PER];
@@ -368,9 +369,10 @@ static int scan_rows_per_lane(int rows) {      // 1, 2, 4, 8 or 16 rows of a col
 }
 static bool aligned16(const void* p) { return (uintptr_t)p % 16 == 0; }
 
+// below: sequences that bring this many tokens or more are left alone (0: none)
 extern "C" int qwb_ssm_scan(const float* xbc, int ldx, const float* dt_raw, int ld_dt, const float* dt_bias, const float* A_log,
                             const float* Dskip, float* state, const int* cu_seqlens, const int* slots, float* y, int B,
-                            int H, int P, int N, int G, int write_state, cudaStream_t stream) {
+                            int H, int P, int N, int G, int write_state, int below, cudaStream_t stream) {
     if (B <= 0) return 0;
     if (H <= 0 || P <= 0 || N <= 0 || G <= 0 || H % G) return qwb_fail(QWB_ERR_ARG, "ssm_scan: %d heads, %d groups, state %d x %d", H, G, N, P);
     const int per = scan_rows_per_lane(N);
@@ -381,7 +383,7 @@ extern "C" int qwb_ssm_scan(const float* xbc, int ldx, const float* dt_raw, int 
     int cw = per <= 4 && P % 4 == 0 ? 4 : (per <= 8 && P % 2 == 0 ? 2 : 1);
     if (cw > QWB_SSM_CW_MAX) cw = QWB_SSM_CW_MAX;
     const dim3 grid((P / cw + QWB_SCAN_WARPS - 1) / QWB_SCAN_WARPS, H, B);
-#define QWB_SSM1(PER, VEC, CW) qwb_launch(ssm_scan_kernel<PER, VEC, (PER <= 4 ? 4 : (PER == 8 ? 2 : 1)), CW>, grid, 32 * QWB_SCAN_WARPS, 0, stream, xbc, ldx, dt_raw, ld_dt, dt_bias, A_log, Dskip, state, cu_seqlens, slots, y, H, P, N, G, write_state)
+#define QWB_SSM1(PER, VEC, CW) qwb_launch(ssm_scan_kernel<PER, VEC, (PER <= 4 ? 4 : (PER == 8 ? 2 : 1)), CW>, grid, 32 * QWB_SCAN_WARPS, 0, stream, xbc, ldx, dt_raw, ld_dt, dt_bias, A_log, Dskip, state, cu_seqlens, slots, y, H, P, N, G, write_state, below)
 #define QWB_SSM(PER, VEC) do { if (cw == 4 && PER <= 4) QWB_SSM1(PER, VEC, (PER <= 4 ? 4 : 1)); else if (cw >= 2 && PER <= 8) QWB_SSM1(PER, VEC, (PER <= 8 ? 2 : 1)); else QWB_SSM1(PER, VEC, 1); } while (0)
     if (per == 1) QWB_SSM(1, false); else if (per == 2) QWB_SSM(2, false);
     else if (per == 4) { if (vec) QWB_SSM(4, true); else QWB_SSM(4, false); }
@@ -402,7 +404,8 @@ extern "C" int qwb_ssm_scan(const float* xbc, int ldx, const float* dt_raw, int 
 // ---------------------------------------------------------------------------------
 __global__ void delta_prep_kernel(float* qkv, int ld, float* __restrict__ kq, const float* __restrict__ b_raw, int ld_b, float* __restrict__ beta,
                                   const float* __restrict__ a_raw, int ld_a, const float* __restrict__ dt_bias, const float* __restrict__ A_log,
-                                  float* __restrict__ decay, int H, int Hk, int K, int decay_k, float unit_eps, float q_scale) {
+                                  float* __restrict__ decay, const int* __restrict__ tok_seq, const int* __restrict__ cu_seqlens, int below, int H, int Hk, int K,
+                                  int decay_k, float unit_eps, float q_scale) {
     pdl_wait();
     pdl_launch_dependents();
     const int t = blockIdx.x;
@@ -426,17 +429,23 @@ __global__ void delta_prep_kernel(float* qkv, int ld, float* __restrict__ kq, co
     }
     for (int i = threadIdx.x; i < H; i += blockDim.x) beta[(size_t)t * H + i] = sigmoid_f(b_raw[(size_t)t * ld_b + i]);
     if (!decay) return;                                             // the chunked form makes its own from the raw ones
+    if (below > 0) {
+        const int b = tok_seq[t];
+        if (cu_seqlens[b + 1] - cu_seqlens[b] >= below) return;
+    }
     for (int i = threadIdx.x; i < H * decay_k; i += blockDim.x)
         decay[(size_t)t * H * decay_k + i] = expf(-expf(A_log[i / decay_k]) * softplus_f(a_raw[(size_t)t * ld_a + i] + dt_bias[i]));
 }
 
+// decay null: none are made; below: those of sequences that bring this many tokens or more are not (0: all are; tok_seq and cu_seqlens
+// are read only with it)
 extern "C" int qwb_delta_prep(float* qkv, int ld, float* kq, const float* b_raw, int ld_b, float* beta, const float* a_raw, int ld_a,
-                              const float* dt_bias, const float* A_log, float* decay, int T, int H, int Hk, int K, int decay_k,
+                              const float* dt_bias, const float* A_log, float* decay, const int* tok_seq, const int* cu_seqlens, int below, int T, int H, int Hk, int K, int decay_k,
                               float unit_eps, float q_scale, cudaStream_t stream) {
     if (T <= 0) return 0;
     if (H <= 0 || Hk <= 0 || K <= 0 || H % Hk) return qwb_fail(QWB_ERR_ARG, "delta_prep: %d heads, %d key heads of %d", H, Hk, K);
     if ((decay_k != K && decay_k != 1) || ld_a < H * decay_k) return qwb_fail(QWB_ERR_ARG, "delta_prep: %d decays a head (1 or %d) in rows of %d", decay_k, K, ld_a);
-    qwb_launch(delta_prep_kernel, T, 128, 0, stream, qkv, ld, kq, b_raw, ld_b, beta, a_raw, ld_a, dt_bias, A_log, decay, H, Hk, K, decay_k, unit_eps, q_scale);
+    qwb_launch(delta_prep_kernel, T, 128, 0, stream, qkv, ld, kq, b_raw, ld_b, beta, a_raw, ld_a, dt_bias, A_log, decay, tok_seq, cu_seqlens, below, H, Hk, K, decay_k, unit_eps, q_scale);
     return qwb_check_launch("delta_prep");
 }
 
@@ -531,7 +540,7 @@ __global__ void __launch_bounds__(32 * QWB_SCAN_WARPS)
 delta_scan_kernel(const float* __restrict__ qkv, int ld, const float* __restrict__ kq, const float* __restrict__ beta,
                   const float* __restrict__ decay, float* __restrict__ state, const int* __restrict__ cu_seqlens,
                   const int* __restrict__ slots, float* __restrict__ o, int H, int Hk, int K, int P, int write_state,
-                  int decay_ts, int decay_k) {
+                  int decay_ts, int decay_k, int below) {
     pdl_wait();
     pdl_launch_dependents();
     const int lane = threadIdx.x & 31;
@@ -539,6 +548,7 @@ delta_scan_kernel(const float* __restrict__ qkv, int ld, const float* __restrict
     if (p0 >= P) return;                                            // P is a multiple of CW: a warp's columns all exist
     const int kh = h / (H / Hk);
     const int t0 = cu_seqlens[b], t1 = cu_seqlens[b + 1];
+    if (below > 0 && t1 - t0 >= below) return;                      // the chunked form's
     const int n0 = lane * PER;
     float* S = state + (((size_t)slots[b] * H + h) * P + p0) * K;
     float s[CW][PER];
@@ -623,9 +633,10 @@ delta_scan_kernel(const float* __restrict__ qkv, int ld, const float* __restrict
     }
 }
 
+// below: sequences that bring this many tokens or more are left alone (0: none)
 extern "C" int qwb_delta_scan(const float* qkv, int ld, const float* kq, const float* beta, const float* decay, float* state,
                               const int* cu_seqlens, const int* slots, float* o, int B, int H, int Hk, int K, int P,
-                              int write_state, int decay_ts, int decay_k, cudaStream_t stream) {
+                              int write_state, int decay_ts, int decay_k, int below, cudaStream_t stream) {
     if (B <= 0) return 0;
     if (H <= 0 || Hk <= 0 || K <= 0 || P <= 0 || H % Hk) return qwb_fail(QWB_ERR_ARG, "delta_scan: %d heads, %d key heads, state %d x %d", H, Hk, K, P);
     if ((decay_k != K && decay_k != 1) || decay_ts < 0 || (decay_ts != 0 && decay_ts < H * decay_k))
@@ -639,7 +650,7 @@ extern "C" int qwb_delta_scan(const float* qkv, int ld, const float* kq, const f
     if (cw > QWB_DELTA_CW_MAX) cw = QWB_DELTA_CW_MAX;
     const dim3 grid((P / cw + QWB_SCAN_WARPS - 1) / QWB_SCAN_WARPS, H, B);
     const bool pc = decay_k > 1 || K == 1;
-#define QWB_DELTA0(PER, VEC, CW, PC) qwb_launch(delta_scan_kernel<PER, VEC, (PER <= 4 ? 4 : (PER == 8 ? 2 : 1)), CW, PC>, grid, 32 * QWB_SCAN_WARPS, 0, stream, qkv, ld, kq, beta, decay, state, cu_seqlens, slots, o, H, Hk, K, P, write_state, decay_ts, decay_k)
+#define QWB_DELTA0(PER, VEC, CW, PC) qwb_launch(delta_scan_kernel<PER, VEC, (PER <= 4 ? 4 : (PER == 8 ? 2 : 1)), CW, PC>, grid, 32 * QWB_SCAN_WARPS, 0, stream, qkv, ld, kq, beta, decay, state, cu_seqlens, slots, o, H, Hk, K, P, write_state, decay_ts, decay_k, below)
 #define QWB_DELTA1(PER, VEC, CW) do { if (pc) QWB_DELTA0(PER, VEC, CW, true); else QWB_DELTA0(PER, VEC, CW, false); } while (0)
 #define QWB_DELTA(PER, VEC) do { if (cw == 4 && PER <= 4) QWB_DELTA1(PER, VEC, (PER <= 4 ? 4 : 1)); else if (cw >= 2 && PER <= 8) QWB_DELTA1(PER, VEC, (PER <= 8 ? 2 : 1)); else QWB_DELTA1(PER, VEC, 1); } while (0)
     if (per == 1) QWB_DELTA(1, false); else if (per == 2) QWB_DELTA(2, false);

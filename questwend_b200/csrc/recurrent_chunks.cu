@@ -16,7 +16,8 @@
 // by cp.async in three stages: while one is multiplied, the next one's rows are weighted in place and the one after is on its
 // way, with one barrier a tile.  Scratch memory holds states and C row by row as the tiles want them (a state's row is a key
 // row here), so that nothing is transposed on the way to a tile.
-// Chunk c of sequence b is place cu_seqlens[b] / 128 + b + c of the scratch memory, which T / 128 + B places hold:
+// A step's sequences of at least `from` tokens go through these kernels, the others through the scan.  Chunk c of the z-th of them,
+// b, is place cu_seqlens[b] / 128 + z + c of the scratch memory, which T / 128 and one for each of them hold:
 //     own / starts [places, H, N, P], total decays [places, H], products [places, G, 128 (j), 128 (i)], C [places, G, N, 128 (i)]
 // The sums of logarithms are 64-bit (only their differences are used).  64 heads of 64 x 128 in 8 groups, with
 // the convolution before it, the scan and now: 2,048 tokens 902 -> 222 us (85 + 14 + 113 us in ncu; the FMA pipe at 44 and 50 %,
@@ -31,7 +32,7 @@ struct ScArgs {
     const float *xbc, *dt_raw, *dt_bias, *A_log, *D;
     const int *cu_seqlens, *slots;
     float *state, *y, *own, *totals, *products, *c_rows;
-    int ldx, ld_dt, H, P, N, G, write_state;
+    int ldx, ld_dt, H, P, N, G, write_state, B, from;
 };
 
 // this head's step sizes [128], sums of log decays [128] and, if wanted, decays [128] (beyond the chunk's n tokens: 0, the last
@@ -71,10 +72,11 @@ ssm_chunk_state_kernel(const ScArgs a, int ptiles, int ntiles) {
     __shared__ __align__(16) float tiles[3][SC_ROWS][SC_LDA + SC_LDB];
     __shared__ float dt[SC_TOKENS], coef[SC_TOKENS];
     __shared__ double G[SC_TOKENS];
-    const int c = blockIdx.x, b = blockIdx.z, tid = threadIdx.x;
+    const int c = blockIdx.x, b = rc_sequence(a.cu_seqlens, a.B, a.from, blockIdx.z), tid = threadIdx.x;
+    if (b < 0) return;
     const int t0 = a.cu_seqlens[b] + c * SC_TOKENS, n = min(SC_TOKENS, a.cu_seqlens[b + 1] - t0);
     if (n <= 0) return;
-    const size_t place = (size_t)(a.cu_seqlens[b] / SC_TOKENS + b + c);
+    const size_t place = (size_t)(a.cu_seqlens[b] / SC_TOKENS + blockIdx.z + c);
     const int inner = a.H * a.P;
     float acc[8][8];
 #pragma unroll
@@ -200,7 +202,9 @@ ssm_chunk_carry_kernel(const ScArgs a, int ptiles) {
     pdl_launch_dependents();
     constexpr int AHEAD = 8;
     __shared__ float turn[32][33];
-    const int h = blockIdx.y, b = blockIdx.z, t0 = a.cu_seqlens[b], n = a.cu_seqlens[b + 1] - t0;
+    const int h = blockIdx.y, b = rc_sequence(a.cu_seqlens, a.B, a.from, blockIdx.z);
+    if (b < 0) return;
+    const int t0 = a.cu_seqlens[b], n = a.cu_seqlens[b + 1] - t0;
     if (n <= 0) return;
     const int n0 = blockIdx.x / ptiles * 32, p0 = blockIdx.x % ptiles * 32, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const size_t size = (size_t)a.P * a.N;
@@ -215,7 +219,7 @@ ssm_chunk_carry_kernel(const ScArgs a, int ptiles) {
     float4 s = make_float4(turn[p][row], turn[p + 1][row], turn[p + 2][row], turn[p + 3][row]);
     if (n0 + row < a.N && p0 + p < a.P) {
         const int chunks = (n + SC_TOKENS - 1) / SC_TOKENS;
-        const size_t place = (size_t)(t0 / SC_TOKENS + b), step = (size_t)a.H * size;
+        const size_t place = (size_t)(t0 / SC_TOKENS + blockIdx.z), step = (size_t)a.H * size;
         float* at = a.own + (place * a.H + h) * size + (size_t)(n0 + row) * a.P + p0 + p;
         const float* total = a.totals + place * a.H + h;
         for (int c0 = 0; c0 < chunks; c0 += AHEAD) {
@@ -251,11 +255,12 @@ ssm_chunk_out_kernel(const ScArgs a, int ptiles) {
     __shared__ __align__(16) float tiles[3][SC_ROWS][SC_LDA + SC_LDB];
     __shared__ float dt[SC_TOKENS], decay[SC_TOKENS];
     __shared__ double G[SC_TOKENS];
-    const int c = blockIdx.x, b = blockIdx.z, tid = threadIdx.x;
+    const int c = blockIdx.x, b = rc_sequence(a.cu_seqlens, a.B, a.from, blockIdx.z), tid = threadIdx.x;
     const int h = blockIdx.y / ptiles, p0 = (blockIdx.y - h * ptiles) * 64;
+    if (b < 0) return;
     const int t0 = a.cu_seqlens[b] + c * SC_TOKENS, n = min(SC_TOKENS, a.cu_seqlens[b + 1] - t0);
     if (n <= 0) return;
-    const size_t place = (size_t)(a.cu_seqlens[b] / SC_TOKENS + b + c);
+    const size_t place = (size_t)(a.cu_seqlens[b] / SC_TOKENS + blockIdx.z + c);
     const int inner = a.H * a.P, g = h / (a.H / a.G);
     const float* X = a.xbc + (size_t)t0 * a.ldx + h * a.P + p0;
     const float* Cg = a.c_rows + (place * a.G + g) * (size_t)a.N * SC_TOKENS;
@@ -350,35 +355,37 @@ ssm_chunk_out_kernel(const ScArgs a, int ptiles) {
     }
 }
 
-// Floats of scratch that qwb_ssm_chunked needs; 0: these sizes are not taken.
-extern "C" long long qwb_ssm_chunked_scratch(int T, int B, int H, int P, int N, int G) {
-    if (T <= 0 || B <= 0 || H <= 0 || P <= 0 || N <= 0 || G <= 0 || H % G || P % 4 || N % 4) return 0;
-    return ((long long)T / SC_TOKENS + B) * ((long long)H * P * N + H + (long long)G * SC_TOKENS * (SC_TOKENS + N)) + 4;
+// Floats of scratch that qwb_ssm_chunked needs; 0: these sizes are not taken (more than a grid holds, or states that the scan refuses).
+#define SC_MAX_N 512
+extern "C" long long qwb_ssm_chunked_scratch(int T, int B, int from, int H, int P, int N, int G) {
+    if (T <= 0 || B <= 0 || H <= 0 || P <= 0 || N <= 0 || G <= 0 || H % G || P % 4 || N % 4 || N > SC_MAX_N) return 0;
+    if (B > 65535 || (long long)H * ((P + 63) / 64) * ((N + 127) / 128) + 3LL * G > 65535) return 0;
+    return ((long long)T / SC_TOKENS + rc_planes(T, B, from)) * ((long long)H * P * N + H + (long long)G * SC_TOKENS * (SC_TOKENS + N)) + 4;
 }
 
-// The same step as qwb_ssm_scan, for 16-byte aligned tensors with rows of a multiple of 4 floats.
+// The same step as qwb_ssm_scan for the sequences that bring at least `from` tokens (0: all), for 16-byte aligned tensors with rows of a
+// multiple of 4 floats.
 extern "C" int qwb_ssm_chunked(const float* xbc, int ldx, const float* dt_raw, int ld_dt, const float* dt_bias, const float* A_log, const float* D,
-                               float* state, const int* cu_seqlens, const int* slots, float* y, float* scratch, int T, int B, int max_new, int H, int P,
+                               float* state, const int* cu_seqlens, const int* slots, float* y, float* scratch, int T, int B, int max_new, int from, int H, int P,
                                int N, int G, int write_state, cudaStream_t stream) {
-    if (T <= 0 || B <= 0 || max_new <= 0) return 0;
-    if (!qwb_ssm_chunked_scratch(T, B, H, P, N, G) || ldx % 4 || ldx < H * P + 2 * G * N || ld_dt < H)
+    if (T <= 0 || B <= 0 || max_new <= 0 || max_new < from) return 0;
+    if (!qwb_ssm_chunked_scratch(T, B, from, H, P, N, G) || ldx % 4 || ldx < H * P + 2 * G * N || ld_dt < H)
         return qwb_fail(QWB_ERR_ARG, "ssm_chunked: %d heads, %d groups, state %d x %d in rows of %d", H, G, N, P, ldx);
     for (const void* p : {(const void*)xbc, (const void*)state, (const void*)y, (const void*)scratch})
         if (!p || !rc_aligned16(p)) return qwb_fail(QWB_ERR_ARG, "ssm_chunked: a tensor is not 16-byte aligned");
-    const int chunks = (max_new + SC_TOKENS - 1) / SC_TOKENS, ptiles = (P + 63) / 64, ntiles = (N + 127) / 128;
-    if (B > 65535 || (long long)H * ptiles * ntiles + 3 * G > 65535) return qwb_fail(QWB_ERR_ARG, "ssm_chunked: %d sequences or %d heads of %d x %d are too many", B, H, N, P);
-    const size_t places = (size_t)T / SC_TOKENS + B;
-    ScArgs a = {xbc, dt_raw, dt_bias, A_log, D, cu_seqlens, slots, state, y, nullptr, nullptr, nullptr, nullptr, ldx, ld_dt, H, P, N, G, write_state};
+    const int chunks = (max_new + SC_TOKENS - 1) / SC_TOKENS, ptiles = (P + 63) / 64, ntiles = (N + 127) / 128, planes = rc_planes(T, B, from);
+    const size_t places = (size_t)T / SC_TOKENS + planes;
+    ScArgs a = {xbc, dt_raw, dt_bias, A_log, D, cu_seqlens, slots, state, y, nullptr, nullptr, nullptr, nullptr, ldx, ld_dt, H, P, N, G, write_state, B, from};
     a.own = scratch;
     a.products = a.own + places * H * P * N;
     a.c_rows = a.products + places * G * SC_TOKENS * SC_TOKENS;
     a.totals = a.c_rows + places * G * N * SC_TOKENS;
-    qwb_launch(ssm_chunk_state_kernel, dim3(chunks, H * ptiles * ntiles + 3 * G, B), 128, 0, stream, a, ptiles, ntiles);
+    qwb_launch(ssm_chunk_state_kernel, dim3(chunks, H * ptiles * ntiles + 3 * G, planes), 128, 0, stream, a, ptiles, ntiles);
     if (int rc = qwb_check_launch("ssm_chunk_state")) return rc;
     const int carry_p = (P + 31) / 32;
-    qwb_launch(ssm_chunk_carry_kernel, dim3((N + 31) / 32 * carry_p, H, B), 256, 0, stream, a, carry_p);
+    qwb_launch(ssm_chunk_carry_kernel, dim3((N + 31) / 32 * carry_p, H, planes), 256, 0, stream, a, carry_p);
     if (int rc = qwb_check_launch("ssm_chunk_carry")) return rc;
-    qwb_launch(ssm_chunk_out_kernel, dim3(chunks, H * ptiles, B), 128, 0, stream, a, ptiles);
+    qwb_launch(ssm_chunk_out_kernel, dim3(chunks, H * ptiles, planes), 128, 0, stream, a, ptiles);
     return qwb_check_launch("ssm_chunk_out");
 }
 
@@ -397,7 +404,7 @@ extern "C" int qwb_ssm_chunked(const float* xbc, int ldx, const float* dt_raw, i
 // sub-blocks of 16: inside one, every pair and channel has an exponential of its own; between two, what decays behind j up to
 // its sub-block's end, what decays in the sub-blocks between, and what decays from the start of i's sub-block to i are three
 // factors of at most 1.  Sums of logarithms (base 2) span what they decay and nothing else.
-// Chunk c of sequence b is place cu_seqlens[b] / 64 + b + c of the scratch memory, which T / 64 + B places hold.
+// Chunk c of the z-th sequence that these kernels take, b, is place cu_seqlens[b] / 64 + z + c of the scratch memory.
 // 16 heads of 128 x 128 with a decay per channel, the convolution before it, the scan and now: 2,048 tokens 955 -> 323 us (prep 121,
 // walk 131, out 49 in ncu), three sequences of 2,900 in all 1,194 -> 472 us; a decay per head, four of 4,096 in all, 1,198 -> 588 us.
 // Bound by what shared memory hands to registers (128 bytes a cycle), the walk more than the others.
@@ -413,14 +420,14 @@ struct DcArgs {
     const float *qkv, *beta, *a_raw, *dt_bias, *A_log;
     const int *cu_seqlens, *slots;
     float *state, *o, *scratch;
-    int ld, ld_a, H, Hk, K, P, decay_k, write_state;
+    int ld, ld_a, H, Hk, K, P, decay_k, write_state, B, from;
 };
 struct DcPlace { float *w, *k_end, *q0, *q_pairs, *u, *decay, *start; };
 __host__ __device__ __forceinline__ size_t dc_floats(int K, int P) {      // of one place and head: a multiple of 4
     return (size_t)3 * K * DC_TOKENS + DC_TOKENS * DC_TOKENS + (size_t)DC_TOKENS * P + K + (size_t)K * P;
 }
-__device__ __forceinline__ DcPlace dc_place(const DcArgs& a, int b, int c, int h) {
-    const size_t place = (size_t)(a.cu_seqlens[b] / DC_TOKENS + b + c);
+__device__ __forceinline__ DcPlace dc_place(const DcArgs& a, int b, int c, int h) {      // in plane blockIdx.z of the grid
+    const size_t place = (size_t)(a.cu_seqlens[b] / DC_TOKENS + blockIdx.z + c);
     DcPlace p;
     p.w = a.scratch + (place * a.H + h) * dc_floats(a.K, a.P);
     p.k_end = p.w + a.K * DC_TOKENS;
@@ -460,7 +467,8 @@ delta_chunk_prep_kernel(const DcArgs a) {
     float* As = gs + DC_TOKENS * DC_MAX_K;                             // beta_i A_ij
     float* totals = As + DC_A_FLOATS;                               // [4][128]
     float* beta = totals + 4 * DC_MAX_K;
-    const int c = blockIdx.x, h = blockIdx.y, b = blockIdx.z, tid = threadIdx.x, K = a.K, P = a.P;
+    const int c = blockIdx.x, h = blockIdx.y, b = rc_sequence(a.cu_seqlens, a.B, a.from, blockIdx.z), tid = threadIdx.x, K = a.K, P = a.P;
+    if (b < 0) return;
     const int t0 = a.cu_seqlens[b] + c * DC_TOKENS, n = min(DC_TOKENS, a.cu_seqlens[b + 1] - t0);
     if (n <= 0) return;
     const DcPlace at = dc_place(a, b, c, h);
@@ -696,7 +704,8 @@ delta_chunk_walk_kernel(const DcArgs a) {
     pdl_launch_dependents();
     extern __shared__ __align__(16) float dc_smem[];
     constexpr int LU = DC_WALK_P + 4;
-    const int h = blockIdx.y, b = blockIdx.z, tid = threadIdx.x, K = a.K, P = a.P, p0 = blockIdx.x * DC_WALK_P, ldw = K + 4;
+    const int h = blockIdx.y, b = rc_sequence(a.cu_seqlens, a.B, a.from, blockIdx.z), tid = threadIdx.x, K = a.K, P = a.P, p0 = blockIdx.x * DC_WALK_P, ldw = K + 4;
+    if (b < 0) return;
     float* Ws = dc_smem;
     float* Ke = Ws + ldw * DC_TOKENS;
     float* Ss = Ke + 2 * K * DC_TOKENS;                             // [16][ldw]
@@ -789,7 +798,9 @@ delta_chunk_out_kernel(const DcArgs a, int ptiles) {
     // a tile: 16 channels or tokens x 128 values, and q of 64 tokens x 16 channels or their pairs with 16 tokens, 16 x 64
     constexpr int ROWS = 16, LDV = 132, LDQ = ROWS + 4, LDP = 68;
     __shared__ __align__(16) float values[3][ROWS * LDV], lefts[3][DC_TOKENS * LDQ];
-    const int c = blockIdx.x, h = blockIdx.y / ptiles, p0 = (blockIdx.y - h * ptiles) * 128, b = blockIdx.z, tid = threadIdx.x, K = a.K, P = a.P;
+    const int c = blockIdx.x, h = blockIdx.y / ptiles, p0 = (blockIdx.y - h * ptiles) * 128, tid = threadIdx.x, K = a.K, P = a.P;
+    const int b = rc_sequence(a.cu_seqlens, a.B, a.from, blockIdx.z);
+    if (b < 0) return;
     const int t0 = a.cu_seqlens[b] + c * DC_TOKENS, n = min(DC_TOKENS, a.cu_seqlens[b + 1] - t0);
     if (n <= 0) return;
     const DcPlace at = dc_place(a, b, c, h);
@@ -869,33 +880,33 @@ delta_chunk_out_kernel(const DcArgs a, int ptiles) {
 }
 
 // Floats of scratch that qwb_delta_chunked needs; 0: these sizes are not taken.
-extern "C" long long qwb_delta_chunked_scratch(int T, int B, int H, int K, int P) {
+extern "C" long long qwb_delta_chunked_scratch(int T, int B, int from, int H, int K, int P) {
     if (T <= 0 || B <= 0 || H <= 0 || K <= 0 || P <= 0 || K % 4 || P % 4 || K > DC_MAX_K) return 0;
-    return ((long long)T / DC_TOKENS + B) * H * (long long)dc_floats(K, P);
+    if (B > 65535 || (long long)H * ((P + 127) / 128) > 65535) return 0;
+    return ((long long)T / DC_TOKENS + rc_planes(T, B, from)) * H * (long long)dc_floats(K, P);
 }
 
-// The same step as qwb_delta_prep and qwb_delta_scan with beta, after qwb_delta_prep made q and k unit vectors and beta; the raw
+// The same step as qwb_delta_prep and qwb_delta_scan with beta for the sequences that bring at least `from` tokens (0: all), after qwb_delta_prep made q and k unit vectors and beta; the raw
 // decays come as qwb_delta_prep takes them.  16-byte aligned tensors, rows of a multiple of 4 floats.
 extern "C" int qwb_delta_chunked(const float* qkv, int ld, const float* beta, const float* a_raw, int ld_a, const float* dt_bias, const float* A_log,
-                                 float* state, const int* cu_seqlens, const int* slots, float* o, float* scratch, int T, int B, int max_new, int H,
+                                 float* state, const int* cu_seqlens, const int* slots, float* o, float* scratch, int T, int B, int max_new, int from, int H,
                                  int Hk, int K, int P, int decay_k, int write_state, cudaStream_t stream) {
-    if (T <= 0 || B <= 0 || max_new <= 0) return 0;
-    if (!qwb_delta_chunked_scratch(T, B, H, K, P) || Hk <= 0 || H % Hk || ld % 4 || ld < 2 * Hk * K + H * P || (decay_k != K && decay_k != 1) || ld_a < H * decay_k)
+    if (T <= 0 || B <= 0 || max_new <= 0 || max_new < from) return 0;
+    if (!qwb_delta_chunked_scratch(T, B, from, H, K, P) || Hk <= 0 || H % Hk || ld % 4 || ld < 2 * Hk * K + H * P || (decay_k != K && decay_k != 1) || ld_a < H * decay_k)
         return qwb_fail(QWB_ERR_ARG, "delta_chunked: %d heads, %d key heads, state %d x %d in rows of %d, %d decays a head", H, Hk, K, P, ld, decay_k);
     for (const void* p : {(const void*)qkv, (const void*)state, (const void*)o, (const void*)scratch})
         if (!p || !rc_aligned16(p)) return qwb_fail(QWB_ERR_ARG, "delta_chunked: a tensor is not 16-byte aligned");
-    const int chunks = (max_new + DC_TOKENS - 1) / DC_TOKENS, ptiles = (P + 127) / 128;
-    if (B > 65535 || (long long)H * ptiles > 65535) return qwb_fail(QWB_ERR_ARG, "delta_chunked: %d sequences or %d heads are too many", B, H);
-    const DcArgs a = {qkv, beta, a_raw, dt_bias, A_log, cu_seqlens, slots, state, o, scratch, ld, ld_a, H, Hk, K, P, decay_k, write_state};
+    const int chunks = (max_new + DC_TOKENS - 1) / DC_TOKENS, ptiles = (P + 127) / 128, planes = rc_planes(T, B, from);
+    const DcArgs a = {qkv, beta, a_raw, dt_bias, A_log, cu_seqlens, slots, state, o, scratch, ld, ld_a, H, Hk, K, P, decay_k, write_state, B, from};
     const size_t smem1 = (3 * DC_TOKENS * DC_MAX_K + DC_A_FLOATS + 4 * DC_MAX_K + DC_TOKENS) * sizeof(float);
     const size_t smem2 = ((3 * K + 4) * DC_TOKENS + DC_WALK_P * (K + 4) + DC_TOKENS * (DC_WALK_P + 4)) * sizeof(float);
     cudaError_t e = cudaFuncSetAttribute(delta_chunk_prep_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem1);
     if (e == cudaSuccess) e = cudaFuncSetAttribute(delta_chunk_walk_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem2);
     if (e != cudaSuccess) return qwb_fail(QWB_ERR_CUDA, "delta_chunked: %s", cudaGetErrorString(e));
-    qwb_launch(delta_chunk_prep_kernel, dim3(chunks, H, B), 256, smem1, stream, a);
+    qwb_launch(delta_chunk_prep_kernel, dim3(chunks, H, planes), 256, smem1, stream, a);
     if (int rc = qwb_check_launch("delta_chunk_prep")) return rc;
-    qwb_launch(delta_chunk_walk_kernel, dim3((P + DC_WALK_P - 1) / DC_WALK_P, H, B), 256, smem2, stream, a);
+    qwb_launch(delta_chunk_walk_kernel, dim3((P + DC_WALK_P - 1) / DC_WALK_P, H, planes), 256, smem2, stream, a);
     if (int rc = qwb_check_launch("delta_chunk_walk")) return rc;
-    qwb_launch(delta_chunk_out_kernel, dim3(chunks, H * ptiles, B), 128, 0, stream, a, ptiles);
+    qwb_launch(delta_chunk_out_kernel, dim3(chunks, H * ptiles, planes), 128, 0, stream, a, ptiles);
     return qwb_check_launch("delta_chunk_out");
 }

@@ -889,18 +889,26 @@ def short_conv(x: torch.Tensor, col0: int, channels: int, weight: torch.Tensor, 
     return out
 
 
-# Tokens of a step's longest sequence from which the recurrence runs in chunks (csrc/recurrent_chunks.cu).  With its
-# convolution, 64 heads of 64 x 128, us, scan / chunks: 64 tokens 33 / 42, 100 tokens 48 / 48, three sequences of 67 80 / 64,
-# 400 tokens 179 / 74.
+# Tokens from which a sequence goes through the recurrence in chunks (csrc/recurrent_chunks.cu), by its own length, whatever else
+# the step brings.  With its convolution, 64 heads of 64 x 128, us, scan / chunks: 64 tokens 33 / 42, 100 tokens 48 / 48, 400 tokens 179 / 74.
+# Steps with both, all by the scan / each its own way: a prompt of 200 beside 63 single tokens 151 / 154, beside 255 444 / 462, one of
+# 2,048 beside 63 952 / 335 (all of them in chunks, a whole chunk each: 861, 3,388, 1,096).
 SSM_CHUNKED_FROM = 96
 CHUNK_SCRATCH_MAX = 1 << 30     # floats of scratch memory that a chunked form may take; a longer prompt runs as a scan
+
+
+def _forms(ctx, chunked_from: int) -> tuple[int, bool]:
+    """How a step whose longest sequence goes through chunks divides its sequences: (from how many tokens on the chunks take them, 0:
+    they take all, whether the scan takes the rest)."""
+    every = getattr(ctx, "min_new", 1) >= chunked_from or ctx.n_seqs == 1
+    return 0 if every else chunked_from, not every
 
 
 def ssm_scan(xbc: torch.Tensor, dt: torch.Tensor, dt_col0: int, dt_bias, a_log, d_skip, state: torch.Tensor, ctx,
              heads: int, vdim: int, n_state: int, groups: int, write_state: bool = True) -> torch.Tensor:
     """The Mamba-2 recurrence over a step's tokens.  ``xbc`` float32 [T, heads * vdim + 2 * groups * n_state] (x | B | C,
     after convolution and SiLU); the raw step sizes are columns ``dt_col0 ..`` of float32 ``dt`` [T, ld]; ``state``
-    float32 [slots, heads, vdim, n_state] (column by column) is read and written back.  Steps with a sequence of at least
+    float32 [slots, heads, vdim, n_state] (column by column) is read and written back.  Sequences of at least
     ``SSM_CHUNKED_FROM`` tokens run in chunks of 128.  Returns y float32 [T, heads * vdim]."""
     _need(xbc, "xbc", torch.float32, 2)
     _need(dt, "dt", torch.float32, 2)
@@ -914,26 +922,31 @@ def ssm_scan(xbc: torch.Tensor, dt: torch.Tensor, dt_col0: int, dt_bias, a_log, 
         if t.numel() != heads:
             raise KernelError(f"ssm_scan: {name} has {t.numel()} entries for {heads} heads")
     y = torch.empty((T, heads * vdim), dtype=torch.float32, device=xbc.device)
+    below = 0
     if ctx.max_new >= SSM_CHUNKED_FROM and xbc.shape[1] % 4 == 0 and not (xbc.data_ptr() % 16 or state.data_ptr() % 16):
         lib, size = _lookup("recurrent_chunks", "qwb_ssm_chunked_scratch")
         size.restype = ctypes.c_longlong
-        floats = size(_i(T), _i(ctx.n_seqs), _i(heads), _i(vdim), _i(n_state), _i(groups))
+        chunks_from, rest = _forms(ctx, SSM_CHUNKED_FROM)
+        floats = size(_i(T), _i(ctx.n_seqs), _i(chunks_from), _i(heads), _i(vdim), _i(n_state), _i(groups))
         if 0 < floats <= CHUNK_SCRATCH_MAX:
             scratch = torch.empty((floats,), dtype=torch.float32, device=xbc.device)
             _call("recurrent_chunks", "qwb_ssm_chunked", _ptr(xbc), _i(xbc.shape[1]), ctypes.c_void_p(dt.data_ptr() + 4 * dt_col0),
                   _i(dt.shape[1]), _ptr(dt_bias), _ptr(a_log), _ptr(d_skip), _ptr(state), _ptr(ctx.cu_seqlens), _ptr(ctx.slots), _ptr(y),
-                  _ptr(scratch), _i(T), _i(ctx.n_seqs), _i(ctx.max_new), _i(heads), _i(vdim), _i(n_state), _i(groups),
+                  _ptr(scratch), _i(T), _i(ctx.n_seqs), _i(ctx.max_new), _i(chunks_from), _i(heads), _i(vdim), _i(n_state), _i(groups),
                   _i(1 if write_state else 0), _stream(), kernels=3)
-            return y
+            if not rest:
+                return y
+            below = chunks_from
     _call("recurrent", "qwb_ssm_scan", _ptr(xbc), _i(xbc.shape[1]), ctypes.c_void_p(dt.data_ptr() + 4 * dt_col0),
           _i(dt.shape[1]), _ptr(dt_bias), _ptr(a_log), _ptr(d_skip), _ptr(state), _ptr(ctx.cu_seqlens), _ptr(ctx.slots),
-          _ptr(y), _i(ctx.n_seqs), _i(heads), _i(vdim), _i(n_state), _i(groups), _i(1 if write_state else 0), _stream())
+          _ptr(y), _i(ctx.n_seqs), _i(heads), _i(vdim), _i(n_state), _i(groups), _i(1 if write_state else 0), _i(below), _stream())
     return y
 
 
-# Tokens of a step's longest sequence from which the delta rule runs in chunks (csrc/recurrent_chunks.cu).  With its
-# convolution, 16 heads of 128 x 128, us, scan / chunks: 64 tokens 44 / 68, 100 tokens (a decay per head) 43 / 68, three sequences
-# of 67 94 / 84, 400 tokens 194 / 94.
+# Tokens from which a sequence goes through the delta rule in chunks (csrc/recurrent_chunks.cu), by its own length.  With its
+# convolution, 16 heads of 128 x 128, us, scan / chunks: 64 tokens 44 / 68, 100 tokens (a decay per head) 43 / 68, 400 tokens 194 / 94.
+# Steps with both, all by the scan / each its own way: 200 beside 63 single tokens 143 / 173 (two kinds of launches one after the other),
+# 2,048 beside 63 1,051 / 395, two of 150 and 160 135 / 89 (all of them in chunks: 609, 864, 83).
 DELTA_CHUNKED_FROM = 144
 
 
@@ -945,7 +958,7 @@ def delta_rule(qkv: torch.Tensor, b_raw: torch.Tensor, b_col0: int, a_raw: torch
     in place, q times ``q_scale``); columns ``b_col0 .. b_col0 + heads`` of ``b_raw`` [T, ld] and ``a_raw``
     [T, heads * key_dim] are the raw write strengths and decays; ``state`` float32 [slots, heads, vdim, key_dim] (column by column).  Returns o float32 [T, heads * vdim].
     ``per_head``: one decay per head instead: the raw decays are columns ``a_col0 .. a_col0 + heads`` of ``a_raw`` [T, ld],
-    ``dt_bias`` has ``heads`` entries.  Steps with a sequence of at least ``DELTA_CHUNKED_FROM`` tokens run in chunks of 64 (keys
+    ``dt_bias`` has ``heads`` entries.  Sequences of at least ``DELTA_CHUNKED_FROM`` tokens run in chunks of 64 (keys
     of up to 128, sizes in multiples of 4)."""
     _need(qkv, "qkv", torch.float32, 2)
     _need(b_raw, "b_raw", torch.float32, 2)
@@ -965,26 +978,30 @@ def delta_rule(qkv: torch.Tensor, b_raw: torch.Tensor, b_col0: int, a_raw: torch
     kq = torch.empty((T, key_heads), dtype=torch.float32, device=dev)
     beta = torch.empty((T, heads), dtype=torch.float32, device=dev)
     raw_decays = (ctypes.c_void_p(a_raw.data_ptr() + 4 * a_col0), _i(a_raw.shape[1]), _ptr(dt_bias), _ptr(a_log))
-    floats = 0
+    floats, chunks_from, rest = 0, 0, True
     if ctx.max_new >= DELTA_CHUNKED_FROM and qkv.shape[1] % 4 == 0 and not (qkv.data_ptr() % 16 or state.data_ptr() % 16):
         size = _lookup("recurrent_chunks", "qwb_delta_chunked_scratch")[1]
         size.restype = ctypes.c_longlong
-        floats = size(_i(T), _i(ctx.n_seqs), _i(heads), _i(key_dim), _i(vdim))
+        chunks_from, rest = _forms(ctx, DELTA_CHUNKED_FROM)
+        floats = size(_i(T), _i(ctx.n_seqs), _i(chunks_from), _i(heads), _i(key_dim), _i(vdim))
     chunked = 0 < floats <= CHUNK_SCRATCH_MAX
-    decay = None if chunked else torch.empty((T, heads * decay_k), dtype=torch.float32, device=dev)
+    if not chunked:
+        chunks_from, rest = 0, True
+    decay = None if not rest else torch.empty((T, heads * decay_k), dtype=torch.float32, device=dev)
     _call("recurrent", "qwb_delta_prep", _ptr(qkv), _i(qkv.shape[1]), _ptr(kq), ctypes.c_void_p(b_raw.data_ptr() + 4 * b_col0),
-          _i(b_raw.shape[1]), _ptr(beta), *raw_decays, _ptr(decay), _i(T), _i(heads), _i(key_heads), _i(key_dim), _i(decay_k), _f(unit_eps),
-          _f(q_scale), _stream())
+          _i(b_raw.shape[1]), _ptr(beta), *raw_decays, _ptr(decay), _ptr(ctx.tok_seq) if chunks_from else _ptr(None), _ptr(ctx.cu_seqlens),
+          _i(chunks_from), _i(T), _i(heads), _i(key_heads), _i(key_dim), _i(decay_k), _f(unit_eps), _f(q_scale), _stream())
     o = torch.empty((T, heads * vdim), dtype=torch.float32, device=dev)
     if chunked:
         scratch = torch.empty((floats,), dtype=torch.float32, device=dev)
         _call("recurrent_chunks", "qwb_delta_chunked", _ptr(qkv), _i(qkv.shape[1]), _ptr(beta), *raw_decays, _ptr(state), _ptr(ctx.cu_seqlens),
-              _ptr(ctx.slots), _ptr(o), _ptr(scratch), _i(T), _i(ctx.n_seqs), _i(ctx.max_new), _i(heads), _i(key_heads), _i(key_dim), _i(vdim),
-              _i(decay_k), _i(1 if write_state else 0), _stream(), kernels=3)
-        return o
+              _ptr(ctx.slots), _ptr(o), _ptr(scratch), _i(T), _i(ctx.n_seqs), _i(ctx.max_new), _i(chunks_from), _i(heads), _i(key_heads),
+              _i(key_dim), _i(vdim), _i(decay_k), _i(1 if write_state else 0), _stream(), kernels=3)
+        if not rest:
+            return o
     _call("recurrent", "qwb_delta_scan", _ptr(qkv), _i(qkv.shape[1]), _ptr(kq), _ptr(beta), _ptr(decay), _ptr(state),
           _ptr(ctx.cu_seqlens), _ptr(ctx.slots), _ptr(o), _i(ctx.n_seqs), _i(heads), _i(key_heads), _i(key_dim), _i(vdim),
-          _i(1 if write_state else 0), _i(heads * decay_k), _i(decay_k), _stream())
+          _i(1 if write_state else 0), _i(heads * decay_k), _i(decay_k), _i(chunks_from), _stream())
     return o
 
 
@@ -1040,7 +1057,7 @@ def retention_scan(qkv: torch.Tensor, cos, sin, rotary_dim: int, decay: torch.Te
         return o
     _call("recurrent", "qwb_delta_scan", _ptr(qkv), _i(qkv.shape[1]), _ptr(kq), _ptr(None), _ptr(decay), _ptr(state),
           _ptr(ctx.cu_seqlens), _ptr(ctx.slots), _ptr(o), _i(ctx.n_seqs), _i(heads), _i(heads), _i(key_dim), _i(vdim),
-          _i(1 if write_state else 0), _i(0), _i(1), _stream())
+          _i(1 if write_state else 0), _i(0), _i(1), _i(0), _stream())
     return o
 
 
@@ -1072,7 +1089,7 @@ def gla_scan(qkv: torch.Tensor, a_raw: torch.Tensor, a_bias: torch.Tensor | None
     o = torch.empty((T, heads * vdim), dtype=torch.float32, device=dev)
     _call("recurrent", "qwb_delta_scan", _ptr(qkv), _i(qkv.shape[1]), _ptr(kq), _ptr(None), _ptr(decay), _ptr(state),
           _ptr(ctx.cu_seqlens), _ptr(ctx.slots), _ptr(o), _i(ctx.n_seqs), _i(heads), _i(heads), _i(key_dim), _i(vdim),
-          _i(1 if write_state else 0), _i(heads * key_dim), _i(key_dim), _stream())
+          _i(1 if write_state else 0), _i(heads * key_dim), _i(key_dim), _i(0), _stream())
     return o
 
 

@@ -246,11 +246,12 @@ def sums_close(got, ref, terms=2 ** -15):
 
 @pytest.mark.parametrize("H, P, N, G", [(2, 64, 128, 1), (4, 4, 4, 2), (3, 68, 132, 3), (8, 32, 64, 2), (2, 128, 256, 1)])
 @pytest.mark.parametrize("pace", [0.01, 1.0, 40.0])
-def test_mamba2_in_chunks(H, P, N, G, pace):
+def test_mamba2_in_chunks(H, P, N, G, pace, monkeypatch):
     """Sequences at the edges of the chunks of 128, from a state, with slow, usual and immediate decays; the scan, which takes
     shorter steps, gives the same; slots of others stay as they are."""
     torch.manual_seed(H + P + N)
-    lens, slots = [1, 64, 127, 128, 129, 300], [4, 2, 7, 1, 5, 3]       # the longest one sends the step into chunks
+    monkeypatch.setattr(ops, "SSM_CHUNKED_FROM", 2)        # all but the shortest
+    lens, slots = [1, 64, 127, 128, 129, 300], [4, 2, 7, 1, 5, 3]
     T, inner = sum(lens), H * P
     step = Steps(lens, slots)
     xbc, dt = torch.randn(T, inner + 2 * G * N, device=DEV), torch.randn(T, H + 5, device=DEV)
@@ -381,10 +382,11 @@ def test_convolutions_of_four_channels_a_thread(taps, C, mode):
 
 @pytest.mark.parametrize("H, Hk, K, P, per_head", [(2, 2, 128, 128, False), (4, 1, 128, 128, True), (2, 1, 4, 4, False), (3, 3, 36, 20, False), (2, 2, 100, 260, True)])
 @pytest.mark.parametrize("pace", [0.01, 1.0, 60.0])
-def test_delta_rule_in_chunks(H, Hk, K, P, per_head, pace):
+def test_delta_rule_in_chunks(H, Hk, K, P, per_head, pace, monkeypatch):
     """Sequences at the edges of the chunks of 64 and their sub-blocks of 16, from a state, with slow, usual and immediate
     decays; the scan gives the same; slots of others stay as they are."""
     torch.manual_seed(H + K + P)
+    monkeypatch.setattr(ops, "DELTA_CHUNKED_FROM", 2)      # all but the shortest
     lens, slots = [1, 15, 16, 17, 63, 64, 65, 200], [4, 2, 7, 1, 5, 3, 8, 9]
     T, n_decay = sum(lens), H if per_head else H * K
     step = Steps(lens, slots)
@@ -456,6 +458,38 @@ def test_delta_rule_in_chunks_with_tokens_that_forget(per_head, rate, forget):
         errors.append([float((got.double() - want).norm() / want.norm()) for got, want in ((o, ref), (state[1], S))])
     for chunks, scan in zip(*errors):
         assert chunks <= 2 * scan + 2.0 ** -23, errors
+
+
+@pytest.mark.parametrize("kind", ["mamba2", "delta", "delta_per_head"])
+@pytest.mark.parametrize("lens", [[200, 1, 1, 1], [1] * 40 + [96, 1, 144, 143, 95, 2, 500] + [1] * 30, [300, 96, 144, 600], [90, 1, 30]])
+def test_recurrences_do_not_look_at_the_rest_of_the_batch(kind, lens):
+    """Whether a sequence goes through the scan or through chunks follows from its own length: its outputs and its state are the same
+    bits alone and beside others, short and long."""
+    torch.manual_seed(len(lens))
+    H, P, K, G, T, B = 4, 64, 64, 2, sum(lens), len(lens)
+    inner, n_decay = H * P, H if kind == "delta_per_head" else H * K
+    xbc, side, a_raw = torch.randn(T, inner + 2 * G * K, device=DEV), torch.randn(T, H, device=DEV), torch.randn(T, n_decay, device=DEV) - 3.0
+    qkv, vec, bias = torch.randn(T, 2 * H * K + inner, device=DEV), torch.randn(H, device=DEV), torch.randn(n_decay, device=DEV)
+    start = 0.3 * torch.randn(B, H, P, K, device=DEV)
+
+    def run(picked, rows_, slots):
+        step, state = Steps(picked, slots), start.clone()
+        step.min_new = min(picked)
+        if kind == "mamba2":
+            out = ops.ssm_scan(xbc[rows_].contiguous(), side[rows_].contiguous(), 0, vec, vec, vec, state, step, H, P, K, G)
+        else:
+            out = ops.delta_rule(qkv[rows_].clone(), side[rows_].contiguous(), 0, a_raw[rows_].contiguous(), bias, vec, state, step, H, H, K, P, 1e-6, K ** -0.5,
+                                 per_head=kind == "delta_per_head")
+        return out, state
+
+    out, state = run(lens, slice(0, T), list(range(B)))
+    seen, at = set(), 0
+    for b, n in enumerate(lens):
+        if n not in seen:
+            alone, after = run([n], slice(at, at + n), [b])
+            assert torch.equal(out[at:at + n], alone) and torch.equal(state[b], after[b]), n
+        seen.add(n)
+        at += n
 
 
 # ----------------------------------------------------------------------------- score maps, single tokens
