@@ -894,7 +894,18 @@ def short_conv(x: torch.Tensor, col0: int, channels: int, weight: torch.Tensor, 
 # Steps with both, all by the scan / each its own way: a prompt of 200 beside 63 single tokens 151 / 154, beside 255 444 / 462, one of
 # 2,048 beside 63 952 / 335 (all of them in chunks, a whole chunk each: 861, 3,388, 1,096).
 SSM_CHUNKED_FROM = 96
-CHUNK_SCRATCH_MAX = 1 << 30     # floats of scratch memory that a chunked form may take; a longer prompt runs as a scan
+CHUNK_SCRATCH_MAX = 1 << 30     # floats of scratch memory that a chunked form may take; a longer prompt runs without
+
+
+def _chunk_scratch(floats: int, device) -> torch.Tensor | None:
+    """Scratch memory for a chunked form, or None where the form does not take the sizes (0 floats), would need too much, or the memory
+    is not there (a cache may have been given all of it): the step then takes the form that it took before there were chunks."""
+    if not 0 < floats <= CHUNK_SCRATCH_MAX:
+        return None
+    try:
+        return torch.empty((floats,), dtype=torch.float32, device=device)
+    except torch.OutOfMemoryError:
+        return None
 
 
 def _forms(ctx, chunked_from: int) -> tuple[int, bool]:
@@ -927,9 +938,8 @@ def ssm_scan(xbc: torch.Tensor, dt: torch.Tensor, dt_col0: int, dt_bias, a_log, 
         lib, size = _lookup("recurrent_chunks", "qwb_ssm_chunked_scratch")
         size.restype = ctypes.c_longlong
         chunks_from, rest = _forms(ctx, SSM_CHUNKED_FROM)
-        floats = size(_i(T), _i(ctx.n_seqs), _i(chunks_from), _i(heads), _i(vdim), _i(n_state), _i(groups))
-        if 0 < floats <= CHUNK_SCRATCH_MAX:
-            scratch = torch.empty((floats,), dtype=torch.float32, device=xbc.device)
+        scratch = _chunk_scratch(size(_i(T), _i(ctx.n_seqs), _i(chunks_from), _i(heads), _i(vdim), _i(n_state), _i(groups)), xbc.device)
+        if scratch is not None:
             _call("recurrent_chunks", "qwb_ssm_chunked", _ptr(xbc), _i(xbc.shape[1]), ctypes.c_void_p(dt.data_ptr() + 4 * dt_col0),
                   _i(dt.shape[1]), _ptr(dt_bias), _ptr(a_log), _ptr(d_skip), _ptr(state), _ptr(ctx.cu_seqlens), _ptr(ctx.slots), _ptr(y),
                   _ptr(scratch), _i(T), _i(ctx.n_seqs), _i(ctx.max_new), _i(chunks_from), _i(heads), _i(vdim), _i(n_state), _i(groups),
@@ -978,22 +988,23 @@ def delta_rule(qkv: torch.Tensor, b_raw: torch.Tensor, b_col0: int, a_raw: torch
     kq = torch.empty((T, key_heads), dtype=torch.float32, device=dev)
     beta = torch.empty((T, heads), dtype=torch.float32, device=dev)
     raw_decays = (ctypes.c_void_p(a_raw.data_ptr() + 4 * a_col0), _i(a_raw.shape[1]), _ptr(dt_bias), _ptr(a_log))
-    floats, chunks_from, rest = 0, 0, True
+    o = torch.empty((T, heads * vdim), dtype=torch.float32, device=dev)
+    scratch, chunks_from, rest, decay = None, 0, True, None
     if ctx.max_new >= DELTA_CHUNKED_FROM and qkv.shape[1] % 4 == 0 and not (qkv.data_ptr() % 16 or state.data_ptr() % 16):
         size = _lookup("recurrent_chunks", "qwb_delta_chunked_scratch")[1]
         size.restype = ctypes.c_longlong
         chunks_from, rest = _forms(ctx, DELTA_CHUNKED_FROM)
-        floats = size(_i(T), _i(ctx.n_seqs), _i(chunks_from), _i(heads), _i(key_dim), _i(vdim))
-    chunked = 0 < floats <= CHUNK_SCRATCH_MAX
-    if not chunked:
+        if rest:                                            # everything else the step needs first: what is left is the scratch's
+            decay = torch.empty((T, heads * decay_k), dtype=torch.float32, device=dev)
+        scratch = _chunk_scratch(size(_i(T), _i(ctx.n_seqs), _i(chunks_from), _i(heads), _i(key_dim), _i(vdim)), dev)
+    if scratch is None:
         chunks_from, rest = 0, True
-    decay = None if not rest else torch.empty((T, heads * decay_k), dtype=torch.float32, device=dev)
+    if rest and decay is None:
+        decay = torch.empty((T, heads * decay_k), dtype=torch.float32, device=dev)
     _call("recurrent", "qwb_delta_prep", _ptr(qkv), _i(qkv.shape[1]), _ptr(kq), ctypes.c_void_p(b_raw.data_ptr() + 4 * b_col0),
           _i(b_raw.shape[1]), _ptr(beta), *raw_decays, _ptr(decay), _ptr(ctx.tok_seq) if chunks_from else _ptr(None), _ptr(ctx.cu_seqlens),
           _i(chunks_from), _i(T), _i(heads), _i(key_heads), _i(key_dim), _i(decay_k), _f(unit_eps), _f(q_scale), _stream())
-    o = torch.empty((T, heads * vdim), dtype=torch.float32, device=dev)
-    if chunked:
-        scratch = torch.empty((floats,), dtype=torch.float32, device=dev)
+    if scratch is not None:
         _call("recurrent_chunks", "qwb_delta_chunked", _ptr(qkv), _i(qkv.shape[1]), _ptr(beta), *raw_decays, _ptr(state), _ptr(ctx.cu_seqlens),
               _ptr(ctx.slots), _ptr(o), _ptr(scratch), _i(T), _i(ctx.n_seqs), _i(ctx.max_new), _i(chunks_from), _i(heads), _i(key_heads),
               _i(key_dim), _i(vdim), _i(decay_k), _i(1 if write_state else 0), _stream(), kernels=3)
@@ -1166,9 +1177,8 @@ def mlstm_scan(proj: torch.Tensor, i_col: int, f_col: int, i_bias: torch.Tensor,
         if key_dim >= MLSTM_TILES_KEYS and T * heads * vdim >= MLSTM_TILES_BLOCKS * 128 * 64 and ld % 4 == 0 and proj.data_ptr() % 16 == 0:
             lib, size = _lookup("mlstm", "qwb_mlstm_tiles_scratch")
             size.restype = ctypes.c_longlong
-            floats = size(_i(T), _i(ctx.n_seqs), _i(heads), _i(key_dim), _i(vdim))
-            if 0 < floats <= CHUNK_SCRATCH_MAX:
-                scratch = torch.empty((floats,), dtype=torch.float32, device=dev)
+            scratch = _chunk_scratch(size(_i(T), _i(ctx.n_seqs), _i(heads), _i(key_dim), _i(vdim)), dev)
+            if scratch is not None:
                 _call("mlstm", "qwb_mlstm_tiles", *inputs, _ptr(scratch), _ptr(raw), _ptr(divisor), *sizes, _f(q_scale), _f(tiny),
                       _i(1 if write_state else 0), _stream(), kernels=4)
                 return raw, divisor

@@ -492,6 +492,39 @@ def test_recurrences_do_not_look_at_the_rest_of_the_batch(kind, lens):
         at += n
 
 
+@pytest.mark.parametrize("kind", ["mamba2", "delta", "mixed"])
+def test_recurrences_without_memory_for_chunks(kind):
+    """Where the scratch memory of the chunks cannot be had, a prompt goes through the scan, as it would without them."""
+    torch.manual_seed(5)
+    H, P, K, G, lens = 16, 64, 256 if kind == "mamba2" else 64, 2, [3000, 1] if kind == "mixed" else [3000]
+    T, B = sum(lens), len(lens)
+    step = Steps(lens, list(range(B)))
+    xbc, side, a_raw = torch.randn(T, H * P + 2 * G * K, device=DEV), torch.randn(T, H, device=DEV), torch.randn(T, H * K, device=DEV) - 3.0
+    qkv, vec, bias = torch.randn(T, 2 * H * K + H * P, device=DEV), torch.randn(H, device=DEV), torch.randn(H * K, device=DEV)
+    start = 0.3 * torch.randn(B, H, P, K, device=DEV)
+
+    def run(x, state):
+        if kind == "mamba2":
+            return ops.ssm_scan(x, side, 0, vec, vec, vec, state, step, H, P, K, G)
+        return ops.delta_rule(x, side, 0, a_raw, bias, vec, state, step, H, H, K, P, 1e-6, K ** -0.5)
+
+    inputs = xbc if kind == "mamba2" else qkv
+    states, xs, outs = [start.clone() for _ in range(3)], [inputs.clone() for _ in range(3)], []
+    outs.append(run(xs[0], states[0]))                      # with chunks
+    step.max_new = 1                                        # the scan
+    outs.append(run(xs[1], states[1]))
+    step.max_new, total = max(lens), torch.cuda.get_device_properties(DEV).total_memory
+    torch.cuda.empty_cache()
+    room = torch.cuda.memory_reserved() + (16 << 20 if kind == "mamba2" else 32 << 20)      # y, or o and the decays: 12 MB each; the scratch is more
+    try:
+        torch.cuda.set_per_process_memory_fraction(room / total, DEV)
+        outs.append(run(xs[2], states[2]))
+    finally:
+        torch.cuda.set_per_process_memory_fraction(1.0, DEV)
+    assert torch.equal(outs[1], outs[2]) and torch.equal(states[1], states[2])
+    sums_close(outs[0], outs[1].double())
+
+
 # ----------------------------------------------------------------------------- score maps, single tokens
 @pytest.mark.parametrize("maps, H, G, dim, vdim", [(2, 16, 4, 64, 128), (2, 2, 2, 8, 8), (2, 15, 3, 40, 72), (1, 10, 1, 128, 128), (2, 4, 1, 128, 120), (1, 3, 3, 24, 16)])
 @pytest.mark.parametrize("softcap, window, chunk, gated", [(0.0, 0, 0, False), (5.0, 0, 0, True), (3.0, 100, 0, False), (2.0, 1, 0, True), (20.0, 0, 96, False)])
