@@ -1137,8 +1137,17 @@ MLSTM_CHUNKED_FROM = 64         # steps whose longest sequence brings at least t
 # tiles are what hides the copies, and at least MLSTM_TILES_BLOCKS blocks of 128 tokens x 64 values, three an SM.  us, 64 / 128
 # tokens a chunk: 4 heads of 256 x 512, 1,000 tokens (249 blocks) 113 / 113, 2,048 233 / 194, 4,096 437 / 374, 4 x 1,024 438 / 367; 4 of
 # 256 x 256, 2,048 tokens (256) 118 / 133, 4,096 240 / 227; 8 of 512 x 256, 1,000 tokens 218 / 233, 2,048 433 / 392; 16 of
-# 128 x 128, 4,096 tokens (1,024) 289 / 295; 4 of 64 x 64, 4,096 tokens 51 / 69.
-MLSTM_TILES_KEYS, MLSTM_TILES_BLOCKS = 256, 512
+# 128 x 128, 4,096 tokens (1,024) 289 / 295; 4 of 64 x 64, 4,096 tokens 51 / 69.  A chunk costs the same however few tokens are in it, so
+# the step must bring at least MLSTM_TILES_FILL tokens a place that its chunks have.  4 heads of 256 x 512: 4 x 512 tokens (102 a place)
+# 231 / 201, 8 x 300 (92) 299 / 299, 16 x 130 (65) 340 / 458, 2,048 beside 4 single tokens (98) 258 / 262, beside 63 (26) 790 / 1,521; 8 of
+# 512 x 256: 4 x 512 434 / 441, 8 x 256 (85) 449 / 574.
+MLSTM_TILES_KEYS, MLSTM_TILES_BLOCKS, MLSTM_TILES_FILL = 256, 512, 100
+
+
+def mlstm_tiles_pay(tokens: int, seqs: int, heads: int, key_dim: int, vdim: int) -> bool:
+    """Whether a step of ``tokens`` tokens of ``seqs`` sequences takes the mLSTM's chunks of 128 tokens rather than those of 64."""
+    return (key_dim >= MLSTM_TILES_KEYS and tokens * heads * vdim >= MLSTM_TILES_BLOCKS * 128 * 64
+            and tokens >= MLSTM_TILES_FILL * (tokens // 128 + seqs))
 
 
 def mlstm_scan(proj: torch.Tensor, i_col: int, f_col: int, i_bias: torch.Tensor, f_bias: torch.Tensor, gate_cap: float,
@@ -1174,7 +1183,7 @@ def mlstm_scan(proj: torch.Tensor, i_col: int, f_col: int, i_bias: torch.Tensor,
               _ptr(ctx.cu_seqlens), _ptr(ctx.slots), _ptr(gate_rows))
     if chunked and not single:
         sizes = (_i(T), _i(ctx.n_seqs), _i(ctx.max_new), _i(heads), _i(key_dim), _i(vdim))
-        if key_dim >= MLSTM_TILES_KEYS and T * heads * vdim >= MLSTM_TILES_BLOCKS * 128 * 64 and ld % 4 == 0 and proj.data_ptr() % 16 == 0:
+        if mlstm_tiles_pay(T, ctx.n_seqs, heads, key_dim, vdim) and ld % 4 == 0 and proj.data_ptr() % 16 == 0:
             lib, size = _lookup("mlstm", "qwb_mlstm_tiles_scratch")
             size.restype = ctypes.c_longlong
             scratch = _chunk_scratch(size(_i(T), _i(ctx.n_seqs), _i(heads), _i(key_dim), _i(vdim)), dev)

@@ -326,8 +326,7 @@ def test_matrix_memory_in_chunks_of_128(H, K, P, forget, monkeypatch):
     """Sequences at the edges of the chunks of 128, from a memory, that fade, last and mix; rows shifted by one float take the
     general form, which gives the same; slots of others stay as they are."""
     torch.manual_seed(H + K + P)
-    monkeypatch.setattr(ops, "MLSTM_TILES_KEYS", 4)
-    monkeypatch.setattr(ops, "MLSTM_TILES_BLOCKS", 0)
+    monkeypatch.setattr(ops, "mlstm_tiles_pay", lambda *sizes: True)
     lens, slots, cap = [1, 64, 127, 128, 129, 300], [4, 2, 7, 1, 5, 3], 15.0
     T, n_qkv, step = sum(lens), H * (2 * K + P), Steps(lens, slots)
     wide = torch.randn(T, -(-(n_qkv + 2 * H) // 4) * 4 + 4, device=DEV)
