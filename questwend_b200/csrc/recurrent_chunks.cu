@@ -27,6 +27,8 @@
 #define SC_ROWS 16                      // rows of a tile
 #define SC_LDA 132
 #define SC_LDB 68
+#define SC_FORGETS -128.f               // the exponential of this is 0 in 32-bit: a log decay below (-infinity too) counts as this much,
+                                        // so that differences of sums are numbers and keep the digits of the other tokens' decays
 
 struct ScArgs {
     const float *xbc, *dt_raw, *dt_bias, *A_log, *D;
@@ -47,8 +49,9 @@ __device__ __forceinline__ void sc_steps(const ScArgs& a, int h, int t0, int n, 
         const int i = 4 * lane + e;
         const float d = i < n ? rc_softplus(a.dt_raw[(size_t)(t0 + i) * a.ld_dt + h] + bias) : 0.f;
         dt[i] = d;
-        if (decay) decay[i] = expf(rate * d);
-        sum += (double)(rate * d);
+        const float fade = i < n ? rate * d : 0.f;
+        if (decay) decay[i] = expf(fade);
+        sum += (double)(fade < SC_FORGETS ? SC_FORGETS : fade);
         own[e] = sum;
     }
     double run = sum;

@@ -281,6 +281,26 @@ def test_mamba2_in_chunks(H, P, N, G, pace, monkeypatch):
     assert torch.equal(state, before)
 
 
+@pytest.mark.parametrize("rate", [10.0, 80.0, 100.0])
+def test_mamba2_in_chunks_with_decays_of_nothing(rate):
+    """Rates so large that a token leaves nothing of the state (e^100 is no 32-bit number: its log decay is -infinity), in all heads or
+    only with large steps: as the scan, which multiplies by a token's own decay."""
+    torch.manual_seed(int(rate))
+    H, P, N, G, T = 4, 64, 128, 2, 300
+    step = Steps([T], [0])
+    xbc, dt = torch.randn(T, H * P + 2 * G * N, device=DEV), torch.randn(T, H, device=DEV) - 3.0
+    dt[:, 1] = -40.0                                        # a step of 4e-18: little of e^40, much of e^50
+    dt[5::9, 1] = 3.0
+    a_log = torch.tensor([rate, rate / 2, 0.0, 1.0], device=DEV)
+    bias, d, start = torch.zeros(H, device=DEV), torch.randn(H, device=DEV), torch.randn(1, H, P, N, device=DEV)
+    results = []
+    for longest in (T, 1):
+        step.max_new, state = longest, start.clone()
+        results.append((ops.ssm_scan(xbc, dt, 0, bias, a_log, d, state, step, H, P, N, G), state))
+    for got, want in zip(*results):
+        sums_close(got, want.double(), 2 ** -18)
+
+
 def matrix_memory(row, at, H, K, P, i_b, f_b, cap, S, top):
     """The mLSTM in 64 bits over one sequence's rows from a memory [H, P + 1, K] and its maxima [H]: (read-outs, divisors, both after it)."""
     row, n, n_qkv, S, top = row.double(), len(row), H * (2 * K + P), S.double().transpose(1, 2), top.double()
