@@ -953,11 +953,12 @@ def ssm_scan(xbc: torch.Tensor, dt: torch.Tensor, dt_col0: int, dt_bias, a_log, 
     return y
 
 
-# Tokens from which a sequence goes through the delta rule in chunks (csrc/recurrent_chunks.cu), by its own length.  With its
-# convolution, 16 heads of 128 x 128, us, scan / chunks: 64 tokens 44 / 68, 100 tokens (a decay per head) 43 / 68, 400 tokens 194 / 94.
-# Steps with both, all by the scan / each its own way: 200 beside 63 single tokens 143 / 173 (two kinds of launches one after the other),
-# 2,048 beside 63 1,051 / 395, two of 150 and 160 135 / 89 (all of them in chunks: 609, 864, 83).
-DELTA_CHUNKED_FROM = 144
+# Tokens from which a sequence goes through the delta rule in chunks (csrc/recurrent_chunks.cu), by its own length.  16 heads of
+# 128 x 128, us, scan / chunks: 64 tokens 44 / 68 and 400 tokens 194 / 101 (with the convolution), 200 tokens 92 / 79, two of 150 and 160
+# 135 / 89.  Beside single tokens, whose scan then waits for the chunks' launches, all by the scan / each its own way: 200 beside 63
+# 143 / 173, beside 255 389 / 426, 2,048 beside 63 1,051 / 395 (all of them in chunks: 609, 2,210, 864).  Alone the chunks are ahead from
+# about 144 tokens on, beside many single ones from about 300: the line lies between.
+DELTA_CHUNKED_FROM = 192
 
 
 def delta_rule(qkv: torch.Tensor, b_raw: torch.Tensor, b_col0: int, a_raw: torch.Tensor, dt_bias, a_log,
