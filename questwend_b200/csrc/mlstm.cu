@@ -564,9 +564,9 @@ struct MlArgs {
     int write_state;
 };
 
-// a head's write strengths, sums of log decays and, if wanted, decays of a chunk's tokens (beyond the n tokens: 0, the last sum, 1);
-// the caller synchronises
-__device__ __forceinline__ void ml_gates(const MlArgs& a, int h, int t0, int n, float* w, double* G, float* decay = nullptr) {
+// a head's write strengths and sums of log decays of a chunk's tokens (beyond the n tokens: 0, the last sum) and, if wanted, the write
+// strengths that are left at the end of a token's tile of 16; the caller synchronises
+__device__ __forceinline__ void ml_gates(const MlArgs& a, int h, int t0, int n, float* w, double* G, float* left = nullptr) {
     const int lane = threadIdx.x;
     if (lane >= 32) return;
     double own[4], sum = 0.0;
@@ -576,7 +576,6 @@ __device__ __forceinline__ void ml_gates(const MlArgs& a, int h, int t0, int n, 
         const size_t at = (size_t)(t0 + i) * a.z.H + h;
         const float d = i < n ? a.log_decay[at] : 0.f;
         w[i] = i < n ? a.write[at] : 0.f;
-        if (decay) decay[i] = expf(d);
         sum += (double)d;
         own[e] = sum;
     }
@@ -589,6 +588,13 @@ __device__ __forceinline__ void ml_gates(const MlArgs& a, int h, int t0, int n, 
     const double before = run - sum;
 #pragma unroll
     for (int e = 0; e < 4; ++e) G[4 * lane + e] = before + own[e];
+    if (!left) return;
+    __syncwarp();
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+        const int i = 4 * lane + e;
+        left[i] = expf((float)(G[i | (ML_ROWS - 1)] - G[i])) * w[i];
+    }
 }
 
 // grid (chunks, H * ptiles * ktiles + 3 H, B), 128 threads: 64 values x 128 key rows of a chunk's own sum, or one of the three
@@ -796,7 +802,7 @@ mlstm_tile_out_kernel(const MlArgs a, int ptiles) {
     pdl_wait();
     pdl_launch_dependents();
     __shared__ __align__(16) float tiles[3][ML_ROWS][ML_LDA + ML_LDB];
-    __shared__ float w[ML_TOKENS], decay[ML_TOKENS];
+    __shared__ float w[ML_TOKENS], left[ML_TOKENS];
     __shared__ double G[ML_TOKENS];
     const int c = blockIdx.x, b = blockIdx.z, tid = threadIdx.x, H = a.z.H, K = a.z.K, P = a.z.P, ld = a.rows.ld;
     const int h = blockIdx.y / ptiles, p0 = (blockIdx.y - h * ptiles) * 64;
@@ -831,17 +837,19 @@ mlstm_tile_out_kernel(const MlArgs a, int ptiles) {
     };
     copy(0);
     copy(1);
-    ml_gates(a, h, t0, n, w, G, decay);
+    ml_gates(a, h, t0, n, w, G, left);
     auto weigh = [&](int t) {                                       // this thread's token's weights of a tile of tokens, over their scores
         if (t < state_tiles || t >= n_tiles) return;
         const int j0 = (t - state_tiles) * ML_ROWS;
         float* col = &tiles[t % 3][0][tid];
-        float e = tid >= j0 + ML_ROWS ? expf((float)(G[tid] - G[j0 + ML_ROWS - 1])) : 0.f;
+        if (tid >= j0 && tid < j0 + ML_ROWS) {                      // its own tile
 #pragma unroll
-        for (int r = ML_ROWS - 1; r >= 0; --r) {
-            if (r < ML_ROWS - 1) e *= decay[j0 + r + 1];
-            if (tid == j0 + r) e = 1.f;
-            col[r * (ML_LDA + ML_LDB)] = tid >= j0 + r ? col[r * (ML_LDA + ML_LDB)] * (e * w[j0 + r]) : 0.f;
+            for (int r = 0; r < ML_ROWS; ++r)
+                col[r * (ML_LDA + ML_LDB)] = tid >= j0 + r ? col[r * (ML_LDA + ML_LDB)] * (expf((float)(G[tid] - G[j0 + r])) * w[j0 + r]) : 0.f;
+        } else {                                                    // what is left at the tile's end, and what decays behind it
+            const float e = tid > j0 ? expf((float)(G[tid] - G[j0 + ML_ROWS - 1])) : 0.f;
+#pragma unroll
+            for (int r = 0; r < ML_ROWS; ++r) col[r * (ML_LDA + ML_LDB)] = tid > j0 ? col[r * (ML_LDA + ML_LDB)] * (e * left[j0 + r]) : 0.f;
         }
     };
     const int ig = (tid >> 3) * 4, pg = (tid & 7) * 4;              // this thread's tokens ig .., 64 + ig ..; values pg .., 32 + pg ..
