@@ -752,7 +752,7 @@ delta_chunk_walk_kernel(const DcArgs a) {
             for (int k = 0; k < 4; ++k) *reinterpret_cast<float2*>(at.start + (size_t)(kg + k) * P + p0 + ps) = make_float2(S[0][k], S[1][k]);
         }
         const float *w = Ws + ig * ldw, *s = Ss + p * ldw;
-        float part[4][2] = {{0.f, 0.f}, {0.f, 0.f}, {0.f, 0.f}, {0.f, 0.f}};
+        float part[4][4] = {};                                      // four chains a sum: shorter ones round less
 #pragma unroll 8
         for (int k = 0; k < K; k += 4) {
             const float4 y = *reinterpret_cast<const float4*>(s + k);
@@ -760,12 +760,12 @@ delta_chunk_walk_kernel(const DcArgs a) {
             for (int i = 0; i < 4; ++i) {
                 const float4 x = *reinterpret_cast<const float4*>(w + 16 * i * ldw + k);
                 part[i][0] += x.x * y.x; part[i][1] += x.y * y.y;
-                part[i][0] += x.z * y.z; part[i][1] += x.w * y.w;
+                part[i][2] += x.z * y.z; part[i][3] += x.w * y.w;
             }
         }
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
-            const float u = own[i] - (part[i][0] + part[i][1]);
+            const float u = own[i] - ((part[i][0] + part[i][1]) + (part[i][2] + part[i][3]));
             Us[(ig + 16 * i) * LU + p] = u;
             if (p_ok) at.u[(size_t)(ig + 16 * i) * P + p0 + p] = u;
         }
