@@ -540,7 +540,7 @@ static int as_launch(const char* what, dim3 grid, const CUtensorMap* maps, const
 static int as_pieces(int n) { return (n + 63) / 64; }
 
 static bool as_latent_fits(int K, int R, int DV) {
-    return K > 0 && R >= 0 && DV > 0 && K % 8 == 0 && R % 8 == 0 && DV % 8 == 0 && DV <= 128 && as_pieces(K) + as_pieces(R) <= 3;
+    return K > 0 && R >= 0 && DV > 0 && K % 8 == 0 && R % 8 == 0 && (K + R) % 16 == 0 && DV % 8 == 0 && DV <= 128 && as_pieces(K) + as_pieces(R) <= 3;
 }
 
 // Prompts that start their sequences: q [T, H, K + R], k_plain [T, H, K], R rotated values at kr + t * ld_kr, v [T, H, DV], out

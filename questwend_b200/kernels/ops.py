@@ -1461,8 +1461,8 @@ def maps_attention(q: torch.Tensor, k_pool, v_pool, page_table, ctx, maps: int, 
     if one_map and ctx.max_new * (H // G) >= 64:
         return attn_prefill(q, k_pool, v_pool, page_table, ctx.cu_seqlens, ctx.pos0, ctx.max_new, scale, window=window, impl="tc",
                             chunk=chunk)
-    if (impl in ("auto", "tc") and scale > 0.0 and ctx.max_new * (H // G) >= 64 and maps_prefill_tc_fits(q.dtype, maps, dim, vdim, H // G)
-            and not any(t.data_ptr() % 16 for t in (q, k_pool, v_pool))):
+    if (impl in ("auto", "tc") and scale > 0.0 and ctx.max_new * (H // G) >= 64 and ctx.max_new * (H // G) <= 65535 * 64
+            and maps_prefill_tc_fits(q.dtype, maps, dim, vdim, H // G) and not any(t.data_ptr() % 16 for t in (q, k_pool, v_pool))):
         _call("attention_streams", "qwb_maps_prefill_tc", _ptr(q), _ptr(k_pool), _ptr(v_pool), _ptr(page_table), _ptr(ctx.cu_seqlens),
               _ptr(ctx.pos0), _ptr(out), _i(ctx.n_seqs), _i(T), _i(ctx.max_new), _i(k_pool.shape[0]), _i(H), _i(G), _i(dim), _i(vdim), _i(width),
               _f(scale), _f(softcap), _i(chunk), _i(window), _f(lam), _i(1 if norm_out else 0), _f(eps), _f(out_scale), *gate_args,
@@ -1692,8 +1692,9 @@ LATENT_PREFILL_TC = True    # prompts take the tcgen05 kernel where it fits; Fal
 
 
 def latent_prefill_tc_fits(dim: int, rot_dim: int, vdim: int) -> bool:
-    """Whether the tcgen05 prompt kernel takes these head sizes: up to three pieces of 64 query values, values of up to 128."""
-    return (LATENT_PREFILL_TC and dim > 0 and rot_dim >= 0 and 0 < vdim <= 128 and not (dim % 8 or rot_dim % 8 or vdim % 8)
+    """Whether the tcgen05 prompt kernel takes these head sizes: up to three pieces of 64 query values, 16 by 16 in all as for the
+    mma.sync kernel, values of up to 128."""
+    return (LATENT_PREFILL_TC and dim > 0 and rot_dim >= 0 and 0 < vdim <= 128 and not (dim % 8 or rot_dim % 8 or vdim % 8 or (dim + rot_dim) % 16)
             and -(-dim // 64) + -(-rot_dim // 64) <= 3)
 
 
