@@ -110,16 +110,20 @@ def test_latent_attention_alone(entry, dtype):
         assert close(g, r, dtype)
 
 
+@pytest.mark.parametrize("streams", [True, False])
 @pytest.mark.parametrize("window", [0, 1, 2, 63, 64, 65, 100])
 @pytest.mark.parametrize("sizes", [dict(heads=3, dim=24, rot_dim=8, vdim=40, kv_rank=40), dict(heads=2, dim=64, rot_dim=16, vdim=64, kv_rank=48),
                                    dict(heads=1, dim=8, rot_dim=8, vdim=8, kv_rank=8, q_rank=8),
                                    dict(heads=2, dim=24, rot_dim=8, vdim=136, kv_rank=16, q_rank=16)])
-def test_whole_prompts_on_the_tensor_cores(sizes, window, monkeypatch):
-    """bfloat16 prompts that start their sequences take the tensor-core kernel (keys and values per head made from the
+def test_whole_prompts_on_the_tensor_cores(sizes, window, streams, monkeypatch):
+    """bfloat16 prompts that start their sequences take a tensor-core kernel, tcgen05 where it fits or mma.sync (keys and values per head made from the
     latents): against the plain implementation, and against the kernel that scores the latents themselves, for windows
     around the key tile of 64 and prompts that cross two tiles, end inside one, or are a single token."""
     from questwend_b200.kernels import ops
     from questwend_b200.parts import latent_attention as la
+    monkeypatch.setattr(ops, "LATENT_PREFILL_TC", streams)
+    if streams != ops.latent_prefill_tc_fits(sizes["dim"], sizes["rot_dim"], sizes["vdim"]):
+        pytest.skip("values of 136 take mma.sync either way")
     entry = mh.latent(window=window, **sizes)
     assert ops.latent_prefill_fits(torch.bfloat16, sizes["dim"], sizes["rot_dim"], sizes["vdim"], sizes["kv_rank"])
     calls = []

@@ -395,10 +395,12 @@ def test_window_edges_show(window):
         assert close(mixers.run([x], plan)[0][0], a, torch.float32), plan[0]
 
 
-def test_whole_prompts_of_latents_take_the_tensor_cores(monkeypatch):
-    """bfloat16 prompts that start their sequences go through the tensor-core kernel, in the layer that owns the rows and in
+@pytest.mark.parametrize("streams", [True, False])
+def test_whole_prompts_of_latents_take_the_tensor_cores(streams, monkeypatch):
+    """bfloat16 prompts that start their sequences go through a tensor-core kernel (tcgen05, or mma.sync), in the layer that owns the rows and in
     the one that reads them; the results agree with the kernel that scores the latents themselves."""
     from questwend_b200.parts import latent_attention as la
+    monkeypatch.setattr(ops, "LATENT_PREFILL_TC", streams)
     layers = [th.latent(heads=3, dim=24, rot_dim=8, vdim=40), th.latent(heads=2, dim=40, rot_dim=8, vdim=16, kv_from=0)]
     w = th.draw_weights(th.config([(l, None) for l in layers], width=WIDTH), 10)
     xs = [pz.round_bf16(np.random.default_rng(n).standard_normal((n, WIDTH))) for n in (150, 64, 20, 1)]
