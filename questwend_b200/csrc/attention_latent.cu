@@ -361,7 +361,8 @@ __global__ void latent_combine_kernel(const float* __restrict__ part_acc, const 
 // heads are the 16 rows of a tile: S = Q K^T over the whole row (L + R values), O += P V with V the same row's first L
 // values, both from one copy of the row in shared memory.  The queries and the probabilities stay 32-bit: each is cut into
 // three bfloat16 numbers whose sum it is (8 + 8 + 8 bits), and each part is multiplied exactly with the bfloat16 row and
-// summed in 32-bit, three products for one.
+// summed in 32-bit, three products for one.  (A cached value that is not finite makes the rows that see it no numbers: the parts'
+// products with it do not add up to an infinity.)
 // Block = 16 warps, one an SM, one run of keys of one sequence, tiles of 32 keys in four buffers (cp.async, three tiles
 // ahead).  For the scores the warps share the row's steps of 16 values (a warp keeps its KW steps of Q in registers; the
 // partial scores meet in shared memory); for the softmax each takes one of the 16 rows; for the output each takes NW tiles of

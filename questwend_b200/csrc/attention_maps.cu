@@ -18,9 +18,11 @@
 //                     first rdims values of every map of q and k, cache write of a step's tokens; q out
 //   maps_row_prep     the same with one norm over the whole projection of q (and of k), and a factor on q by its position
 //   maps_prefill      any number of new tokens per sequence (float and bfloat16, any sizes up to 256)
-//   maps_prefill_mma  bfloat16 prompts on the tensor cores
+//   maps_prefill_mma  bfloat16 prompts on the tensor cores (mma.sync); those with two maps and sizes that fit take
+//                     maps_prefill_tc (attention_streams.cu, tcgen05) instead
 //   maps_decode       one new token per sequence: runs of pages, one block of threads a run, then maps_merge, which also
 //                     takes the difference and the norm
+//   maps_decode_mma   the same over a bfloat16 cache on the tensor cores (mma.sync), keys of up to 256 values and values of up to 128
 #include "common.cuh"
 
 #include <type_traits>
@@ -1196,6 +1198,8 @@ __global__ void maps_decode_kernel(const T* __restrict__ q, const T* __restrict_
 // and no ldmatrix.  q is zero outside a row's own map, so that one product over a whole key row gives every row its map's score.
 // Probabilities stay 32-bit: each is cut into three bfloat16 numbers whose sum it is; the tile's other eight rows take the second
 // one, a product of its own the third.  What a lane holds of the scores is what it needs of the probabilities.
+// A cached value that is not finite gives a result that is no number, also where it belongs to the head's other map (0 times it) or is
+// seen with a probability whose smaller parts are 0; the plain kernel leaves an infinity.
 // Bound by the chain of a group (about 700 instructions a warp, twelve warps an SM): a third stage, which leaves room for eight,
 // is slower.  16 heads of 2 x 64 over 4 key/value heads, values of 128, with the merge, replayed from a graph, before
 // (maps_decode_kernel, plain FMA) and now: 8 sequences of about 8,000 keys 74.4 -> 43.9 us (123 MB), 32 of 300 23.9 -> 16.3 us, one of

@@ -1,8 +1,9 @@
 // Long prompts through the recurrences of recurrent.cu in chunks: inside a chunk the tokens meet in small matrix products,
-// from chunk to chunk only the state is carried.  Everything is 32-bit (plain multiply-adds; the tensor cores have no product
-// of 32-bit operands, and six products of bfloat16 parts in place of one would run no faster on mma.sync: 554 / 6 TFLOP/s
-// against 72).  Decays enter as sums of their logarithms, always of tokens between two others, so every exponential is of a
-// number that is at most 0: nothing overflows, and what underflows is below the smallest float in truth too.
+// from chunk to chunk only the state is carried.  Everything is 32-bit, in plain multiply-adds: the tensor cores have no product
+// of 32-bit operands, and six products of bfloat16 parts in place of one, at mma.sync's rate 92 TFLOP/s (554 / 6) against 72, would
+// gain little once the parts are made; on tcgen05 they would be faster, which is not written.  Decays enter as sums of their
+// logarithms, always of tokens between two others, so every exponential is of a number that is at most 0: nothing overflows, and
+// what underflows is below the smallest float in truth too.
 #include "chunks.cuh"
 
 // ---------------------------------------------------------------------------------
@@ -408,8 +409,8 @@ extern "C" int qwb_ssm_chunked(const float* xbc, int ldx, const float* dt_raw, i
 // its sub-block's end, what decays in the sub-blocks between, and what decays from the start of i's sub-block to i are three
 // factors of at most 1.  Sums of logarithms (base 2) span what they decay and nothing else.
 // Chunk c of the z-th sequence that these kernels take, b, is place cu_seqlens[b] / 64 + z + c of the scratch memory.
-// 16 heads of 128 x 128 with a decay per channel, the convolution before it, the scan and now: 2,048 tokens 955 -> 323 us (prep 121,
-// walk 131, out 49 in ncu), three sequences of 2,900 in all 1,194 -> 472 us; a decay per head, four of 4,096 in all, 1,198 -> 588 us.
+// 16 heads of 128 x 128 with a decay per channel, the convolution before it, the scan and now: 2,048 tokens 955 -> 328 us (prep 124,
+// walk 133, out 49 in ncu), three sequences of 2,900 in all 1,194 -> 485 us; a decay per head, four of 4,096 in all, 1,198 -> 594 us.
 // Bound by what shared memory hands to registers (128 bytes a cycle), the walk more than the others.
 // Scratch of a place and head:
 //     W [64][K] | k e_end [64][K] | q e_0 [64][K] | Q [64 (j)][64 (i)] | U, then u [64][P] | decay of the chunk [K] | S0 [K][P]
