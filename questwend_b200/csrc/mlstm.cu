@@ -545,8 +545,8 @@ mlstm_chunk_out_kernel(MlstmRows rows, const float* __restrict__ log_decay, cons
 // sequence b in the scratch memory: cu_seqlens[b] / 128 + b + c of T / 128 + B:
 //     own / starts [places, H, K, P], their normalisers [places, H, K], scores [places, H, 128 (j), 128 (i)], q [places, H, K, 128 (i)],
 //     total decays [places, H]
-// Bound by the 16 floats that 64 multiply-adds want from shared memory, at 0.46 of the FMA rate; half as many chunks are half the
-// bytes that the carries move.  4,096 tokens, 4 heads of 256 x 512, us: state 156, carry 36, out 190; in all 388 where
+// Bound by the 16 floats that 64 multiply-adds want from shared memory, at 0.44 of the FMA rate; half as many chunks are half the
+// bytes that the carries move.  4,096 tokens, 4 heads of 256 x 512, us: state 158, carry 37, out 189; in all 388 where
 // chunks of 64 tokens take 437.  Few blocks, keys below 256, or sequences that fill few of the chunks leave the 64-token form the faster one.
 // ---------------------------------------------------------------------------------
 #define ML_TOKENS 128

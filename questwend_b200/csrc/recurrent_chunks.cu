@@ -409,8 +409,8 @@ extern "C" int qwb_ssm_chunked(const float* xbc, int ldx, const float* dt_raw, i
 // its sub-block's end, what decays in the sub-blocks between, and what decays from the start of i's sub-block to i are three
 // factors of at most 1.  Sums of logarithms (base 2) span what they decay and nothing else.
 // Chunk c of the z-th sequence that these kernels take, b, is place cu_seqlens[b] / 64 + z + c of the scratch memory.
-// 16 heads of 128 x 128 with a decay per channel, the convolution before it, the scan and now: 2,048 tokens 955 -> 328 us (prep 124,
-// walk 133, out 49 in ncu), three sequences of 2,900 in all 1,194 -> 485 us; a decay per head, four of 4,096 in all, 1,198 -> 594 us.
+// 16 heads of 128 x 128 with a decay per channel, the convolution before it, the scan and now: 2,048 tokens 955 -> 328 us (prep 123,
+// walk 133, out 49 in ncu), three sequences of 2,900 in all 1,194 -> 484 us; a decay per head, four of 4,096 in all, 1,198 -> 596 us.
 // Bound by what shared memory hands to registers (128 bytes a cycle), the walk more than the others.
 // Scratch of a place and head:
 //     W [64][K] | k e_end [64][K] | q e_0 [64][K] | Q [64 (j)][64 (i)] | U, then u [64][P] | decay of the chunk [K] | S0 [K][P]

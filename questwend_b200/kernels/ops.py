@@ -1141,7 +1141,7 @@ MLSTM_CHUNKED_FROM = 64         # steps whose longest sequence brings at least t
 # 128 x 128, 4,096 tokens (1,024) 289 / 295; 4 of 64 x 64, 4,096 tokens 51 / 69.  A chunk costs the same however few tokens are in it, so
 # the step must bring at least MLSTM_TILES_FILL tokens a place that its chunks have.  4 heads of 256 x 512: 4 x 512 tokens (102 a place)
 # 231 / 201, 8 x 300 (92) 299 / 299, 16 x 130 (65) 340 / 458, 2,048 beside 4 single tokens (98) 258 / 262, beside 63 (26) 790 / 1,521; 8 of
-# 512 x 256: 4 x 512 434 / 441, 8 x 256 (85) 449 / 574.
+# 512 x 256: 4 x 512 434 / 441, 8 x 256 (85) 449 / 574.  (The chunks of 128 take 4 % more since their weights are two exponentials each.)
 MLSTM_TILES_KEYS, MLSTM_TILES_BLOCKS, MLSTM_TILES_FILL = 256, 512, 100
 
 
