@@ -1136,13 +1136,13 @@ def gated_part_norm(y: torch.Tensor, gate: torch.Tensor, gate_col0: int, weight:
 MLSTM_CHUNKED_FROM = 64         # steps whose longest sequence brings at least this many tokens take the chunked form
 # Its chunks of 128 tokens (csrc/mlstm.cu: mlstm_tile_*), for sizes and rows in multiples of 4: keys of at least MLSTM_TILES_KEYS, whose
 # tiles are what hides the copies, and at least MLSTM_TILES_BLOCKS blocks of 128 tokens x 64 values, three an SM.  us, 64 / 128
-# tokens a chunk: 4 heads of 256 x 512, 1,000 tokens (249 blocks) 113 / 113, 2,048 233 / 194, 4,096 437 / 374, 4 x 1,024 438 / 367; 4 of
-# 256 x 256, 2,048 tokens (256) 118 / 133, 4,096 240 / 227; 8 of 512 x 256, 1,000 tokens 218 / 233, 2,048 433 / 392; 16 of
-# 128 x 128, 4,096 tokens (1,024) 289 / 295; 4 of 64 x 64, 4,096 tokens 51 / 69.  A chunk costs the same however few tokens are in it, so
-# the step must bring at least MLSTM_TILES_FILL tokens a place that its chunks have.  4 heads of 256 x 512: 4 x 512 tokens (102 a place)
-# 231 / 201, 8 x 300 (92) 299 / 299, 16 x 130 (65) 340 / 458, 2,048 beside 4 single tokens (98) 258 / 262, beside 63 (26) 790 / 1,521; 8 of
-# 512 x 256: 4 x 512 434 / 441, 8 x 256 (85) 449 / 574.  (The chunks of 128 take 4 % more since their weights are two exponentials each.)
-MLSTM_TILES_KEYS, MLSTM_TILES_BLOCKS, MLSTM_TILES_FILL = 256, 512, 100
+# tokens a chunk: 4 heads of 256 x 512, 1,000 tokens (250 blocks) 113 / 123, 2,048 231 / 203, 4,096 442 / 387, 4 x 1,024 439 / 383; 4 of
+# 256 x 256, 2,048 tokens (256) 119 / 142, 4,096 240 / 238; 8 of 512 x 256, 1,000 tokens 218 / 241, 2,048 434 / 402; 16 of
+# 128 x 128, 4,096 tokens (1,024) 289 / 309; 4 of 64 x 64, 4,096 tokens 51 / 69.  A chunk costs the same however few tokens are in it, so
+# the step must bring at least MLSTM_TILES_FILL tokens a place that its chunks have.  4 heads of 256 x 512: 4 x 700 tokens (112 a place)
+# 324 / 308, 4 x 512 (102) 230 / 208, 8 x 300 (92) 297 / 316, 16 x 130 (65) 339 / 459, 2,048 beside 4 single tokens (98) 256 / 265, beside 63
+# (26) 785 / 1,511; 8 of 512 x 256: 4 x 700 602 / 607, 4 x 512 433 / 446, 8 x 256 (85) 447 / 574.
+MLSTM_TILES_KEYS, MLSTM_TILES_BLOCKS, MLSTM_TILES_FILL = 256, 512, 105
 
 
 def mlstm_tiles_pay(tokens: int, seqs: int, heads: int, key_dim: int, vdim: int) -> bool:

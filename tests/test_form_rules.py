@@ -5,7 +5,7 @@ from questwend_b200.kernels import ops
 
 
 @pytest.mark.parametrize("lens, heads, key_dim, vdim, tiles", [
-    ([4096], 4, 256, 512, True), ([1024] * 4, 4, 256, 512, True), ([512] * 4, 8, 512, 256, True), ([1000], 4, 256, 512, False),
+    ([4096], 4, 256, 512, True), ([1024] * 4, 4, 256, 512, True), ([700] * 4, 8, 512, 256, True), ([512] * 4, 8, 512, 256, False), ([1000], 4, 256, 512, False),
     ([4096], 16, 128, 128, False), ([2048] + [1] * 16, 4, 256, 512, False), ([4096] + [1] * 63, 8, 512, 256, False), ([130] * 16, 4, 256, 512, False),
     ([256] * 8, 8, 512, 256, False)])
 def test_matrix_memory_takes_long_chunks_only_where_they_are_filled(lens, heads, key_dim, vdim, tiles):
