@@ -14,7 +14,7 @@
 //   mlstm_chunked   long prompts in chunks of 64 tokens: every chunk's own sum of outer products, the carries, the outputs
 //   mlstm_tiles     the same in chunks of 128 tokens, for large memories and many tokens
 // Each leaves S^T q and the denominator; the norm that follows divides.
-#include "chunks.cuh"
+#include "chunk_tc.cuh"
 
 #define QWB_MLSTM_CHUNK 64
 #define QWB_MLSTM_WARPS 4
@@ -539,380 +539,138 @@ mlstm_chunk_out_kernel(MlstmRows rows, const float* __restrict__ log_decay, cons
 }
 
 // ---------------------------------------------------------------------------------
-// The same in chunks of 128 tokens, for key and value sizes in multiples of 4 (aligned): the tiles of 16 rows in three stages, the
-// 8 x 8 sums a thread and the layouts of the chunked Mamba-2 recurrence (recurrent_chunks.cu), with keys, queries, gates and a
-// normaliser per head; the scores q . k are made once per head and chunk instead of once per tile of values.  Place of chunk c of
-// sequence b in the scratch memory: cu_seqlens[b] / 128 + b + c of T / 128 + B:
-//     own / starts [places, H, K, P], their normalisers [places, H, K], scores [places, H, 128 (j), 128 (i)], q [places, H, K, 128 (i)],
+// The same in chunks of 128 tokens on tcgen05 (chunk_tc.cuh), for key and value sizes in multiples of 4 (aligned), with a normaliser per
+// head; the scores q . k are made once per head and chunk instead of once per tile of values.  Place of chunk c of sequence b in the
+// scratch memory: cu_seqlens[b] / 128 + b + c of T / 128 + B:
+//     own / starts [places, H, P / 4, K, 4], scores [places, H, 32, 128 (i), 4 (j)], gates [places, H], normalisers [places, H, K],
 //     total decays [places, H]
-// Bound by the 16 floats that 64 multiply-adds want from shared memory, at 0.44 of the FMA rate; half as many chunks are half the
-// bytes that the carries move.  4,096 tokens, 4 heads of 256 x 512, us: state 158, carry 37, out 189; in all 388 where
-// chunks of 64 tokens take 437.  Few blocks, keys below 256, or sequences that fill few of the chunks leave the 64-token form the faster one.
+// 4,096 tokens, 4 heads of 256 x 512, us: gates of the tokens 17, of the chunks 14, state 71, carries 24, outputs 87; in all 217 where the same
+// chunks took 395 in plain multiply-adds (state 152, carries 38, outputs 182) and those of 64 tokens take 447.  Error against 64 bits 2.1e-7
+// (3.6e-7 before).
 // ---------------------------------------------------------------------------------
-#define ML_TOKENS 128
-#define ML_ROWS 16
-#define ML_LDA 132
-#define ML_LDB 68
+#define ML_TOKENS CT_TOKENS
 
 struct MlArgs {
     MlstmRows rows;
     const float *log_decay, *write, *m_run;
     const int *cu_seqlens, *slots;
-    float *state, *m_state, *own, *own_n, *scores, *q_rows, *totals, *raw, *divisor;
+    float *state, *m_state, *own, *own_n, *scores, *totals, *raw, *divisor;
+    CtGates* gates;
+    int* error;
     MlstmSizes z;
     float q_scale, tiny;
     int write_state;
 };
 
-// a head's write strengths and sums of log decays of a chunk's tokens (beyond the n tokens: 0, the last sum) and, if wanted, the write
-// strengths that are left at the end of a token's tile of 16; the caller synchronises
-__device__ __forceinline__ void ml_gates(const MlArgs& a, int h, int t0, int n, float* w, double* G, float* left = nullptr) {
-    const int lane = threadIdx.x;
-    if (lane >= 32) return;
-    double own[4], sum = 0.0;
+// a chunk's place, first token and tokens (0: none)
+__device__ __forceinline__ int ml_chunk(const MlArgs& a, size_t& place, int& t0) {
+    const int b = blockIdx.z, c = blockIdx.x;
+    t0 = a.cu_seqlens[b] + c * ML_TOKENS;
+    place = (size_t)(a.cu_seqlens[b] / ML_TOKENS + b + c);
+    return min(ML_TOKENS, a.cu_seqlens[b + 1] - t0);
+}
+__device__ __forceinline__ CtRows ml_rows(const MlArgs& a, int t0, int n, int h) {
+    const float* x = a.rows.x + (size_t)t0 * a.rows.ld;
+    return {x + h * a.z.K, x + (a.z.H + h) * a.z.K, x + 2 * a.z.H * a.z.K + h * a.z.P, a.rows.ld, n};
+}
+
+// grid (chunks, H, B), 1,024 threads: a chunk's gates, and its own sum of the normaliser, 32 tokens and a key row a thread (16.6 us with
+// all 128 tokens, 4,096 tokens of 4 heads of 256 x 512)
+__global__ void __launch_bounds__(1024)
+mlstm_tile_gates_kernel(const MlArgs a) {
+    pdl_wait();
+    pdl_launch_dependents();
+    __shared__ float coef[ML_TOKENS], part[4][256];
+    int t0;
+    size_t place;
+    const int n = ml_chunk(a, place, t0), h = blockIdx.y, i = threadIdx.x, K = a.z.K, column = i & 255, group = i >> 8;
+    if (n <= 0) return;
+    const size_t at = (size_t)(t0 + i) * a.z.H + h, head = place * a.z.H + h;
+    ct_gates(i < n ? a.log_decay[at] : 0.f, i < n ? a.write[at] : 0.f, a.gates + head, a.totals + head, coef);
+    const CtRows r = ml_rows(a, t0, n, h);
+    for (int k0 = 0; k0 < K; k0 += 256) {
+        const int k = k0 + column;
+        float sum = 0.f;
 #pragma unroll
-    for (int e = 0; e < 4; ++e) {
-        const int i = 4 * lane + e;
-        const size_t at = (size_t)(t0 + i) * a.z.H + h;
-        const float d = i < n ? a.log_decay[at] : 0.f;
-        w[i] = i < n ? a.write[at] : 0.f;
-        sum += (double)d;
-        own[e] = sum;
-    }
-    double run = sum;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const double up = __shfl_up_sync(0xffffffffu, run, o);
-        if (lane >= o) run += up;
-    }
-    const double before = run - sum;
-#pragma unroll
-    for (int e = 0; e < 4; ++e) G[4 * lane + e] = before + own[e];
-    if (!left) return;
-    __syncwarp();
-#pragma unroll
-    for (int e = 0; e < 4; ++e) {
-        const int i = 4 * lane + e;
-        left[i] = expf((float)(G[i | (ML_ROWS - 1)] - G[i])) * w[i];
+        for (int e = 0; e < 32; ++e) {
+            const int j = 32 * group + e;
+            if (j < n && k < K) sum += coef[j] * r.k[(size_t)j * r.ld + k];
+        }
+        __syncthreads();
+        part[group][column] = sum;
+        __syncthreads();
+        if (group == 0 && k < K) a.own_n[head * K + k] = (part[0][column] + part[1][column]) + (part[2][column] + part[3][column]);
     }
 }
 
-// grid (chunks, H * ptiles * ktiles + 3 H, B), 128 threads: 64 values x 128 key rows of a chunk's own sum, or one of the three
-// 64 x 64 quarters with j <= i of a head's scores
-__global__ void __launch_bounds__(128)
+// grid (chunks, 2 H + H * ptiles * ktiles, B): the scores of a head's chunk with 64 of its tokens, or 64 values x 128 key rows of its own sum
+__global__ void __launch_bounds__(CT_THREADS, 2)
 mlstm_tile_state_kernel(const MlArgs a, int ptiles, int ktiles) {
     pdl_wait();
     pdl_launch_dependents();
-    constexpr int KB = 32;
-    __shared__ __align__(16) float tiles[3][ML_ROWS][ML_LDA + ML_LDB];
-    __shared__ float w[ML_TOKENS], coef[ML_TOKENS];
-    __shared__ double G[ML_TOKENS];
-    const int c = blockIdx.x, b = blockIdx.z, tid = threadIdx.x, H = a.z.H, K = a.z.K, P = a.z.P, ld = a.rows.ld;
-    const int t0 = a.cu_seqlens[b] + c * ML_TOKENS, n = min(ML_TOKENS, a.cu_seqlens[b + 1] - t0);
+    const int H = a.z.H, K = a.z.K, P = a.z.P, i = (int)blockIdx.y - 2 * H;
+    int t0;
+    size_t place;
+    const int n = ml_chunk(a, place, t0);
     if (n <= 0) return;
-    const size_t place = (size_t)(a.cu_seqlens[b] / ML_TOKENS + b + c);
-    float acc[8][8];
-#pragma unroll
-    for (int i = 0; i < 8; ++i)
-#pragma unroll
-        for (int j = 0; j < 8; ++j) acc[i][j] = 0.f;
-    const int n_state = H * ptiles * ktiles;
-    if ((int)blockIdx.y >= n_state) {                               // scores
-        const int h = ((int)blockIdx.y - n_state) / 3, quarter = ((int)blockIdx.y - n_state) % 3;
-        const int i0 = quarter == 0 ? 0 : 64, j0 = quarter == 2 ? 64 : 0;
-        if (i0 >= n) return;
-        float (*As)[68] = reinterpret_cast<float (*)[68]>(&tiles[0][0][0]), (*Bs)[68] = As + KB;
-        const float* Qh = a.rows.x + (size_t)t0 * ld + h * K;
-        const float* Kh = Qh + H * K;
-        const int ig = (tid >> 4) * 4, jg = (tid & 15) * 4;
-        for (int k0 = 0; k0 < K; k0 += KB) {
-            __syncthreads();
-            for (int idx = tid; idx < 64 * (KB / 4); idx += 128) {  // lanes walk tokens: the transposed stores do not collide
-                const int i = idx & 63, k = (idx >> 6) * 4;
-                const float4 qv = rc_load4(Qh + (size_t)(i0 + i) * ld + k0 + k, i0 + i < n && k0 + k < K);
-                const float4 kv = rc_load4(Kh + (size_t)(j0 + i) * ld + k0 + k, j0 + i < n && k0 + k < K);
-                As[k][i] = qv.x; As[k + 1][i] = qv.y; As[k + 2][i] = qv.z; As[k + 3][i] = qv.w;
-                Bs[k][i] = kv.x; Bs[k + 1][i] = kv.y; Bs[k + 2][i] = kv.z; Bs[k + 3][i] = kv.w;
-            }
-            __syncthreads();
-            if (quarter < 2)                                        // q, a key row a row, for the output blocks
-                for (int idx = tid; idx < KB * 16; idx += 128) {
-                    const int k = idx >> 4, e = (idx & 15) * 4;
-                    if (k0 + k < K) *reinterpret_cast<float4*>(a.q_rows + ((place * H + h) * K + k0 + k) * ML_TOKENS + i0 + e) = *reinterpret_cast<const float4*>(&As[k][e]);
-                }
-#pragma unroll 8
-            for (int k = 0; k < KB; ++k) {
-                const float4 x0 = *reinterpret_cast<const float4*>(&As[k][ig]), x1 = *reinterpret_cast<const float4*>(&As[k][32 + ig]);
-                const float4 y = *reinterpret_cast<const float4*>(&Bs[k][jg]);
-                const float xv[8] = {x0.x, x0.y, x0.z, x0.w, x1.x, x1.y, x1.z, x1.w}, yv[4] = {y.x, y.y, y.z, y.w};
-#pragma unroll
-                for (int i = 0; i < 8; ++i)
-#pragma unroll
-                    for (int j = 0; j < 4; ++j) acc[i][j] += xv[i] * yv[j];
-            }
-        }
-        float* out = a.scores + (place * H + h) * ML_TOKENS * ML_TOKENS;
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            float* row = out + (size_t)(j0 + jg + j) * ML_TOKENS + i0;
-            *reinterpret_cast<float4*>(row + ig) = make_float4(acc[0][j], acc[1][j], acc[2][j], acc[3][j]);
-            *reinterpret_cast<float4*>(row + 32 + ig) = make_float4(acc[4][j], acc[5][j], acc[6][j], acc[7][j]);
-        }
+    if (i < 0) {
+        const int h = blockIdx.y / 2, j0 = blockIdx.y % 2 * 64;
+        if (j0 < n) ct_pairs(ml_rows(a, t0, n, h), K, j0, a.scores + (place * H + h) * ML_TOKENS * ML_TOKENS, a.error);
         return;
     }
-    const int h = blockIdx.y / (ptiles * ktiles), tile = blockIdx.y - h * ptiles * ktiles, p0 = tile / ktiles * 64, k0 = tile % ktiles * 128;
-    ml_gates(a, h, t0, n, w, G);
-    __syncthreads();
-    coef[tid] = expf((float)(G[ML_TOKENS - 1] - G[tid])) * w[tid];
-    if (tid == 0 && tile == 0) a.totals[place * H + h] = expf((float)G[ML_TOKENS - 1]);
-    const float* V = a.rows.x + (size_t)t0 * ld + 2 * H * K + h * P + p0;
-    const float* Kh = a.rows.x + (size_t)t0 * ld + (H + h) * K + k0;
-    const int pg = (tid >> 4) * 4, kg = (tid & 15) * 4;
-    const int n_tiles = (n + ML_ROWS - 1) / ML_ROWS;
-    auto copy = [&](int t) {                                        // one commit group a tile, also beyond the last
-        if (t < n_tiles) {
-            float (*to)[ML_LDA + ML_LDB] = tiles[t % 3];
-#pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                const int r = (tid >> 5) + 4 * i, e = (tid & 31) * 4, j = t * ML_ROWS + r;
-                const bool ok = j < n && k0 + e < K;
-                rc_copy16(&to[r][e], Kh + (ok ? (size_t)j * ld + e : 0), ok);
-            }
-#pragma unroll
-            for (int i = 0; i < 2; ++i) {
-                const int r = (tid >> 4) + 8 * i, e = (tid & 15) * 4, j = t * ML_ROWS + r;
-                const bool ok = j < n && p0 + e < P;
-                rc_copy16(&to[r][ML_LDA + e], V + (ok ? (size_t)j * ld + e : 0), ok);
-            }
-        }
-        rc_commit();
-    };
-    auto weigh = [&](int t) {                                       // the values by their tokens' write strengths up to the chunk's end
-        if (t >= n_tiles) return;
-#pragma unroll
-        for (int i = 0; i < 2; ++i) {
-            const int r = (tid >> 4) + 8 * i;
-            float4* v = reinterpret_cast<float4*>(&tiles[t % 3][r][ML_LDA + (tid & 15) * 4]);
-            const float f = coef[t * ML_ROWS + r];
-            const float4 x = *v;
-            *v = make_float4(f * x.x, f * x.y, f * x.z, f * x.w);
-        }
-    };
-    copy(0);
-    copy(1);
-    rc_wait<1>();
-    __syncthreads();                                                // the write strengths are there too
-    weigh(0);
-    float norm = 0.f;                                               // of key row k0 + tid, by the first tile of values
-    for (int t = 0; t < n_tiles; ++t) {
-        rc_wait<0>();
-        __syncthreads();
-        copy(t + 2);
-        weigh(t + 1);
-        const float* rows = &tiles[t % 3][0][0];
-        rc_outer<ML_ROWS>(acc, rows, ML_LDA + ML_LDB, kg, 64 + kg, rows + ML_LDA, ML_LDA + ML_LDB, pg, 32 + pg);
-        if (p0 == 0) {
-#pragma unroll
-            for (int r = 0; r < ML_ROWS; ++r) norm += coef[t * ML_ROWS + r] * rows[r * (ML_LDA + ML_LDB) + tid];
-        }
-    }
-    float* U = a.own + (place * H + h) * (size_t)P * K;
-#pragma unroll
-    for (int i = 0; i < 8; ++i) {
-        const int k = k0 + (i >> 2) * 64 + kg + (i & 3);
-        if (k >= K) continue;
-#pragma unroll
-        for (int half = 0; half < 2; ++half) {
-            const int p = p0 + 32 * half + pg;
-            if (p < P) *reinterpret_cast<float4*>(U + (size_t)k * P + p) = make_float4(acc[i][4 * half], acc[i][4 * half + 1], acc[i][4 * half + 2], acc[i][4 * half + 3]);
-        }
-    }
-    if (p0 == 0 && k0 + tid < K) a.own_n[(place * H + h) * K + k0 + tid] = norm;
+    const int h = i / (ptiles * ktiles), tile = i - h * ptiles * ktiles;
+    ct_state(ml_rows(a, t0, n, h), a.gates + place * H + h, K, P, tile % ktiles * 128, tile / ktiles * 64, a.own + (place * H + h) * (size_t)P * K, a.error);
 }
 
-// grid (tiles of 32 key rows x 32 values + tiles of 256 normaliser values, H, B), 256 threads: through the sequence's chunks in order
-__global__ void __launch_bounds__(256)
-mlstm_tile_carry_kernel(const MlArgs a, int ptiles, int matrix_tiles) {
+// grid (blocks of 1,024 of a head's state + tiles of 256 normaliser values, H, B): through the sequence's chunks in order
+__global__ void __launch_bounds__(256, 4)
+mlstm_tile_carry_kernel(const MlArgs a, int matrix_blocks) {
     pdl_wait();
     pdl_launch_dependents();
-    constexpr int AHEAD = 8;
-    __shared__ float turn[32][33];
     const int h = blockIdx.y, b = blockIdx.z, H = a.z.H, K = a.z.K, P = a.z.P, t0 = a.cu_seqlens[b], n = a.cu_seqlens[b + 1] - t0;
     if (n <= 0) return;
-    const int chunks = (n + ML_TOKENS - 1) / ML_TOKENS, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int chunks = (n + ML_TOKENS - 1) / ML_TOKENS;
     const size_t place = (size_t)(t0 / ML_TOKENS + b), head = (size_t)a.slots[b] * H + h;
     const float* total = a.totals + place * H + h;
     float* S = a.state + head * (P + 1) * K;
-    if ((int)blockIdx.x >= matrix_tiles) {                          // the normaliser, and the running maxima
-        const int k = ((int)blockIdx.x - matrix_tiles) * 256 + threadIdx.x;
-        if (k < K) {
-            float s = S[(size_t)P * K + k];
-            float* at = a.own_n + (place * H + h) * K + k;
-            for (int c = 0; c < chunks; ++c) {
-                const float u = at[(size_t)c * H * K];
-                at[(size_t)c * H * K] = s;
-                s = total[(size_t)c * H] * s + u;
-            }
-            if (a.write_state) S[(size_t)P * K + k] = s;
-        }
-        if (a.write_state && (int)blockIdx.x == matrix_tiles)
-            for (int p = threadIdx.x; p <= P; p += 256) a.m_state[head * (P + 1) + p] = a.m_run[(size_t)(t0 + n - 1) * H + h];
+    if ((int)blockIdx.x < matrix_blocks) {
+        ct_carry(a.own + (place * H + h) * (size_t)P * K, (size_t)H * P * K, total, H, chunks, S, K, P, blockIdx.x * 256 + threadIdx.x, a.write_state);
         return;
     }
-    const int k0 = blockIdx.x / ptiles * 32, p0 = blockIdx.x % ptiles * 32;
-    const size_t size = (size_t)P * K;
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        const int p = warp + 8 * i;
-        turn[p][lane] = p0 + p < P && k0 + lane < K ? S[(size_t)(p0 + p) * K + k0 + lane] : 0.f;
-    }
-    __syncthreads();
-    const int row = threadIdx.x >> 3, p = (threadIdx.x & 7) * 4;
-    float4 s = make_float4(turn[p][row], turn[p + 1][row], turn[p + 2][row], turn[p + 3][row]);
-    if (k0 + row < K && p0 + p < P) {
-        const size_t step = (size_t)H * size;
-        float* at = a.own + (place * H + h) * size + (size_t)(k0 + row) * P + p0 + p;
-        for (int c0 = 0; c0 < chunks; c0 += AHEAD) {
-            float4 u[AHEAD];
-            float d[AHEAD];
-#pragma unroll
-            for (int i = 0; i < AHEAD; ++i)
-                if (c0 + i < chunks) { u[i] = *reinterpret_cast<const float4*>(at + (c0 + i) * step); d[i] = total[(size_t)(c0 + i) * H]; }
-#pragma unroll
-            for (int i = 0; i < AHEAD; ++i)
-                if (c0 + i < chunks) {
-                    *reinterpret_cast<float4*>(at + (c0 + i) * step) = s;
-                    s = make_float4(d[i] * s.x + u[i].x, d[i] * s.y + u[i].y, d[i] * s.z + u[i].z, d[i] * s.w + u[i].w);
-                }
+    const int k = ((int)blockIdx.x - matrix_blocks) * 256 + threadIdx.x;            // the normaliser, and the running maxima
+    if (k < K) {
+        float s = S[(size_t)P * K + k];
+        float* at = a.own_n + (place * H + h) * K + k;
+        for (int c = 0; c < chunks; ++c) {
+            const float u = at[(size_t)c * H * K];
+            at[(size_t)c * H * K] = s;
+            s = total[(size_t)c * H] * s + u;
         }
+        if (a.write_state) S[(size_t)P * K + k] = s;
     }
-    if (!a.write_state) return;
-    turn[p][row] = s.x; turn[p + 1][row] = s.y; turn[p + 2][row] = s.z; turn[p + 3][row] = s.w;
-    __syncthreads();
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        const int q = warp + 8 * i;
-        if (p0 + q < P && k0 + lane < K) S[(size_t)(p0 + q) * K + k0 + lane] = turn[q][lane];
-    }
+    if (a.write_state && (int)blockIdx.x == matrix_blocks)
+        for (int p = threadIdx.x; p <= P; p += 256) a.m_state[head * (P + 1) + p] = a.m_run[(size_t)(t0 + n - 1) * H + h];
 }
 
-// grid (chunks, H * ptiles, B), 128 threads: a chunk's 128 tokens x 64 values; a head's first tile of values also makes the divisors
-__global__ void __launch_bounds__(128, 4)
+// grid (chunks, H * ptiles, B): a chunk's 128 tokens x 64 values; a head's first tile of values also makes the divisors
+__global__ void __launch_bounds__(CT_THREADS, 2)
 mlstm_tile_out_kernel(const MlArgs a, int ptiles) {
     pdl_wait();
     pdl_launch_dependents();
-    __shared__ __align__(16) float tiles[3][ML_ROWS][ML_LDA + ML_LDB];
-    __shared__ float w[ML_TOKENS], left[ML_TOKENS];
-    __shared__ double G[ML_TOKENS];
-    const int c = blockIdx.x, b = blockIdx.z, tid = threadIdx.x, H = a.z.H, K = a.z.K, P = a.z.P, ld = a.rows.ld;
-    const int h = blockIdx.y / ptiles, p0 = (blockIdx.y - h * ptiles) * 64;
-    const int t0 = a.cu_seqlens[b] + c * ML_TOKENS, n = min(ML_TOKENS, a.cu_seqlens[b + 1] - t0);
+    const int H = a.z.H, K = a.z.K, P = a.z.P, h = blockIdx.y / ptiles, p0 = (blockIdx.y - h * ptiles) * 64;
+    int t0;
+    size_t place;
+    const int n = ml_chunk(a, place, t0);
     if (n <= 0) return;
-    const size_t place = (size_t)(a.cu_seqlens[b] / ML_TOKENS + b + c);
-    const float* V = a.rows.x + (size_t)t0 * ld + 2 * H * K + h * P + p0;
-    const float* Qh = a.q_rows + (place * H + h) * (size_t)K * ML_TOKENS;
-    const float* S0 = a.own + (place * H + h) * (size_t)P * K + p0;
-    const float* N0 = a.own_n + (place * H + h) * K;
-    const float* scores = a.scores + (place * H + h) * ML_TOKENS * ML_TOKENS;
-    const int state_tiles = (K + ML_ROWS - 1) / ML_ROWS, n_tiles = state_tiles + (n + ML_ROWS - 1) / ML_ROWS;
-    auto copy = [&](int t) {                                        // one commit group a tile, also beyond the last
-        if (t < n_tiles) {
-            const bool from_state = t < state_tiles;
-            const int row0 = (from_state ? t : t - state_tiles) * ML_ROWS, limit = from_state ? K : n;
-            float (*to)[ML_LDA + ML_LDB] = tiles[t % 3];
-#pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                const int r = (tid >> 5) + 4 * i, e = (tid & 31) * 4;
-                const bool ok = row0 + r < limit;
-                rc_copy16(&to[r][e], (from_state ? Qh : scores) + (ok ? (size_t)(row0 + r) * ML_TOKENS + e : 0), ok);
-            }
-#pragma unroll
-            for (int i = 0; i < 2; ++i) {
-                const int r = (tid >> 4) + 8 * i, e = (tid & 15) * 4;
-                const bool ok = row0 + r < limit && p0 + e < P;
-                rc_copy16(&to[r][ML_LDA + e], from_state ? S0 + (ok ? (size_t)(row0 + r) * P + e : 0) : V + (ok ? (size_t)(row0 + r) * ld + e : 0), ok);
-            }
-        }
-        rc_commit();
-    };
-    copy(0);
-    copy(1);
-    ml_gates(a, h, t0, n, w, G, left);
-    auto weigh = [&](int t) {                                       // this thread's token's weights of a tile of tokens, over their scores
-        if (t < state_tiles || t >= n_tiles) return;
-        const int j0 = (t - state_tiles) * ML_ROWS;
-        float* col = &tiles[t % 3][0][tid];
-        if (tid >= j0 && tid < j0 + ML_ROWS) {                      // its own tile
-#pragma unroll
-            for (int r = 0; r < ML_ROWS; ++r)
-                col[r * (ML_LDA + ML_LDB)] = tid >= j0 + r ? col[r * (ML_LDA + ML_LDB)] * (expf((float)(G[tid] - G[j0 + r])) * w[j0 + r]) : 0.f;
-        } else {                                                    // what is left at the tile's end, and what decays behind it
-            const float e = tid > j0 ? expf((float)(G[tid] - G[j0 + ML_ROWS - 1])) : 0.f;
-#pragma unroll
-            for (int r = 0; r < ML_ROWS; ++r) col[r * (ML_LDA + ML_LDB)] = tid > j0 ? col[r * (ML_LDA + ML_LDB)] * (e * left[j0 + r]) : 0.f;
-        }
-    };
-    const int ig = (tid >> 3) * 4, pg = (tid & 7) * 4;              // this thread's tokens ig .., 64 + ig ..; values pg .., 32 + pg ..
-    float acc[8][8], norm = 0.f;                                    // norm: n . q of token tid
-#pragma unroll
-    for (int i = 0; i < 8; ++i)
-#pragma unroll
-        for (int j = 0; j < 8; ++j) acc[i][j] = 0.f;
-    for (int t = 0; t < n_tiles; ++t) {
-        rc_wait<0>();
-        __syncthreads();                                            // tiles t and t + 1 are there (t's rows weighted)
-        copy(t + 2);
-        weigh(t + 1);
-        const float* rows = &tiles[t % 3][0][0];
-        if (t == state_tiles) {                                     // what came from the state fades with the chunk's decays
-#pragma unroll
-            for (int i = 0; i < 8; ++i) {
-                const float f = expf((float)G[(i >> 2) * 64 + ig + (i & 3)]);
-#pragma unroll
-                for (int j = 0; j < 8; ++j) acc[i][j] *= f;
-            }
-            norm *= expf((float)G[tid]);
-        }
-        if (p0 == 0) {
-#pragma unroll
-            for (int r = 0; r < ML_ROWS; ++r) {
-                const float q = rows[r * (ML_LDA + ML_LDB) + tid];
-                norm += t >= state_tiles ? q : (t * ML_ROWS + r < K ? q * N0[t * ML_ROWS + r] : 0.f);
-            }
-        }
-        if (t < state_tiles + 64 / ML_ROWS) {
-            rc_outer<ML_ROWS>(acc, rows, ML_LDA + ML_LDB, ig, 64 + ig, rows + ML_LDA, ML_LDA + ML_LDB, pg, 32 + pg);
-        } else {                                                    // tokens of the chunk's second half: the first half sees nothing
-#pragma unroll 8
-            for (int r = 0; r < ML_ROWS; ++r) {
-                const float* row = rows + r * (ML_LDA + ML_LDB);
-                const float4 x = *reinterpret_cast<const float4*>(row + 64 + ig);
-                const float4 y0 = *reinterpret_cast<const float4*>(row + ML_LDA + pg), y1 = *reinterpret_cast<const float4*>(row + ML_LDA + 32 + pg);
-                const float xv[4] = {x.x, x.y, x.z, x.w}, yv[8] = {y0.x, y0.y, y0.z, y0.w, y1.x, y1.y, y1.z, y1.w};
-#pragma unroll
-                for (int i = 0; i < 4; ++i)
-#pragma unroll
-                    for (int j = 0; j < 8; ++j) acc[4 + i][j] += xv[i] * yv[j];
-            }
-        }
-    }
-#pragma unroll
-    for (int i = 0; i < 8; ++i) {
-        const int t = (i >> 2) * 64 + ig + (i & 3);
-        if (t >= n) continue;
-        float* out = a.raw + ((size_t)(t0 + t) * H + h) * P + p0;
-#pragma unroll
-        for (int half = 0; half < 2; ++half) {
-            const int p = 32 * half + pg;
-            if (p0 + p < P)
-                *reinterpret_cast<float4*>(out + p) = make_float4(acc[i][4 * half] * a.q_scale, acc[i][4 * half + 1] * a.q_scale, acc[i][4 * half + 2] * a.q_scale,
-                                                                  acc[i][4 * half + 3] * a.q_scale);
-        }
-    }
-    if (p0 == 0 && tid < n) {
-        const size_t at = (size_t)(t0 + tid) * H + h;
-        a.divisor[at] = fmaxf(fabsf(norm * a.q_scale), expf(-a.m_run[at])) + a.tiny;
-    }
+    ct_out(ml_rows(a, t0, n, h), a.own + (place * H + h) * (size_t)P * K, a.scores + (place * H + h) * ML_TOKENS * ML_TOKENS, a.gates + place * H + h, 0.f, K, P, p0,
+           p0 == 0 ? a.own_n + (place * H + h) * K : nullptr, a.error,
+           [&](int i, int p, float4 v) {
+               *reinterpret_cast<float4*>(a.raw + ((size_t)(t0 + i) * H + h) * P + p) = make_float4(v.x * a.q_scale, v.y * a.q_scale, v.z * a.q_scale, v.w * a.q_scale);
+           },
+           [&](int i, float v) {
+               const size_t at = (size_t)(t0 + i) * H + h;
+               a.divisor[at] = fmaxf(fabsf(v * a.q_scale), expf(-a.m_run[at])) + a.tiny;
+           });
 }
 
 // ---------------------------------------------------------------------------------
@@ -1018,36 +776,42 @@ extern "C" int qwb_mlstm_chunked(const float* x, int ld, int i_col, int f_col, c
 extern "C" long long qwb_mlstm_tiles_scratch(int T, int B, int H, int K, int P) {
     if (T <= 0 || B <= 0 || H <= 0 || K <= 0 || P <= 0 || K % 4 || P % 4) return 0;
     if ((long long)H * ((P + 63) / 64) * ((K + 127) / 128) + 3LL * H > 65535) return 0;     // more blocks than a grid takes: the other form
-    return ((long long)T / ML_TOKENS + B) * H * ((long long)P * K + K + ML_TOKENS * ML_TOKENS + (long long)K * ML_TOKENS + 1) + 4;
+    return ((long long)T / ML_TOKENS + B) * H * ((long long)P * K + K + ML_TOKENS * ML_TOKENS + CT_GATE_FLOATS + 1) + 4;
 }
 
 // The same step in chunks of 128 tokens, for 16-byte aligned tensors with rows of a multiple of 4 floats; scratch: qwb_mlstm_tiles_scratch floats.
+// *error: set where a kernel's wait ran out.
 extern "C" int qwb_mlstm_tiles(const float* x, int ld, int i_col, int f_col, const float* i_bias, const float* f_bias, float cap, float* state,
                                float* m_state, const int* cu_seqlens, const int* slots, float* gate_rows, float* scratch, float* raw, float* divisor,
-                               int T, int B, int max_new, int H, int K, int P, float q_scale, float tiny, int write_state, cudaStream_t stream) {
+                               int T, int B, int max_new, int H, int K, int P, float q_scale, float tiny, int write_state, int* error, cudaStream_t stream) {
     if (T <= 0 || B <= 0 || max_new <= 0) return 0;
     const MlstmSizes z{H, K, P};
     const MlstmRows rows{x, ld, i_col, f_col};
     const MlstmGates gates{i_bias, f_bias, cap};
     if (int rc = check_mlstm("mlstm_tiles", z, rows, B)) return rc;
     const int chunks = (max_new + ML_TOKENS - 1) / ML_TOKENS, ptiles = (P + 63) / 64, ktiles = (K + 127) / 128;
-    if (!(cap > 0.f) || !gate_rows || !scratch || !qwb_mlstm_tiles_scratch(T, B, H, K, P) || ld % 4)
+    if (!(cap > 0.f) || !gate_rows || !scratch || !error || !qwb_mlstm_tiles_scratch(T, B, H, K, P) || ld % 4)
         return qwb_fail(QWB_ERR_ARG, "mlstm_tiles: cap %g, %d heads of %d x %d in rows of %d", (double)cap, H, K, P, ld);
     if (!mlstm_aligned(x) || !mlstm_aligned(scratch) || !mlstm_aligned(raw)) return qwb_fail(QWB_ERR_ARG, "mlstm_tiles: a tensor is not 16-byte aligned");
     float *log_decay = gate_rows, *write = gate_rows + (size_t)T * H, *m_run = gate_rows + 2 * (size_t)T * H;
     qwb_launch(mlstm_gates_kernel, dim3(H, B), mlstm_gate_threads(T), 0, stream, rows, gates, (const float*)m_state, cu_seqlens, slots, log_decay, write, m_run, H, P);
     if (int rc = qwb_check_launch("mlstm_gates")) return rc;
     const size_t heads = ((size_t)T / ML_TOKENS + B) * H;
-    MlArgs a = {rows, log_decay, write, m_run, cu_seqlens, slots, state, m_state, scratch, nullptr, nullptr, nullptr, nullptr, raw, divisor, z, q_scale, tiny, write_state};
+    MlArgs a = {rows, log_decay, write, m_run, cu_seqlens, slots, state, m_state, scratch, nullptr, nullptr, nullptr, raw, divisor, nullptr, error, z, q_scale, tiny, write_state};
     a.scores = a.own + heads * P * K;
-    a.q_rows = a.scores + heads * ML_TOKENS * ML_TOKENS;
-    a.own_n = a.q_rows + heads * K * ML_TOKENS;
+    a.gates = reinterpret_cast<CtGates*>(a.scores + heads * ML_TOKENS * ML_TOKENS);
+    a.own_n = reinterpret_cast<float*>(a.gates + heads);
     a.totals = a.own_n + heads * K;
-    qwb_launch(mlstm_tile_state_kernel, dim3(chunks, H * ptiles * ktiles + 3 * H, B), 128, 0, stream, a, ptiles, ktiles);
+    cudaError_t e = cudaFuncSetAttribute(mlstm_tile_state_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, CT_SMEM);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(mlstm_tile_out_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, CT_SMEM);
+    if (e != cudaSuccess) return qwb_fail(QWB_ERR_CUDA, "mlstm_tiles: %s", cudaGetErrorString(e));
+    qwb_launch(mlstm_tile_gates_kernel, dim3(chunks, H, B), 1024, 0, stream, a);
+    if (int rc = qwb_check_launch("mlstm_tile_gates")) return rc;
+    qwb_launch(mlstm_tile_state_kernel, dim3(chunks, 2 * H + H * ptiles * ktiles, B), CT_THREADS, CT_SMEM, stream, a, ptiles, ktiles);
     if (int rc = qwb_check_launch("mlstm_tile_state")) return rc;
-    const int ctiles = (P + 31) / 32, matrix_tiles = (K + 31) / 32 * ctiles;
-    qwb_launch(mlstm_tile_carry_kernel, dim3(matrix_tiles + (K + 255) / 256, H, B), 256, 0, stream, a, ctiles, matrix_tiles);
+    const int matrix_blocks = (K * (P / 4) + 255) / 256;
+    qwb_launch(mlstm_tile_carry_kernel, dim3(matrix_blocks + (K + 255) / 256, H, B), 256, 0, stream, a, matrix_blocks);
     if (int rc = qwb_check_launch("mlstm_tile_carry")) return rc;
-    qwb_launch(mlstm_tile_out_kernel, dim3(chunks, H * ptiles, B), 128, 0, stream, a, ptiles);
+    qwb_launch(mlstm_tile_out_kernel, dim3(chunks, H * ptiles, B), CT_THREADS, CT_SMEM, stream, a, ptiles);
     return qwb_check_launch("mlstm_tile_out");
 }

@@ -1,362 +1,115 @@
 // Long prompts through the recurrences of recurrent.cu in chunks: inside a chunk the tokens meet in small matrix products,
-// from chunk to chunk only the state is carried.  Everything is 32-bit, in plain multiply-adds: the tensor cores have no product
-// of 32-bit operands, and six products of bfloat16 parts in place of one, at mma.sync's rate 92 TFLOP/s (554 / 6) against 72, would
-// gain little once the parts are made; on tcgen05 they would be faster, which is not written.  Decays enter as sums of their
+// from chunk to chunk only the state is carried.  Everything is 32-bit: Mamba-2's products on the tensor cores as sums of products of
+// bfloat16 parts (chunk_tc.cuh), the delta rule's in plain multiply-adds.  Decays enter as sums of their
 // logarithms, always of tokens between two others, so every exponential is of a number that is at most 0: nothing overflows, and
 // what underflows is below the smallest float in truth too.
-#include "chunks.cuh"
+#include "chunk_tc.cuh"
 
 // ---------------------------------------------------------------------------------
 // Mamba-2 in chunks of 128 tokens.  With G_i the sum of a head's log decays (a dt) in the chunk up to token i and S0 the state
 // at its start,
 //     y_i   = e^(G_i) S0 C_i + sum_{j <= i} e^(G_i - G_j) dt_j (C_i . B_j) x_j + D x_i
 //     S_end = e^(G_end) S0 + sum_j e^(G_end - G_j) dt_j x_j B_j^T
-// Three kernels: every chunk's own sum of outer products, and, in the same launch, the products C_i . B_j, which the heads of a
-// group share; the carries, which run through a sequence's chunks and replace each sum by the state that its chunk starts from;
-// the outputs.  A thread keeps 8 x 8 sums: four 16-byte loads from shared memory for 64 multiply-adds.  Tiles of 16 rows come
-// by cp.async in three stages: while one is multiplied, the next one's rows are weighted in place and the one after is on its
-// way, with one barrier a tile.  Scratch memory holds states and C row by row as the tiles want them (a state's row is a key
-// row here), so that nothing is transposed on the way to a tile.
+// Four kernels on chunk_tc.cuh: the gates; every chunk's own sum of outer products and, in the same launch, the products C_i . B_j,
+// which the heads of a group share; the carries; the outputs.
 // A step's sequences of at least `from` tokens go through these kernels, the others through the scan.  Chunk c of the z-th of them,
 // b, is place cu_seqlens[b] / 128 + z + c of the scratch memory, which T / 128 and one for each of them hold:
-//     own / starts [places, H, N, P], total decays [places, H], products [places, G, 128 (j), 128 (i)], C [places, G, N, 128 (i)]
-// The sums of logarithms are 64-bit (only their differences are used).  64 heads of 64 x 128 in 8 groups, with
-// the convolution before it, the scan and now: 2,048 tokens 902 -> 222 us (85 + 14 + 113 us in ncu; the FMA pipe at 44 and 50 %,
-// issue slots at 57 and 65 %), 4,096 tokens 1,804 -> 428 us, four sequences of 3,000 in all 1,115 -> 351 us.
+//     own / starts [places, H, P / 4, N, 4], products [places, G, 32, 128 (i), 4 (j)], gates [places, H], total decays [places, H]
+// The sums of logarithms are 64-bit (only their differences are used).  64 heads of 64 x 128 in 8 groups, 2,048 tokens, us: gates 5,
+// state 39, carries 13, outputs 60; with the convolution before it 153 where 8 x 8 sums a thread in plain multiply-adds took 233 (state 81,
+// carries 10, outputs 107: bound by what shared memory hands to registers).  Error against 64 bits 1.2e-7 as before.
 // ---------------------------------------------------------------------------------
-#define SC_TOKENS 128
-#define SC_ROWS 16                      // rows of a tile
-#define SC_LDA 132
-#define SC_LDB 68
+#define SC_TOKENS CT_TOKENS
 #define SC_FORGETS -128.f               // the exponential of this is 0 in 32-bit: a log decay below (-infinity too) counts as this much,
                                         // so that differences of sums are numbers and keep the digits of the other tokens' decays
 
 struct ScArgs {
     const float *xbc, *dt_raw, *dt_bias, *A_log, *D;
     const int *cu_seqlens, *slots;
-    float *state, *y, *own, *totals, *products, *c_rows;
+    float *state, *y, *own, *products, *totals;
+    CtGates* gates;
+    int* error;
     int ldx, ld_dt, H, P, N, G, write_state, B, from;
 };
 
-// this head's step sizes [128], sums of log decays [128] and, if wanted, decays [128] (beyond the chunk's n tokens: 0, the last
-// sum, 1); the caller synchronises
-__device__ __forceinline__ void sc_steps(const ScArgs& a, int h, int t0, int n, float* dt, double* G, float* decay = nullptr) {
-    const int lane = threadIdx.x;
-    if (lane >= 32) return;
-    const float rate = -expf(a.A_log[h]), bias = a.dt_bias[h];
-    double own[4], sum = 0.0;
-#pragma unroll
-    for (int e = 0; e < 4; ++e) {
-        const int i = 4 * lane + e;
-        const float d = i < n ? rc_softplus(a.dt_raw[(size_t)(t0 + i) * a.ld_dt + h] + bias) : 0.f;
-        dt[i] = d;
-        const float fade = i < n ? rate * d : 0.f;
-        if (decay) decay[i] = expf(fade);
-        sum += (double)(fade < SC_FORGETS ? SC_FORGETS : fade);
-        own[e] = sum;
-    }
-    double run = sum;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const double up = __shfl_up_sync(0xffffffffu, run, o);
-        if (lane >= o) run += up;
-    }
-    const double before = run - sum;
-#pragma unroll
-    for (int e = 0; e < 4; ++e) G[4 * lane + e] = before + own[e];
+// a chunk's place, first token and tokens (0: none)
+__device__ __forceinline__ int sc_chunk(const ScArgs& a, size_t& place, int& t0) {
+    const int b = rc_sequence(a.cu_seqlens, a.B, a.from, blockIdx.z), c = blockIdx.x;
+    if (b < 0) return 0;
+    t0 = a.cu_seqlens[b] + c * SC_TOKENS;
+    place = (size_t)(a.cu_seqlens[b] / SC_TOKENS + blockIdx.z + c);
+    return min(SC_TOKENS, a.cu_seqlens[b + 1] - t0);
+}
+__device__ __forceinline__ CtRows sc_rows(const ScArgs& a, int t0, int n, int h, int g) {
+    const float *x = a.xbc + (size_t)t0 * a.ldx, *bs = x + a.H * a.P + g * a.N;
+    return {bs + a.G * a.N, bs, x + h * a.P, a.ldx, n};
 }
 
-// grid (chunks, H * ptiles * ntiles + 3 G, B), 128 threads.  A state block makes 64 values (p) x 128 state rows (n); a product
-// block one of the three 64 x 64 quarters with j <= i of a group's products.
-__global__ void __launch_bounds__(128)
+// grid (chunks, H, B), 128 threads
+__global__ void __launch_bounds__(SC_TOKENS)
+ssm_chunk_gates_kernel(const ScArgs a) {
+    pdl_wait();
+    pdl_launch_dependents();
+    __shared__ float coef[SC_TOKENS];
+    int t0;
+    size_t place;
+    const int n = sc_chunk(a, place, t0), h = blockIdx.y, i = threadIdx.x;
+    if (n <= 0) return;
+    float dt = 0.f, fade = 0.f;
+    if (i < n) {
+        dt = rc_softplus(a.dt_raw[(size_t)(t0 + i) * a.ld_dt + h] + a.dt_bias[h]);
+        fade = -expf(a.A_log[h]) * dt;
+        if (fade < SC_FORGETS) fade = SC_FORGETS;
+    }
+    ct_gates(fade, dt, a.gates + place * a.H + h, a.totals + place * a.H + h, coef);
+}
+
+// grid (chunks, 2 G + H * ptiles * ntiles, B): the products of a group's chunk with 64 of its tokens, or 64 values x 128 state rows of a head's own sum
+__global__ void __launch_bounds__(CT_THREADS, 2)
 ssm_chunk_state_kernel(const ScArgs a, int ptiles, int ntiles) {
     pdl_wait();
     pdl_launch_dependents();
-    constexpr int KB = 32;                                          // state rows of a tile of the products
-    __shared__ __align__(16) float tiles[3][SC_ROWS][SC_LDA + SC_LDB];
-    __shared__ float dt[SC_TOKENS], coef[SC_TOKENS];
-    __shared__ double G[SC_TOKENS];
-    const int c = blockIdx.x, b = rc_sequence(a.cu_seqlens, a.B, a.from, blockIdx.z), tid = threadIdx.x;
-    if (b < 0) return;
-    const int t0 = a.cu_seqlens[b] + c * SC_TOKENS, n = min(SC_TOKENS, a.cu_seqlens[b + 1] - t0);
+    int t0;
+    size_t place;
+    const int n = sc_chunk(a, place, t0), i = (int)blockIdx.y - 2 * a.G;
     if (n <= 0) return;
-    const size_t place = (size_t)(a.cu_seqlens[b] / SC_TOKENS + blockIdx.z + c);
-    const int inner = a.H * a.P;
-    float acc[8][8];
-#pragma unroll
-    for (int i = 0; i < 8; ++i)
-#pragma unroll
-        for (int j = 0; j < 8; ++j) acc[i][j] = 0.f;
-
-    const int n_state = a.H * ptiles * ntiles;
-    if ((int)blockIdx.y >= n_state) {                               // products
-        const int g = ((int)blockIdx.y - n_state) / 3, quarter = ((int)blockIdx.y - n_state) % 3;
-        const int i0 = quarter == 0 ? 0 : 64, j0 = quarter == 2 ? 64 : 0;
-        if (i0 >= n) return;
-        float (*As)[68] = reinterpret_cast<float (*)[68]>(&tiles[0][0][0]), (*Bs)[68] = As + KB;
-        const float* Bg = a.xbc + (size_t)t0 * a.ldx + inner + g * a.N;
-        const float* Cg = Bg + a.G * a.N;
-        // 64 (i) x 64 (j) by 128 threads: i groups of 8 (tid >> 4), j groups of 4 (tid & 15)
-        const int ig = (tid >> 4) * 4, jg = (tid & 15) * 4;
-        for (int k0 = 0; k0 < a.N; k0 += KB) {
-            __syncthreads();
-            for (int idx = tid; idx < 64 * (KB / 4); idx += 128) {  // lanes walk tokens: the transposed stores do not collide
-                const int i = idx & 63, k = (idx >> 6) * 4;
-                const float4 cv = rc_load4(Cg + (size_t)(i0 + i) * a.ldx + k0 + k, i0 + i < n && k0 + k < a.N);
-                const float4 bv = rc_load4(Bg + (size_t)(j0 + i) * a.ldx + k0 + k, j0 + i < n && k0 + k < a.N);
-                As[k][i] = cv.x; As[k + 1][i] = cv.y; As[k + 2][i] = cv.z; As[k + 3][i] = cv.w;
-                Bs[k][i] = bv.x; Bs[k + 1][i] = bv.y; Bs[k + 2][i] = bv.z; Bs[k + 3][i] = bv.w;
-            }
-            __syncthreads();
-            if (quarter < 2)                                        // C, a state row a row, for the output blocks
-                for (int idx = tid; idx < KB * 16; idx += 128) {
-                    const int k = idx >> 4, e = (idx & 15) * 4;
-                    if (k0 + k < a.N)
-                        *reinterpret_cast<float4*>(a.c_rows + ((place * a.G + g) * a.N + k0 + k) * SC_TOKENS + i0 + e) = *reinterpret_cast<const float4*>(&As[k][e]);
-                }
-#pragma unroll 8
-            for (int k = 0; k < KB; ++k) {
-                const float4 x0 = *reinterpret_cast<const float4*>(&As[k][ig]), x1 = *reinterpret_cast<const float4*>(&As[k][32 + ig]);
-                const float4 y = *reinterpret_cast<const float4*>(&Bs[k][jg]);
-                const float xv[8] = {x0.x, x0.y, x0.z, x0.w, x1.x, x1.y, x1.z, x1.w}, yv[4] = {y.x, y.y, y.z, y.w};
-#pragma unroll
-                for (int i = 0; i < 8; ++i)
-#pragma unroll
-                    for (int j = 0; j < 4; ++j) acc[i][j] += xv[i] * yv[j];
-            }
-        }
-        float* out = a.products + (place * a.G + g) * SC_TOKENS * SC_TOKENS;
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            float* row = out + (size_t)(j0 + jg + j) * SC_TOKENS + i0;
-            *reinterpret_cast<float4*>(row + ig) = make_float4(acc[0][j], acc[1][j], acc[2][j], acc[3][j]);
-            *reinterpret_cast<float4*>(row + 32 + ig) = make_float4(acc[4][j], acc[5][j], acc[6][j], acc[7][j]);
-        }
+    if (i < 0) {
+        const int g = blockIdx.y / 2, j0 = blockIdx.y % 2 * 64;
+        if (j0 < n) ct_pairs(sc_rows(a, t0, n, 0, g), a.N, j0, a.products + (place * a.G + g) * SC_TOKENS * SC_TOKENS, a.error);
         return;
     }
-    const int h = blockIdx.y / (ptiles * ntiles), tile = blockIdx.y - h * ptiles * ntiles, p0 = tile / ntiles * 64, n0 = tile % ntiles * 128;
-    sc_steps(a, h, t0, n, dt, G);
-    __syncthreads();
-    coef[tid] = expf((float)(G[SC_TOKENS - 1] - G[tid])) * dt[tid];
-    if (tid == 0 && tile == 0) a.totals[place * a.H + h] = expf((float)G[SC_TOKENS - 1]);
-    const float* X = a.xbc + (size_t)t0 * a.ldx + h * a.P + p0;
-    const float* Bh = a.xbc + (size_t)t0 * a.ldx + inner + (h / (a.H / a.G)) * a.N + n0;
-    const int pg = (tid >> 4) * 4, ng = (tid & 15) * 4;
-    const int n_tiles = (n + SC_ROWS - 1) / SC_ROWS;
-    auto copy = [&](int t) {                                        // one commit group a tile, also beyond the last
-        if (t < n_tiles) {
-            float (*tile_rows)[SC_LDA + SC_LDB] = tiles[t % 3];
-#pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                const int r = (tid >> 5) + 4 * i, e = (tid & 31) * 4, j = t * SC_ROWS + r;
-                const bool ok = j < n && n0 + e < a.N;
-                rc_copy16(&tile_rows[r][e], Bh + (ok ? (size_t)j * a.ldx + e : 0), ok);
-            }
-#pragma unroll
-            for (int i = 0; i < 2; ++i) {
-                const int r = (tid >> 4) + 8 * i, e = (tid & 15) * 4, j = t * SC_ROWS + r;
-                const bool ok = j < n && p0 + e < a.P;
-                rc_copy16(&tile_rows[r][SC_LDA + e], X + (ok ? (size_t)j * a.ldx + e : 0), ok);
-            }
-        }
-        rc_commit();
-    };
-    auto weigh = [&](int t) {                                       // the values by their tokens' write strengths up to the chunk's end
-        if (t >= n_tiles) return;
-#pragma unroll
-        for (int i = 0; i < 2; ++i) {
-            const int r = (tid >> 4) + 8 * i;
-            float4* v = reinterpret_cast<float4*>(&tiles[t % 3][r][SC_LDA + (tid & 15) * 4]);
-            const float f = coef[t * SC_ROWS + r];
-            const float4 x = *v;
-            *v = make_float4(f * x.x, f * x.y, f * x.z, f * x.w);
-        }
-    };
-    copy(0);
-    copy(1);
-    rc_wait<1>();
-    __syncthreads();                                                // the write strengths are there too
-    weigh(0);
-    for (int t = 0; t < n_tiles; ++t) {
-        rc_wait<0>();                                               // tile t + 1
-        __syncthreads();
-        copy(t + 2);
-        weigh(t + 1);
-        const float* rows = &tiles[t % 3][0][0];
-        rc_outer<SC_ROWS>(acc, rows, SC_LDA + SC_LDB, ng, 64 + ng, rows + SC_LDA, SC_LDA + SC_LDB, pg, 32 + pg);
-    }
-    float* U = a.own + (place * a.H + h) * (size_t)a.P * a.N;
-#pragma unroll
-    for (int i = 0; i < 8; ++i) {
-        const int m = n0 + (i >> 2) * 64 + ng + (i & 3);
-        if (m >= a.N) continue;
-#pragma unroll
-        for (int half = 0; half < 2; ++half) {
-            const int p = p0 + 32 * half + pg;
-            if (p < a.P) *reinterpret_cast<float4*>(U + (size_t)m * a.P + p) = make_float4(acc[i][4 * half], acc[i][4 * half + 1], acc[i][4 * half + 2], acc[i][4 * half + 3]);
-        }
-    }
+    const int h = i / (ptiles * ntiles), tile = i - h * ptiles * ntiles;
+    ct_state(sc_rows(a, t0, n, h, h / (a.H / a.G)), a.gates + place * a.H + h, a.N, a.P, tile % ntiles * 128, tile / ntiles * 64,
+             a.own + (place * a.H + h) * (size_t)a.P * a.N, a.error);
 }
 
-// grid (tiles of 32 state rows x 32 values, H, B), 256 threads: four neighbouring values of a state row a thread, through the
-// sequence's chunks in order.  The state itself lies column by column and is turned in shared memory.
-__global__ void __launch_bounds__(256)
-ssm_chunk_carry_kernel(const ScArgs a, int ptiles) {
+// grid (N * P / 1,024, H, B)
+__global__ void __launch_bounds__(256, 4)
+ssm_chunk_carry_kernel(const ScArgs a) {
     pdl_wait();
     pdl_launch_dependents();
-    constexpr int AHEAD = 8;
-    __shared__ float turn[32][33];
     const int h = blockIdx.y, b = rc_sequence(a.cu_seqlens, a.B, a.from, blockIdx.z);
     if (b < 0) return;
     const int t0 = a.cu_seqlens[b], n = a.cu_seqlens[b + 1] - t0;
     if (n <= 0) return;
-    const int n0 = blockIdx.x / ptiles * 32, p0 = blockIdx.x % ptiles * 32, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const size_t size = (size_t)a.P * a.N;
-    float* S = a.state + ((size_t)a.slots[b] * a.H + h) * size;
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        const int p = warp + 8 * i;
-        turn[p][lane] = p0 + p < a.P && n0 + lane < a.N ? S[(size_t)(p0 + p) * a.N + n0 + lane] : 0.f;
-    }
-    __syncthreads();
-    const int row = threadIdx.x >> 3, p = (threadIdx.x & 7) * 4;
-    float4 s = make_float4(turn[p][row], turn[p + 1][row], turn[p + 2][row], turn[p + 3][row]);
-    if (n0 + row < a.N && p0 + p < a.P) {
-        const int chunks = (n + SC_TOKENS - 1) / SC_TOKENS;
-        const size_t place = (size_t)(t0 / SC_TOKENS + blockIdx.z), step = (size_t)a.H * size;
-        float* at = a.own + (place * a.H + h) * size + (size_t)(n0 + row) * a.P + p0 + p;
-        const float* total = a.totals + place * a.H + h;
-        for (int c0 = 0; c0 < chunks; c0 += AHEAD) {
-            float4 u[AHEAD];
-            float d[AHEAD];
-#pragma unroll
-            for (int i = 0; i < AHEAD; ++i)
-                if (c0 + i < chunks) { u[i] = *reinterpret_cast<const float4*>(at + (c0 + i) * step); d[i] = total[(size_t)(c0 + i) * a.H]; }
-#pragma unroll
-            for (int i = 0; i < AHEAD; ++i)
-                if (c0 + i < chunks) {
-                    *reinterpret_cast<float4*>(at + (c0 + i) * step) = s;
-                    s = make_float4(d[i] * s.x + u[i].x, d[i] * s.y + u[i].y, d[i] * s.z + u[i].z, d[i] * s.w + u[i].w);
-                }
-        }
-    }
-    if (!a.write_state) return;
-    turn[p][row] = s.x; turn[p + 1][row] = s.y; turn[p + 2][row] = s.z; turn[p + 3][row] = s.w;
-    __syncthreads();
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        const int q = warp + 8 * i;
-        if (p0 + q < a.P && n0 + lane < a.N) S[(size_t)(p0 + q) * a.N + n0 + lane] = turn[q][lane];
-    }
+    const size_t place = (size_t)(t0 / SC_TOKENS + blockIdx.z), size = (size_t)a.P * a.N;
+    ct_carry(a.own + (place * a.H + h) * size, a.H * size, a.totals + place * a.H + h, a.H, (n + SC_TOKENS - 1) / SC_TOKENS,
+             a.state + ((size_t)a.slots[b] * a.H + h) * size, a.N, a.P, blockIdx.x * 256 + threadIdx.x, a.write_state);
 }
 
-// grid (chunks, H * ptiles, B), 128 threads: a chunk's 128 tokens x 64 values.  A thread weighs its token's products with a
-// tile of tokens j, e^(G_i - G_j) dt_j, from the tile's last token to its first: one exponential, then a decay a token.
-__global__ void __launch_bounds__(128, 4)
+// grid (chunks, H * ptiles, B): a chunk's 128 tokens x 64 values
+__global__ void __launch_bounds__(CT_THREADS, 2)
 ssm_chunk_out_kernel(const ScArgs a, int ptiles) {
     pdl_wait();
     pdl_launch_dependents();
-    __shared__ __align__(16) float tiles[3][SC_ROWS][SC_LDA + SC_LDB];
-    __shared__ float dt[SC_TOKENS], decay[SC_TOKENS];
-    __shared__ double G[SC_TOKENS];
-    const int c = blockIdx.x, b = rc_sequence(a.cu_seqlens, a.B, a.from, blockIdx.z), tid = threadIdx.x;
-    const int h = blockIdx.y / ptiles, p0 = (blockIdx.y - h * ptiles) * 64;
-    if (b < 0) return;
-    const int t0 = a.cu_seqlens[b] + c * SC_TOKENS, n = min(SC_TOKENS, a.cu_seqlens[b + 1] - t0);
+    int t0;
+    size_t place;
+    const int n = sc_chunk(a, place, t0), h = blockIdx.y / ptiles, p0 = (blockIdx.y - h * ptiles) * 64, g = h / (a.H / a.G);
     if (n <= 0) return;
-    const size_t place = (size_t)(a.cu_seqlens[b] / SC_TOKENS + blockIdx.z + c);
-    const int inner = a.H * a.P, g = h / (a.H / a.G);
-    const float* X = a.xbc + (size_t)t0 * a.ldx + h * a.P + p0;
-    const float* Cg = a.c_rows + (place * a.G + g) * (size_t)a.N * SC_TOKENS;
-    const float* S0 = a.own + (place * a.H + h) * (size_t)a.P * a.N + p0;
-    const float* products = a.products + (place * a.G + g) * SC_TOKENS * SC_TOKENS;
-    const int state_tiles = (a.N + SC_ROWS - 1) / SC_ROWS, n_tiles = state_tiles + (n + SC_ROWS - 1) / SC_ROWS;
-    auto copy = [&](int t) {                                        // one commit group a tile, also beyond the last
-        if (t < n_tiles) {
-            const bool from_state = t < state_tiles;
-            const int row0 = (from_state ? t : t - state_tiles) * SC_ROWS, limit = from_state ? a.N : n;
-            float (*tile_rows)[SC_LDA + SC_LDB] = tiles[t % 3];
-#pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                const int r = (tid >> 5) + 4 * i, e = (tid & 31) * 4;
-                const bool ok = row0 + r < limit;
-                rc_copy16(&tile_rows[r][e], (from_state ? Cg : products) + (ok ? (size_t)(row0 + r) * SC_TOKENS + e : 0), ok);
-            }
-#pragma unroll
-            for (int i = 0; i < 2; ++i) {
-                const int r = (tid >> 4) + 8 * i, e = (tid & 15) * 4;
-                const bool ok = row0 + r < limit && p0 + e < a.P;
-                rc_copy16(&tile_rows[r][SC_LDA + e], from_state ? S0 + (ok ? (size_t)(row0 + r) * a.P + e : 0) : X + (ok ? (size_t)(row0 + r) * a.ldx + e : 0), ok);
-            }
-        }
-        rc_commit();
-    };
-    copy(0);
-    copy(1);
-    sc_steps(a, h, t0, n, dt, G, decay);
-    auto weigh = [&](int t) {                                       // this thread's token's weights of a tile of tokens, over their products
-        if (t < state_tiles || t >= n_tiles) return;
-        const int j0 = (t - state_tiles) * SC_ROWS;
-        float* col = &tiles[t % 3][0][tid];
-        float e = tid >= j0 + SC_ROWS ? expf((float)(G[tid] - G[j0 + SC_ROWS - 1])) : 0.f;
-#pragma unroll
-        for (int r = SC_ROWS - 1; r >= 0; --r) {
-            if (r < SC_ROWS - 1) e *= decay[j0 + r + 1];
-            if (tid == j0 + r) e = 1.f;
-            col[r * (SC_LDA + SC_LDB)] = tid >= j0 + r ? col[r * (SC_LDA + SC_LDB)] * (e * dt[j0 + r]) : 0.f;
-        }
-    };
-    const int ig = (tid >> 3) * 4, pg = (tid & 7) * 4;              // this thread's tokens ig .., 64 + ig ..; values pg .., 32 + pg ..
-    float acc[8][8];
-#pragma unroll
-    for (int i = 0; i < 8; ++i)
-#pragma unroll
-        for (int j = 0; j < 8; ++j) acc[i][j] = 0.f;
-    for (int t = 0; t < n_tiles; ++t) {
-        rc_wait<0>();
-        __syncthreads();                                            // tiles t and t + 1 are there (t's rows weighted)
-        copy(t + 2);
-        weigh(t + 1);
-        const float* rows = &tiles[t % 3][0][0];
-        if (t == state_tiles) {                                     // what came from the state fades with the chunk's decays
-#pragma unroll
-            for (int i = 0; i < 8; ++i) {
-                const float f = expf((float)G[(i >> 2) * 64 + ig + (i & 3)]);
-#pragma unroll
-                for (int j = 0; j < 8; ++j) acc[i][j] *= f;
-            }
-        }
-        if (t < state_tiles + 64 / SC_ROWS) {
-            rc_outer<SC_ROWS>(acc, rows, SC_LDA + SC_LDB, ig, 64 + ig, rows + SC_LDA, SC_LDA + SC_LDB, pg, 32 + pg);
-        } else {                                                    // tokens of the chunk's second half: the first half sees nothing
-#pragma unroll 8
-            for (int r = 0; r < SC_ROWS; ++r) {
-                const float* row = rows + r * (SC_LDA + SC_LDB);
-                const float4 x = *reinterpret_cast<const float4*>(row + 64 + ig);
-                const float4 y0 = *reinterpret_cast<const float4*>(row + SC_LDA + pg), y1 = *reinterpret_cast<const float4*>(row + SC_LDA + 32 + pg);
-                const float xv[4] = {x.x, x.y, x.z, x.w}, yv[8] = {y0.x, y0.y, y0.z, y0.w, y1.x, y1.y, y1.z, y1.w};
-#pragma unroll
-                for (int i = 0; i < 4; ++i)
-#pragma unroll
-                    for (int j = 0; j < 8; ++j) acc[4 + i][j] += xv[i] * yv[j];
-            }
-        }
-    }
-    const float skip = a.D[h];
-#pragma unroll
-    for (int i = 0; i < 8; ++i) {
-        const int t = (i >> 2) * 64 + ig + (i & 3);
-        if (t >= n) continue;
-        float* out = a.y + (size_t)(t0 + t) * inner + h * a.P + p0;
-#pragma unroll
-        for (int half = 0; half < 2; ++half) {
-            const int p = 32 * half + pg;
-            if (p0 + p >= a.P) continue;
-            const float4 x = *reinterpret_cast<const float4*>(X + (size_t)t * a.ldx + p);
-            *reinterpret_cast<float4*>(out + p) = make_float4(acc[i][4 * half] + skip * x.x, acc[i][4 * half + 1] + skip * x.y,
-                                                              acc[i][4 * half + 2] + skip * x.z, acc[i][4 * half + 3] + skip * x.w);
-        }
-    }
+    const CtRows rows = sc_rows(a, t0, n, h, g);
+    float* y = a.y + (size_t)t0 * a.H * a.P + h * a.P;
+    ct_out(rows, a.own + (place * a.H + h) * (size_t)a.P * a.N, a.products + (place * a.G + g) * SC_TOKENS * SC_TOKENS, a.gates + place * a.H + h, a.D[h], a.N, a.P,
+           p0, nullptr, a.error, [&](int i, int p, float4 v) { *reinterpret_cast<float4*>(y + (size_t)i * a.H * a.P + p) = v; }, [](int, float) {});
 }
 
 // Floats of scratch that qwb_ssm_chunked needs; 0: these sizes are not taken (more than a grid holds, or states that the scan refuses).
@@ -364,32 +117,36 @@ ssm_chunk_out_kernel(const ScArgs a, int ptiles) {
 extern "C" long long qwb_ssm_chunked_scratch(int T, int B, int from, int H, int P, int N, int G) {
     if (T <= 0 || B <= 0 || H <= 0 || P <= 0 || N <= 0 || G <= 0 || H % G || P % 4 || N % 4 || N > SC_MAX_N) return 0;
     if (B > 65535 || (long long)H * ((P + 63) / 64) * ((N + 127) / 128) + 3LL * G > 65535) return 0;
-    return ((long long)T / SC_TOKENS + rc_planes(T, B, from)) * ((long long)H * P * N + H + (long long)G * SC_TOKENS * (SC_TOKENS + N)) + 4;
+    return ((long long)T / SC_TOKENS + rc_planes(T, B, from)) * ((long long)H * ((long long)P * N + CT_GATE_FLOATS + 1) + (long long)G * SC_TOKENS * SC_TOKENS) + 4;
 }
 
 // The same step as qwb_ssm_scan for the sequences that bring at least `from` tokens (0: all), for 16-byte aligned tensors with rows of a
-// multiple of 4 floats.
+// multiple of 4 floats.  *error: set where a kernel's wait ran out.
 extern "C" int qwb_ssm_chunked(const float* xbc, int ldx, const float* dt_raw, int ld_dt, const float* dt_bias, const float* A_log, const float* D,
                                float* state, const int* cu_seqlens, const int* slots, float* y, float* scratch, int T, int B, int max_new, int from, int H, int P,
-                               int N, int G, int write_state, cudaStream_t stream) {
+                               int N, int G, int write_state, int* error, cudaStream_t stream) {
     if (T <= 0 || B <= 0 || max_new <= 0 || max_new < from) return 0;
-    if (!qwb_ssm_chunked_scratch(T, B, from, H, P, N, G) || ldx % 4 || ldx < H * P + 2 * G * N || ld_dt < H)
+    if (!qwb_ssm_chunked_scratch(T, B, from, H, P, N, G) || ldx % 4 || ldx < H * P + 2 * G * N || ld_dt < H || !error)
         return qwb_fail(QWB_ERR_ARG, "ssm_chunked: %d heads, %d groups, state %d x %d in rows of %d", H, G, N, P, ldx);
     for (const void* p : {(const void*)xbc, (const void*)state, (const void*)y, (const void*)scratch})
         if (!p || !rc_aligned16(p)) return qwb_fail(QWB_ERR_ARG, "ssm_chunked: a tensor is not 16-byte aligned");
     const int chunks = (max_new + SC_TOKENS - 1) / SC_TOKENS, ptiles = (P + 63) / 64, ntiles = (N + 127) / 128, planes = rc_planes(T, B, from);
     const size_t places = (size_t)T / SC_TOKENS + planes;
-    ScArgs a = {xbc, dt_raw, dt_bias, A_log, D, cu_seqlens, slots, state, y, nullptr, nullptr, nullptr, nullptr, ldx, ld_dt, H, P, N, G, write_state, B, from};
+    ScArgs a = {xbc, dt_raw, dt_bias, A_log, D, cu_seqlens, slots, state, y, nullptr, nullptr, nullptr, nullptr, error, ldx, ld_dt, H, P, N, G, write_state, B, from};
     a.own = scratch;
     a.products = a.own + places * H * P * N;
-    a.c_rows = a.products + places * G * SC_TOKENS * SC_TOKENS;
-    a.totals = a.c_rows + places * G * N * SC_TOKENS;
-    qwb_launch(ssm_chunk_state_kernel, dim3(chunks, H * ptiles * ntiles + 3 * G, planes), 128, 0, stream, a, ptiles, ntiles);
+    a.gates = reinterpret_cast<CtGates*>(a.products + places * G * SC_TOKENS * SC_TOKENS);
+    a.totals = reinterpret_cast<float*>(a.gates + places * H);
+    cudaError_t e = cudaFuncSetAttribute(ssm_chunk_state_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, CT_SMEM);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(ssm_chunk_out_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, CT_SMEM);
+    if (e != cudaSuccess) return qwb_fail(QWB_ERR_CUDA, "ssm_chunked: %s", cudaGetErrorString(e));
+    qwb_launch(ssm_chunk_gates_kernel, dim3(chunks, H, planes), SC_TOKENS, 0, stream, a);
+    if (int rc = qwb_check_launch("ssm_chunk_gates")) return rc;
+    qwb_launch(ssm_chunk_state_kernel, dim3(chunks, 2 * G + H * ptiles * ntiles, planes), CT_THREADS, CT_SMEM, stream, a, ptiles, ntiles);
     if (int rc = qwb_check_launch("ssm_chunk_state")) return rc;
-    const int carry_p = (P + 31) / 32;
-    qwb_launch(ssm_chunk_carry_kernel, dim3((N + 31) / 32 * carry_p, H, planes), 256, 0, stream, a, carry_p);
+    qwb_launch(ssm_chunk_carry_kernel, dim3((N * (P / 4) + 255) / 256, H, planes), 256, 0, stream, a);
     if (int rc = qwb_check_launch("ssm_chunk_carry")) return rc;
-    qwb_launch(ssm_chunk_out_kernel, dim3(chunks, H * ptiles, planes), 128, 0, stream, a, ptiles);
+    qwb_launch(ssm_chunk_out_kernel, dim3(chunks, H * ptiles, planes), CT_THREADS, CT_SMEM, stream, a, ptiles);
     return qwb_check_launch("ssm_chunk_out");
 }
 

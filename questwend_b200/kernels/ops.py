@@ -943,7 +943,7 @@ def ssm_scan(xbc: torch.Tensor, dt: torch.Tensor, dt_col0: int, dt_bias, a_log, 
             _call("recurrent_chunks", "qwb_ssm_chunked", _ptr(xbc), _i(xbc.shape[1]), ctypes.c_void_p(dt.data_ptr() + 4 * dt_col0),
                   _i(dt.shape[1]), _ptr(dt_bias), _ptr(a_log), _ptr(d_skip), _ptr(state), _ptr(ctx.cu_seqlens), _ptr(ctx.slots), _ptr(y),
                   _ptr(scratch), _i(T), _i(ctx.n_seqs), _i(ctx.max_new), _i(chunks_from), _i(heads), _i(vdim), _i(n_state), _i(groups),
-                  _i(1 if write_state else 0), _stream(), kernels=3)
+                  _i(1 if write_state else 0), _ptr(gemm_tc_error_word(xbc.device)), _stream(), kernels=4)
             if not rest:
                 return y
             below = chunks_from
@@ -1190,7 +1190,7 @@ def mlstm_scan(proj: torch.Tensor, i_col: int, f_col: int, i_bias: torch.Tensor,
             scratch = _chunk_scratch(size(_i(T), _i(ctx.n_seqs), _i(heads), _i(key_dim), _i(vdim)), dev)
             if scratch is not None:
                 _call("mlstm", "qwb_mlstm_tiles", *inputs, _ptr(scratch), _ptr(raw), _ptr(divisor), *sizes, _f(q_scale), _f(tiny),
-                      _i(1 if write_state else 0), _stream(), kernels=4)
+                      _i(1 if write_state else 0), _ptr(gemm_tc_error_word(dev)), _stream(), kernels=5)
                 return raw, divisor
         lib = _lookup("mlstm", "qwb_mlstm_scratch_floats")[0]
         lib.qwb_mlstm_scratch_floats.restype = ctypes.c_longlong

@@ -380,6 +380,49 @@ def test_matrix_memory_in_chunks_of_128(H, K, P, forget, monkeypatch):
     assert torch.equal(st, before) and torch.equal(m, m_before)
 
 
+@pytest.mark.parametrize("kind", ["mamba2", "mlstm"])
+@pytest.mark.parametrize("H, K, P", [(2, 36, 20), (4, 128, 64), (2, 260, 132)])
+def test_products_of_three_parts_keep_32_bits(kind, H, K, P, monkeypatch):
+    """Sequences at the edges of the eights, stages and chunks.  Without cancellation every digit of a sum can be compared: six products of
+    parts leave 2^-23 of a term, cut sums of two and rounded ones of up to 13 about 2^-22, gates and decays (of at most 4) about 2^-21; a part
+    less would be off by 2^-17."""
+    torch.manual_seed(H + K + P)
+    lens, slots = [7, 8, 9, 31, 32, 33, 96, 97, 160], [4, 2, 7, 1, 5, 3, 0, 6, 8]
+    T, step, near = sum(lens), Steps(lens, slots), lambda got, ref: ((got.double() - ref).abs() / ref.abs()).max().item() <= 2.0 ** -19
+    if kind == "mamba2":
+        monkeypatch.setattr(ops, "SSM_CHUNKED_FROM", 2)
+        G, inner = 2, H * P
+        xbc, dt = 0.1 + torch.rand(T, inner + 2 * G * K, device=DEV), torch.randn(T, H, device=DEV)
+        bias, a_log, d, start = torch.zeros(H, device=DEV), torch.full((H,), -4.0, device=DEV), torch.rand(H, device=DEV), torch.rand(9, H, P, K, device=DEV)
+        state = start.clone()
+        y = ops.ssm_scan(xbc, dt, 0, bias, a_log, d, state, step, H, P, K, G)
+    else:
+        monkeypatch.setattr(ops, "mlstm_tiles_pay", lambda *sizes: True)
+        n_qkv = H * (2 * K + P)
+        proj = 0.1 + torch.rand(T, -(-(n_qkv + 2 * H) // 4) * 4, device=DEV)
+        proj[:, n_qkv + H:n_qkv + 2 * H] += 5.0
+        zero, start, m_start = torch.zeros(H, device=DEV), torch.rand(9, H, P + 1, K, device=DEV), torch.rand(9, H, 1, device=DEV).repeat(1, 1, P + 1)
+        state, m = start.clone(), m_start.clone()
+        y, div = ops.mlstm_scan(proj, n_qkv, n_qkv + H, zero, zero, 15.0, state, m, step, H, K, P, K ** -0.5, 1e-6)
+    t = 0
+    for n, slot in zip(lens, slots):
+        if kind == "mamba2":
+            S, ref = start[slot].double(), torch.empty(n, inner, dtype=F64, device=DEV)
+            for i in range(n):
+                row = xbc[t + i].double()
+                x, (b, c) = row[:inner].view(H, P), (row[inner + k * G * K:inner + (k + 1) * G * K].view(G, K).repeat_interleave(H // G, 0) for k in (0, 1))
+                s = torch.nn.functional.softplus(dt[t + i].double(), threshold=100.0)
+                S = torch.exp(-math.exp(-4.0) * s)[:, None, None] * S + (s[:, None] * x)[:, :, None] * b[:, None, :]
+                ref[i] = ((S @ c[:, :, None])[..., 0] + d.double()[:, None] * x).reshape(-1)
+        else:
+            ref, div_ref, S, _ = matrix_memory(proj[t:t + n], n_qkv, H, K, P, zero, zero, 15.0, start[slot], m_start[slot, :, 0])
+            ref = ref.reshape(n, -1)
+            assert near(div[t:t + n], div_ref.reshape(n, H))
+        assert near(y[t:t + n], ref) and near(state[slot], S.reshape(state[slot].shape))
+        t += n
+    ops.gemm_tc_check(DEV)
+
+
 @pytest.mark.parametrize("forget", [3.0, 5.0])
 def test_chunks_of_128_round_as_little_as_those_of_64(forget, monkeypatch):
     """Against 64 bits the mLSTM's two chunked forms are off by the same: their sums and weights have about as many roundings."""
