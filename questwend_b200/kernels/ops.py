@@ -1134,21 +1134,27 @@ def gated_part_norm(y: torch.Tensor, gate: torch.Tensor, gate_col0: int, weight:
 
 # ----------------------------------------------------------------------------- matrix memory with exponential gates
 MLSTM_CHUNKED_FROM = 64         # steps whose longest sequence brings at least this many tokens take the chunked form
-# Its chunks of 128 tokens (csrc/mlstm.cu: mlstm_tile_*), for sizes and rows in multiples of 4: keys of at least MLSTM_TILES_KEYS, whose
-# tiles are what hides the copies, and at least MLSTM_TILES_BLOCKS blocks of 128 tokens x 64 values, three an SM.  us, 64 / 128
-# tokens a chunk: 4 heads of 256 x 512, 1,000 tokens (250 blocks) 113 / 123, 2,048 231 / 203, 4,096 442 / 387, 4 x 1,024 439 / 383; 4 of
-# 256 x 256, 2,048 tokens (256) 119 / 142, 4,096 240 / 238; 8 of 512 x 256, 1,000 tokens 218 / 241, 2,048 434 / 402; 16 of
-# 128 x 128, 4,096 tokens (1,024) 289 / 309; 4 of 64 x 64, 4,096 tokens 51 / 69.  A chunk costs the same however few tokens are in it, so
-# the step must bring at least MLSTM_TILES_FILL tokens a place that its chunks have.  4 heads of 256 x 512: 4 x 700 tokens (112 a place)
-# 324 / 308, 4 x 512 (102) 230 / 208, 8 x 300 (92) 297 / 316, 16 x 130 (65) 339 / 459, 2,048 beside 4 single tokens (98) 256 / 265, beside 63
-# (26) 785 / 1,511; 8 of 512 x 256: 4 x 700 602 / 607, 4 x 512 433 / 446, 8 x 256 (85) 447 / 574.
+# Its chunks of 128 tokens (csrc/mlstm.cu: mlstm_tile_*, on tcgen05), for sizes and rows in multiples of 4, against those of 64: a chunk costs
+# about the same in both however few tokens are in it, so they win wherever sequences fill more than one of 64; with small memories the
+# fifth launch costs what the products save.  us, 64 / 128 tokens a chunk: 4 heads of 256 x 512, 64 tokens 65 / 51, 500 80 / 60, 2,048 243 / 125,
+# 4,096 447 / 217, 8 x 300 (92 tokens a place that its chunks have) 307 / 170, 8 x 64 (42) 87 / 81, 2,048 beside 63 single tokens (26) 795 / 867;
+# 8 of 512 x 256, 1,000 tokens 227 / 132, 16 x 130 (65) 647 / 398; 2 of 256 x 512, 100 tokens 62 / 51; 16 of 128 x 128, 100 tokens 48 / 45, 1,000
+# 81 / 69, 4,096 298 / 220, 16 x 130 (65) 217 / 187, 8 x 64 (42) 58 / 64; 4 of 64 x 64, 100 tokens 34 / 42, 4,096 60 / 65.
 MLSTM_TILES_KEYS, MLSTM_TILES_BLOCKS, MLSTM_TILES_FILL = 256, 512, 105
+MLSTM_TILES_MEMORY, MLSTM_TILES_WIDE = 1 << 18, 1 << 16        # values of all heads' memories; of one that is worth half-filled chunks
 
 
 def mlstm_tiles_pay(tokens: int, seqs: int, heads: int, key_dim: int, vdim: int) -> bool:
-    """Whether a step of ``tokens`` tokens of ``seqs`` sequences takes the mLSTM's chunks of 128 tokens rather than those of 64."""
+    """Whether a step is long enough, and its chunks full enough, for chunks of 128 tokens whatever the memories' values."""
     return (key_dim >= MLSTM_TILES_KEYS and tokens * heads * vdim >= MLSTM_TILES_BLOCKS * 128 * 64
             and tokens >= MLSTM_TILES_FILL * (tokens // 128 + seqs))
+
+
+def _mlstm_tiles(tokens: int, seqs: int, heads: int, key_dim: int, vdim: int) -> bool:
+    """Whether a step of ``tokens`` tokens of ``seqs`` sequences takes the mLSTM's chunks of 128 tokens rather than those of 64."""
+    fill = 40 if key_dim * vdim >= MLSTM_TILES_WIDE else 60
+    return (mlstm_tiles_pay(tokens, seqs, heads, key_dim, vdim)
+            or (min(key_dim, vdim) >= 128 and heads * key_dim * vdim >= MLSTM_TILES_MEMORY and tokens >= fill * (tokens // 128 + seqs)))
 
 
 def mlstm_scan(proj: torch.Tensor, i_col: int, f_col: int, i_bias: torch.Tensor, f_bias: torch.Tensor, gate_cap: float,
@@ -1184,7 +1190,7 @@ def mlstm_scan(proj: torch.Tensor, i_col: int, f_col: int, i_bias: torch.Tensor,
               _ptr(ctx.cu_seqlens), _ptr(ctx.slots), _ptr(gate_rows))
     if chunked and not single:
         sizes = (_i(T), _i(ctx.n_seqs), _i(ctx.max_new), _i(heads), _i(key_dim), _i(vdim))
-        if mlstm_tiles_pay(T, ctx.n_seqs, heads, key_dim, vdim) and ld % 4 == 0 and proj.data_ptr() % 16 == 0:
+        if _mlstm_tiles(T, ctx.n_seqs, heads, key_dim, vdim) and ld % 4 == 0 and proj.data_ptr() % 16 == 0:
             lib, size = _lookup("mlstm", "qwb_mlstm_tiles_scratch")
             size.restype = ctypes.c_longlong
             scratch = _chunk_scratch(size(_i(T), _i(ctx.n_seqs), _i(heads), _i(key_dim), _i(vdim)), dev)
