@@ -12,13 +12,15 @@
 //
 // The products read each chosen expert's rows straight from the stacked weights (Wu [E, F, D], gated: [E, 2F, D] with the
 // gate rows first; Wd [E, D, F]): a warp per few rows, 32-bit sums.  This is the form for a step of few tokens, where every
-// token's experts are streamed once, and for the 32-bit engine.  Many bfloat16 tokens are sorted by expert instead
+// token's experts are streamed once, and for the 32-bit engine.  moe_stream reads an expert once for all of its tokens, on mma.sync, from
+// about as many choices on as there are experts.  Many bfloat16 tokens are sorted by expert instead
 // and go through a library grouped product; moe_sort, moe_spread, moe_act and moe_combine are the kernels around it.
 #include "common.cuh"
 
 #define QWB_MOE_MAX_TOP 16
 #define QWB_MOE_MAX_EXPERTS 1024
 #define MOE_UP_BLOCKS 5         // blocks of moe_up an SM by registers: more loads on their way beat a few spills in the shared expert's part
+#define MOE_SHARED_WARPS 4      // of moe_down, at most
 #define QWB_MOE_GATED 16        // activation code of the gated form, silu(gate) * up; others: qwb_activate's codes
 
 // ---------------------------------------------------------------------------------
@@ -211,15 +213,17 @@ moe_up_kernel(const T* __restrict__ x, const T* __restrict__ wu, const int* __re
     }
 }
 
-// grid (ceil(D / NR), T), a warp per choice and one for the shared expert: NR outputs of one token; the warps' products
-// are weighted and summed in the order of the choices, the shared expert last.  out may be added onto (`onto`).
+// grid (ceil(D / NR), T), a warp per choice and one or more for the shared expert: NR outputs of one token; the warps' products
+// are weighted and summed in the order of the choices, the shared expert last.  out may be added onto (`onto`).  A shared expert
+// about s times as wide as the others is cut into s warps' shares for one or two tokens, where a block waits for its longest warp (6 of 64
+// experts of 2,048 x 1,408 and one of 2,816, us: 1 token 10.2 -> 8.7, 2 19.5 -> 18.1, but 4 29.3 -> 30.8, 8 50.9 -> 53.6).
 template <typename T, int NR>
 __global__ void moe_down_kernel(const T* __restrict__ act, const T* __restrict__ wd, const int* __restrict__ chosen,
                                 const float* __restrict__ weight, const T* __restrict__ act_s, const T* __restrict__ wsd,
                                 const float* __restrict__ gate, float* out, int D, int F, int Fs, int top, int onto) {
     pdl_wait();
     pdl_launch_dependents();
-    __shared__ float part[QWB_MOE_MAX_TOP + 1][NR];
+    __shared__ float part[QWB_MOE_MAX_TOP + MOE_SHARED_WARPS][NR];
     const int t = blockIdx.y, d = blockIdx.x * NR;
     const int k = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int nr = min(NR, D - d);
@@ -229,7 +233,8 @@ __global__ void moe_down_kernel(const T* __restrict__ act, const T* __restrict__
         lane_dots<T, NR, 1>(wd + ((size_t)chosen[slot] * D + d) * F, F, nr, act + slot * F, 0, 1, F, lane, acc);
         mul = weight ? weight[slot] : 1.f;
     } else {
-        lane_dots<T, NR, 1>(wsd + (size_t)d * Fs, Fs, nr, act_s + (size_t)t * Fs, 0, 1, Fs, lane, acc);
+        const int warps = (blockDim.x >> 5) - top, share = warps == 1 ? Fs : (Fs / 8 + warps - 1) / warps * 8, from = min(Fs, (k - top) * share);
+        lane_dots<T, NR, 1>(wsd + (size_t)d * Fs + from, Fs, nr, act_s + (size_t)t * Fs + from, 0, 1, min(share, Fs - from), lane, acc);
         mul = gate ? gate[t] : 1.f;
     }
 #pragma unroll
@@ -257,8 +262,249 @@ static void launch_moe_experts(const void* x, const void* wu, const void* wd, co
         qwb_launch(moe_up_kernel<T, 1>, g1, 256, 0, stream, (const T*)x, (const T*)wu, chosen, weight_in, (T*)act, (const T*)wsu, (T*)act_s, n_tok, D, F, Fs, top, kind);
     else
         qwb_launch(moe_up_kernel<T, 2>, g1, 256, 0, stream, (const T*)x, (const T*)wu, chosen, weight_in, (T*)act, (const T*)wsu, (T*)act_s, n_tok, D, F, Fs, top, kind);
-    qwb_launch(moe_down_kernel<T, 4>, g2, 32 * (top + (Fs > 0 ? 1 : 0)), 0, stream, (const T*)act, (const T*)wd, chosen, weight, (const T*)act_s,
+    int shared_warps = Fs > 0 ? 1 : 0;
+    if (n_tok <= 2 && Fs > F && Fs % 8 == 0) shared_warps = min((Fs + F / 2) / F, MOE_SHARED_WARPS);
+    qwb_launch(moe_down_kernel<T, 4>, g2, 32 * (top + shared_warps), 0, stream, (const T*)act, (const T*)wd, chosen, weight, (const T*)act_s,
                (const T*)wsd, gate, out, D, F, Fs, top, onto);
+}
+
+// ---------------------------------------------------------------------------------
+// The same for bfloat16 and sizes in multiples of 8, an expert's rows once for all the tokens that chose it: 16 rows of one expert a
+// block on mma.sync (the rows are its 16-row operand, eight tokens its 8-column one), the contraction cut over the block's four warps.
+// A step of few tokens is bound by the weights' bytes: a thread asks for 8 x 16 bytes of its two rows before the first product, seven
+// blocks an SM, and the weights pass L1 by.  moe_lists finds the experts that are chosen and the copies of tokens that chose them, in order,
+// so that a block's first weights are asked for one round trip after its start.  `down` leaves a row of D sums for every copy and for the
+// shared expert of every token, which moe_merge adds up in the order of the choices.
+// 32 tokens, 6 of 64 experts of 2,048 x 1,408 and a shared one, us: a row for each copy 328, the library's grouped products 224; here 168 with
+// every block going through the choices by itself, 151 with lists, 136 with four instead of eight blocks of 32 values on their way, seven
+// instead of four blocks an SM and early starts (the weights at 6.55 TB/s: 107).  8 tokens 104 -> 92.
+// ---------------------------------------------------------------------------------
+#define MS_WARPS 4
+#define MS_AHEAD 4              // blocks of 32 values of two rows that are on their way
+#define MS_MAX_COPIES 2048
+#define MS_LINK_ROWS 128        // tokens up to which the four kernels start early
+
+__device__ __forceinline__ uint4 ms_weight(const uint4* p) {
+    uint4 v;
+    asm volatile("ld.global.nc.L1::no_allocate.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
+    return v;
+}
+__device__ __forceinline__ void ms_mma(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+                 : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+// acc += rows lo and hi (of this lane; null: zeros) times NT x 8 vectors (vector(j): this lane's of the j-th eight, or null; called behind the
+// rows' first loads), n values each (a multiple of 8), this warp's share.  A lane's 16 bytes are eight neighbouring values of the rows and
+// the same eight of the vectors.
+template <int NT, class Vector>
+__device__ __forceinline__ void ms_tile(float (&acc)[NT][4], const bf16* lo, const bf16* hi, Vector vector, int n) {
+    const int warp = threadIdx.x >> 5, t = threadIdx.x & 3, pieces = n / 8;
+    const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
+    for (int b0 = warp; 4 * b0 < pieces; b0 += MS_WARPS * MS_AHEAD) {
+        uint4 w0[MS_AHEAD], w1[MS_AHEAD], v[NT == 1 ? MS_AHEAD : 1];
+#pragma unroll
+        for (int u = 0; u < MS_AHEAD; ++u) {
+            const int p = 4 * (b0 + MS_WARPS * u) + t;
+            w0[u] = lo && p < pieces ? ms_weight(reinterpret_cast<const uint4*>(lo) + p) : zero;
+            w1[u] = hi && p < pieces ? ms_weight(reinterpret_cast<const uint4*>(hi) + p) : zero;
+        }
+        const bf16* x[NT];
+#pragma unroll
+        for (int j = 0; j < NT; ++j) x[j] = vector(j);
+        if (NT == 1) {
+#pragma unroll
+            for (int u = 0; u < MS_AHEAD; ++u) {
+                const int p = 4 * (b0 + MS_WARPS * u) + t;
+                v[u] = x[0] && p < pieces ? reinterpret_cast<const uint4*>(x[0])[p] : zero;
+            }
+        }
+#pragma unroll
+        for (int u = 0; u < MS_AHEAD; ++u) {
+            const int p = 4 * (b0 + MS_WARPS * u) + t;
+#pragma unroll
+            for (int j = 0; j < NT; ++j) {
+                const uint4 y = NT == 1 ? v[u] : (x[j] && p < pieces ? reinterpret_cast<const uint4*>(x[j])[p] : zero);
+                ms_mma(acc[j], w0[u].x, w1[u].x, w0[u].y, w1[u].y, y.x, y.y);
+                ms_mma(acc[j], w0[u].z, w1[u].z, w0[u].w, w1[u].w, y.z, y.w);
+            }
+        }
+    }
+}
+
+// What moe_lists leaves: the experts that are chosen, in order, where each one's copies begin (and the last one's end), the copies.
+struct MsLists { int n; int expert[QWB_MOE_MAX_EXPERTS], begin[QWB_MOE_MAX_EXPERTS + 1], copies[MS_MAX_COPIES]; };
+
+struct MsArgs {
+    const bf16 *in, *in_s, *w, *w_s;        // vectors of copies (up: of tokens) and of the shared expert's tokens; experts' and shared weights
+    const MsLists* lists;
+    const float* weight_in;
+    bf16 *act, *act_s;                      // up
+    float *y, *y_s;                         // down
+    int T, top, K, K_s, rows, rows_s, kind;
+};
+
+// one block of 1,024 threads; a warp counts, then lists, the copies of every 32nd expert
+__global__ void __launch_bounds__(1024)
+moe_lists_kernel(const int* chosen, MsLists* lists, int S, int E) {
+    pdl_launch_dependents();            // the trigger first: see qwb_launch_link
+    pdl_wait();
+    __shared__ int choice[MS_MAX_COPIES], count[QWB_MOE_MAX_EXPERTS], warps[2][32];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    for (int c = tid; c < S; c += 1024) choice[c] = __ldcg(chosen + c);
+    __syncthreads();
+    for (int e = warp; e < E; e += 32) {
+        int total = 0;
+        for (int c = 0; c < S; c += 32) total += __popc(__ballot_sync(0xffffffffu, c + lane < S && choice[c + lane] == e));
+        if (lane == 0) count[e] = total;
+    }
+    __syncthreads();
+    const int mine = tid < E ? count[tid] : 0;
+    int copies = mine, active = mine > 0;                           // sums over the experts up to this one
+    for (int o = 1; o < 32; o <<= 1) {
+        const int a = __shfl_up_sync(0xffffffffu, copies, o), b = __shfl_up_sync(0xffffffffu, active, o);
+        if (lane >= o) { copies += a; active += b; }
+    }
+    if (lane == 31) { warps[0][warp] = copies; warps[1][warp] = active; }
+    __syncthreads();
+    for (int w = 0; w < warp; ++w) { copies += warps[0][w]; active += warps[1][w]; }
+    if (mine) { lists->expert[active - 1] = tid; lists->begin[active] = copies; }
+    if (tid == 0) lists->begin[0] = 0;
+    if (tid == 1023) lists->n = active;
+    if (tid < E) count[tid] = copies - mine;
+    __syncthreads();
+    for (int e = warp; e < E; e += 32) {
+        int at = count[e];
+        for (int c = 0; c < S; c += 32) {
+            const bool is = c + lane < S && choice[c + lane] == e;
+            const unsigned all = __ballot_sync(0xffffffffu, is);
+            if (is) lists->copies[at + __popc(all & ((1u << lane) - 1u))] = c + lane;
+            at += __popc(all);
+        }
+    }
+}
+
+// One 16-row tile with the vectors from `first` on, NT x 8 of them at a time
+template <int NT, bool DOWN>
+__device__ __forceinline__ void ms_rows(const MsArgs& a, bool shared, const bf16* lo, const bf16* hi, int f0, const int* copies, int n, int first, float* part) {
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3, K = shared ? a.K_s : a.K;
+    int copy[NT];
+#pragma unroll
+    for (int j = 0; j < NT; ++j) copy[j] = first + 8 * j + g < n ? (shared ? first + 8 * j + g : __ldcg(copies + first + 8 * j + g)) : -1;
+    float acc[NT][4] = {};
+    ms_tile<NT>(acc, lo, hi, [&](int j) -> const bf16* {
+        return copy[j] < 0 ? nullptr : (shared ? a.in_s + (size_t)copy[j] * K : a.in + (size_t)(DOWN ? copy[j] : copy[j] / a.top) * K);
+    }, K);
+#pragma unroll
+    for (int j = 0; j < NT; ++j)
+#pragma unroll
+        for (int r = 0; r < 4; ++r) part[((warp * NT + j) * 4 + r) * 32 + lane] = acc[j][r];
+    __syncthreads();
+    const int r = warp;                                             // thread: register r of every tile's lane
+    const bool gated = !DOWN && !shared && a.kind == QWB_MOE_GATED;
+#pragma unroll
+    for (int j = 0; j < NT; ++j) {
+        auto sum = [&](int reg) {
+            float v = 0.f;
+#pragma unroll
+            for (int w = 0; w < MS_WARPS; ++w) v += part[((w * NT + j) * 4 + reg) * 32 + lane];
+            return v;
+        };
+        const int i = first + 8 * j + 2 * t + (r & 1), row = g + 8 * (r >> 1);
+        if (i >= n || (gated && r >= 2)) continue;
+        const int c = shared ? i : __ldcg(copies + i), f = f0 + row;
+        if (f >= (shared ? a.rows_s : a.rows)) continue;
+        float v = sum(r);
+        if (DOWN) {
+            (shared ? a.y_s : a.y)[(size_t)c * a.rows + f] = v;
+        } else {
+            const float w = a.weight_in && !shared ? a.weight_in[c] : 1.f;
+            v *= w;
+            if (gated) v = v / (1.f + expf(-v)) * (sum(r + 2) * w);
+            else v = qwb_activate(v, shared && a.kind == QWB_MOE_GATED ? 3 : a.kind);
+            (shared ? a.act_s + (size_t)c * a.rows_s : a.act + (size_t)c * a.rows)[f] = from_f32<bf16>(v);
+        }
+    }
+    __syncthreads();
+}
+
+// Blocks: the shared expert's tiles, then (slot, tile).  A tile is 16 rows, of a gated expert 8 gate rows and their 8 up rows.
+template <bool DOWN>
+__global__ void __launch_bounds__(32 * MS_WARPS, 7)
+moe_stream_kernel(const MsArgs a, int tiles, int tiles_s) {
+    pdl_launch_dependents();            // the trigger first: see qwb_launch_link
+    pdl_wait();
+    __shared__ float part[MS_WARPS * 4 * 4 * 32];
+    const int lane = threadIdx.x & 31, g = lane >> 2;
+    const bool shared = (int)blockIdx.x < tiles_s, gated = !DOWN && !shared && a.kind == QWB_MOE_GATED;
+    const int item = (int)blockIdx.x - tiles_s, slot = item / tiles, tile = shared ? blockIdx.x : item - slot * tiles;
+    const int* copies = nullptr;
+    int n = a.T, e = 0;
+    if (!shared) {
+        const int begin = __ldcg(a.lists->begin + slot), end = __ldcg(a.lists->begin + slot + 1);
+        e = __ldcg(a.lists->expert + slot);
+        if (slot >= __ldcg(&a.lists->n)) return;
+        copies = a.lists->copies + begin;
+        n = end - begin;
+    }
+    const int rows = shared ? a.rows_s : a.rows, f0 = tile * (gated ? 8 : 16), K = shared ? a.K_s : a.K;
+    const bf16* w = shared ? a.w_s : a.w + (size_t)e * (gated ? 2 * rows : rows) * K;
+    const int r0 = f0 + g, r1 = gated ? rows + f0 + g : f0 + g + 8;
+    const bf16 *lo = r0 < rows ? w + (size_t)r0 * K : nullptr, *hi = (gated ? r0 : r1) < rows ? w + (size_t)r1 * K : nullptr;
+    for (int first = 0; first < n;) {
+        if (n - first <= 8) { ms_rows<1, DOWN>(a, shared, lo, hi, f0, copies, n, first, part); first += 8; }
+        else if (n - first <= 16) { ms_rows<2, DOWN>(a, shared, lo, hi, f0, copies, n, first, part); first += 16; }
+        else { ms_rows<4, DOWN>(a, shared, lo, hi, f0, copies, n, first, part); first += 32; }
+    }
+}
+
+// grid (ceil(D / 1,024), T), 256 threads: four outputs of a token a thread, from the rows of its copies
+__global__ void __launch_bounds__(256)
+moe_merge_kernel(const float* y, const float* y_s, const float* weight, const float* gate, float* out, int D, int top, int onto) {
+    pdl_launch_dependents();            // the trigger first: see qwb_launch_link
+    pdl_wait();
+    const int t = blockIdx.y, d = (blockIdx.x * 256 + threadIdx.x) * 4;
+    if (d >= D) return;
+    float4 total = make_float4(0.f, 0.f, 0.f, 0.f);
+    auto add = [&](const float* row, float w) {
+        const float4 v = *reinterpret_cast<const float4*>(row + d);
+        total.x += w * v.x; total.y += w * v.y; total.z += w * v.z; total.w += w * v.w;
+    };
+#pragma unroll 4
+    for (int k = 0; k < top; ++k) add(y + ((size_t)t * top + k) * D, weight ? weight[(size_t)t * top + k] : 1.f);
+    if (y_s) add(y_s + (size_t)t * D, gate ? gate[t] : 1.f);
+    float4* o = reinterpret_cast<float4*>(out + (size_t)t * D + d);
+    if (onto) { const float4 v = *o; total.x += v.x; total.y += v.y; total.z += v.z; total.w += v.w; }
+    *o = total;
+}
+
+// As qwb_moe_experts for bfloat16 and sizes in multiples of 8, every tensor 16-byte aligned; y [T * top + (Fs > 0 ? T : 0), D]: scratch,
+// with qwb_moe_lists_floats() more behind it.
+extern "C" int qwb_moe_lists_floats() { return (int)(sizeof(MsLists) / sizeof(float)) + 4; }
+extern "C" int qwb_moe_stream(const void* x, const void* wu, const void* wd, const int* chosen, const float* weight, int on_input, const void* wsu, const void* wsd,
+                              const float* gate, void* act, void* act_s, float* y, float* out, int T, int E, int D, int F, int Fs, int top, int kind, int onto,
+                              cudaStream_t stream) {
+    if (T <= 0) return 0;
+    if (D <= 0 || F <= 0 || Fs < 0 || top <= 0 || top > QWB_MOE_MAX_TOP || E <= 0 || E > QWB_MOE_MAX_EXPERTS || D % 8 || F % 8 || Fs % 8 || T > MS_MAX_COPIES / top)
+        return qwb_fail(QWB_ERR_ARG, "moe_stream: %d tokens x %d choices of %d experts, width %d, expert width %d, shared %d", T, top, E, D, F, Fs);
+    if (Fs > 0 && (!wsu || !wsd || !act_s)) return qwb_fail(QWB_ERR_ARG, "moe_stream: a shared expert without its matrices");
+    if (kind != QWB_MOE_GATED && !qwb_activation_known(kind)) return qwb_fail(QWB_ERR_ARG, "moe_stream: unknown activation %d", kind);
+    for (const void* p : {x, wu, wd, wsu, wsd, (const void*)act, (const void*)act_s, (const void*)y, (const void*)out})
+        if ((uintptr_t)p % 16) return qwb_fail(QWB_ERR_ARG, "moe_stream: a tensor is not 16-byte aligned");
+    const int slots = T * top < E ? T * top : E;
+    const int up_tiles = kind == QWB_MOE_GATED ? F / 8 : (F + 15) / 16, up_shared = (Fs + 15) / 16, down_tiles = (D + 15) / 16, down_shared = Fs > 0 ? down_tiles : 0;
+    MsLists* lists = reinterpret_cast<MsLists*>(y + (size_t)T * (top + (Fs > 0 ? 1 : 0)) * D);
+    float* y_s = Fs > 0 ? y + (size_t)T * top * D : nullptr;
+    const MsArgs up = {(const bf16*)x, (const bf16*)x, (const bf16*)wu, (const bf16*)wsu, lists, on_input ? weight : nullptr, (bf16*)act, (bf16*)act_s, nullptr, nullptr,
+                       T, top, D, D, F, Fs, kind};
+    const MsArgs down = {(const bf16*)act, (const bf16*)act_s, (const bf16*)wd, (const bf16*)wsd, lists, nullptr, nullptr, nullptr, y, y_s, T, top, F, Fs, D, D, kind};
+    qwb_launch_link(T, MS_LINK_ROWS, moe_lists_kernel, 1, 1024, 0, stream, chosen, lists, T * top, E);
+    if (int rc = qwb_check_launch("moe_lists")) return rc;
+    qwb_launch_link(T, MS_LINK_ROWS, moe_stream_kernel<false>, up_shared + slots * up_tiles, 32 * MS_WARPS, 0, stream, up, up_tiles, up_shared);
+    if (int rc = qwb_check_launch("moe_stream up")) return rc;
+    qwb_launch_link(T, MS_LINK_ROWS, moe_stream_kernel<true>, down_shared + slots * down_tiles, 32 * MS_WARPS, 0, stream, down, down_tiles, down_shared);
+    if (int rc = qwb_check_launch("moe_stream down")) return rc;
+    qwb_launch_link(T, MS_LINK_ROWS, moe_merge_kernel, dim3((D + 1023) / 1024, T), 256, 0, stream, (const float*)y, (const float*)y_s, on_input ? nullptr : weight, gate, out, D, top, onto);
+    return qwb_check_launch("moe_merge");
 }
 
 // weight [T, top]: on the experts' inputs (on_input) or outputs.

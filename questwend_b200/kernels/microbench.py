@@ -304,7 +304,7 @@ def bench_moe(T, D, F, E, top, shared, activation, iters, dtype=torch.bfloat16) 
     gate = torch.rand(T, device=DEV) if shared else None
     # one choice for every copy of the inputs, so that the chosen experts do not stay in L2
     routes = [ops.moe_route(torch.randn(T, E, device=DEV), top, True, scores="sigmoid") for _ in range(8)]
-    grouped = ops.moe_grouped_fits(x, up, down)
+    grouped = ops.moe_grouped_fits(x, up, down, top, shared)
     if grouped:
         out = torch.zeros(T, D, device=DEV)
         fn = lambda i: ops.moe_experts_grouped(x, up, down, *routes[i % 8], activation, shared=out if shared else None, gate=gate)

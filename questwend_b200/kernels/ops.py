@@ -1838,6 +1838,23 @@ def _moe_sizes(what, x, w_up, w_down, chosen, weight, kind):
     return T, D, E, F, top
 
 
+MOE_STREAM_COPIES = 2048    # csrc/moe.cu: MS_MAX_COPIES
+# When bfloat16 tokens' experts are read once for all the tokens that chose them: with this many choices and three for four experts, where
+# the copies' rereading begins to cost more than the lists and the merge of that form, or from this many tokens on.  us, a row of the
+# weights for each copy / once for all / the library's grouped product: 6 of 64 experts of 2,048 x 1,408 and a shared one, 4 tokens 59 / 72 / -, 8
+# 103 / 92 / -, 16 178 / 122 / 206, 32 330 / 136 / 224, 128 - / 211 / 234, 160 - / 256 / 233; the same gated, no shared one, 4 72 / 81 / -, 8 122 / 114 / -,
+# 32 448 / 196 / 267, 128 - / 259 / 278, 160 - / 326 / 292; 8 of 128 gated of 2,048 x 768, 8 96 / 106 / -, 12 133 / 135 / -, 32 329 / 218 / 278, 128 - / 275 /
+# 298; 8 of 256 of these, 16 178 / 180 / 230, 24 257 / 252 / 312, 128 - / 491 / 520; 2 of 8 gated of 4,096 x 2,048, 5 69 / 74 / -, 6 92 / 76 / -, 32 366 / 87 /
+# 141, 64 - / 137 / 133; 4 of 32 and a shared one of 2,048 x 1,408, 6 57 / 53 / -, 128 - / 185 / 202.
+MOE_STREAM_MIN_CHOICES, MOE_STREAM_MIN_TOKENS = 12, 17
+
+
+def moe_stream_fits(D: int, F: int, Fs: int, top: int) -> bool:
+    """Whether bfloat16 experts of these sizes have the form that reads an expert's weights once for all the tokens that chose it (each
+    tensor at a multiple of 16 bytes)."""
+    return D % 8 == 0 and F % 8 == 0 and Fs % 8 == 0 and top <= MOE_MAX_TOP
+
+
 def moe_experts(x: torch.Tensor, w_up: torch.Tensor, w_down: torch.Tensor, chosen: torch.Tensor, weight: torch.Tensor,
                 activation: str = "gated_silu", shared_up: torch.Tensor | None = None, shared_down: torch.Tensor | None = None,
                 gate: torch.Tensor | None = None, out: torch.Tensor | None = None, weight_on_input: bool = False) -> torch.Tensor:
@@ -1864,23 +1881,35 @@ def moe_experts(x: torch.Tensor, w_up: torch.Tensor, w_down: torch.Tensor, chose
         out = torch.empty((T, D), dtype=torch.float32, device=x.device)
     act = torch.empty((T * top, F), dtype=x.dtype, device=x.device)
     act_s = torch.empty((T, Fs), dtype=x.dtype, device=x.device) if Fs else None
-    per = max(1, _MOE_SLOTS_PER_LAUNCH // (top + 1))
+    stream = x.dtype == torch.bfloat16 and (4 * T * top >= max(3 * E, 4 * MOE_STREAM_MIN_CHOICES) or T >= MOE_STREAM_MIN_TOKENS) and moe_stream_fits(D, F, Fs, top) and not any(
+        t.data_ptr() % 16 for t in (x, w_up, w_down, out, shared_up, shared_down) if t is not None)
+    per = MOE_STREAM_COPIES // top if stream else max(1, _MOE_SLOTS_PER_LAUNCH // (top + 1))
+    if stream:
+        y = torch.empty((min(per, T) * (top + (1 if Fs else 0)) * D + _lookup("moe", "qwb_moe_lists_floats")[1](),), dtype=torch.float32, device=x.device)
     for t0 in range(0, T, per):
         n = min(per, T - t0)
         cut = (lambda t: None if t is None else t[t0:t0 + n])
+        if stream:
+            _call("moe", "qwb_moe_stream", _ptr(cut(x)), _ptr(w_up), _ptr(w_down), _ptr(cut(chosen)), _ptr(cut(weight)), _i(1 if weight_on_input else 0), _ptr(shared_up),
+                  _ptr(shared_down), _ptr(cut(gate)), _ptr(act[t0 * top:(t0 + n) * top]), _ptr(cut(act_s)), _ptr(y), _ptr(cut(out)), _i(n), _i(E), _i(D), _i(F), _i(Fs),
+                  _i(top), _i(MOE_ACTIVATIONS[activation]), _i(1 if onto else 0), _stream(), kernels=4)
+            continue
         _call("moe", "qwb_moe_experts", _ptr(cut(x)), _ptr(w_up), _ptr(w_down), _ptr(cut(chosen)), _ptr(cut(weight)), _i(1 if weight_on_input else 0), _ptr(shared_up),
               _ptr(shared_down), _ptr(cut(gate)), _ptr(act[t0 * top:(t0 + n) * top]), _ptr(cut(act_s)), _ptr(cut(out)), _i(_dt(x.dtype)),
               _i(n), _i(D), _i(F), _i(Fs), _i(top), _i(MOE_ACTIVATIONS[activation]), _i(1 if onto else 0), _stream(), kernels=2)
     return out
 
 
-MOE_GROUPED_MIN_TOKENS = 17     # from here on bfloat16 tokens are sorted by expert and go through the library's grouped product
+# From here on, or from this many choices an expert on, bfloat16 tokens are sorted by expert and go through the library's grouped product
+# (figures: MOE_STREAM_MIN_TOKENS); the last number where a shared expert's width leaves only the form that reads weights for each copy.
+MOE_GROUPED_MIN_TOKENS, MOE_GROUPED_MIN_CHOICES, MOE_GROUPED_MIN_TOKENS_ODD = 129, 16, 17
 
 
-def moe_grouped_fits(x: torch.Tensor, w_up: torch.Tensor, w_down: torch.Tensor) -> bool:
+def moe_grouped_fits(x: torch.Tensor, w_up: torch.Tensor, w_down: torch.Tensor, top: int = 1, shared_size: int = 0) -> bool:
     """Whether a step's tokens take the sorted, grouped form (else the expert-streaming kernels do)."""
-    D, F = w_down.shape[1], w_down.shape[2]
-    return (x.dtype == torch.bfloat16 and x.shape[0] >= MOE_GROUPED_MIN_TOKENS and D % 8 == 0 and F % 8 == 0
+    T, (E, D, F) = x.shape[0], w_down.shape
+    many = T >= MOE_GROUPED_MIN_TOKENS or (T >= MOE_GROUPED_MIN_TOKENS_ODD and (T * top > MOE_GROUPED_MIN_CHOICES * E or shared_size % 8 != 0))
+    return (x.dtype == torch.bfloat16 and many and D % 8 == 0 and F % 8 == 0
             and hasattr(torch, "_grouped_mm"))
 
 

@@ -119,7 +119,7 @@ class RoutedExperts(FeedForward):
                                weight_scale=self.weight_scale, gate=self.shared_gate)
         on_input = self.weight_on == "input"
         chosen, weight, gate = routed if self.shared_gate else (*routed, None)
-        if ops.moe_grouped_fits(x, self.w_up, self.w_down):
+        if ops.moe_grouped_fits(x, self.w_up, self.w_down, self.top, self.shared):
             shared = None
             if self.shared:
                 shared = linear(linear_act(x, self.w_shared_up, None, self.activation, self.runtime.dtype), self.w_shared_down)

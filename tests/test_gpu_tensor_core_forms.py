@@ -662,3 +662,39 @@ def test_score_maps_of_single_tokens_from_any_address(maps, H, G, dim, vdim):
     ctx = SimpleNamespace(single_token=True, n_seqs=len(lens), max_new=1, max_len=max(lens), seq_len=torch.tensor(lens, device=DEV).int())
     a, b = (ops.maps_attention(x, k_pool, v_pool, table, ctx, maps, dim ** -0.5, lam=0.4) for x in (q, shifted))
     assert ((a.double() - b.double()).abs() <= 2.0 ** -7 * a.double().abs() + 2e-5).all()      # two roundings of nearly the same numbers
+
+
+# ----------------------------------------------------------------------------- experts
+@pytest.mark.parametrize("T, E, top, D, F, Fs, activation", [(1, 3, 1, 8, 8, 0, "relu2"), (7, 64, 6, 264, 40, 72, "gelu"), (9, 5, 5, 72, 24, 16, "silu"), (17, 130, 8, 2048, 136, 0, "gated_silu"),
+                                                            (40, 2, 1, 136, 264, 520, "relu2"), (33, 4, 2, 40, 8, 0, "gated_silu"), (140, 6, 16 // 4, 64, 72, 8, "relu2"), (600, 9, 4, 24, 16, 40, "silu")])
+@pytest.mark.parametrize("on_input", [False, True])
+def test_experts_read_once_for_all_their_tokens(T, E, top, D, F, Fs, activation, on_input, monkeypatch):
+    """Experts with no token, one eight, more than four eights and all tokens; rows, features and contractions that end inside a tile; a
+    shared expert with a gate; more tokens than a launch takes.  The form that reads the weights for each copy gives the same."""
+    torch.manual_seed(T + E + F)
+    gated, r16 = activation == "gated_silu", lambda x: x.to(torch.bfloat16).double()
+    x, up, down = (torch.randn(*s, device=DEV).mul(f).to(torch.bfloat16) for s, f in (((T, D), 1.0), ((E, (2 if gated else 1) * F, D), D ** -0.5), ((E, D, F), F ** -0.5)))
+    su, sd, gate = (None, None, None) if not Fs else (torch.randn(Fs, D, device=DEV).mul(D ** -0.5).to(torch.bfloat16), torch.randn(D, Fs, device=DEV).mul(Fs ** -0.5).to(torch.bfloat16), torch.rand(T, device=DEV))
+    logits = torch.randn(T, E, device=DEV)
+    logits[:, 0] += 3.0                                     # most tokens choose the first one, few the last
+    logits[:, -1] -= 3.0 * (E > top)
+    chosen, weight = ops.moe_route(logits, top)
+    act = {"relu2": lambda z: torch.relu(z).square(), "gelu": lambda z: torch.nn.functional.gelu(z, approximate="tanh"), "silu": torch.nn.functional.silu}
+    ref = torch.zeros(T, D, dtype=F64, device=DEV)
+    for k in range(top):
+        w = weight[:, k].double()[:, None]
+        z = torch.einsum("tfd,td->tf", up[chosen[:, k].long()].double(), x.double()) * (w if on_input else 1.0)
+        a = torch.nn.functional.silu(z[:, :F]) * z[:, F:] if gated else act[activation](z)
+        ref += torch.einsum("tdf,tf->td", down[chosen[:, k].long()].double(), r16(a)) * (1.0 if on_input else w)
+    if Fs:
+        ref += gate.double()[:, None] * (r16(act[activation](x.double() @ su.double().T)) @ sd.double().T)
+    base = torch.randn(T, D, device=DEV)
+    for least in (1, 10 ** 6):                              # every step in that form; none that brings fewer choices than experts
+        monkeypatch.setattr(ops, "MOE_STREAM_MIN_TOKENS", least)
+        if least > 1:
+            monkeypatch.setattr(ops, "moe_stream_fits", lambda *sizes: False)
+        for out in (None, base.clone()):
+            got = ops.moe_experts(x, up, down, chosen, weight, activation, su, sd, gate, out=out, weight_on_input=on_input)
+            want = ref + base.double() if out is not None else ref
+            # an activation that lies at the border of two bfloat16 numbers may be rounded the other way: 2^-8 of one of F terms
+            assert torch.isfinite(got).all() and (got.double() - want).norm() <= 2 ** -9 * ref.norm() and (got.double() - want).abs().max() <= 2 ** -6 * (1 + ref.abs().max())
