@@ -12,9 +12,11 @@ from __future__ import annotations
 import ctypes
 import hashlib
 import os
+import importlib.util
 import shutil
 import subprocess
 import sys
+import sysconfig
 import tempfile
 import threading
 import time
@@ -171,3 +173,62 @@ def load_module(module: str) -> ctypes.CDLL:
         lib.qwb_last_error.restype = ctypes.c_char_p
         _loaded[module] = lib
         return lib
+
+
+# ----------------------------------------------------------------------------- the way from Python to the launchers (csrc/host_call.cpp)
+HOST_MODULE = "qwb_host_call"
+
+
+def _host_command(out: str) -> list[str]:
+    import torch
+    root = os.path.dirname(torch.__file__)
+    cuda = os.environ.get("CUDA_HOME") or "/usr/local/cuda"
+    return [shutil.which("g++") or "g++", "-O2", "-std=c++17", "-shared", "-fPIC", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch.compiled_with_cxx11_abi())}",
+            "-I", os.path.join(root, "include"), "-I", os.path.join(root, "include", "torch", "csrc", "api", "include"),
+            "-I", sysconfig.get_paths()["include"], "-I", os.path.join(cuda, "include"), "-o", out, os.path.join(CSRC, "host_call.cpp"),
+            "-L", os.path.join(root, "lib"), "-ltorch_python", "-ltorch_cpu", "-lc10"]
+
+
+def _host_stamp() -> str:
+    import torch
+    with open(os.path.join(CSRC, "host_call.cpp"), "rb") as f:
+        return hashlib.sha256(f.read() + f"{torch.__version__} {sys.version}".encode()).hexdigest()
+
+
+def _host_path() -> str:
+    return os.path.join(build_dir(), f"{HOST_MODULE}.so")
+
+
+def host_calls_built() -> bool:
+    try:
+        with open(_host_path() + ".stamp") as f:
+            return os.path.exists(_host_path()) and f.read().strip() == _host_stamp()
+    except OSError:
+        return False
+
+
+def compile_host_calls() -> None:
+    """Compile csrc/host_call.cpp against this torch and Python, if that is not done."""
+    if host_calls_built():
+        return
+    tmp = f"{_host_path()}.{os.getpid()}.tmp"
+    proc = subprocess.run(_host_command(tmp), stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True)
+    if proc.returncode != 0:
+        raise KernelBuildError(f"g++ failed for csrc/host_call.cpp:\n{proc.stdout}")
+    os.replace(tmp, _host_path())
+    with open(_host_path() + ".stamp", "w") as f:
+        f.write(_host_stamp())
+
+
+def host_calls():
+    """The module of csrc/host_call.cpp, or None where it is not built for this torch and Python: calls then go through ctypes."""
+    if not host_calls_built():
+        return None
+    try:
+        spec = importlib.util.spec_from_file_location(HOST_MODULE, _host_path())
+        module = importlib.util.module_from_spec(spec)
+        spec.loader.exec_module(module)
+        return module
+    except ImportError as e:
+        _log(f"{_host_path()} cannot be loaded ({e}): calls go through ctypes")
+        return None

@@ -9,10 +9,11 @@ from __future__ import annotations
 
 import ctypes
 import math
+import operator
 
 import torch
 
-from .build import load_module
+from .build import host_calls, load_module
 
 DT_F32, DT_BF16 = 0, 1
 PAGE_SIZE = 64          # tokens per cache page
@@ -33,18 +34,28 @@ def _dt(t: torch.dtype) -> int:
 _raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)
 
 
-def _stream() -> ctypes.c_void_p:
+def _stream():
     """The current stream of the current device (also inside a graph capture, which runs on a stream of its own)."""
     if _raw_stream is not None:                      # the handle itself: a tenth of the cost of making a Stream object
-        return ctypes.c_void_p(_raw_stream(torch.cuda.current_device()))
-    return ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+        return _address(_raw_stream(torch.cuda.current_device()))
+    return _address(torch.cuda.current_stream().cuda_stream)
 
 
-def _ptr(t: torch.Tensor | None) -> ctypes.c_void_p:
-    return ctypes.c_void_p(0 if t is None else t.data_ptr())
+# A launcher's arguments: tensors (None: a null pointer), other addresses, whole numbers, 32-bit floats; and the outputs' memory.  Through
+# csrc/host_call.cpp, where it is built, they go as they are (20 arguments 0.8 us, an output 1.7); ctypes wants an object each (4.8 and 4.4).
+_HOST = host_calls()
+if _HOST is not None:
+    _ptr, _i, _f, _address, _empty = _HOST.same, operator.index, float, _HOST.same, _HOST.empty
+else:
+    _i, _f, _address, _empty = ctypes.c_int, ctypes.c_float, ctypes.c_void_p, torch.empty
+
+    def _ptr(t: torch.Tensor | None) -> ctypes.c_void_p:
+        return ctypes.c_void_p(0 if t is None else t.data_ptr())
 
 
 def _need(t: torch.Tensor, name: str, dtype=None, ndim=None):
+    if _HOST is not None and _HOST.fits(t, dtype, ndim):
+        return
     if not t.is_cuda:
         raise KernelError(f"{name}: must be a CUDA tensor (this library has no CPU path)")
     if not t.is_contiguous():
@@ -62,13 +73,14 @@ def _column_gate(what: str, gate: torch.Tensor | None, col0: int, T: int, H: int
     _need(gate, "gate", torch.float32, 2)
     if gate.shape[0] != T or col0 < 0 or col0 + H > gate.shape[1]:
         raise KernelError(f"{what}: gate {tuple(gate.shape)} from column {col0} for {T} tokens of {H} heads")
-    return ctypes.c_void_p(gate.data_ptr() + 4 * col0), _i(gate.shape[1])
+    return _address(gate.data_ptr() + 4 * col0), _i(gate.shape[1])
 
 
 LAUNCHES = [0]          # kernels of this library launched so far (through these entry points)
 
 
 _FUNCTIONS: dict = {}    # (module, name) -> (library, its function), looked up once
+_ADDRESSES: dict = {}    # (module, name) -> the function's address
 
 
 def _lookup(module: str, fn: str):
@@ -76,19 +88,23 @@ def _lookup(module: str, fn: str):
     if entry is None:
         lib = load_module(module)
         entry = _FUNCTIONS[module, fn] = (lib, getattr(lib, fn))
+        _ADDRESSES[module, fn] = ctypes.cast(entry[1], ctypes.c_void_p).value
     return entry
 
 
 def _call(module: str, fn: str, *args, kernels: int = 1):
-    entry = _lookup(module, fn)
-    rc = entry[1](*args)
+    name = module, fn
+    if _HOST is None:
+        rc = _lookup(module, fn)[1](*args)
+    else:
+        address = _ADDRESSES.get(name)
+        if address is None:
+            _lookup(module, fn)
+            address = _ADDRESSES[name]
+        rc = _HOST.call(address, *args)
     LAUNCHES[0] += kernels
     if rc != 0:
-        raise KernelError(entry[0].qwb_last_error().decode("utf-8", "replace") or f"{fn} failed with code {rc}")
-
-
-_i = ctypes.c_int
-_f = ctypes.c_float
+        raise KernelError(_FUNCTIONS[name][0].qwb_last_error().decode("utf-8", "replace") or f"{fn} failed with code {rc}")
 
 
 # ----------------------------------------------------------------------------- elementwise
@@ -106,7 +122,7 @@ def embed_gather(ids: torch.Tensor, table: torch.Tensor, bad_token: torch.Tensor
         NP = pos_table.shape[0]
         if pos_table.shape[1] != D or positions.numel() != T:
             raise KernelError(f"embed_gather: position table {tuple(pos_table.shape)}, {positions.numel()} positions for {T} rows of {D}")
-    out = torch.empty((T, D), dtype=torch.float32, device=table.device)
+    out = _empty((T, D), dtype=torch.float32, device=table.device)
     _call("elementwise", "qwb_embed_gather", _ptr(ids), _ptr(table), _i(_dt(table.dtype)), _ptr(positions if NP else None),
           _ptr(pos_table), _ptr(out), _i(T), _i(D), _i(V), _i(NP), _ptr(bad_token), _f(scale), _stream())
     return out
@@ -152,7 +168,7 @@ def rmsnorm(x: torch.Tensor, weight: torch.Tensor, eps: float, out_dtype: torch.
     if rows is not None:
         _need(rows, "rows", torch.int32, 1)
         n_rows = rows.numel()
-    out = torch.empty((n_rows, D), dtype=out_dtype, device=x.device)
+    out = _empty((n_rows, D), dtype=out_dtype, device=x.device)
     if isinstance(delta, SplitSum):
         if tuple(delta.planes.shape[1:]) != (T, D):
             raise KernelError(f"rmsnorm: planes {tuple(delta.planes.shape)} do not match x {tuple(x.shape)}")
@@ -195,7 +211,7 @@ def silu_mul(gate_up: torch.Tensor, out_dtype: torch.dtype, interleave: int = 0,
     T, F2 = gate_up.shape
     if F2 % 2:
         raise KernelError(f"silu_mul: {F2} columns cannot be split into gate and up")
-    out = torch.empty((T, F2 // 2), dtype=out_dtype, device=gate_up.device)
+    out = _empty((T, F2 // 2), dtype=out_dtype, device=gate_up.device)
     _call("elementwise", "qwb_silu_mul", _ptr(gate_up), _ptr(out), _i(_dt(out_dtype)), _i(T), _i(F2 // 2), _i(interleave),
           _i(GATE_ACTIVATIONS[activation]), _f(limit), _stream())
     return out
@@ -223,7 +239,7 @@ def rmsnorm_onto(h: torch.Tensor, y: torch.Tensor, weight: torch.Tensor, eps: fl
         raise KernelError(f"rmsnorm_onto: h {tuple(h.shape)}, y {tuple(y.shape)}, weight of {weight.numel()}")
     cast = None
     if cast_dtype is not None and cast_dtype != torch.float32:
-        cast = torch.empty((T, D), dtype=cast_dtype, device=h.device)
+        cast = _empty((T, D), dtype=cast_dtype, device=h.device)
     _call("elementwise", "qwb_rmsnorm_onto", _ptr(y), _ptr(weight), _ptr(h), _ptr(cast),
           _i(_dt(cast_dtype) if cast is not None else DT_F32), _i(T), _i(D), _f(eps), _stream())
     if cast_dtype is None:
@@ -244,7 +260,7 @@ def rmsnorm_mix(h: torch.Tensor, y: torch.Tensor, weight: torch.Tensor, eps: flo
         raise KernelError(f"rmsnorm_mix: y {tuple(y.shape)}, weight of {weight.numel()} for a stream {tuple(h.shape)}")
     cast = None
     if cast_dtype is not None and cast_dtype != torch.float32:
-        cast = torch.empty((T, D), dtype=cast_dtype, device=h.device)
+        cast = _empty((T, D), dtype=cast_dtype, device=h.device)
     _call("elementwise", "qwb_rmsnorm_mix", _ptr(y), _ptr(weight), _ptr(h), _ptr(cast),
           _i(_dt(cast.dtype) if cast is not None else DT_F32), _i(T), _i(D), _f(eps), _f(alpha), _stream())
     if cast_dtype is None:
@@ -283,8 +299,8 @@ def bias_act(x: torch.Tensor, bias: torch.Tensor | None, activation: str, out_dt
     whole = F == ld
     if whole and out_dtype == torch.float32 and bias is None and activation == "none":
         return x
-    out = x if (out_dtype == torch.float32 and whole) else torch.empty((T, F), dtype=out_dtype, device=x.device)
-    _call("elementwise", "qwb_bias_act", ctypes.c_void_p(x.data_ptr() + 4 * col0), _i(ld), _ptr(bias), _ptr(out),
+    out = x if (out_dtype == torch.float32 and whole) else _empty((T, F), dtype=out_dtype, device=x.device)
+    _call("elementwise", "qwb_bias_act", _address(x.data_ptr() + 4 * col0), _i(ld), _ptr(bias), _ptr(out),
           _i(_dt(out_dtype)), _i(T), _i(F), _i(ACTIVATIONS[activation]), _ptr(params), _stream())
     return out
 
@@ -317,7 +333,7 @@ def layernorm(x: torch.Tensor, weight: torch.Tensor | None, eps: float, out_dtyp
         n_rows = rows.numel()
     out = None
     if weight is not None:
-        out = torch.empty((n_rows, D), dtype=out_dtype, device=x.device)
+        out = _empty((n_rows, D), dtype=out_dtype, device=x.device)
     _call("layernorm", "qwb_layernorm", _ptr(x), _ptr(add), _ptr(add_weight), _f(eps if add_eps is None else add_eps),
           _i(1 if write_sum else 0), _ptr(weight), _ptr(out), _i(_dt(out_dtype) if out is not None else DT_F32), _ptr(rows),
           _i(n_rows), _i(D), _f(eps), _stream())
@@ -339,7 +355,7 @@ def rope_table(positions: torch.Tensor, inv_freq: torch.Tensor, factor: float = 
     _need(positions, "positions", torch.int32, 1)
     _need(inv_freq, "inv_freq", torch.float64, 1)
     T, half = positions.numel(), inv_freq.numel()
-    cos = torch.empty((T, half), dtype=torch.float32, device=positions.device)
+    cos = _empty((T, half), dtype=torch.float32, device=positions.device)
     sin = torch.empty_like(cos)
     _call("rope_kv", "qwb_rope_table", _ptr(positions), _ptr(inv_freq), _ptr(cos), _ptr(sin), _i(T), _i(half),
           ctypes.c_double(factor), _stream())
@@ -375,7 +391,7 @@ def qk_norm_rope_store(qkv: torch.Tensor, q_weight, k_weight, cos, sin, tok_seq,
     _need(tok_seq, "tok_seq", torch.int32, 1)
     _need(tok_pos, "tok_pos", torch.int32, 1)
     _need(page_table, "page_table", torch.int32, 2)
-    q_out = torch.empty((T, n_heads, head_dim), dtype=k_pool.dtype, device=qkv.device)
+    q_out = _empty((T, n_heads, head_dim), dtype=k_pool.dtype, device=qkv.device)
     _call("rope_kv", "qwb_qk_norm_rope_store", _ptr(qkv), _ptr(q_weight), _ptr(k_weight), _ptr(cos), _ptr(sin),
           _ptr(tok_seq), _ptr(tok_pos), _ptr(page_table), _ptr(q_out), _ptr(k_pool), _ptr(v_pool),
           _i(_dt(k_pool.dtype)), _i(T), _i(n_heads), _i(n_kv_heads), _i(head_dim), _i(rotary_dim), _f(eps),
@@ -423,7 +439,7 @@ def attn_prefill(q, k_pool, v_pool, page_table, cu_seqlens, pos0, max_new: int, 
     if cu_seqlens.numel() != B + 1 or page_table.shape[0] < B:
         raise KernelError("attn_prefill: cu_seqlens / page_table do not fit the batch")
     vd = v_pool.shape[3]
-    out = torch.empty((T, Hq * vd), dtype=q.dtype, device=q.device)
+    out = _empty((T, Hq * vd), dtype=q.dtype, device=q.device)
     group = Hq // max(1, k_pool.shape[1])
     # the tcgen05 kernel works on tiles of 128 rows: it pays from a few dozen new tokens per sequence on
     use_tc = impl == "tc" or (impl == "auto" and max_new * group >= 64 and
@@ -501,10 +517,10 @@ def attn_decode(q, k_pool, v_pool, page_table, seq_len, scale: float, max_len: i
     held = (64 if vd <= 64 else 128) if use_mma else hd         # values of a partial result
     need = attn_decode_scratch_floats(B, Hq, held, max_runs) if max_runs > 1 else 0
     if need and (scratch is None or scratch.numel() < need):
-        scratch = torch.empty(need, dtype=torch.float32, device=q.device)
+        scratch = _empty(need, dtype=torch.float32, device=q.device)
     if scratch is not None:
         _need(scratch, "scratch", torch.float32)
-    out = torch.empty((B, Hq * vd), dtype=q.dtype, device=q.device)
+    out = _empty((B, Hq * vd), dtype=q.dtype, device=q.device)
     if use_mma:
         _call("attention_mma", "qwb_attn_mma_decode", _ptr(q), _ptr(k_pool), _ptr(v_pool), _ptr(page_table),
               _ptr(seq_len), _ptr(scratch), _ptr(out), _i(B), _i(Hq), _i(k_pool.shape[1]), _i(hd), _i(vd), _i(k_pool.shape[2]),
@@ -555,8 +571,8 @@ def attn_decode_fused(qkv: torch.Tensor, q_weight, k_weight, cos, sin, eps: floa
     max_runs = max(1, mma_decode_runs(max_len, runs_target, run_pages_max))
     need = attn_decode_scratch_floats(B, n_heads, head_dim, max_runs) if max_runs > 1 else 0
     if need and (scratch is None or scratch.numel() < need):
-        scratch = torch.empty(need, dtype=torch.float32, device=qkv.device)
-    out = torch.empty((B, n_heads * head_dim), dtype=torch.bfloat16, device=qkv.device)
+        scratch = _empty(need, dtype=torch.float32, device=qkv.device)
+    out = _empty((B, n_heads * head_dim), dtype=torch.bfloat16, device=qkv.device)
     _call("attention_mma", "qwb_attn_mma_decode_fused", _ptr(qkv), _ptr(q_weight), _ptr(k_weight), _ptr(cos), _ptr(sin),
           _f(eps), _i(1 if store_kv else 0), _ptr(k_pool), _ptr(v_pool), _ptr(page_table), _ptr(seq_len), _ptr(scratch),
           _ptr(out), _i(B), _i(n_heads), _i(n_kv_heads), _i(head_dim), _i(k_pool.shape[2]), _i(page_table.shape[1]),
@@ -579,7 +595,7 @@ def gemm_small(x: torch.Tensor, weight: torch.Tensor, residual: torch.Tensor | N
     if weight.shape[1] != K:
         raise KernelError(f"gemm_small: x has {K} columns, the weight {weight.shape[1]}")
     if out is None:
-        out = residual if residual is not None else torch.empty((M, N), dtype=torch.float32, device=x.device)
+        out = residual if residual is not None else _empty((M, N), dtype=torch.float32, device=x.device)
     _need(out, "out", torch.float32, 2)
     if residual is not None:
         _need(residual, "residual", torch.float32, 2)
@@ -605,7 +621,7 @@ def gemm_stream(x: torch.Tensor, weight: torch.Tensor, residual: torch.Tensor | 
     if weight.shape[1] != K:
         raise KernelError(f"gemm_stream: x has {K} columns, the weight {weight.shape[1]}")
     if out is None:
-        out = residual if residual is not None else torch.empty((M, N), dtype=torch.float32, device=x.device)
+        out = residual if residual is not None else _empty((M, N), dtype=torch.float32, device=x.device)
     _need(out, "out", torch.float32, 2)
     if residual is not None:
         _need(residual, "residual", torch.float32, 2)
@@ -624,7 +640,7 @@ def gemm_stream_swiglu(x: torch.Tensor, weight: torch.Tensor, config: tuple | No
     if weight.shape[1] != K or weight.shape[0] % 2:
         raise KernelError(f"gemm_stream_swiglu: x is {tuple(x.shape)}, the weight {tuple(weight.shape)}")
     F = weight.shape[0] // 2
-    out = torch.empty((M, F), dtype=torch.bfloat16, device=x.device)
+    out = _empty((M, F), dtype=torch.bfloat16, device=x.device)
     u, w = config or (0, 0)
     _call("gemm_stream", "qwb_gemm_stream_swiglu", _ptr(x), _ptr(weight), _ptr(out), _i(M), _i(F), _i(K), _i(u), _i(w), _stream())
     return out
@@ -645,7 +661,7 @@ def gemm_ring(x: torch.Tensor, weight: torch.Tensor, residual: torch.Tensor | No
     if weight.shape[1] != K:
         raise KernelError(f"gemm_ring: x has {K} columns, the weight {weight.shape[1]}")
     if out is None:
-        out = residual if residual is not None else torch.empty((M, N), dtype=torch.float32, device=x.device)
+        out = residual if residual is not None else _empty((M, N), dtype=torch.float32, device=x.device)
     _need(out, "out", torch.float32, 2)
     if residual is not None:
         _need(residual, "residual", torch.float32, 2)
@@ -737,7 +753,7 @@ def gemm_ring_split(x: torch.Tensor, weight: torch.Tensor, plan=None) -> SplitSu
         if plan is None:
             raise KernelError(f"gemm_ring_split: no split plan for a weight of {N} x {K}")
     blocks, n_planes, plane_count = plan
-    planes = torch.empty((n_planes, M, N), dtype=torch.float32, device=x.device)
+    planes = _empty((n_planes, M, N), dtype=torch.float32, device=x.device)
     _call("gemm_ring", "qwb_gemm_ring_split", _ptr(x), _ptr(weight), _ptr(planes), _i(M), _i(N), _i(K), _i(blocks),
           _ptr(gemm_tc_error_word(x.device)), _stream())
     return SplitSum(planes, plane_count)
@@ -751,7 +767,7 @@ def gemm_ring_swiglu(x: torch.Tensor, weight: torch.Tensor) -> torch.Tensor:
     if weight.shape[1] != K or weight.shape[0] % 2:
         raise KernelError(f"gemm_ring_swiglu: x is {tuple(x.shape)}, the weight {tuple(weight.shape)}")
     F = weight.shape[0] // 2
-    out = torch.empty((M, F), dtype=torch.bfloat16, device=x.device)
+    out = _empty((M, F), dtype=torch.bfloat16, device=x.device)
     _call("gemm_ring", "qwb_gemm_ring_swiglu", _ptr(x), _ptr(weight), _ptr(out), _i(M), _i(F), _i(K),
           _ptr(gemm_tc_error_word(x.device)), _stream())
     return out
@@ -765,7 +781,7 @@ def gemm_ring_xielu(x: torch.Tensor, weight: torch.Tensor, params: torch.Tensor)
     M, K = x.shape
     if weight.shape[1] != K or params.numel() != 2:
         raise KernelError(f"gemm_ring_xielu: x is {tuple(x.shape)}, the weight {tuple(weight.shape)}, {params.numel()} numbers")
-    out = torch.empty((M, weight.shape[0]), dtype=torch.bfloat16, device=x.device)
+    out = _empty((M, weight.shape[0]), dtype=torch.bfloat16, device=x.device)
     _call("gemm_ring", "qwb_gemm_ring_xielu", _ptr(x), _ptr(weight), _ptr(out), _ptr(params), _i(M), _i(weight.shape[0]), _i(K),
           _ptr(gemm_tc_error_word(x.device)), _stream())
     return out
@@ -821,7 +837,7 @@ def gemm_tc(x: torch.Tensor, weight: torch.Tensor, epilogue: str = "store", out:
     if out is None:
         if epilogue == "add":
             raise KernelError("gemm_tc: the 'add' epilogue needs the tensor to add onto")
-        out = torch.empty((M, N), dtype=out_dtype, device=x.device)
+        out = _empty((M, N), dtype=out_dtype, device=x.device)
     _need(out, "out", out_dtype, 2)
     if tuple(out.shape) != (M, N):
         raise KernelError(f"gemm_tc: out is {tuple(out.shape)}, expected {(M, N)}")
@@ -842,7 +858,7 @@ def gemm_tc_xielu(x: torch.Tensor, weight: torch.Tensor, params: torch.Tensor, t
     N = weight.shape[0]
     if weight.shape[1] != K or params.numel() != 2:
         raise KernelError(f"gemm_tc_xielu: x {tuple(x.shape)}, weight {tuple(weight.shape)}, {params.numel()} numbers")
-    out = torch.empty((M, N), dtype=torch.bfloat16, device=x.device)
+    out = _empty((M, N), dtype=torch.bfloat16, device=x.device)
     _call("gemm_tc", "qwb_gemm_tc_xielu", _ptr(x), _ptr(weight), _ptr(out), _ptr(params), _i(M), _i(N), _i(K), _i(tile_n),
           _ptr(gemm_tc_error_word(x.device)), _stream())
     return out
@@ -879,8 +895,8 @@ def short_conv(x: torch.Tensor, col0: int, channels: int, weight: torch.Tensor, 
             _need(t, name, torch.float32, 1)
             if t.numel() != channels:
                 raise KernelError(f"short_conv: {name} of {t.numel()} for {channels} channels")
-    out = torch.empty((T, channels), dtype=out_dtype, device=x.device)
-    _call("recurrent", "qwb_short_conv", ctypes.c_void_p(x.data_ptr() + 4 * col0), _i(ld), _ptr(weight), _ptr(bias),
+    out = _empty((T, channels), dtype=out_dtype, device=x.device)
+    _call("recurrent", "qwb_short_conv", _address(x.data_ptr() + 4 * col0), _i(ld), _ptr(weight), _ptr(bias),
           _ptr(in_bias), _ptr(tail), _ptr(ctx.tok_seq), _ptr(ctx.cu_seqlens), _ptr(ctx.slots), _ptr(out), _i(_dt(out_dtype)),
           _i(T), _i(ctx.n_seqs), _i(channels), _i(taps), _i(2 if plus_input else (1 if activation else 0)),
           _i(1 if update_tail else 0),
@@ -903,7 +919,7 @@ def _chunk_scratch(floats: int, device) -> torch.Tensor | None:
     if not 0 < floats <= CHUNK_SCRATCH_MAX:
         return None
     try:
-        return torch.empty((floats,), dtype=torch.float32, device=device)
+        return _empty((floats,), dtype=torch.float32, device=device)
     except torch.OutOfMemoryError:
         return None
 
@@ -932,7 +948,7 @@ def ssm_scan(xbc: torch.Tensor, dt: torch.Tensor, dt_col0: int, dt_bias, a_log, 
         _need(t, name, torch.float32, 1)
         if t.numel() != heads:
             raise KernelError(f"ssm_scan: {name} has {t.numel()} entries for {heads} heads")
-    y = torch.empty((T, heads * vdim), dtype=torch.float32, device=xbc.device)
+    y = _empty((T, heads * vdim), dtype=torch.float32, device=xbc.device)
     below = 0
     if ctx.max_new >= SSM_CHUNKED_FROM and xbc.shape[1] % 4 == 0 and not (xbc.data_ptr() % 16 or state.data_ptr() % 16):
         lib, size = _lookup("recurrent_chunks", "qwb_ssm_chunked_scratch")
@@ -940,14 +956,14 @@ def ssm_scan(xbc: torch.Tensor, dt: torch.Tensor, dt_col0: int, dt_bias, a_log, 
         chunks_from, rest = _forms(ctx, SSM_CHUNKED_FROM)
         scratch = _chunk_scratch(size(_i(T), _i(ctx.n_seqs), _i(chunks_from), _i(heads), _i(vdim), _i(n_state), _i(groups)), xbc.device)
         if scratch is not None:
-            _call("recurrent_chunks", "qwb_ssm_chunked", _ptr(xbc), _i(xbc.shape[1]), ctypes.c_void_p(dt.data_ptr() + 4 * dt_col0),
+            _call("recurrent_chunks", "qwb_ssm_chunked", _ptr(xbc), _i(xbc.shape[1]), _address(dt.data_ptr() + 4 * dt_col0),
                   _i(dt.shape[1]), _ptr(dt_bias), _ptr(a_log), _ptr(d_skip), _ptr(state), _ptr(ctx.cu_seqlens), _ptr(ctx.slots), _ptr(y),
                   _ptr(scratch), _i(T), _i(ctx.n_seqs), _i(ctx.max_new), _i(chunks_from), _i(heads), _i(vdim), _i(n_state), _i(groups),
                   _i(1 if write_state else 0), _ptr(gemm_tc_error_word(xbc.device)), _stream(), kernels=4)
             if not rest:
                 return y
             below = chunks_from
-    _call("recurrent", "qwb_ssm_scan", _ptr(xbc), _i(xbc.shape[1]), ctypes.c_void_p(dt.data_ptr() + 4 * dt_col0),
+    _call("recurrent", "qwb_ssm_scan", _ptr(xbc), _i(xbc.shape[1]), _address(dt.data_ptr() + 4 * dt_col0),
           _i(dt.shape[1]), _ptr(dt_bias), _ptr(a_log), _ptr(d_skip), _ptr(state), _ptr(ctx.cu_seqlens), _ptr(ctx.slots),
           _ptr(y), _i(ctx.n_seqs), _i(heads), _i(vdim), _i(n_state), _i(groups), _i(1 if write_state else 0), _i(below), _stream())
     return y
@@ -986,23 +1002,23 @@ def delta_rule(qkv: torch.Tensor, b_raw: torch.Tensor, b_col0: int, a_raw: torch
         raise KernelError(f"delta_rule: qkv {tuple(qkv.shape)}, b {tuple(b_raw.shape)}, a {tuple(a_raw.shape)}, state "
                           f"{tuple(state.shape)} do not fit {heads} heads ({key_heads} key heads) of {key_dim} x {vdim}")
     dev = qkv.device
-    kq = torch.empty((T, key_heads), dtype=torch.float32, device=dev)
-    beta = torch.empty((T, heads), dtype=torch.float32, device=dev)
-    raw_decays = (ctypes.c_void_p(a_raw.data_ptr() + 4 * a_col0), _i(a_raw.shape[1]), _ptr(dt_bias), _ptr(a_log))
-    o = torch.empty((T, heads * vdim), dtype=torch.float32, device=dev)
+    kq = _empty((T, key_heads), dtype=torch.float32, device=dev)
+    beta = _empty((T, heads), dtype=torch.float32, device=dev)
+    raw_decays = (_address(a_raw.data_ptr() + 4 * a_col0), _i(a_raw.shape[1]), _ptr(dt_bias), _ptr(a_log))
+    o = _empty((T, heads * vdim), dtype=torch.float32, device=dev)
     scratch, chunks_from, rest, decay = None, 0, True, None
     if ctx.max_new >= DELTA_CHUNKED_FROM and qkv.shape[1] % 4 == 0 and not (qkv.data_ptr() % 16 or state.data_ptr() % 16):
         size = _lookup("recurrent_chunks", "qwb_delta_chunked_scratch")[1]
         size.restype = ctypes.c_longlong
         chunks_from, rest = _forms(ctx, DELTA_CHUNKED_FROM)
         if rest:                                            # everything else the step needs first: what is left is the scratch's
-            decay = torch.empty((T, heads * decay_k), dtype=torch.float32, device=dev)
+            decay = _empty((T, heads * decay_k), dtype=torch.float32, device=dev)
         scratch = _chunk_scratch(size(_i(T), _i(ctx.n_seqs), _i(chunks_from), _i(heads), _i(key_dim), _i(vdim)), dev)
     if scratch is None:
         chunks_from, rest = 0, True
     if rest and decay is None:
-        decay = torch.empty((T, heads * decay_k), dtype=torch.float32, device=dev)
-    _call("recurrent", "qwb_delta_prep", _ptr(qkv), _i(qkv.shape[1]), _ptr(kq), ctypes.c_void_p(b_raw.data_ptr() + 4 * b_col0),
+        decay = _empty((T, heads * decay_k), dtype=torch.float32, device=dev)
+    _call("recurrent", "qwb_delta_prep", _ptr(qkv), _i(qkv.shape[1]), _ptr(kq), _address(b_raw.data_ptr() + 4 * b_col0),
           _i(b_raw.shape[1]), _ptr(beta), *raw_decays, _ptr(decay), _ptr(ctx.tok_seq) if chunks_from else _ptr(None), _ptr(ctx.cu_seqlens),
           _i(chunks_from), _i(T), _i(heads), _i(key_heads), _i(key_dim), _i(decay_k), _f(unit_eps), _f(q_scale), _stream())
     if scratch is not None:
@@ -1053,16 +1069,16 @@ def retention_scan(qkv: torch.Tensor, cos, sin, rotary_dim: int, decay: torch.Te
             if tuple(t.shape) != (T, rotary_dim // 2):
                 raise KernelError(f"retention_scan: table {name} {tuple(t.shape)} for {T} tokens and {rotary_dim} turned values")
     dev = qkv.device
-    kq = torch.empty((T, heads), dtype=torch.float32, device=dev)
+    kq = _empty((T, heads), dtype=torch.float32, device=dev)
     _call("recurrent", "qwb_turn_qk_prep", _ptr(qkv), _i(qkv.shape[1]), _ptr(kq), _ptr(cos), _ptr(sin), _i(T), _i(heads),
           _i(key_dim), _i(rotary_dim), _f(q_scale), _f(k_scale), _stream())
-    o = torch.empty((T, heads * vdim), dtype=torch.float32, device=dev)
+    o = _empty((T, heads * vdim), dtype=torch.float32, device=dev)
     if chunked is None:
         chunked = ctx.max_new >= RETENTION_CHUNKED_FROM
     if chunked and qkv.shape[1] % 4 == 0 and retention_chunked_fits(key_dim, vdim):
         # long prompts: chunks of 64 tokens side by side (three kernels) instead of a chain through every token
         n_chunks = -(-ctx.max_new // RETENTION_CHUNK)
-        scratch = torch.empty((2, ctx.n_seqs * n_chunks, heads, vdim, key_dim), dtype=torch.float32, device=dev)
+        scratch = _empty((2, ctx.n_seqs * n_chunks, heads, vdim, key_dim), dtype=torch.float32, device=dev)
         _call("recurrent", "qwb_retention_chunked", _ptr(qkv), _i(qkv.shape[1]), _ptr(decay), _ptr(state), _ptr(ctx.cu_seqlens),
               _ptr(ctx.slots), _ptr(scratch), _ptr(o), _i(ctx.n_seqs), _i(ctx.max_new), _i(heads), _i(key_dim), _i(vdim),
               _i(1 if write_state else 0), _stream(), kernels=3)
@@ -1094,11 +1110,11 @@ def gla_scan(qkv: torch.Tensor, a_raw: torch.Tensor, a_bias: torch.Tensor | None
         if a_bias.numel() != heads * key_dim:
             raise KernelError(f"gla_scan: a bias of {a_bias.numel()} for {heads} heads of {key_dim}")
     dev = qkv.device
-    kq = torch.empty((T, heads), dtype=torch.float32, device=dev)
-    decay = torch.empty((T, heads * key_dim), dtype=torch.float32, device=dev)
+    kq = _empty((T, heads), dtype=torch.float32, device=dev)
+    decay = _empty((T, heads * key_dim), dtype=torch.float32, device=dev)
     _call("recurrent", "qwb_gla_prep", _ptr(qkv), _i(qkv.shape[1]), _ptr(kq), _ptr(a_raw), _ptr(a_bias), _ptr(decay), _i(T),
           _i(heads), _i(key_dim), _f(q_scale), _f(tau), _stream())
-    o = torch.empty((T, heads * vdim), dtype=torch.float32, device=dev)
+    o = _empty((T, heads * vdim), dtype=torch.float32, device=dev)
     _call("recurrent", "qwb_delta_scan", _ptr(qkv), _i(qkv.shape[1]), _ptr(kq), _ptr(None), _ptr(decay), _ptr(state),
           _ptr(ctx.cu_seqlens), _ptr(ctx.slots), _ptr(o), _i(ctx.n_seqs), _i(heads), _i(heads), _i(key_dim), _i(vdim),
           _i(1 if write_state else 0), _i(heads * key_dim), _i(key_dim), _i(0), _stream())
@@ -1125,8 +1141,8 @@ def gated_part_norm(y: torch.Tensor, gate: torch.Tensor, gate_col0: int, weight:
         _need(divisor, "divisor", torch.float32, 2)
         if tuple(divisor.shape) != (T, n_parts):
             raise KernelError(f"gated_part_norm: divisor {tuple(divisor.shape)} for {T} rows of {n_parts} parts")
-    out = torch.empty((T, D), dtype=out_dtype, device=y.device)
-    _call("recurrent", "qwb_gated_part_norm", _ptr(y), ctypes.c_void_p(gate.data_ptr() + 4 * gate_col0), _i(gate.shape[1]),
+    out = _empty((T, D), dtype=out_dtype, device=y.device)
+    _call("recurrent", "qwb_gated_part_norm", _ptr(y), _address(gate.data_ptr() + 4 * gate_col0), _i(gate.shape[1]),
           _ptr(weight), _i(weight.numel()), _ptr(divisor), _ptr(out), _i(_dt(out_dtype)), _i(T), _i(n_parts), _i(D // n_parts), _f(eps),
           _i(0 if gate_first else (2 if gate_activation == "silu" else 1)), _stream())
     return out
@@ -1180,10 +1196,10 @@ def mlstm_scan(proj: torch.Tensor, i_col: int, f_col: int, i_bias: torch.Tensor,
         if t.numel() != heads:
             raise KernelError(f"mlstm_scan: {name} of {t.numel()} for {heads} heads")
     dev = proj.device
-    raw = torch.empty((T, heads * vdim), dtype=torch.float32, device=dev)
-    divisor = torch.empty((T, heads), dtype=torch.float32, device=dev)
+    raw = _empty((T, heads * vdim), dtype=torch.float32, device=dev)
+    divisor = _empty((T, heads), dtype=torch.float32, device=dev)
     single = ctx.single_token and T == ctx.n_seqs
-    gate_rows = None if single else torch.empty((3, T, heads), dtype=torch.float32, device=dev)
+    gate_rows = None if single else _empty((3, T, heads), dtype=torch.float32, device=dev)
     if chunked is None:
         chunked = ctx.max_new >= MLSTM_CHUNKED_FROM
     inputs = (_ptr(proj), _i(ld), _i(i_col), _i(f_col), _ptr(i_bias), _ptr(f_bias), _f(gate_cap), _ptr(state), _ptr(m_state),
@@ -1200,7 +1216,7 @@ def mlstm_scan(proj: torch.Tensor, i_col: int, f_col: int, i_bias: torch.Tensor,
                 return raw, divisor
         lib = _lookup("mlstm", "qwb_mlstm_scratch_floats")[0]
         lib.qwb_mlstm_scratch_floats.restype = ctypes.c_longlong
-        scratch = torch.empty((lib.qwb_mlstm_scratch_floats(_i(ctx.n_seqs), _i(ctx.max_new), _i(heads), _i(key_dim), _i(vdim)),),
+        scratch = _empty((lib.qwb_mlstm_scratch_floats(_i(ctx.n_seqs), _i(ctx.max_new), _i(heads), _i(key_dim), _i(vdim)),),
                               dtype=torch.float32, device=dev)
         _call("mlstm", "qwb_mlstm_chunked", *inputs, _ptr(scratch), _ptr(raw), _ptr(divisor), *sizes, _f(q_scale), _f(tiny),
               _i(1 if write_state else 0), _stream(), kernels=4)
@@ -1228,7 +1244,7 @@ def block_gates(u: torch.Tensor, w_a: torch.Tensor, b_a: torch.Tensor, w_i: torc
         _need(b, name + " bias", torch.float32)
         if blocks * n != C or tuple(w.shape) != (blocks, n, n) or b.numel() != C:
             raise KernelError(f"block_gates: {name} {tuple(w.shape)} with bias of {b.numel()} for {C} channels")
-    r = torch.empty((T, C), dtype=torch.float32, device=u.device)
+    r = _empty((T, C), dtype=torch.float32, device=u.device)
     i = torch.empty_like(r)
     _call("rglru", "qwb_block_gates", _ptr(u), _ptr(w_a), _ptr(b_a), _ptr(w_i), _ptr(b_i), _ptr(r), _ptr(i), _i(_dt(w_a.dtype)),
           _i(T), _i(C), _i(blocks), _stream())
@@ -1253,15 +1269,15 @@ def rglru_scan(u: torch.Tensor, r: torch.Tensor, i: torch.Tensor, lam: torch.Ten
                           f"{tuple(state.shape)}, y {tuple(y.shape)} from column {y_col0}")
     if y_bias is not None:
         _need(y_bias, "y_bias", torch.float32, 1)
-    out = torch.empty((T, C), dtype=out_dtype, device=u.device)
+    out = _empty((T, C), dtype=out_dtype, device=u.device)
     chunk = max_chunks = 0
     tables = scratch = None
     if ctx.max_new >= RGLRU_CHUNKED_FROM:
         chunk = RGLRU_CHUNK
         max_chunks = -(-T // chunk) + ctx.n_seqs
-        tables = torch.empty((2 * max_chunks + ctx.n_seqs + 1,), dtype=torch.int32, device=u.device)
-        scratch = torch.empty((2 * max_chunks * C,), dtype=torch.float32, device=u.device)
-    _call("rglru", "qwb_rglru_scan", _ptr(u), _ptr(r), _ptr(i), _ptr(lam), ctypes.c_void_p(y.data_ptr() + 4 * y_col0),
+        tables = _empty((2 * max_chunks + ctx.n_seqs + 1,), dtype=torch.int32, device=u.device)
+        scratch = _empty((2 * max_chunks * C,), dtype=torch.float32, device=u.device)
+    _call("rglru", "qwb_rglru_scan", _ptr(u), _ptr(r), _ptr(i), _ptr(lam), _address(y.data_ptr() + 4 * y_col0),
           _i(y.shape[1]), _ptr(y_bias), _ptr(state), _ptr(ctx.cu_seqlens), _ptr(ctx.slots), _ptr(out), _i(_dt(out_dtype)),
           _i(ctx.n_seqs), _i(C), _f(sharpness), _i(1 if write_state else 0), _i(chunk), _i(max_chunks), _ptr(tables),
           _ptr(scratch), _stream(), kernels=4 if chunk else 1)
@@ -1295,7 +1311,7 @@ def pool_prep(qkv: torch.Tensor, q_weight, k_weight, cos_qk, sin_qk, cos_v, sin_
             _need(t, name, torch.float32, 2)
             if tuple(t.shape) != (T, n // 2):
                 raise KernelError(f"pool_prep: table {name} {tuple(t.shape)} for {T} tokens and {n} turned values")
-    q = torch.empty((T, n_heads, dim), dtype=k_pool.dtype, device=qkv.device)
+    q = _empty((T, n_heads, dim), dtype=k_pool.dtype, device=qkv.device)
     _call("attention_pool", "qwb_pool_prep", _ptr(qkv), _ptr(q_weight), _ptr(k_weight), _ptr(cos_qk), _ptr(sin_qk), _ptr(cos_v),
           _ptr(sin_v), _ptr(ctx.tok_seq), _ptr(ctx.tok_pos), _ptr(page_table), _i(page_table.shape[1]), _ptr(q), _ptr(k_pool),
           _ptr(v_pool), _i(_dt(k_pool.dtype)), _i(T), _i(n_heads), _i(n_kv_heads), _i(dim), _i(vdim),
@@ -1329,7 +1345,7 @@ def pool_attention(q: torch.Tensor, k_pool, v_pool, pk_pool, pv_pool, page_table
     _need(q, "q", k_pool.dtype, 3)
     T, H, dim = q.shape
     G, vdim = k_pool.shape[1], v_pool.shape[3]
-    out = torch.empty((T, H * vdim), dtype=q.dtype, device=q.device)
+    out = _empty((T, H * vdim), dtype=q.dtype, device=q.device)
     width = page_table.shape[1]
     if block_table is not None and block_table.shape[1] != width:
         raise KernelError("pool_attention: the two page tables differ in width")
@@ -1338,7 +1354,7 @@ def pool_attention(q: torch.Tensor, k_pool, v_pool, pk_pool, pv_pool, page_table
         block_runs = ctypes.c_int(0)
         n_runs = lib.qwb_pool_decode_runs(_i(ctx.max_len), _i(window), _i(pool), ctypes.byref(block_runs))
         lib.qwb_pool_decode_scratch_floats.restype = ctypes.c_longlong
-        scratch = torch.empty((lib.qwb_pool_decode_scratch_floats(_i(T), _i(H), _i(vdim), _i(n_runs)),), dtype=torch.float32,
+        scratch = _empty((lib.qwb_pool_decode_scratch_floats(_i(T), _i(H), _i(vdim), _i(n_runs)),), dtype=torch.float32,
                               device=q.device)
         _call("attention_pool", "qwb_pool_decode", _ptr(q), _ptr(k_pool), _ptr(v_pool), _ptr(pk_pool), _ptr(pv_pool),
               _ptr(page_table), _ptr(block_table), _ptr(ctx.seq_len), _ptr(cos_v), _ptr(sin_v), _ptr(scratch), _ptr(out),
@@ -1397,7 +1413,7 @@ def maps_prep(qkv: torch.Tensor, bias, q_weight, k_weight, cos, sin, ctx, page_t
             _need(t, name, torch.float32, 2)
             if tuple(t.shape) != (T, rotary_dim // 2):
                 raise KernelError(f"maps_prep: table {name} {tuple(t.shape)} for {T} tokens and {rotary_dim} turned values")
-    q = torch.empty((T, n_heads, maps * dim), dtype=k_pool.dtype, device=qkv.device)
+    q = _empty((T, n_heads, maps * dim), dtype=k_pool.dtype, device=qkv.device)
     if whole_norm:
         _call("attention_maps", "qwb_maps_row_prep", _ptr(qkv), _i(ld), _ptr(bias), _ptr(q_weight), _ptr(k_weight), _ptr(cos), _ptr(sin),
               _ptr(ctx.tok_seq), _ptr(ctx.tok_pos), _ptr(page_table), _i(page_table.shape[1]), _ptr(q), _ptr(k_pool), _ptr(v_pool),
@@ -1445,7 +1461,7 @@ def maps_attention(q: torch.Tensor, k_pool, v_pool, page_table, ctx, maps: int, 
     if kdim % maps or k_pool.shape[3] != kdim:
         raise KernelError(f"maps_attention: q {tuple(q.shape)} and keys {tuple(k_pool.shape)} with {maps} maps")
     dim = kdim // maps
-    out = torch.empty((T, H * vdim), dtype=q.dtype, device=q.device)
+    out = _empty((T, H * vdim), dtype=q.dtype, device=q.device)
     width = page_table.shape[1]
     gate_args = _column_gate("maps_attention", gate, gate_col0, T, H)
     one_map = (maps == 1 and softcap <= 0.0 and not norm_out and gate is None and not (chunk and window) and impl in ("auto", "tc")
@@ -1454,9 +1470,9 @@ def maps_attention(q: torch.Tensor, k_pool, v_pool, page_table, ctx, maps: int, 
         return attn_decode(q, k_pool, v_pool, page_table, ctx.seq_len, scale, ctx.max_len, window=window, impl="mma")
     if ctx.single_token and dim % MAPS_FAST_STEP == 0 and vdim % MAPS_FAST_STEP == 0:
         lib = _lookup("attention_maps", "qwb_maps_decode_runs")[0]
-        n_runs = lib.qwb_maps_decode_runs(_ptr(q), _i(_dt(q.dtype)), _i(maps), _i(dim), _i(vdim), _i(ctx.max_len), _i(chunk), _i(window))
+        n_runs = lib.qwb_maps_decode_runs(ctypes.c_void_p(q.data_ptr()), _i(_dt(q.dtype)), _i(maps), _i(dim), _i(vdim), _i(ctx.max_len), _i(chunk), _i(window))
         lib.qwb_maps_decode_scratch_floats.restype = ctypes.c_longlong
-        scratch = torch.empty((lib.qwb_maps_decode_scratch_floats(_i(T), _i(H), _i(maps), _i(vdim), _i(n_runs)),),
+        scratch = _empty((lib.qwb_maps_decode_scratch_floats(_i(T), _i(H), _i(maps), _i(vdim), _i(n_runs)),),
                               dtype=torch.float32, device=q.device)
         _call("attention_maps", "qwb_maps_decode", _ptr(q), _ptr(k_pool), _ptr(v_pool), _ptr(page_table), _ptr(ctx.seq_len),
               _ptr(scratch), _ptr(out), _i(_dt(q.dtype)), _i(T), _i(H), _i(G), _i(maps), _i(dim), _i(vdim), _i(width), _f(scale),
@@ -1530,7 +1546,7 @@ def bias_prep(qkv: torch.Tensor, bias, q_weight, k_weight, cos, sin, ctx, page_t
             _need(t, name, torch.float32, 2)
             if tuple(t.shape) != (T, rotary_dim // 2):
                 raise KernelError(f"bias_prep: table {name} {tuple(t.shape)} for {T} tokens and {rotary_dim} turned values")
-    q = torch.empty((T, n_heads, dim), dtype=k_pool.dtype, device=qkv.device)
+    q = _empty((T, n_heads, dim), dtype=k_pool.dtype, device=qkv.device)
     _call("attention_bias", "qwb_bias_prep", _ptr(qkv), _ptr(bias), _ptr(q_weight), _ptr(k_weight), _ptr(cos), _ptr(sin),
           _ptr(ctx.tok_seq), _ptr(ctx.tok_pos), _ptr(page_table), _i(page_table.shape[1]), _ptr(q), _ptr(k_pool), _ptr(v_pool),
           _i(_dt(k_pool.dtype)), _i(T), _i(n_heads), _i(n_kv_heads), _i(dim), _i(vdim), _i(rotary_dim),
@@ -1585,13 +1601,13 @@ def bias_attention(q: torch.Tensor, k_pool, v_pool, page_table, ctx, scale: floa
         lib = _lookup("attention_bias", "qwb_bias_decode_runs")[0]
         n_runs = lib.qwb_bias_decode_runs(_i(ctx.max_len), _i(window))
         lib.qwb_bias_decode_mixed_scratch_floats.restype = ctypes.c_longlong
-        scratch = torch.empty((lib.qwb_bias_decode_mixed_scratch_floats(_i(T), _i(H), _i(vdim), _i(n_runs)),),
+        scratch = _empty((lib.qwb_bias_decode_mixed_scratch_floats(_i(T), _i(H), _i(vdim), _i(n_runs)),),
                               dtype=torch.float32, device=q.device)
-        out = torch.empty((T, H * vdim), dtype=q.dtype, device=q.device)
+        out = _empty((T, H * vdim), dtype=q.dtype, device=q.device)
         _call("attention_bias", "qwb_bias_decode_mixed", _ptr(q), _ptr(k_pool), _ptr(v_pool), _ptr(page_table), _ptr(ctx.seq_len),
               _ptr(scratch), _ptr(out), _i(_dt(q.dtype)), _i(T), _i(H), _i(G), _i(dim), _i(vdim), _i(width), _f(scale),
               _ptr(head_scale), _f(softcap), _ptr(slopes), _i(window), _ptr(sinks), _ptr(head_mix),
-              ctypes.c_void_p(gate.data_ptr() + 4 * gate_col0) if gate is not None else _ptr(None),
+              _address(gate.data_ptr() + 4 * gate_col0) if gate is not None else _ptr(None),
               _i(gate.shape[1] if gate is not None else 0), _i(n_runs), _stream(), kernels=4)
         return out
     all_values = head_mix is not None
@@ -1599,12 +1615,12 @@ def bias_attention(q: torch.Tensor, k_pool, v_pool, page_table, ctx, scale: floa
     C = G if all_values else 1
     width = page_table.shape[1]
     dev = q.device
-    att = torch.empty((T, H, C, vdim) if raw else (T, H * vdim), dtype=torch.float32 if raw else q.dtype, device=dev)
+    att = _empty((T, H, C, vdim) if raw else (T, H * vdim), dtype=torch.float32 if raw else q.dtype, device=dev)
     if ctx.single_token and dim % BIAS_ATTN_FAST_STEP == 0 and vdim % BIAS_ATTN_FAST_STEP == 0:
         lib = _lookup("attention_bias", "qwb_bias_decode_runs")[0]
         n_runs = lib.qwb_bias_decode_runs(_i(ctx.max_len), _i(window))
         lib.qwb_bias_decode_scratch_floats.restype = ctypes.c_longlong
-        scratch = torch.empty((lib.qwb_bias_decode_scratch_floats(_i(T), _i(H), _i(C), _i(vdim), _i(n_runs)),),
+        scratch = _empty((lib.qwb_bias_decode_scratch_floats(_i(T), _i(H), _i(C), _i(vdim), _i(n_runs)),),
                               dtype=torch.float32, device=dev)
         _call("attention_bias", "qwb_bias_decode", _ptr(q), _ptr(k_pool), _ptr(v_pool), _ptr(page_table), _ptr(ctx.seq_len),
               _ptr(scratch), _ptr(att), _i(_dt(q.dtype)), _i(1 if raw else 0), _i(T), _i(H), _i(G), _i(1 if all_values else 0),
@@ -1628,9 +1644,9 @@ def bias_attention(q: torch.Tensor, k_pool, v_pool, page_table, ctx, scale: floa
               _i(window), _ptr(sinks), _stream())
     if not raw:
         return att
-    out = torch.empty((T, H * vdim), dtype=q.dtype, device=dev)
+    out = _empty((T, H * vdim), dtype=q.dtype, device=dev)
     _call("attention_bias", "qwb_bias_head_mix", _ptr(att), _ptr(head_mix),
-          ctypes.c_void_p(gate.data_ptr() + 4 * gate_col0) if gate is not None else _ptr(None),
+          _address(gate.data_ptr() + 4 * gate_col0) if gate is not None else _ptr(None),
           _i(gate.shape[1] if gate is not None else 0), _ptr(out), _i(_dt(q.dtype)), _i(T), _i(H), _i(G),
           _i(1 if all_values else 0), _i(vdim), _stream())
     return out
@@ -1674,13 +1690,13 @@ def latent_prep(q: torch.Tensor, dkv: torch.Tensor | None, c_weight: torch.Tenso
                           f"{heads} heads of {dim} + {rot_dim}, latent {rank}")
     q_plain = q_rot = q_full = row_new = None
     if whole_heads:
-        q_full = torch.empty((T, heads, dim + rot_dim), dtype=pool.dtype, device=q.device)
-        row_new = torch.empty((T, rank + rot_dim), dtype=pool.dtype, device=q.device) if dkv is not None else None
+        q_full = _empty((T, heads, dim + rot_dim), dtype=pool.dtype, device=q.device)
+        row_new = _empty((T, rank + rot_dim), dtype=pool.dtype, device=q.device) if dkv is not None else None
     else:
-        q_plain = torch.empty((heads, T, dim), dtype=pool.dtype, device=q.device)
-        q_rot = torch.empty((T, heads, rot_dim), dtype=torch.float32, device=q.device)
+        q_plain = _empty((heads, T, dim), dtype=pool.dtype, device=q.device)
+        q_rot = _empty((T, heads, rot_dim), dtype=torch.float32, device=q.device)
     _call("attention_latent", "qwb_latent_prep", _ptr(q), _i(q.shape[1]),
-          ctypes.c_void_p(dkv.data_ptr() + 4 * dkv_col0) if dkv is not None else _ptr(None), _i(dkv.shape[1] if dkv is not None else 0), _ptr(c_weight), _ptr(cos), _ptr(sin), _ptr(ctx.tok_seq),
+          _address(dkv.data_ptr() + 4 * dkv_col0) if dkv is not None else _ptr(None), _i(dkv.shape[1] if dkv is not None else 0), _ptr(c_weight), _ptr(cos), _ptr(sin), _ptr(ctx.tok_seq),
           _ptr(ctx.tok_pos), _ptr(page_table), _ptr(pool), _i(_dt(pool.dtype)), _ptr(q_plain), _ptr(q_rot), _ptr(q_full),
           _ptr(row_new), _i(T), _i(heads), _i(dim), _i(rot_dim), _i(rank), _i(half), _f(eps), _i(pool.shape[2]),
           _i(page_table.shape[1]), _i(1 if store else 0), _stream())
@@ -1720,16 +1736,16 @@ def latent_prefill(q: torch.Tensor, k_plain: torch.Tensor, rows: torch.Tensor, v
         raise KernelError(f"latent_prefill: q {tuple(q.shape)}, k {tuple(k_plain.shape)}, rows {tuple(rows.shape)}, v {tuple(v.shape)}")
     if sink is not None:
         _need(sink, "sink", torch.float32, 1)
-    out = torch.empty((T, heads * vdim), dtype=torch.bfloat16, device=q.device)
+    out = _empty((T, heads * vdim), dtype=torch.bfloat16, device=q.device)
     ld = rows.shape[1]
     if scale > 0.0 and ld % 8 == 0 and latent_prefill_tc_fits(dim, rot_dim, vdim):
         _call("attention_streams", "qwb_latent_prefill_tc", _ptr(q), _ptr(k_plain),
-              ctypes.c_void_p(rows.data_ptr() + 2 * (ld - rot_dim)), _i(ld), _ptr(v), _ptr(ctx.cu_seqlens), _ptr(sink), _ptr(out),
+              _address(rows.data_ptr() + 2 * (ld - rot_dim)), _i(ld), _ptr(v), _ptr(ctx.cu_seqlens), _ptr(sink), _ptr(out),
               _i(ctx.n_seqs), _i(T), _i(ctx.max_new), _i(heads), _i(dim), _i(rot_dim), _i(vdim), _f(scale), _i(window),
               *_column_gate("latent_prefill", gate, gate_col0, T, heads), _ptr(gemm_tc_error_word(q.device)), _stream())
         return out
     _call("attention_latent_mma", "qwb_latent_prefill_mma", _ptr(q), _ptr(k_plain),
-          ctypes.c_void_p(rows.data_ptr() + 2 * (ld - rot_dim)), _i(ld), _ptr(v), _ptr(ctx.cu_seqlens), _ptr(sink), _ptr(out),
+          _address(rows.data_ptr() + 2 * (ld - rot_dim)), _i(ld), _ptr(v), _ptr(ctx.cu_seqlens), _ptr(sink), _ptr(out),
           _i(ctx.n_seqs), _i(ctx.max_new), _i(heads), _i(dim), _i(rot_dim), _i(vdim), _f(scale), _i(window),
           *_column_gate("latent_prefill", gate, gate_col0, T, heads), _stream())
     return out
@@ -1740,7 +1756,7 @@ def latent_heads_out(values: torch.Tensor, dtype: torch.dtype, gate: torch.Tenso
     ``gate_col0 + h`` of the float32 matrix ``gate`` [T, ld] if that is given."""
     _need(values, "values", torch.float32, 3)
     H, T, P = values.shape
-    out = torch.empty((T, H * P), dtype=dtype, device=values.device)
+    out = _empty((T, H * P), dtype=dtype, device=values.device)
     _call("attention_latent", "qwb_latent_heads_out", _ptr(values), *_column_gate("latent_heads_out", gate, gate_col0, T, H), _ptr(out),
           _i(_dt(dtype)), _i(T), _i(H), _i(P), _stream())
     return out
@@ -1764,7 +1780,7 @@ def latent_attention(q_abs: torch.Tensor, q_rot: torch.Tensor, pool: torch.Tenso
         _need(sink, "sink", torch.float32, 1)
         if sink.numel() != H:
             raise KernelError(f"latent_attention: {sink.numel()} sinks for {H} heads")
-    out = torch.empty((H, T, L), dtype=pool.dtype, device=q_abs.device)
+    out = _empty((H, T, L), dtype=pool.dtype, device=q_abs.device)
     max_runs, scratch = 0, None
     if ctx.single_token and T == ctx.n_seqs and not (pool.data_ptr() % 16 or q_abs.data_ptr() % 8 or q_rot.data_ptr() % 8):
         # bfloat16 rows in sizes that the tensor-core kernel takes: runs by each sequence's own length, then a merge
@@ -1772,7 +1788,7 @@ def latent_attention(q_abs: torch.Tensor, q_rot: torch.Tensor, pool: torch.Tenso
                                                                                  _i(ctx.max_len), _i(window))
     if max_runs:
         if max_runs > 1:
-            scratch = torch.empty((max_runs * T * H * (L + 2),), dtype=torch.float32, device=q_abs.device)
+            scratch = _empty((max_runs * T * H * (L + 2),), dtype=torch.float32, device=q_abs.device)
         _call("attention_latent", "qwb_latent_decode_mma", _ptr(q_abs), _ptr(q_rot), _ptr(pool), _ptr(page_table), _ptr(ctx.pos0),
               _ptr(sink), _ptr(out), _i(T), _i(H), _i(L), _i(R), _i(pool.shape[2]), _i(page_table.shape[1]), _f(scale), _i(window),
               _i(max_runs), _ptr(scratch), _stream(), kernels=2 if max_runs > 1 else 1)
@@ -1781,7 +1797,7 @@ def latent_attention(q_abs: torch.Tensor, q_rot: torch.Tensor, pool: torch.Tenso
         # one token per sequence over more than one run of keys: a block a run (cut by the key's index, so a sequence's
         # result does not depend on the batch), then a merge; ctx.max_len bounds every sequence's length
         max_runs = -(-ctx.max_len // LATENT_RUN_KEYS)
-        scratch = torch.empty((max_runs * T * H * (L + 2),), dtype=torch.float32, device=q_abs.device)
+        scratch = _empty((max_runs * T * H * (L + 2),), dtype=torch.float32, device=q_abs.device)
     _call("attention_latent", "qwb_latent_attn", _ptr(q_abs), _ptr(q_rot), _ptr(pool), _ptr(page_table), _ptr(ctx.cu_seqlens),
           _ptr(ctx.pos0), _ptr(sink), _ptr(out), _i(_dt(pool.dtype)), _i(ctx.n_seqs), _i(T), _i(ctx.max_new), _i(H), _i(L),
           _i(R), _i(pool.shape[2]), _i(page_table.shape[1]), _f(scale), _i(window), _i(max_runs), _ptr(scratch), _stream(),
@@ -1813,9 +1829,9 @@ def moe_route(logits: torch.Tensor, top: int, renormalize: bool = False, experts
         _need(correction, "correction", torch.float32, 1)
         if correction.numel() != E:
             raise KernelError(f"moe_route: correction of {correction.numel()} for {E} experts")
-    chosen = torch.empty((T, top), dtype=torch.int32, device=logits.device)
-    weight = torch.empty((T, top), dtype=torch.float32, device=logits.device)
-    gate_out = torch.empty((T,), dtype=torch.float32, device=logits.device) if gate else None
+    chosen = _empty((T, top), dtype=torch.int32, device=logits.device)
+    weight = _empty((T, top), dtype=torch.float32, device=logits.device)
+    gate_out = _empty((T,), dtype=torch.float32, device=logits.device) if gate else None
     _call("moe", "qwb_moe_route", _ptr(logits), _i(ld), _ptr(correction), _ptr(chosen), _ptr(weight), _ptr(gate_out), _i(T), _i(E),
           _i(top), _i(MOE_SCORES.index(scores)), _i(groups), _i(keep), _i(1 if renormalize else 0), _f(sum_eps), _f(weight_scale), _stream())
     return (chosen, weight, gate_out) if gate else (chosen, weight)
@@ -1878,14 +1894,14 @@ def moe_experts(x: torch.Tensor, w_up: torch.Tensor, w_down: torch.Tensor, chose
         if tuple(out.shape) != (T, D):
             raise KernelError(f"moe_experts: out {tuple(out.shape)} for {T} x {D}")
     else:
-        out = torch.empty((T, D), dtype=torch.float32, device=x.device)
-    act = torch.empty((T * top, F), dtype=x.dtype, device=x.device)
-    act_s = torch.empty((T, Fs), dtype=x.dtype, device=x.device) if Fs else None
+        out = _empty((T, D), dtype=torch.float32, device=x.device)
+    act = _empty((T * top, F), dtype=x.dtype, device=x.device)
+    act_s = _empty((T, Fs), dtype=x.dtype, device=x.device) if Fs else None
     stream = x.dtype == torch.bfloat16 and (4 * T * top >= max(3 * E, 4 * MOE_STREAM_MIN_CHOICES) or T >= MOE_STREAM_MIN_TOKENS) and moe_stream_fits(D, F, Fs, top) and not any(
         t.data_ptr() % 16 for t in (x, w_up, w_down, out, shared_up, shared_down) if t is not None)
     per = MOE_STREAM_COPIES // top if stream else max(1, _MOE_SLOTS_PER_LAUNCH // (top + 1))
     if stream:
-        y = torch.empty((min(per, T) * (top + (1 if Fs else 0)) * D + _lookup("moe", "qwb_moe_lists_floats")[1](),), dtype=torch.float32, device=x.device)
+        y = _empty((min(per, T) * (top + (1 if Fs else 0)) * D + _lookup("moe", "qwb_moe_lists_floats")[1](),), dtype=torch.float32, device=x.device)
     for t0 in range(0, T, per):
         n = min(per, T - t0)
         cut = (lambda t: None if t is None else t[t0:t0 + n])
@@ -1918,7 +1934,7 @@ def moe_sort(chosen: torch.Tensor, experts: int):
     where each expert's run ends)."""
     _need(chosen, "chosen", torch.int32, 2)
     place = torch.empty_like(chosen)
-    ends = torch.empty((experts,), dtype=torch.int32, device=chosen.device)
+    ends = _empty((experts,), dtype=torch.int32, device=chosen.device)
     _call("moe", "qwb_moe_sort", _ptr(chosen), _ptr(place), _ptr(ends), _i(chosen.numel()), _i(experts), _stream())
     return place, ends
 
@@ -1940,16 +1956,16 @@ def moe_experts_grouped(x: torch.Tensor, w_up: torch.Tensor, w_down: torch.Tenso
             if tuple(t.shape) != shape:
                 raise KernelError(f"moe_experts_grouped: {name} {tuple(t.shape)}, wanted {shape}")
     place, ends = moe_sort(chosen, E)
-    xs = torch.empty((T * top, D), dtype=torch.bfloat16, device=x.device)
-    row_weight = torch.empty((T * top,), dtype=torch.float32, device=x.device) if weight_on_input else None
+    xs = _empty((T * top, D), dtype=torch.bfloat16, device=x.device)
+    row_weight = _empty((T * top,), dtype=torch.float32, device=x.device) if weight_on_input else None
     _call("moe", "qwb_moe_spread", _ptr(x), _ptr(place), _ptr(xs), _ptr(weight if weight_on_input else None), _ptr(row_weight), _i(T), _i(D), _i(top), _stream())
     u = torch._grouped_mm(xs, w_up.transpose(1, 2), offs=ends).contiguous()
-    act = torch.empty((T * top, F), dtype=torch.bfloat16, device=x.device)
+    act = _empty((T * top, F), dtype=torch.bfloat16, device=x.device)
     _call("moe", "qwb_moe_act", _ptr(u), _ptr(row_weight), _ptr(act), _i(T * top), _i(F), _i(MOE_ACTIVATIONS[activation]), _stream())
     y = torch._grouped_mm(act, w_down.transpose(1, 2), offs=ends).contiguous()
     onto = out is not None
     if not onto:
-        out = torch.empty((T, D), dtype=torch.float32, device=x.device)
+        out = _empty((T, D), dtype=torch.float32, device=x.device)
     _call("moe", "qwb_moe_combine", _ptr(y), _ptr(place), _ptr(None if weight_on_input else weight), _ptr(shared), _ptr(gate), _ptr(out), _i(T), _i(D), _i(top),
           _i(1 if onto else 0), _stream())
     return out
@@ -1979,13 +1995,13 @@ def sample(logits: torch.Tensor, temperature: float, top_k: int = 0, top_p: floa
     if seed_from is not None:
         _need(seed_from, "seed_from", torch.int64, 1)
     if out is None:
-        out = torch.empty((B,), dtype=torch.int32, device=logits.device)
+        out = _empty((B,), dtype=torch.int32, device=logits.device)
     # few rows and a small top-k: the kernels cut every row into chunks and want scratch memory for what the chunks find
-    scratch_bytes = (_lookup("sampling", "qwb_sample_scratch_bytes")[1](_i(B), _i(V), _f(temperature), _i(top_k), _f(top_p))
+    scratch_bytes = (_lookup("sampling", "qwb_sample_scratch_bytes")[1](_i(B), _i(V), ctypes.c_float(temperature), _i(top_k), ctypes.c_float(top_p))
                      if split else 0)
     scratch = counters = None
     if scratch_bytes:
-        scratch = torch.empty((scratch_bytes,), dtype=torch.uint8, device=logits.device)
+        scratch = _empty((scratch_bytes,), dtype=torch.uint8, device=logits.device)
         if temperature > 0:
             counters = _sample_counters(logits.device, B)
     _call("sampling", "qwb_sample", _ptr(logits), _i(B), _i(V), _ptr(recent), _i(window), _f(repeat_penalty),

@@ -1,0 +1,79 @@
+"""The way from Python to the launchers: arguments arrive as ctypes would pass them, outputs are torch.empty's."""
+import ctypes
+import shutil
+import subprocess
+
+import pytest
+import torch
+
+from questwend_b200.kernels import build
+
+SOURCE = """
+#include <string.h>
+static unsigned char seen[512];
+int take(void* a, int b, float c, double d, long long e, void* g, int h, int i, int j, unsigned k, float l, unsigned long long m, int n, float o, void* p, int q) {
+    unsigned char* s = seen;
+#define KEEP(x) memcpy(s, &x, sizeof x); s += sizeof x
+    KEEP(a); KEEP(b); KEEP(c); KEEP(d); KEEP(e); KEEP(g); KEEP(h); KEEP(i); KEEP(j); KEEP(k); KEEP(l); KEEP(m); KEEP(n); KEEP(o); KEEP(p); KEEP(q);
+    return (int)(s - seen);
+}
+int refuse(void) { return -7; }
+void* what(void) { return seen; }
+"""
+
+
+@pytest.fixture(scope="module")
+def host():
+    if not shutil.which("g++") and not build.host_calls_built():
+        pytest.skip("no g++")
+    build.compile_host_calls()
+    module = build.host_calls()
+    assert module is not None
+    return module
+
+
+@pytest.fixture(scope="module")
+def lib(tmp_path_factory):
+    if not shutil.which("gcc"):
+        pytest.skip("no gcc")
+    d = tmp_path_factory.mktemp("c")
+    (d / "take.c").write_text(SOURCE)
+    subprocess.run(["gcc", "-O1", "-shared", "-fPIC", "-o", str(d / "take.so"), str(d / "take.c")], check=True)
+    lib = ctypes.CDLL(str(d / "take.so"))
+    lib.what.restype = ctypes.c_void_p
+    return lib
+
+
+def test_arguments_arrive_as_through_ctypes(host, lib):
+    t, u = torch.arange(6.0)[2:], torch.zeros(3, dtype=torch.bfloat16)
+    address = lambda name: ctypes.cast(getattr(lib, name), ctypes.c_void_p).value
+    n = lib.take(ctypes.c_void_p(t.data_ptr()), ctypes.c_int(-3), ctypes.c_float(1e-6), ctypes.c_double(-2.25), ctypes.c_longlong(-(2 ** 40)), ctypes.c_void_p(0), ctypes.c_int(1),
+                 ctypes.c_int(2 ** 31 - 1), ctypes.c_int(0), ctypes.c_uint(2 ** 32 - 5), ctypes.c_float(0.1), ctypes.c_ulonglong(2 ** 64 - 2), ctypes.c_int(9),
+                 ctypes.c_float(-0.0), ctypes.c_void_p(u.data_ptr()), ctypes.c_int(77))
+    want = ctypes.string_at(lib.what(), n)
+    ctypes.memset(lib.what(), 0, n)
+    args = (t, -3, 1e-6, ctypes.c_double(-2.25), ctypes.c_longlong(-(2 ** 40)), None, True, 2 ** 31 - 1, False, ctypes.c_uint(2 ** 32 - 5), 0.1, ctypes.c_ulonglong(2 ** 64 - 2), 9,
+            ctypes.c_float(-0.0), torch.nn.Parameter(u, requires_grad=False), 77)
+    assert host.call(address("take"), *args) == n and ctypes.string_at(lib.what(), n) == want
+    assert host.call(address("refuse")) == -7
+    for bad in (("x",), ([1],), (1j,), tuple(range(57)), (0.5,) * 9):
+        with pytest.raises((TypeError, AttributeError)):
+            host.call(address("refuse"), *bad)
+    with pytest.raises(ValueError):
+        host.call(0)
+
+
+def test_tensors_that_fit_and_outputs(host):
+    assert not host.fits(torch.zeros(2), torch.float32, 1) and not host.fits(None, None, None) and not host.fits("x", None, 1)      # none on a GPU
+    for shape, dtype in (((2, 3), torch.bfloat16), ((), torch.int32), ((0, 5), torch.float64), (4, torch.uint8), ([2, 2], torch.float32)):
+        for device in (torch.device("cpu"), "cpu"):
+            t = host.empty(shape, dtype=dtype, device=device)
+            want = torch.empty(shape, dtype=dtype, device=device)
+            assert t.shape == want.shape and t.dtype == dtype and t.device == want.device and t.is_contiguous() and not t.requires_grad
+    for bad in (dict(dtype=torch.float32, device="nowhere"), dict(dtype=3, device="cpu")):
+        with pytest.raises((TypeError, RuntimeError)):
+            host.empty((2,), **bad)
+    with pytest.raises(RuntimeError):
+        host.empty((-1,), dtype=torch.float32, device=torch.device("cpu"))
+    x = object()
+    assert host.same(x) is x
