@@ -1,4 +1,4 @@
-// What the chunked recurrences share: copies into shared memory and the sums of a thread's 8 x 8 outputs.
+// What the chunked recurrences share: copies into shared memory, and which sequences they take.
 #pragma once
 
 #include "common.cuh"
@@ -31,20 +31,4 @@ __device__ __forceinline__ int rc_sequence(const int* __restrict__ cu_seqlens, i
         z -= n;
     }
     return -1;
-}
-
-// acc[8][8] += a[8] x b[8] for `STEPS` rows of two tiles in shared memory: row r of the first at A + r * lda, whose values
-// a0 .. a0 + 3 and a1 .. a1 + 3 are this thread's, and the same for B.
-template <int STEPS>
-__device__ __forceinline__ void rc_outer(float (&acc)[8][8], const float* A, int lda, int a0, int a1, const float* B, int ldb, int b0, int b1) {
-#pragma unroll 8
-    for (int r = 0; r < STEPS; ++r) {
-        const float4 x0 = *reinterpret_cast<const float4*>(A + r * lda + a0), x1 = *reinterpret_cast<const float4*>(A + r * lda + a1);
-        const float4 y0 = *reinterpret_cast<const float4*>(B + r * ldb + b0), y1 = *reinterpret_cast<const float4*>(B + r * ldb + b1);
-        const float x[8] = {x0.x, x0.y, x0.z, x0.w, x1.x, x1.y, x1.z, x1.w}, y[8] = {y0.x, y0.y, y0.z, y0.w, y1.x, y1.y, y1.z, y1.w};
-#pragma unroll
-        for (int i = 0; i < 8; ++i)
-#pragma unroll
-            for (int j = 0; j < 8; ++j) acc[i][j] += x[i] * y[j];
-    }
 }

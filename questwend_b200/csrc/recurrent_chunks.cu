@@ -170,7 +170,7 @@ extern "C" int qwb_ssm_chunked(const float* xbc, int ldx, const float* dt_raw, i
 // walk 133, out 49 in ncu), three sequences of 2,900 in all 1,194 -> 484 us; a decay per head, four of 4,096 in all, 1,198 -> 596 us.
 // Bound by what shared memory hands to registers (128 bytes a cycle), the walk more than the others.
 // Scratch of a place and head:
-//     W [64][K] | k e_end [64][K] | q e_0 [64][K] | Q [64 (j)][64 (i)] | U, then u [64][P] | decay of the chunk [K] | S0 [K][P]
+//     W [64][K] | k e_end [64][K] | q e_0 [64][K] | Q [64 (i)][64 (j)] | U, then u [64][P] | decay of the chunk [K] | S0 [K][P]
 // ---------------------------------------------------------------------------------
 #define DC_TOKENS 64
 #define DC_SUB 16
@@ -181,6 +181,7 @@ struct DcArgs {
     const float *qkv, *beta, *a_raw, *dt_bias, *A_log;
     const int *cu_seqlens, *slots;
     float *state, *o, *scratch;
+    int* error;
     int ld, ld_a, H, Hk, K, P, decay_k, write_state, B, from;
 };
 struct DcPlace { float *w, *k_end, *q0, *q_pairs, *u, *decay, *start; };
@@ -269,37 +270,49 @@ delta_chunk_prep_kernel(const DcArgs a) {
         }
     }
     __syncthreads();
-    // pairs of one sub-block, four threads a token j: i goes down the tokens from j on, and what decays on the way is summed from j
+    // pairs of one sub-block, eight threads two tokens j: i goes down the tokens from j on, and what decays on the way is summed from j
     // on, never taken as the difference of two sums from the sub-block's start (after a token that forgets, the difference has
-    // lost the digits of those that keep, and after a logarithm of -infinity it is no number)
-    const int lane4 = (tid & 3) * 4;
+    // lost the digits of those that keep, and after a logarithm of -infinity it is no number).  Bound by the 16-byte loads, which cost
+    // the same however many threads read one address: with four threads a token they served one j each, not two (29,000 of the
+    // block's 75,000 cycles).
     {
-        const int j = tid >> 2, end = (j / DC_SUB + 1) * DC_SUB;
-        float4 kj[DC_MAX_K / 16], sum[DC_MAX_K / 16];
+        const int lane8 = (tid & 7) * 4, j0 = 8 * warp + ((tid >> 3) & 3), end = (j0 / DC_SUB + 1) * DC_SUB;       // tokens j0 and j0 + 4
+        float4 kj[2][DC_MAX_K / 32], sum[2][DC_MAX_K / 32];
 #pragma unroll
-        for (int c = 0; c < DC_MAX_K / 16; ++c) {
-            kj[c] = lane4 + 16 * c < K ? *reinterpret_cast<const float4*>(ks + dc_at(j, lane4 + 16 * c)) : make_float4(0.f, 0.f, 0.f, 0.f);
-            sum[c] = make_float4(0.f, 0.f, 0.f, 0.f);
-        }
+        for (int e = 0; e < 2; ++e)
+#pragma unroll
+            for (int c = 0; c < DC_MAX_K / 32; ++c) {
+                kj[e][c] = lane8 + 32 * c < K ? *reinterpret_cast<const float4*>(ks + dc_at(j0 + 4 * e, lane8 + 32 * c)) : make_float4(0.f, 0.f, 0.f, 0.f);
+                sum[e][c] = make_float4(0.f, 0.f, 0.f, 0.f);
+            }
 #pragma unroll 1
         for (int i = 8 * warp; i < end; ++i) {                      // from the first of the warp's eight tokens on
-            float sa = 0.f, sq = 0.f;
+            float sa[2] = {0.f, 0.f}, sq[2] = {0.f, 0.f};
 #pragma unroll
-            for (int c = 0; c < DC_MAX_K / 16; ++c) {
-                if (lane4 + 16 * c >= K) continue;
-                const int pi = dc_at(i, lane4 + 16 * c);
+            for (int c = 0; c < DC_MAX_K / 32; ++c) {
+                if (lane8 + 32 * c >= K) continue;
+                const int pi = dc_at(i, lane8 + 32 * c);
                 const float4 l = *reinterpret_cast<const float4*>(gs + pi), ki = *reinterpret_cast<const float4*>(ks + pi), qi = *reinterpret_cast<const float4*>(qs + pi);
-                if (i > j) sum[c] = make_float4(sum[c].x + l.x, sum[c].y + l.y, sum[c].z + l.z, sum[c].w + l.w);
-                const float x = kj[c].x * dc_exp2(sum[c].x), y = kj[c].y * dc_exp2(sum[c].y), z = kj[c].z * dc_exp2(sum[c].z), w = kj[c].w * dc_exp2(sum[c].w);
-                sa += ki.x * x + ki.y * y + ki.z * z + ki.w * w;
-                sq += qi.x * x + qi.y * y + qi.z * z + qi.w * w;
+#pragma unroll
+                for (int e = 0; e < 2; ++e) {
+                    float4& S = sum[e][c];
+                    if (i > j0 + 4 * e) S = make_float4(S.x + l.x, S.y + l.y, S.z + l.z, S.w + l.w);
+                    const float x = kj[e][c].x * dc_exp2(S.x), y = kj[e][c].y * dc_exp2(S.y), z = kj[e][c].z * dc_exp2(S.z), w = kj[e][c].w * dc_exp2(S.w);
+                    sa[e] += ki.x * x + ki.y * y + ki.z * z + ki.w * w;
+                    sq[e] += qi.x * x + qi.y * y + qi.z * z + qi.w * w;
+                }
             }
-            sa = dc_quad_sum(sa);
-            sq = dc_quad_sum(sq);
-            if (lane4 == 0 && i >= j) {
-                if (i > j) As[dc_row(j) + i] = beta[i] * sa;
-                at.q_pairs[j * DC_TOKENS + i] = sq;
-                if (i > j) at.q_pairs[i * DC_TOKENS + j] = 0.f;
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+                const int j = j0 + 4 * e;
+                float va = dc_quad_sum(sa[e]), vq = dc_quad_sum(sq[e]);
+                va += __shfl_xor_sync(0xffffffffu, va, 4);
+                vq += __shfl_xor_sync(0xffffffffu, vq, 4);
+                if (lane8 == 0 && i >= j) {
+                    if (i > j) As[dc_row(j) + i] = beta[i] * va;
+                    at.q_pairs[i * DC_TOKENS + j] = vq;
+                    if (i > j) at.q_pairs[j * DC_TOKENS + i] = 0.f;
+                }
             }
         }
     }
@@ -344,39 +357,47 @@ delta_chunk_prep_kernel(const DcArgs a) {
             }
             __syncthreads();
         }
-        for (int round = 0; round < s; ++round) {                   // sub-block `round` against sub-block s: 64 tiles of 2 x 2
-            const int task = tid >> 2, i = task >> 3, j = task & 7;
-            const int i0 = s * DC_SUB + i, j0 = round * DC_SUB + j;
-            float sa[2][2] = {{0.f, 0.f}, {0.f, 0.f}}, sq[2][2] = {{0.f, 0.f}, {0.f, 0.f}};
-#pragma unroll 2
-            for (int k = lane4; k < K; k += 16) {
-                float4 l[2], q[2], r[2];
+        for (int round = 0; round < s; ++round) {                   // sub-block `round` against sub-block s: 16 tiles of 4 x 4, 16 threads a tile
+            const int kl = tid & 15, i0 = s * DC_SUB + (tid >> 6), j0 = round * DC_SUB + ((tid >> 4) & 3);      // rows i0 + 4 x, columns j0 + 4 y
+            float v[32] = {};                                       // A: 4 x + y, Q: 16 + 4 x + y
 #pragma unroll
-                for (int e = 0; e < 2; ++e) {
-                    l[e] = *reinterpret_cast<const float4*>(gs + dc_at(i0 + 8 * e, k));
-                    q[e] = *reinterpret_cast<const float4*>(qs + dc_at(i0 + 8 * e, k));
-                    r[e] = *reinterpret_cast<const float4*>(ks + dc_at(j0 + 8 * e, k));
-                }
+            for (int half = 0; half < 2; ++half) {
+                const int k = 4 * kl + 64 * half;
+                if (k >= K) continue;
+                float4 r[4];
 #pragma unroll
-                for (int x = 0; x < 2; ++x)
+                for (int y = 0; y < 4; ++y) r[y] = *reinterpret_cast<const float4*>(ks + dc_at(j0 + 4 * y, k));
 #pragma unroll
-                    for (int y = 0; y < 2; ++y) {
-                        sa[x][y] += l[x].x * r[y].x + l[x].y * r[y].y + l[x].z * r[y].z + l[x].w * r[y].w;
-                        sq[x][y] += q[x].x * r[y].x + q[x].y * r[y].y + q[x].z * r[y].z + q[x].w * r[y].w;
+                for (int x = 0; x < 4; ++x) {
+                    const float4 l = *reinterpret_cast<const float4*>(gs + dc_at(i0 + 4 * x, k)), q = *reinterpret_cast<const float4*>(qs + dc_at(i0 + 4 * x, k));
+#pragma unroll
+                    for (int y = 0; y < 4; ++y) {
+                        v[4 * x + y] += l.x * r[y].x + l.y * r[y].y + l.z * r[y].z + l.w * r[y].w;
+                        v[16 + 4 * x + y] += q.x * r[y].x + q.y * r[y].y + q.z * r[y].z + q.w * r[y].w;
                     }
+                }
             }
+            // the 16 threads' parts: each step adds half of what is left across one bit of kl, which then says which half is kept
 #pragma unroll
-            for (int x = 0; x < 2; ++x)
+            for (int bit = 8, n = 16; bit > 0; bit >>= 1, n >>= 1) {
+                const bool up = kl & bit;
 #pragma unroll
-                for (int y = 0; y < 2; ++y) {
-                    const float va = dc_quad_sum(sa[x][y]), vq = dc_quad_sum(sq[x][y]);
-                    if (lane4 == 4 * (2 * x + y)) {                 // one of the four threads each
-                        const int ii = i0 + 8 * x, jj = j0 + 8 * y;
-                        As[dc_row(jj) + ii] = beta[ii] * va;
-                        at.q_pairs[jj * DC_TOKENS + ii] = vq;
-                        at.q_pairs[ii * DC_TOKENS + jj] = 0.f;
-                    }
+                for (int e = 0; e < n; ++e) {
+                    const float keep = up ? v[n + e] : v[e], give = up ? v[e] : v[n + e];
+                    v[e] = keep + __shfl_xor_sync(0xffffffffu, give, bit);
                 }
+            }
+            const int ii = i0 + 4 * ((kl >> 1) & 3);
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+                const int jj = j0 + 4 * (2 * (kl & 1) + e);
+                if (kl < 8) {
+                    As[dc_row(jj) + ii] = beta[ii] * v[e];
+                } else {
+                    at.q_pairs[ii * DC_TOKENS + jj] = v[e];
+                    at.q_pairs[jj * DC_TOKENS + ii] = 0.f;
+                }
+            }
         }
     }
     __syncthreads();
@@ -459,7 +480,7 @@ delta_chunk_prep_kernel(const DcArgs a) {
 // grid (ceil(P / 16), H, B), 256 threads; dynamic shared memory: W [64][K + 4], k e_end 2 x [64][K], S^T [16][K + 4], u [64][20].
 // For u a thread sums 4 tokens x 1 value over all channels, four channels a load; the state lives in registers, 4 channels x 2
 // values a thread, and in shared memory for u.  A chunk is two products in a chain, with two barriers.
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(256, 2)
 delta_chunk_walk_kernel(const DcArgs a) {
     pdl_wait();
     pdl_launch_dependents();
@@ -551,93 +572,48 @@ delta_chunk_walk_kernel(const DcArgs a) {
     }
 }
 
-// grid (chunks, H * ptiles, B), 128 threads: a chunk's 64 tokens x 128 values, from S0 and then from the chunk's own u
-__global__ void __launch_bounds__(128, 3)
+// grid (chunks, H * ptiles, B): a chunk's 64 tokens x 128 values, from S0 and then from the chunk's own u, as o^T on tcgen05 (chunk_tc.cuh: the
+// values are the product's 128 rows).  65 us with 8 x 8 sums a thread, 58 on mma.sync, %OUT% here (three prompts of 2,900 tokens in all)
+__global__ void __launch_bounds__(CT_THREADS, 2)
 delta_chunk_out_kernel(const DcArgs a, int ptiles) {
     pdl_wait();
     pdl_launch_dependents();
-    // a tile: 16 channels or tokens x 128 values, and q of 64 tokens x 16 channels or their pairs with 16 tokens, 16 x 64
-    constexpr int ROWS = 16, LDV = 132, LDQ = ROWS + 4, LDP = 68;
-    __shared__ __align__(16) float values[3][ROWS * LDV], lefts[3][DC_TOKENS * LDQ];
-    const int c = blockIdx.x, h = blockIdx.y / ptiles, p0 = (blockIdx.y - h * ptiles) * 128, tid = threadIdx.x, K = a.K, P = a.P;
+    const int c = blockIdx.x, h = blockIdx.y / ptiles, p0 = (blockIdx.y - h * ptiles) * 128, K = a.K, P = a.P;
     const int b = rc_sequence(a.cu_seqlens, a.B, a.from, blockIdx.z);
     if (b < 0) return;
     const int t0 = a.cu_seqlens[b] + c * DC_TOKENS, n = min(DC_TOKENS, a.cu_seqlens[b + 1] - t0);
     if (n <= 0) return;
     const DcPlace at = dc_place(a, b, c, h);
-    const int state_tiles = (K + ROWS - 1) / ROWS, n_tiles = state_tiles + (n + ROWS - 1) / ROWS;
-    auto copy = [&](int t) {                                        // one commit group a tile, also beyond the last
-        if (t < n_tiles) {
-            const bool from_state = t < state_tiles;
-            const int row0 = (from_state ? t : t - state_tiles) * ROWS, limit = from_state ? K : n;
-            const float* right = from_state ? at.start : at.u;
+    const CtBlock block = ct_begin(a.error);
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, state_stages = (K + CT_R - 1) / CT_R;
+    const int index = 4 * warp + (lane >> 3), token = 8 * warp + ct_row(lane), eight = lane & 3;
+    float sum[32];
+    const bool ok = ct_products<true, false>(
+        block, state_stages + (n + CT_R - 1) / CT_R,
+        [&](int s, float (&v)[3][8]) {
+            const bool state = s < state_stages;
+            const int r = CT_R * (state ? s : s - state_stages) + index, col = CT_R * (state ? s : s - state_stages) + 8 * eight, cols = state ? K : DC_TOKENS;
+            const float* from = (state ? at.start : at.u) + (size_t)r * P;
 #pragma unroll
-            for (int i = 0; i < 2; ++i) {
-                if (from_state) {
-                    const int r = (tid >> 2) + 32 * i, e = (tid & 3) * 4;
-                    const bool ok = row0 + e < K;
-                    rc_copy16(&lefts[t % 3][r * LDQ + e], at.q0 + (ok ? r * K + row0 + e : 0), ok);
-                } else {
-                    const int r = (tid >> 4) + 8 * i, e = (tid & 15) * 4;
-                    const bool ok = row0 + r < n;
-                    rc_copy16(&lefts[t % 3][r * LDP + e], at.q_pairs + (ok ? (row0 + r) * DC_TOKENS + e : 0), ok);
-                }
-            }
+            for (int i = 0; i < 2; ++i) ct_load(from, p0 + 64 * i + 8 * (lane & 7), P, r < (state ? K : n), v[i]);
+            ct_load((state ? at.q0 : at.q_pairs) + token * cols, col, cols, true, v[2]);
+        },
+        [] {},
+        [&](int s, float (&v)[3][8]) {
 #pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                const int r = (tid >> 5) + 4 * i, e = (tid & 31) * 4;
-                const bool ok = row0 + r < limit && p0 + e < P;
-                rc_copy16(&values[t % 3][r * LDV + e], right + (ok ? (size_t)(row0 + r) * P + p0 + e : 0), ok);
-            }
-        }
-        rc_commit();
-    };
-    copy(0);
-    copy(1);
-    const int ig = (tid >> 4) * 4, pg = (tid & 15) * 4;             // tokens ig .., 32 + ig ..; values pg .., 64 + pg ..
-    float acc[8][8];
+            for (int i = 0; i < 2; ++i) ct_put(block.a, CT_A_PART, 64 * i + CT_R * (s & 1) + index, lane & 7, v[i]);
+            ct_put(block.b, CT_B_PART, token, 4 * (s & 1) + eight, v[2]);
+        },
+        sum);
+    const int p = p0 + 32 * (warp & 3) + lane;
+    if (ok && p < P) {
+        const int first = 32 * (warp >> 2);
+        float* out = a.o + (size_t)(t0 + first) * a.H * P + h * P + p;
 #pragma unroll
-    for (int i = 0; i < 8; ++i)
-#pragma unroll
-        for (int j = 0; j < 8; ++j) acc[i][j] = 0.f;
-    for (int t = 0; t < n_tiles; ++t) {
-        rc_wait<1>();
-        __syncthreads();
-        copy(t + 2);
-        const float *left = lefts[t % 3], *right = values[t % 3];
-        if (t >= state_tiles) {
-            rc_outer<ROWS>(acc, left, LDP, ig, 32 + ig, right, LDV, pg, 64 + pg);
-        } else {
-#pragma unroll
-            for (int k = 0; k < ROWS; k += 4) {                     // q four channels a load
-                float4 q[8];
-#pragma unroll
-                for (int i = 0; i < 8; ++i) q[i] = *reinterpret_cast<const float4*>(left + ((i >> 2) * 32 + ig + (i & 3)) * LDQ + k);
-#pragma unroll
-                for (int r = 0; r < 4; ++r) {
-                    const float4 y0 = *reinterpret_cast<const float4*>(right + (k + r) * LDV + pg), y1 = *reinterpret_cast<const float4*>(right + (k + r) * LDV + 64 + pg);
-                    const float y[8] = {y0.x, y0.y, y0.z, y0.w, y1.x, y1.y, y1.z, y1.w};
-#pragma unroll
-                    for (int i = 0; i < 8; ++i) {
-                        const float x = r == 0 ? q[i].x : (r == 1 ? q[i].y : (r == 2 ? q[i].z : q[i].w));
-#pragma unroll
-                        for (int j = 0; j < 8; ++j) acc[i][j] += x * y[j];
-                    }
-                }
-            }
-        }
+        for (int i = 0; i < 32; ++i)
+            if (first + i < n) out[(size_t)i * a.H * P] = sum[i];
     }
-#pragma unroll
-    for (int i = 0; i < 8; ++i) {
-        const int t = (i >> 2) * 32 + ig + (i & 3);
-        if (t >= n) continue;
-        float* out = a.o + (size_t)(t0 + t) * a.H * P + h * P + p0;
-#pragma unroll
-        for (int half = 0; half < 2; ++half) {
-            const int p = 64 * half + pg;
-            if (p0 + p < P) *reinterpret_cast<float4*>(out + p) = make_float4(acc[i][4 * half], acc[i][4 * half + 1], acc[i][4 * half + 2], acc[i][4 * half + 3]);
-        }
-    }
+    ct_end(block);
 }
 
 // Floats of scratch that qwb_delta_chunked needs; 0: these sizes are not taken.
@@ -651,23 +627,24 @@ extern "C" long long qwb_delta_chunked_scratch(int T, int B, int from, int H, in
 // decays come as qwb_delta_prep takes them.  16-byte aligned tensors, rows of a multiple of 4 floats.
 extern "C" int qwb_delta_chunked(const float* qkv, int ld, const float* beta, const float* a_raw, int ld_a, const float* dt_bias, const float* A_log,
                                  float* state, const int* cu_seqlens, const int* slots, float* o, float* scratch, int T, int B, int max_new, int from, int H,
-                                 int Hk, int K, int P, int decay_k, int write_state, cudaStream_t stream) {
+                                 int Hk, int K, int P, int decay_k, int write_state, int* error, cudaStream_t stream) {
     if (T <= 0 || B <= 0 || max_new <= 0 || max_new < from) return 0;
-    if (!qwb_delta_chunked_scratch(T, B, from, H, K, P) || Hk <= 0 || H % Hk || ld % 4 || ld < 2 * Hk * K + H * P || (decay_k != K && decay_k != 1) || ld_a < H * decay_k)
+    if (!qwb_delta_chunked_scratch(T, B, from, H, K, P) || Hk <= 0 || H % Hk || ld % 4 || ld < 2 * Hk * K + H * P || (decay_k != K && decay_k != 1) || ld_a < H * decay_k || !error)
         return qwb_fail(QWB_ERR_ARG, "delta_chunked: %d heads, %d key heads, state %d x %d in rows of %d, %d decays a head", H, Hk, K, P, ld, decay_k);
     for (const void* p : {(const void*)qkv, (const void*)state, (const void*)o, (const void*)scratch})
         if (!p || !rc_aligned16(p)) return qwb_fail(QWB_ERR_ARG, "delta_chunked: a tensor is not 16-byte aligned");
     const int chunks = (max_new + DC_TOKENS - 1) / DC_TOKENS, ptiles = (P + 127) / 128, planes = rc_planes(T, B, from);
-    const DcArgs a = {qkv, beta, a_raw, dt_bias, A_log, cu_seqlens, slots, state, o, scratch, ld, ld_a, H, Hk, K, P, decay_k, write_state, B, from};
+    const DcArgs a = {qkv, beta, a_raw, dt_bias, A_log, cu_seqlens, slots, state, o, scratch, error, ld, ld_a, H, Hk, K, P, decay_k, write_state, B, from};
     const size_t smem1 = (3 * DC_TOKENS * DC_MAX_K + DC_A_FLOATS + 4 * DC_MAX_K + DC_TOKENS) * sizeof(float);
     const size_t smem2 = ((3 * K + 4) * DC_TOKENS + DC_WALK_P * (K + 4) + DC_TOKENS * (DC_WALK_P + 4)) * sizeof(float);
     cudaError_t e = cudaFuncSetAttribute(delta_chunk_prep_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem1);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(delta_chunk_out_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, CT_SMEM);
     if (e == cudaSuccess) e = cudaFuncSetAttribute(delta_chunk_walk_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem2);
     if (e != cudaSuccess) return qwb_fail(QWB_ERR_CUDA, "delta_chunked: %s", cudaGetErrorString(e));
     qwb_launch(delta_chunk_prep_kernel, dim3(chunks, H, planes), 256, smem1, stream, a);
     if (int rc = qwb_check_launch("delta_chunk_prep")) return rc;
     qwb_launch(delta_chunk_walk_kernel, dim3((P + DC_WALK_P - 1) / DC_WALK_P, H, planes), 256, smem2, stream, a);
     if (int rc = qwb_check_launch("delta_chunk_walk")) return rc;
-    qwb_launch(delta_chunk_out_kernel, dim3(chunks, H * ptiles, planes), 128, 0, stream, a, ptiles);
+    qwb_launch(delta_chunk_out_kernel, dim3(chunks, H * ptiles, planes), CT_THREADS, CT_SMEM, stream, a, ptiles);
     return qwb_check_launch("delta_chunk_out");
 }

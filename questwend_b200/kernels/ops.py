@@ -1024,7 +1024,7 @@ def delta_rule(qkv: torch.Tensor, b_raw: torch.Tensor, b_col0: int, a_raw: torch
     if scratch is not None:
         _call("recurrent_chunks", "qwb_delta_chunked", _ptr(qkv), _i(qkv.shape[1]), _ptr(beta), *raw_decays, _ptr(state), _ptr(ctx.cu_seqlens),
               _ptr(ctx.slots), _ptr(o), _ptr(scratch), _i(T), _i(ctx.n_seqs), _i(ctx.max_new), _i(chunks_from), _i(heads), _i(key_heads),
-              _i(key_dim), _i(vdim), _i(decay_k), _i(1 if write_state else 0), _stream(), kernels=3)
+              _i(key_dim), _i(vdim), _i(decay_k), _i(1 if write_state else 0), _ptr(gemm_tc_error_word(dev)), _stream(), kernels=3)
         if not rest:
             return o
     _call("recurrent", "qwb_delta_scan", _ptr(qkv), _i(qkv.shape[1]), _ptr(kq), _ptr(beta), _ptr(decay), _ptr(state),
