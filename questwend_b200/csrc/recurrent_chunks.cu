@@ -478,8 +478,11 @@ delta_chunk_prep_kernel(const DcArgs a) {
 }
 
 // grid (ceil(P / 16), H, B), 256 threads; dynamic shared memory: W [64][K + 4], k e_end 2 x [64][K], S^T [16][K + 4], u [64][20].
-// For u a thread sums 4 tokens x 1 value over all channels, four channels a load; the state lives in registers, 4 channels x 2
-// values a thread, and in shared memory for u.  A chunk is two products in a chain, with two barriers.
+// For u a thread sums 4 tokens x 4 values over a quarter of the channels, for the state 4 channels x 4 values over half of the tokens, and
+// threads that hold parts of the same sums exchange halves of them by shuffles: 64 multiply-adds for eight 16-byte loads and 16 for two,
+// where one value (16 for five) and two values a thread (8 for one and a half) were bound by the loads (8,200 of a chunk's 8,500 cycles).
+// The state lives in registers, 4 channels x 2 values a thread, and in shared memory for u.  A chunk is two products in a chain, with two
+// barriers.
 __global__ void __launch_bounds__(256, 2)
 delta_chunk_walk_kernel(const DcArgs a) {
     pdl_wait();
@@ -508,9 +511,10 @@ delta_chunk_walk_kernel(const DcArgs a) {
     const size_t step = a.H * dc_floats(K, P);
     copy(Ws, ldw, at.w, true);
     copy(Ke, K, at.k_end, true);
-    const int p = (tid & 3) + 4 * (warp & 3), ig = ((tid >> 2) & 7) + 8 * (warp >> 2);      // u: value p, tokens ig, ig + 16, ig + 32, ig + 48
-    const int ps = (tid & 7) * 2, kg = (tid >> 3) * 4;              // state: values ps, ps + 1, channels kg ..
-    const bool p_ok = p0 + p < P, s_ok = p0 + ps < P && kg < K;
+    const int lane = tid & 31, kq = lane >> 3, tg = (lane & 7) + 8 * (warp & 1), pv = 4 * (warp >> 1);     // u: tokens tg + 16 i, values pv .., channels 16 . + 4 kq ..
+    const int mine = tg + 16 * kq;                                  // the token whose four sums this thread ends up with
+    const int half = lane >> 4, kg = 4 * (4 * warp + ((lane >> 2) & 3)), pg = 4 * (lane & 3), ps = pg + 2 * half;    // state: channels kg .., of values pg .. in the end ps, ps + 1
+    const bool p_ok = p0 + pv < P, s_ok = p0 + ps < P && kg < K;
     float S[2][4];
 #pragma unroll
     for (int e = 0; e < 2; ++e) {
@@ -519,9 +523,7 @@ delta_chunk_walk_kernel(const DcArgs a) {
         if (kg < K) *reinterpret_cast<float4*>(Ss + (ps + e) * ldw + kg) = v;
     }
     for (int c = 0; c < chunks; ++c) {
-        float own[4];                                               // U, asked for early
-#pragma unroll
-        for (int i = 0; i < 4; ++i) own[i] = p_ok ? at.u[(size_t)(ig + 16 * i) * P + p0 + p] : 0.f;
+        const float4 own = rc_load4(at.u + (size_t)mine * P + p0 + pv, p_ok);      // U, asked for early
         const float4 fade = rc_load4(at.decay + kg, kg < K);
         rc_wait<0>();                                               // W and k e_end
         __syncthreads();                                            // and S is whole; the last chunk's k e_end is read
@@ -530,37 +532,55 @@ delta_chunk_walk_kernel(const DcArgs a) {
 #pragma unroll
             for (int k = 0; k < 4; ++k) *reinterpret_cast<float2*>(at.start + (size_t)(kg + k) * P + p0 + ps) = make_float2(S[0][k], S[1][k]);
         }
-        const float *w = Ws + ig * ldw, *s = Ss + p * ldw;
-        float part[4][4] = {};                                      // four chains a sum: shorter ones round less
-#pragma unroll 8
-        for (int k = 0; k < K; k += 4) {
-            const float4 y = *reinterpret_cast<const float4*>(s + k);
+        {
+            const float *w = Ws + tg * ldw, *s = Ss + pv * ldw;
+            float part[16] = {};                                    // 4 i + e
+#pragma unroll 2
+            for (int k = 4 * kq; k < K; k += 16) {
+                float4 x[4];
 #pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                const float4 x = *reinterpret_cast<const float4*>(w + 16 * i * ldw + k);
-                part[i][0] += x.x * y.x; part[i][1] += x.y * y.y;
-                part[i][2] += x.z * y.z; part[i][3] += x.w * y.w;
+                for (int i = 0; i < 4; ++i) x[i] = *reinterpret_cast<const float4*>(w + 16 * i * ldw + k);
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                    const float4 y = *reinterpret_cast<const float4*>(s + e * ldw + k);
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) part[4 * i + e] += x[i].x * y.x + x[i].y * y.y + x[i].z * y.z + x[i].w * y.w;
+                }
             }
-        }
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            const float u = own[i] - ((part[i][0] + part[i][1]) + (part[i][2] + part[i][3]));
-            Us[(ig + 16 * i) * LU + p] = u;
-            if (p_ok) at.u[(size_t)(ig + 16 * i) * P + p0 + p] = u;
+            for (int bit = 16, n = 8; bit >= 8; bit >>= 1, n >>= 1) {        // half of what is left across one bit of the lane, which says which is kept
+                const bool up = lane & bit;
+#pragma unroll
+                for (int e = 0; e < n; ++e) {
+                    const float keep = up ? part[n + e] : part[e], give = up ? part[e] : part[n + e];
+                    part[e] = keep + __shfl_xor_sync(0xffffffffu, give, bit);
+                }
+            }
+            const float4 u = make_float4(own.x - part[0], own.y - part[1], own.z - part[2], own.w - part[3]);
+            *reinterpret_cast<float4*>(Us + mine * LU + pv) = u;
+            if (p_ok) *reinterpret_cast<float4*>(at.u + (size_t)mine * P + p0 + pv) = u;
         }
         __syncthreads();                                            // u is whole; W is read
         copy(Ws, ldw, at.w + step, c + 1 < chunks);
 #pragma unroll
         for (int e = 0; e < 2; ++e) { S[e][0] *= fade.x; S[e][1] *= fade.y; S[e][2] *= fade.z; S[e][3] *= fade.w; }
-        if (kg < K) {
-            const float* ke = Ke + (c & 1) * K * DC_TOKENS + kg;
-#pragma unroll 16
-            for (int j = 0; j < DC_TOKENS; ++j) {
-                const float4 x = *reinterpret_cast<const float4*>(ke + j * K);
-                const float2 y = *reinterpret_cast<const float2*>(Us + j * LU + ps);
-                S[0][0] += x.x * y.x; S[0][1] += x.y * y.x; S[0][2] += x.z * y.x; S[0][3] += x.w * y.x;
-                S[1][0] += x.x * y.y; S[1][1] += x.y * y.y; S[1][2] += x.z * y.y; S[1][3] += x.w * y.y;
+        const float* ke = Ke + (c & 1) * K * DC_TOKENS + (kg < K ? kg : 0);
+        float sum[16] = {};                                         // 8 (value / 2) + 4 (value % 2) + channel
+#pragma unroll 8
+        for (int j = half * (DC_TOKENS / 2); j < (half + 1) * (DC_TOKENS / 2); ++j) {
+            const float4 x = *reinterpret_cast<const float4*>(ke + j * K), y = *reinterpret_cast<const float4*>(Us + j * LU + pg);
+            const float yv[4] = {y.x, y.y, y.z, y.w};
+#pragma unroll
+            for (int e = 0; e < 4; ++e) { sum[4 * e] += x.x * yv[e]; sum[4 * e + 1] += x.y * yv[e]; sum[4 * e + 2] += x.z * yv[e]; sum[4 * e + 3] += x.w * yv[e]; }
+        }
+#pragma unroll
+        for (int e = 0; e < 2; ++e)
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                const float keep = half ? sum[8 + 4 * e + k] : sum[4 * e + k], give = half ? sum[4 * e + k] : sum[8 + 4 * e + k];
+                S[e][k] += keep + __shfl_xor_sync(0xffffffffu, give, 16);
             }
+        if (kg < K) {
 #pragma unroll
             for (int e = 0; e < 2; ++e) *reinterpret_cast<float4*>(Ss + (ps + e) * ldw + kg) = make_float4(S[e][0], S[e][1], S[e][2], S[e][3]);
         }
@@ -573,7 +593,7 @@ delta_chunk_walk_kernel(const DcArgs a) {
 }
 
 // grid (chunks, H * ptiles, B): a chunk's 64 tokens x 128 values, from S0 and then from the chunk's own u, as o^T on tcgen05 (chunk_tc.cuh: the
-// values are the product's 128 rows).  65 us with 8 x 8 sums a thread, 58 on mma.sync, %OUT% here (three prompts of 2,900 tokens in all)
+// values are the product's 128 rows).  65 us with 8 x 8 sums a thread, 58 on mma.sync, 42 here (three prompts of 2,900 tokens in all)
 __global__ void __launch_bounds__(CT_THREADS, 2)
 delta_chunk_out_kernel(const DcArgs a, int ptiles) {
     pdl_wait();
