@@ -13,10 +13,15 @@
 // relative to the row's largest score so far, as with the mma.sync kernels: the largest probability is 1 and exact in bfloat16.  A
 // reference that is moved only past 2^8 is faster (8,192 tokens 529 us where this takes 577, one latent prompt the same) but rounds
 // the largest probability too: errors of 0.00213 and 0.00260 of the results in place of 0.00207 and 0.00252, more where few keys weigh.
-// A stream waits for its product only when a row of a warp moves its reference; otherwise it may be two tiles ahead.  With two streams in one block the tensor cores work on one while the other is
+// With two streams in one block the tensor cores work on one while the other is
 // in its softmax, what two blocks an SM give attention_tc.cu, but the Q, K and V tiles of 192-value keys would not leave room for
-// a second block (2 x 48 KB of Q, K and V in three stages: 216 KB), and K and V cross L2 once for 256 rows.  Warp 0 loads, warp 1
-// issues the products, warps 2-5 and 6-9 are the streams' softmax warps.  Every wait is bounded.
+// a second block (2 x 48 KB of Q, K and V in three stages: 216 KB), and K and V cross L2 once for 256 rows.  Every wait is bounded.
+//
+// Warps, in groups of four that have registers of their own (setmaxnreg): 0 loads, 1 and 2 issue a stream's products each, 4-7 and 8-11 are the
+// streams' softmax warps, 12-15 multiply O by what a row's reference has moved: in most tiles some row of a warp's 32 moves it, and a
+// softmax warp that did this itself waited for the product before, 780 to 1,830 of a tile's 3,000 cycles.  One warp for both streams'
+// products spent 3,500 cycles a tile (65 to 80 a product, about 200 a wait, passed or not).  With capped scores the softmax's multiply-adds
+// fill the schedulers and want the registers: there its warps move O themselves (8,192 tokens 673 us, with warps for it 760).
 //
 // Sizes that are no multiples of 64 are filled up by the TMA loads with zeros.  In the last tile, rows of V behind the last
 // key that the block sees are overwritten with zeros before the product: they can belong to another sequence, and what stands
@@ -24,15 +29,19 @@
 // the zeros of the rows before it: up to 127 earlier tokens of a latent prompt (64-row tiles: 63) and 128 / (heads a group) - 1 of
 // one with two maps.
 //
-// Bound by the tensor cores' products of 64 keys (clocks in a block: the issuing warp is busy all of the time, a softmax warp two
-// thirds of a tile's waiting for scores).  16 heads, replayed from a graph, with the mma.sync kernels, with P in shared memory, and
-// now: latent 128 + 64 / 128, one prompt of 4,096: 816 -> 155 -> 108 us, of 600: 55 -> 19 -> 16 us; two maps of 64 over 4
-// key/value heads, values of 128, 8,192 tokens: 2,447 -> 707 -> 577 us (cap 50: 3,261 -> 795 -> 693), 2,048 tokens with a window of
-// 1,024: 170 -> 52 -> 48 us.  Of the last step P in tensor memory and the third and fourth stage gave 5 to 10 %, the elected lane
-// in place of `lane == 0` the rest.
+// Bound by the issue of products of 64 keys and the softmax's chain, near each other.  16 heads: latent 128 + 64 / 128, one prompt of 4,096, with
+// the mma.sync kernels 816 us, one issuing warp 112, now 92 (600 tokens 55 -> 19.7 -> 19.0); two maps of 64 over 4 key/value heads, values of 128,
+// 8,192 tokens: 2,447 -> 583 -> 507 us (cap 50: 3,261 -> 696 -> 673), 2,048 tokens with a window of 1,024: 170 -> 51 -> 45 us.
 #include "attention_tc.cuh"
 
-#define AS_THREADS 320
+#define AS_THREADS(apart) ((apart) ? 512 : 384)
+// Registers a thread of the loader's and issuers' warps, of the streams' softmax warps, of the warps that move O: as many in all as the block is
+// launched with (128 a thread, all of an SM's), which is what setmaxnreg has to give.
+#define AS_LAUNCH_REGS 128
+#define AS_FEW_REGS 56
+#define AS_SOFTMAX_REGS 184
+#define AS_MOVE_REGS 88
+static_assert(AS_FEW_REGS + 2 * AS_SOFTMAX_REGS + AS_MOVE_REGS == 4 * AS_LAUNCH_REGS, "four groups of 128 threads");
 #define AS_MAX_STAGES 4
 #define AS_SMEM (227 * 1024)
 
@@ -41,6 +50,43 @@ __device__ __forceinline__ void as_mma_ts(uint32_t tmem_d, uint32_t tmem_a, uint
     asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
                  "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, {%5, %5, %5, %5}, p;\n\t}"
                  ::"r"(tmem_d), "r"(tmem_a), "l"(desc_b), "r"(idesc), "r"(accumulate), "r"(0u) : "memory");
+}
+// as at_ld32 and at_st32, without their waits
+__device__ __forceinline__ void as_ld32(uint32_t taddr, uint32_t* r) {
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x32.b32 "
+                 "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
+                 "%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
+                   "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]),
+                   "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]),
+                   "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
+                 : "r"(taddr));
+}
+__device__ __forceinline__ void as_st32(uint32_t taddr, const uint32_t* r) {
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], "
+                 "{%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16, "
+                 "%17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31, %32};"
+                 ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]),
+                   "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]),
+                   "r"(r[16]), "r"(r[17]), "r"(r[18]), "r"(r[19]), "r"(r[20]), "r"(r[21]), "r"(r[22]), "r"(r[23]),
+                   "r"(r[24]), "r"(r[25]), "r"(r[26]), "r"(r[27]), "r"(r[28]), "r"(r[29]), "r"(r[30]), "r"(r[31])
+                 : "memory");
+}
+// VD sums of this lane's row times alpha
+template <int VD>
+__device__ __forceinline__ void as_rescale(uint32_t taddr, float alpha) {
+#pragma unroll
+    for (int c = 0; c < VD; c += 64) {                  // two loads and two stores on their way together
+        uint32_t ov[2][32];
+        as_ld32(taddr + c, ov[0]);
+        as_ld32(taddr + c + 32, ov[1]);
+        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+        for (int e = 0; e < 64; ++e) ov[e / 32][e % 32] = __float_as_uint(__uint_as_float(ov[e / 32][e % 32]) * alpha);
+        as_st32(taddr + c, ov[0]);
+        as_st32(taddr + c + 32, ov[1]);
+    }
+    asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
 }
 __device__ __forceinline__ uint64_t as_two(float lo, float hi) {
     uint64_t v;
@@ -83,7 +129,7 @@ struct AsSmem {
     static constexpr size_t Q_BYTES = (size_t)2 * KA * AT_ROWS * 128;                       // stream by stream, [128 rows][128 bytes] a piece
     static constexpr size_t K_BYTES = (size_t)(MAPS ? 2 : 1) * KA * AT_KEYS * 128;          // (map by map,) [64 keys][128 bytes] a piece
     static constexpr size_t V_BYTES = (size_t)VA * AT_KEYS * 128;
-    static constexpr size_t MORE = 512 + (MAPS ? 4 * AT_ROWS * sizeof(float) : 0);          // barriers; what the maps' streams exchange
+    static constexpr size_t MORE = 512 + 4 * AT_ROWS * sizeof(float);                       // barriers; factors of rows, see below
     static constexpr int FIT = (int)((AS_SMEM - MORE - Q_BYTES) / (K_BYTES + V_BYTES));
     static constexpr int STAGES = FIT < AS_MAX_STAGES ? FIT : AS_MAX_STAGES;
     static constexpr size_t TILES = Q_BYTES + STAGES * (K_BYTES + V_BYTES);
@@ -102,11 +148,12 @@ struct AsArgs {
 };
 
 template <int KA, int VA, bool MAPS, bool CAP>
-__global__ void __launch_bounds__(AS_THREADS, 1)
+__global__ void __launch_bounds__(AS_THREADS(!CAP), 1)
 attn_streams_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_q2, const __grid_constant__ CUtensorMap map_k,
                     const __grid_constant__ CUtensorMap map_k2, const __grid_constant__ CUtensorMap map_v, const AsArgs p) {
     using Smem = AsSmem<KA, VA, MAPS>;
     constexpr int VD = 64 * VA, STAGES = Smem::STAGES;
+    constexpr bool APART = !CAP;
     constexpr uint32_t K_BYTES = Smem::K_BYTES, V_BYTES = Smem::V_BYTES;
     extern __shared__ __align__(1024) unsigned char smem_raw[];
     if (at_smem(smem_raw) & 1023u) {                    // never seen; refuse rather than compute with a wrong layout
@@ -125,8 +172,11 @@ attn_streams_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
     uint64_t* s_full = v_empty + STAGES;
     uint64_t* p_full = s_full + 4;
     uint64_t* o_full = p_full + 4;
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(o_full + 4);
-    float* swap = reinterpret_cast<float*>(smem_raw + Smem::TILES + 512);       // MAPS: [2][128] factors, [2][128] sums of squares
+    uint64_t* a_full = o_full + 4;
+    uint64_t* c_full = a_full + 4;
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(c_full + 4);
+    // per stream two rows of 128: what a row's sums are multiplied by, of even and odd tiles; MAPS, in the end: factors and sums of squares
+    float* swap = reinterpret_cast<float*>(smem_raw + Smem::TILES + 512);
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int b = blockIdx.z;
@@ -157,10 +207,13 @@ attn_streams_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
     if (threadIdx.x == 0) {
         at_bar_init(q_full, 1);
         for (int s = 0; s < STAGES; ++s) {
-            at_bar_init(&k_full[s], 1); at_bar_init(&k_empty[s], 1);
-            at_bar_init(&v_full[s], 1); at_bar_init(&v_empty[s], 1);
+            at_bar_init(&k_full[s], 1); at_bar_init(&k_empty[s], 2);                   // both streams have read a tile
+            at_bar_init(&v_full[s], 1); at_bar_init(&v_empty[s], 2);
         }
-        for (int i = 0; i < 4; ++i) { at_bar_init(&s_full[i], 1); at_bar_init(&p_full[i], 4); at_bar_init(&o_full[i], 1); }
+        for (int i = 0; i < 4; ++i) {
+            at_bar_init(&s_full[i], 1); at_bar_init(&p_full[i], 4); at_bar_init(&o_full[i], 1);
+            at_bar_init(&a_full[i], 4); at_bar_init(&c_full[i], 4);
+        }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == 1) {
@@ -175,6 +228,9 @@ attn_streams_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
     pdl_wait();
     pdl_launch_dependents();
 
+    // what a warp does follows from its group of four, so that each group's registers are its own
+    if (warp < 4) {
+        if (APART) asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(AS_FEW_REGS));
     if (warp == 0) {
         if (lane == 0) {
             if (MAPS) {                                 // rows (token, head of the group): boxes of [128 / G tokens][G heads][1 map][64 d]
@@ -239,80 +295,107 @@ attn_streams_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
                 for (int j = max(0, v_issued - STAGES); j < v_issued; ++j) at_wait(&v_full[j % STAGES], (j / STAGES) & 1);
             }
         }
-    } else if (warp == 1) {                             // all lanes wait, one issues
+    } else if (warp == 1 || warp == 2) {                // a stream's products: all lanes wait, one issues
         constexpr uint32_t idesc_s = at_idesc(AT_ROWS, AT_KEYS, false), idesc_o = at_idesc(AT_ROWS, VD, true);
+        const int x = warp - 1;
         auto all = [](bool ok) -> bool { return __all_sync(0xffffffffu, ok); };
         bool ok = all(at_wait(q_full, 0));
-        auto issue_s = [&](int x, int j) -> bool {      // S of stream x for tile j, two tiles ahead of its product with V
+        auto active = [&](int j) { return j >= from(x) && j < to(x); };
+        // S for tile j, two tiles ahead of its product with V: the buffer's last scores were read, and its P used by a product issued
+        // before.  A tile that the stream does not see is waited for all the same, so that it is given back in its turn.
+        auto issue_s = [&](int j) -> bool {
             const int i = j - from(x), s = j % STAGES;
-            bool good = at_wait(&k_full[s], (j / STAGES) & 1);
-            if (!all(good)) return false;               // the buffer's last scores were read, and its P used by a product issued before
+            if (!all(at_wait(&k_full[s], (j / STAGES) & 1))) return false;
             at_fence_after();
             if (at_elect()) {
-                const unsigned char* qt = q_tile + (size_t)x * KA * AT_ROWS * 128;
-                const unsigned char* kt = k_tiles + (size_t)s * K_BYTES + (MAPS ? (size_t)x * KA * AT_KEYS * 128 : 0);
+                if (active(j)) {
+                    const unsigned char* qt = q_tile + (size_t)x * KA * AT_ROWS * 128;
+                    const unsigned char* kt = k_tiles + (size_t)s * K_BYTES + (MAPS ? (size_t)x * KA * AT_KEYS * 128 : 0);
 #pragma unroll
-                for (int k = 0; k < 4 * KA; ++k) {
-                    const uint64_t da = at_desc_kmajor(qt + (size_t)(k / 4) * AT_ROWS * 128) + 2 * (k % 4);
-                    const uint64_t db = at_desc_kmajor(kt + (size_t)(k / 4) * AT_KEYS * 128) + 2 * (k % 4);
-                    at_mma(tmem + 128 * x + 64 * (i & 1), da, db, idesc_s, k > 0 ? 1u : 0u);
+                    for (int k = 0; k < 4 * KA; ++k) {
+                        const uint64_t da = at_desc_kmajor(qt + (size_t)(k / 4) * AT_ROWS * 128) + 2 * (k % 4);
+                        const uint64_t db = at_desc_kmajor(kt + (size_t)(k / 4) * AT_KEYS * 128) + 2 * (k % 4);
+                        at_mma(tmem + 128 * x + 64 * (i & 1), da, db, idesc_s, k > 0 ? 1u : 0u);
+                    }
+                    at_commit(&s_full[2 * x + (i & 1)]);
+                    at_commit(&k_empty[s]);
+                } else {
+                    at_arrive(&k_empty[s]);
                 }
-                at_commit(&s_full[2 * x + (i & 1)]);
             }
             __syncwarp();
             return true;
         };
-        auto active = [&](int x, int j) { return j >= from(x) && j < to(x); };
-        for (int j = 0; j < 2 && j < n_tiles && ok; ++j) {
-#pragma unroll
-            for (int x = 0; x < 2 && ok; ++x)
-                if (active(x, j)) ok = issue_s(x, j);
-            if (ok && at_elect()) at_commit(&k_empty[j % STAGES]);
-        }
+        for (int j = 0; j < 2 && j < n_tiles && ok; ++j) ok = issue_s(j);
         for (int j = 0; j < n_tiles && ok; ++j) {
-            const int s = j % STAGES;
+            const int s = j % STAGES, i = j - from(x);
             unsigned char* vt = v_tiles + (size_t)s * V_BYTES;
             ok = all(at_wait(&v_full[s], (j / STAGES) & 1));
             if (!ok) break;
-            const int kept = k_last + 1 - (first_tile + j) * AT_KEYS;
-            if (kept < AT_KEYS) {                       // the last tile: rows behind the last key
-                for (int i = lane; i < (AT_KEYS - kept) * VA * 8; i += 32) {
-                    const int r = kept + i / (VA * 8), c = i % (VA * 8);
-                    *reinterpret_cast<uint4*>(vt + (size_t)(c / 8) * AT_KEYS * 128 + r * 128 + (c % 8) * 16) = make_uint4(0, 0, 0, 0);
-                }
-                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-                __syncwarp();
-            }
-#pragma unroll
-            for (int x = 0; x < 2 && ok; ++x) {
-                if (active(x, j)) {
-                    const int i = j - from(x);
-                    ok = all(at_wait(&p_full[2 * x + (i & 1)], (i >> 1) & 1));
-                    if (!ok) break;
-                    at_fence_after();
-                    if (at_elect()) {
-#pragma unroll
-                        for (int k = 0; k < AT_KEYS / 16; ++k) {
-                            const uint64_t db = at_desc_mnmajor(vt + (size_t)k * 16 * 128, AT_KEYS * 128);
-                            as_mma_ts(tmem + 256 + 128 * x, tmem + 128 * x + 64 * (i & 1) + 8 * k, db, idesc_o, (i > 0 || k > 0) ? 1u : 0u);
-                        }
-                        at_commit(&o_full[2 * x + (i & 1)]);
+            if (active(j)) {
+                const int kept = k_last + 1 - (first_tile + j) * AT_KEYS;
+                if (kept < AT_KEYS) {                   // the last tile: rows behind the last key (both streams' warps write the same)
+                    for (int e = lane; e < (AT_KEYS - kept) * VA * 8; e += 32) {
+                        const int r = kept + e / (VA * 8), c = e % (VA * 8);
+                        *reinterpret_cast<uint4*>(vt + (size_t)(c / 8) * AT_KEYS * 128 + r * 128 + (c % 8) * 16) = make_uint4(0, 0, 0, 0);
                     }
+                    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
                     __syncwarp();
                 }
-                if (j + 2 < n_tiles && active(x, j + 2)) ok = issue_s(x, j + 2);
+                ok = all(at_wait(&p_full[2 * x + (i & 1)], (i >> 1) & 1) && (!APART || at_wait(&c_full[2 * x + (i & 1)], (i >> 1) & 1)));
+                if (!ok) break;
+                at_fence_after();
             }
-            if (ok && at_elect()) {
-                at_commit(&v_empty[s]);
-                if (j + 2 < n_tiles) at_commit(&k_empty[(j + 2) % STAGES]);
+            if (at_elect()) {
+                if (active(j)) {
+#pragma unroll
+                    for (int k = 0; k < AT_KEYS / 16; ++k) {
+                        const uint64_t db = at_desc_mnmajor(vt + (size_t)k * 16 * 128, AT_KEYS * 128);
+                        as_mma_ts(tmem + 256 + 128 * x, tmem + 128 * x + 64 * (i & 1) + 8 * k, db, idesc_o, (i > 0 || k > 0) ? 1u : 0u);
+                    }
+                    at_commit(&o_full[2 * x + (i & 1)]);
+                    at_commit(&v_empty[s]);
+                } else {
+                    at_arrive(&v_empty[s]);
+                }
             }
+            __syncwarp();
+            if (j + 2 < n_tiles) ok = issue_s(j + 2);
         }
         if (!ok && at_elect()) {
             atomicExch(p.error, 2);
-            for (int i = 0; i < 4; ++i) { at_commit(&s_full[i]); at_commit(&o_full[i]); }
+            for (int i = 2 * x; i < 2 * x + 2; ++i) { at_commit(&s_full[i]); at_commit(&o_full[i]); }
         }
+    }
+    } else if (APART && warp >= 12) {
+        asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(AS_MOVE_REGS));
+        // O of both streams relative to the rows' new references, while the softmax warps go on
+        const int lane_group = warp & 3, r = 32 * lane_group + lane;
+        const uint32_t lane_off = (uint32_t)(32 * lane_group) << 16;
+        bool ok = true;
+        for (int j = 0; j < n_tiles && ok; ++j) {       // in the order in which the products are issued
+#pragma unroll
+            for (int x = 0; x < 2 && ok; ++x) {
+                if (j < from(x) || j >= to(x)) continue;
+                const int i = j - from(x), at = 2 * x + (i & 1);
+                ok = at_wait(&a_full[at], (i >> 1) & 1);
+                if (!ok) break;
+                const float alpha = swap[at * AT_ROWS + r];
+                if (i > 0 && __any_sync(0xffffffffu, alpha != 1.f)) {
+                    ok = at_wait(&o_full[at ^ 1], ((i - 1) >> 1) & 1);      // what the products before have written
+                    at_fence_after();
+                    if (!ok) break;
+                    as_rescale<VD>(tmem + 256 + 128 * x + lane_off, alpha);
+                }
+                at_fence_before();
+                __syncwarp();
+                if (lane == 0) at_arrive(&c_full[at]);
+            }
+        }
+        if (!ok && lane == 0) atomicExch(p.error, 4);
     } else {
-        const int x = (warp - 2) >> 2, lane_group = warp & 3;
+        if (APART) asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(AS_SOFTMAX_REGS));
+        const int x = (warp - 4) >> 2, lane_group = warp & 3;
         const int r = 32 * lane_group + lane;                                          // this thread's row = tensor-memory lane
         const int tok = MAPS ? q0 + r / p.G : q0 + AT_ROWS * x + r, head = MAPS ? (int)blockIdx.x * p.G + r % p.G : (int)blockIdx.x;
         const bool row_ok = to(x) > 0 && tok < n_new && (!MAPS || r < p.tok_per_block * p.G);
@@ -392,6 +475,11 @@ attn_streams_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
             const float alpha = rescale ? at_exp2((m_ref - m_new) * sl2) : 1.f;        // m_ref = -inf gives 0
             const float base = m_new == -INFINITY ? 0.f : m_new * sl2;
             m_ref = m_new;
+            if (APART) {                                                                // read before the tile after the next has scores
+                swap[(2 * x + (i & 1)) * AT_ROWS + r] = alpha;
+                __syncwarp();
+                if (lane == 0) at_arrive(&a_full[2 * x + (i & 1)]);
+            }
             uint32_t pk[32];                                                            // two keys' probabilities each
             float sum[4] = {l * alpha, 0.f, 0.f, 0.f};
             auto probabilities = [&](auto argument) {
@@ -421,18 +509,11 @@ attn_streams_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
                 });
             }
             l = (sum[0] + sum[1]) + (sum[2] + sum[3]);
-            if (i > 0 && __any_sync(0xffffffffu, rescale)) {                            // a row of this warp moves its reference: rescale O,
+            if (!APART && i > 0 && __any_sync(0xffffffffu, rescale)) {                  // a row of this warp moves its reference: rescale O,
                 ok = at_wait(&o_full[2 * x + ((i - 1) & 1)], ((i - 1) >> 1) & 1);       // which the product before this one has written
                 at_fence_after();
                 if (!ok) { if (lane == 0) atomicExch(p.error, 4); break; }
-#pragma unroll 1
-                for (int c = 0; c < VD; c += 32) {
-                    uint32_t ov[32];
-                    at_ld32(tmem_o + lane_off + c, ov);
-#pragma unroll
-                    for (int e = 0; e < 32; ++e) ov[e] = __float_as_uint(__uint_as_float(ov[e]) * alpha);
-                    at_st32(tmem_o + lane_off + c, ov);
-                }
+                as_rescale<VD>(tmem_o + lane_off, alpha);
             }
             at_st32(tmem_s + (i & 1) * 64 + lane_off, pk);                              // P over the scores it came from
             at_fence_before();
@@ -475,11 +556,11 @@ attn_streams_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
             }
         } else {
             // both streams' threads of a row form half of the difference's columns each; every thread passes both barriers
-            swap[x * AT_ROWS + r] = (l > 0.f ? 1.f / l : 0.f) * (x ? p.lambda : 1.f);
+            swap[2 * x * AT_ROWS + r] = (l > 0.f ? 1.f / l : 0.f) * (x ? p.lambda : 1.f);
             at_fence_before();
             asm volatile("bar.sync 1, 256;" ::: "memory");
             at_fence_after();
-            const float f0 = swap[r], f1 = swap[AT_ROWS + r];
+            const float f0 = swap[r], f1 = swap[2 * AT_ROWS + r];
             float v[VA][32], squares = 0.f;
 #pragma unroll
             for (int a = 0; a < VA; ++a) {
@@ -493,9 +574,9 @@ attn_streams_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
                     squares += v[a][e] * v[a][e];
                 }
             }
-            swap[2 * AT_ROWS + x * AT_ROWS + r] = squares;
+            swap[(2 * x + 1) * AT_ROWS + r] = squares;
             asm volatile("bar.sync 1, 256;" ::: "memory");
-            const float total = swap[2 * AT_ROWS + r] + swap[3 * AT_ROWS + r];
+            const float total = swap[AT_ROWS + r] + swap[3 * AT_ROWS + r];
             const float mul = (p.norm_out ? rsqrtf(total / (float)p.vd + p.eps) * p.out_scale : 1.f) * gate;
             if (ok) {
 #pragma unroll
@@ -532,7 +613,10 @@ static int as_launch(const char* what, dim3 grid, const CUtensorMap* maps, const
     auto kernel = attn_streams_kernel<KA, VA, MAPS, CAP>;
     cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return qwb_fail(QWB_ERR_CUDA, "%s: %s", what, cudaGetErrorString(e));
-    e = qwb_launch(kernel, grid, AS_THREADS, smem, stream, maps[0], maps[1], maps[2], maps[3], maps[4], args);
+    static const int regs = [&] { cudaFuncAttributes f; return cudaFuncGetAttributes(&f, kernel) == cudaSuccess ? f.numRegs : 0; }();
+    if (!CAP && regs != AS_LAUNCH_REGS)                         // built otherwise: the warps would wait for registers that there are not
+        return qwb_fail(QWB_ERR_CUDA, "%s: built with %d registers a thread, not %d", what, regs, AS_LAUNCH_REGS);
+    e = qwb_launch(kernel, grid, AS_THREADS(!CAP), smem, stream, maps[0], maps[1], maps[2], maps[3], maps[4], args);
     if (e != cudaSuccess) return qwb_fail(QWB_ERR_CUDA, "%s: launch failed: %s", what, cudaGetErrorString(e));
     return qwb_check_launch(what);
 }
