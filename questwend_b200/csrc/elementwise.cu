@@ -277,6 +277,51 @@ rmsnorm_rows_kernel(const float* x, const float* delta, const float* planes, con
     }
 }
 
+// Many rows of up to 1,024 values: a warp a row, eight rows a block, no barrier.  A block a row is bound by its start, its two
+// barriers and one load a thread; a warp has the whole row in flight.  us, a block a row -> a warp a row, norm alone and with
+// the residual's sum (bf16 out, rows in L2): 3,001 rows of 1,024  6.9 -> 3.7, 7.8 -> 6.2; 2,048 of 1,024  5.1 -> 3.6, 5.9 -> 5.3;
+// 1,024 of 512  3.2 -> 2.6, 3.5 -> 3.0; 512 of 256  2.3 -> 2.0, 2.4 -> 2.2.  A warp's own chain is the longer one, so a chip that
+// blocks of a row do not fill several times keeps those: 1,024 of 1,024  3.2 and 3.4, 3.6 and 4.5; 512 of 512  2.3 and 2.4,
+// 2.4 and 2.9; 384 of 256  2.1 and 2.1, 2.2 and 2.2.
+#define RMS_WARPS 8
+#define RMS_WARPS_FROM(D) ((D) * 3 / 2 > 512 ? (D) * 3 / 2 : 512)
+template <typename TOut>
+__global__ void __launch_bounds__(32 * RMS_WARPS)
+rmsnorm_warps_kernel(const float* x, const float* delta, float* sum_out, const float* __restrict__ w, TOut* __restrict__ out, const int* __restrict__ rows, int n_rows,
+                     int D, float eps, float delta_scale) {
+    pdl_wait();
+    pdl_launch_dependents();
+    const int r = blockIdx.x * RMS_WARPS + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+    if (r >= n_rows) return;
+    const size_t src = (size_t)(rows ? rows[r] : r) * D;
+    float4 v[8];
+#pragma unroll
+    for (int k = 0; k < 8; ++k) v[k] = lane + 32 * k < D / 4 ? reinterpret_cast<const float4*>(x + src)[lane + 32 * k] : make_float4(0.f, 0.f, 0.f, 0.f);
+    if (delta) {
+#pragma unroll
+        for (int k = 0; k < 8; ++k)
+            if (lane + 32 * k < D / 4) {
+                const float4 d = reinterpret_cast<const float4*>(delta + src)[lane + 32 * k];
+                v[k].x += delta_scale * d.x; v[k].y += delta_scale * d.y; v[k].z += delta_scale * d.z; v[k].w += delta_scale * d.w;
+            }
+    }
+    float ss = 0.f;
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+        if (sum_out && lane + 32 * k < D / 4) reinterpret_cast<float4*>(sum_out + src)[lane + 32 * k] = v[k];
+        ss += v[k].x * v[k].x + v[k].y * v[k].y + v[k].z * v[k].z + v[k].w * v[k].w;
+    }
+    const float scale = rsqrtf(warp_sum(ss) / (float)D + eps);
+    TOut* o = out + (size_t)r * D;
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+        const int i = lane + 32 * k;
+        if (i >= D / 4) break;
+        const float4 g = reinterpret_cast<const float4*>(w)[i];
+        Pack4<TOut>::store(o + 4 * i, v[k].x * scale * g.x, v[k].y * scale * g.y, v[k].z * scale * g.z, v[k].w * scale * g.w);
+    }
+}
+
 template <typename TOut>
 static int launch_rmsnorm(const float* x, const float* delta, const float* planes, const unsigned char* plane_count,
                           size_t plane_stride, float* sum_out, const float* w, TOut* out, const int* rows,
@@ -287,7 +332,9 @@ static int launch_rmsnorm(const float* x, const float* delta, const float* plane
     const int work = vec ? D / 4 : D;
     const int block = work >= 1024 ? 256 : (work >= 256 ? 128 : 64);
     cudaError_t e = cudaSuccess;
-    if (vec && D / 4 <= 4 * 256) {
+    if (vec && D / 4 <= 8 * 32 && !planes && n_rows >= RMS_WARPS_FROM(D)) {
+        qwb_launch(rmsnorm_warps_kernel<TOut>, (n_rows + RMS_WARPS - 1) / RMS_WARPS, 32 * RMS_WARPS, 0, stream, x, delta, sum_out, w, out, rows, n_rows, D, eps, delta_scale);
+    } else if (vec && D / 4 <= 4 * 256) {
         qwb_launch_link(n_rows, QWB_LINK_ROWS_NORM, rmsnorm_rows_kernel<TOut, 4>, n_rows, 256, 0, stream, x, delta, planes, plane_count, plane_stride, sum_out, w, out, rows, D, eps, delta_scale);
     } else if (vec && D / 4 <= 8 * 256) {
         qwb_launch_link(n_rows, QWB_LINK_ROWS_NORM, rmsnorm_rows_kernel<TOut, 8>, n_rows, 256, 0, stream, x, delta, planes, plane_count, plane_stride, sum_out, w, out, rows, D, eps, delta_scale);

@@ -64,6 +64,22 @@ def test_rmsnorm(D, out_dtype):
     close(out, pm.rms_norm((f64(x) + f64(delta))[[6, 0, 3]], f64(w), eps), out_dtype)
 
 
+@pytest.mark.parametrize("n, D", [(511, 4), (512, 4), (517, 100), (512, 256), (768, 512), (1535, 1024), (1537, 1024), (1537, 1020), (2049, 1028)])
+def test_rmsnorm_of_many_rows(n, D):
+    g = torch.Generator().manual_seed(n + D)
+    x, delta = (torch.randn(n, D, generator=g) * 3).to(DEV), torch.randn(n, D, generator=g).to(DEV)
+    w = (1 + 0.1 * torch.randn(D, generator=g)).to(DEV)
+    for out_dtype in DTYPES:
+        close(ops.rmsnorm(x, w, 1e-5, out_dtype), pm.rms_norm(f64(x), f64(w), 1e-5), out_dtype)
+        x2 = x.clone()
+        out = ops.rmsnorm(x2, w, 1e-5, out_dtype, delta=delta, write_sum=True)
+        assert torch.equal(x2, x + delta)
+        close(out, pm.rms_norm(f64(x) + f64(delta), f64(w), 1e-5), out_dtype)
+        rows = torch.randperm(n, generator=g).to(torch.int32).to(DEV)
+        out = ops.rmsnorm(x, w, 1e-5, out_dtype, delta=delta, rows=rows)
+        close(out, pm.rms_norm((f64(x) + f64(delta))[rows.tolist()], f64(w), 1e-5), out_dtype)
+
+
 def test_rmsnorm_refuses_a_row_that_does_not_fit():
     with pytest.raises(KernelError, match="shared memory"):
         ops.rmsnorm(torch.zeros(1, 60000, device=DEV), torch.ones(60000, device=DEV), 1e-6, torch.float32)
