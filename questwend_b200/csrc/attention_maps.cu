@@ -1393,13 +1393,15 @@ maps_decode_mma_kernel(const bf16* __restrict__ q, const bf16* __restrict__ k_po
 // Per (query head, sequence): each map's a = sum_r acc_r e^(m_r - M) / sum_r l_r e^(m_r - M), M = max_r m_r, over the
 // sequence's runs in index order; then the difference of the maps, the norm and the factor.  grid (H, B), 128 threads a map:
 // a map's first warp makes its weights e^(m_r - M) / L once for all columns, while the first runs' values are on their way.
+// Launched early: its blocks stand ready while the last runs are read, and what comes after it may start as well.  The call,
+// 8 sequences of 8,192: 45.6 -> 44.8 us, one of 1,000: 11.3 -> 10.3.  So the runs' parts are no __restrict__ pointers.
 template <typename T>
 __global__ void __launch_bounds__(128 * QWB_MAPS_MAX)
-maps_merge_kernel(const float* __restrict__ part_acc, const float* __restrict__ part_m, const float* __restrict__ part_l,
+maps_merge_kernel(const float* part_acc, const float* part_m, const float* part_l,
                   const int* __restrict__ seq_len, T* __restrict__ out, int H, int maps, int vdim, MapsMask mask, int n_runs, int max_runs,
                   float lambda, int norm_out, float eps, float out_scale, MapsGate gate) {
-    pdl_wait();
     pdl_launch_dependents();
+    pdl_wait();
     constexpr int AHEAD = 16;
     __shared__ float red[32];
     __shared__ float wts[QWB_MAPS_MAX][QWB_MAPS_MAX_RUNS], second[2 * 128];
@@ -1516,7 +1518,7 @@ static int launch_maps_decode(const void* q, const void* k_pool, const void* v_p
                    H, G, maps, dim, vdim, table_width, scale, softcap, mask, n_runs);
     }
     if (int rc = qwb_check_launch("maps_decode")) return rc;
-    qwb_launch(maps_merge_kernel<T>, dim3(H, B), 128 * maps, 0, stream, (const float*)part_acc, (const float*)part_m, (const float*)part_l,
+    qwb_launch_early(maps_merge_kernel<T>, dim3(H, B), 128 * maps, 0, stream, (const float*)part_acc, (const float*)part_m, (const float*)part_l,
                seq_len, (T*)out, H, maps, vdim, mask, n_runs, mma ? MD_MAX_RUNS : QWB_MAPS_MAX_RUNS, lambda, norm_out, eps, out_scale, gate);
     return qwb_check_launch("maps_merge");
 }
