@@ -1,4 +1,4 @@
-// The way from Python to the kernels' launchers: a Python module of four functions.  A step of few tokens is a handful of launches of a few
+// The way from Python to the kernels' launchers: a Python module of five functions.  A step of few tokens is a handful of launches of a few
 // microseconds each, and through ctypes making a launcher's arguments (an object each), checking its tensors and asking for its outputs took
 // longer than the launches: one token through Mamba-2's convolution and recurrence 27 us of the host for 6 us of the GPU.
 //
@@ -7,6 +7,8 @@
 //     fits(tensor, dtype, dimensions)     whether it is a contiguous CUDA tensor of this type (None: any) and number of dimensions (None: any)
 //     empty(shape, dtype=, device=)       torch.empty for these arguments
 //     same(x)                             x
+//     fill(array, numbers)                a list's whole numbers into a contiguous array of as many 32-bit ones; False where the list holds anything
+//                                         else, or a number that does not fit: the array then holds any part of them
 //
 // Launchers take integers, pointers, floats and doubles and return an int.  On x86-64 (System V) integers and pointers go into six registers
 // and then onto the stack, in their order, floats and doubles into eight registers of their own, so one function type with many integers
@@ -165,10 +167,29 @@ PyObject* same(PyObject*, PyObject* x) {
     return x;
 }
 
+PyObject* fill(PyObject*, PyObject* const* args, Py_ssize_t n) {
+    if (n != 2 || !PyList_CheckExact(args[1])) Py_RETURN_FALSE;
+    Py_buffer to;
+    if (PyObject_GetBuffer(args[0], &to, PyBUF_WRITABLE | PyBUF_FORMAT | PyBUF_C_CONTIGUOUS)) return nullptr;
+    const Py_ssize_t count = PyList_GET_SIZE(args[1]);
+    bool ok = to.itemsize == 4 && to.len == 4 * count && to.format && std::strcmp(to.format, "i") == 0;
+    int32_t* out = static_cast<int32_t*>(to.buf);
+    for (Py_ssize_t i = 0; ok && i < count; ++i) {
+        PyObject* o = PyList_GET_ITEM(args[1], i);
+        int overflow = 0;
+        const long v = PyLong_CheckExact(o) ? PyLong_AsLongAndOverflow(o, &overflow) : INT64_MAX;
+        ok = !overflow && v >= INT32_MIN && v <= INT32_MAX;
+        if (ok) out[i] = (int32_t)v;
+    }
+    PyBuffer_Release(&to);
+    return PyBool_FromLong(ok);
+}
+
 PyMethodDef methods[] = {{"call", (PyCFunction)(void*)call, METH_FASTCALL, nullptr},
                          {"fits", (PyCFunction)(void*)fits, METH_FASTCALL, nullptr},
                          {"empty", (PyCFunction)(void*)empty, METH_FASTCALL | METH_KEYWORDS, nullptr},
                          {"same", same, METH_O, nullptr},
+                         {"fill", (PyCFunction)(void*)fill, METH_FASTCALL, nullptr},
                          {nullptr, nullptr, 0, nullptr}};
 PyModuleDef module_def = {PyModuleDef_HEAD_INIT, "qwb_host_call", nullptr, -1, methods, nullptr, nullptr, nullptr, nullptr};
 

@@ -23,7 +23,7 @@ from ..config.base import ModelConfig
 from ..config.registry import get_architecture, load_config
 from ..kernels import build as kernel_build
 from ..kernels import ops
-from ..kernels.ops import PAGE_SIZE
+from ..kernels.ops import PAGE_SIZE, fill_int32
 from ..parts.base import Runtime, StepContext
 from ..parts.linear import require_true_fp32
 from ..weights.loader import load_tensors
@@ -83,10 +83,11 @@ def build_step_context(cache: CacheManager, entries: list, vocab_size: int, devi
     w = 0
     for b, e in enumerate(entries):
         n = n_new[b]
-        try:
-            ids[t:t + n] = e.tokens
-        except (TypeError, ValueError, OverflowError):
-            raise EngineError(f"slot {e.slot}: token ids must be integers") from None
+        if not fill_int32(ids[t:t + n], e.tokens):
+            try:
+                ids[t:t + n] = e.tokens
+            except (TypeError, ValueError, OverflowError):
+                raise EngineError(f"slot {e.slot}: token ids must be integers") from None
         tok_seq[t:t + n] = b
         tok_pos[t:t + n] = np.arange(pos0[b], pos0[b] + n)
         cu[b] = t

@@ -77,3 +77,14 @@ def test_tensors_that_fit_and_outputs(host):
         host.empty((-1,), dtype=torch.float32, device=torch.device("cpu"))
     x = object()
     assert host.same(x) is x
+
+
+def test_lists_into_arrays(host):
+    import numpy as np
+    a = np.zeros(5, dtype=np.int32)
+    assert host.fill(a[1:4], [2 ** 31 - 1, -(2 ** 31), 7]) and a.tolist() == [0, 2 ** 31 - 1, -(2 ** 31), 7, 0] and host.fill(a[:0], [])
+    for array, numbers in ((a, [1, 2]), (a[:2], (1, 2)), (a[:2], [1, 2.0]), (a[:2], [1, True]), (a[:2], [1, 2 ** 31]), (a[:2], [1, -(2 ** 80)]), (a[:2], [1, np.int32(2)]),
+                           (np.zeros(2, dtype=np.int64), [1, 2]), (np.zeros(2, dtype=np.float32), [1, 2])):
+        assert host.fill(array, numbers) is False
+    with pytest.raises((BufferError, ValueError)):
+        host.fill(np.zeros(4, dtype=np.int32)[::2], [1, 2])
