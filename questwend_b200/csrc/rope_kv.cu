@@ -118,15 +118,19 @@ template <> struct Pack4Store<bf16> {
 
 // The same for head size 128 rotated over all 128 values, the common case.  Half a warp takes a head: lane L of the 16
 // holds values 4L..4L+3 and 64+4L..64+4L+3, so that a value and its rotation partner (64 places away) lie in one lane
-// and only the sum of squares crosses lanes (four shuffles).  A block takes one token: its eight warps share the
-// token's pairs of heads (warp w: pairs w, w + 8, ...), up to three pairs' loads on their way before the first is used
-// (all of a warp's for a token of 48 heads), the token's cos and sin, position and page looked up once.  A v head runs
+// and only the sum of squares crosses lanes (four shuffles).  A block takes one token: its four warps share the
+// token's pairs of heads (warp w: pairs w, w + 4, ...), one or two pairs' loads on their way at a time, the token's cos and
+// sin, position and page looked up once.  A v head runs
 // through the same arithmetic with a factor, weights and cosines of one and sines of zero: x * 1 - x' * 0 is x.
-// 2,048 tokens of 32 + 2 x 8 heads: 16.8 us (4.5 TB/s); with a whole warp per head and the partner by shuffle 19.7 us (the kernel
-// issued instructions 58 % of the time and moved 29 % of what the memory can), with a block per four heads 27.6 us.
-#define RK_WARPS 8
-#define RK_PAIRS_AT_ONCE 3
-template <typename TOut>
+// What a block waits for is the chain of its first loads, so small blocks with few registers, of which many stand on an SM, do
+// more than loads in flight: 3,001 tokens of 16 + 2 x 8 heads 15.2 us with eight warps and three pairs at a time, 11.4 with
+// four and two, 11.4 with one; of 64 + 2 x 8 heads 36.1, 34.1 and 36.5; 800 tokens of 32 + 2 x 8 heads 6.7, 6.3 and 5.8, one
+// token 2.4, 2.2 and 2.0 (inputs in L2).  Before, with a whole warp per head and the partner by shuffle 19.7 us (2,048 tokens of 32 + 2 x 8 heads;
+// it issued instructions 58 % of the time and moved 29 % of what the memory can), against 16.8 with half a warp per head, and 27.6 us with a block per four heads.
+#define RK_WARPS 4
+#define RK_BLOCKS 1184              // as many are wanted of a call
+#define RK_PAIRS_TOKENS 1536        // from so many on two pairs at a time
+template <typename TOut, int RK_PAIRS_AT_ONCE>
 __global__ void __launch_bounds__(RK_WARPS * 32)
 qk_norm_rope_store_hd128_kernel(const float* __restrict__ qkv, const float* __restrict__ q_weight,
                                 const float* __restrict__ k_weight, const float* __restrict__ cos_t,
@@ -220,19 +224,19 @@ extern "C" int qwb_qk_norm_rope_store(const float* qkv, const float* q_weight, c
                       (uintptr_t)k_pool % 16 == 0 && (uintptr_t)v_pool % 16 == 0 && (uintptr_t)cos_t % 16 == 0 &&
                       (uintptr_t)sin_t % 16 == 0 && (!q_weight || (uintptr_t)q_weight % 16 == 0) &&
                       (!k_weight || (uintptr_t)k_weight % 16 == 0);
-    // hd128 kernel: a block a token; with few tokens up to six blocks share a token's heads, so that there are blocks for the SMs
+    // hd128 kernel: a block a token; with few tokens up to a block per four pairs share a token's heads, so that there are blocks for the SMs
     int share = 1;
-    if (T < 592) {
-        share = (592 + T - 1) / T;
+    if (T < RK_BLOCKS) {
+        share = (RK_BLOCKS + T - 1) / T;
         const int most = ((Hq + 2 * Hkv + 1) / 2 + RK_WARPS - 1) / RK_WARPS;
         if (share > most) share = most;
     }
     if (fast && dtype == QWB_DT_F32)
-        qwb_launch(qk_norm_rope_store_hd128_kernel<float>, dim3(T, share), RK_WARPS * 32, 0, stream, qkv, q_weight, k_weight, cos_t, sin_t,
+        qwb_launch(T < RK_PAIRS_TOKENS ? qk_norm_rope_store_hd128_kernel<float, 1> : qk_norm_rope_store_hd128_kernel<float, 2>, dim3(T, share), RK_WARPS * 32, 0, stream, qkv, q_weight, k_weight, cos_t, sin_t,
                    tok_seq, tok_pos, page_table, (float*)q_out, (float*)k_pool, (float*)v_pool, Hq, Hkv, eps, page_size,
                    table_width, store_kv);
     else if (fast && dtype == QWB_DT_BF16)
-        qwb_launch(qk_norm_rope_store_hd128_kernel<bf16>, dim3(T, share), RK_WARPS * 32, 0, stream, qkv, q_weight, k_weight, cos_t, sin_t,
+        qwb_launch(T < RK_PAIRS_TOKENS ? qk_norm_rope_store_hd128_kernel<bf16, 1> : qk_norm_rope_store_hd128_kernel<bf16, 2>, dim3(T, share), RK_WARPS * 32, 0, stream, qkv, q_weight, k_weight, cos_t, sin_t,
                    tok_seq, tok_pos, page_table, (bf16*)q_out, (bf16*)k_pool, (bf16*)v_pool, Hq, Hkv, eps, page_size,
                    table_width, store_kv);
     else if (dtype == QWB_DT_F32)
