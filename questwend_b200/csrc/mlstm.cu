@@ -26,10 +26,14 @@ struct MlstmRows { const float* x; int ld, i_col, f_col; };
 struct MlstmGates { const float *i_bias, *f_bias; float cap; };
 
 __device__ __forceinline__ float mlstm_log_sigmoid(float z) { return z > 0.f ? -log1pf(expf(-z)) : z - log1pf(expf(z)); }
+// a token's two gates from their raw values, and from its row
+__device__ __forceinline__ void mlstm_log_gates(MlstmGates g, float raw_i, float raw_f, float bias_i, float bias_f, float& i, float& f) {
+    i = g.cap * tanhf((raw_i + bias_i) / g.cap);
+    f = mlstm_log_sigmoid(g.cap * tanhf((raw_f + bias_f) / g.cap));
+}
 __device__ __forceinline__ void mlstm_log_gates(MlstmRows rows, MlstmGates g, int t, int h, float& i, float& f) {
     const float* row = rows.x + (size_t)t * rows.ld;
-    i = g.cap * tanhf((row[rows.i_col + h] + g.i_bias[h]) / g.cap);
-    f = mlstm_log_sigmoid(g.cap * tanhf((row[rows.f_col + h] + g.f_bias[h]) / g.cap));
+    mlstm_log_gates(g, row[rows.i_col + h], row[rows.f_col + h], g.i_bias[h], g.f_bias[h], i, f);
 }
 
 // ---------------------------------------------------------------------------------
@@ -38,7 +42,8 @@ __device__ __forceinline__ void mlstm_log_gates(MlstmRows rows, MlstmGates g, in
 // over a warp's tokens and then over the warps.  With the rounded maxima, log_decay = m + f - m' telescopes exactly.
 // Outputs [T, H].  What it costs is a sequence's chain of passes, each its loads, its logarithms and its scans one after the
 // other: 256 tokens a pass took 4,096 tokens through 16 passes (4 heads of 64 x 64 in chunks, 59.6 us in all), 1,024 take
-// them through four (51.7).  Short steps are as fast as they were: a block has no more warps than the step fills.
+// them through four (51.7).  Short steps are as fast as they were: a block has no more warps than the step fills.  A pass's raw gates
+// are asked for while the pass before is scanned: 17.2 -> 14.8 us of 4,096 tokens.
 // ---------------------------------------------------------------------------------
 #define QWB_MLSTM_GATE_THREADS 1024
 
@@ -52,7 +57,7 @@ __device__ __forceinline__ void mlstm_scan_maps(double& F, double& X) {
     }
 }
 
-__global__ void __launch_bounds__(QWB_MLSTM_GATE_THREADS)
+__global__ void __launch_bounds__(QWB_MLSTM_GATE_THREADS, 1)
 mlstm_gates_kernel(MlstmRows rows, MlstmGates gates, const float* __restrict__ m_state, const int* __restrict__ cu_seqlens,
                    const int* __restrict__ slots, float* __restrict__ log_decay, float* __restrict__ write, float* __restrict__ m_run, int H, int P) {
     pdl_wait();
@@ -61,14 +66,22 @@ mlstm_gates_kernel(MlstmRows rows, MlstmGates gates, const float* __restrict__ m
     __shared__ float last_m[32];
     const int h = blockIdx.x, b = blockIdx.y, warp = threadIdx.x >> 5, lane = threadIdx.x & 31, warps = blockDim.x >> 5;
     const int t0 = cu_seqlens[b], t1 = cu_seqlens[b + 1];
+    const float* raw = rows.x + h;
+    const float bias_i = gates.i_bias[h], bias_f = gates.f_bias[h];
+    float raw_i = 0.f, raw_f = 0.f;
+    if (t0 + (int)threadIdx.x < t1) { raw_i = raw[(size_t)(t0 + threadIdx.x) * rows.ld + rows.i_col]; raw_f = raw[(size_t)(t0 + threadIdx.x) * rows.ld + rows.f_col]; }
     double carry = (double)m_state[((size_t)slots[b] * H + h) * (P + 1)];
     for (int base = t0; base < t1; base += blockDim.x) {
         const int t = base + threadIdx.x;
         float i = 0.f, f = 0.f;
         double F = 0.0, X = -INFINITY;                              // beyond the end: the map that changes nothing
         if (t < t1) {
-            mlstm_log_gates(rows, gates, t, h, i, f);
+            mlstm_log_gates(gates, raw_i, raw_f, bias_i, bias_f, i, f);
             F = (double)f; X = (double)i;
+        }
+        if (t + blockDim.x < t1) {                                  // the next pass's, while this one's scans run
+            raw_i = raw[(size_t)(t + blockDim.x) * rows.ld + rows.i_col];
+            raw_f = raw[(size_t)(t + blockDim.x) * rows.ld + rows.f_col];
         }
         mlstm_scan_maps(F, X);
         if (lane == 31) { tot_f[warp] = F; tot_x[warp] = X; }
@@ -574,33 +587,34 @@ __device__ __forceinline__ CtRows ml_rows(const MlArgs& a, int t0, int n, int h)
     return {x + h * a.z.K, x + (a.z.H + h) * a.z.K, x + 2 * a.z.H * a.z.K + h * a.z.P, a.rows.ld, n};
 }
 
-// grid (chunks, H, B), 1,024 threads: a chunk's gates, and its own sum of the normaliser, 32 tokens and a key row a thread (16.6 us with
-// all 128 tokens, 4,096 tokens of 4 heads of 256 x 512)
-__global__ void __launch_bounds__(1024)
-mlstm_tile_gates_kernel(const MlArgs a) {
+// grid (chunks, H * ktiles, B), 1,024 threads: a chunk's gates, and its own sum of the normaliser over 128 key rows, 16 tokens and a key
+// row a thread.  Each block makes the gates (all write the same); the keys are asked for before that, and a thread's 16 fit its
+// registers.  A chain of waits either way: 14.0 us with a block a head, 32 tokens a thread and the keys asked for behind the
+// gates, 9.2 now (4,096 tokens of 4 heads of 256 x 512).
+__global__ void __launch_bounds__(1024, 1)
+mlstm_tile_gates_kernel(const MlArgs a, int ktiles) {
     pdl_wait();
     pdl_launch_dependents();
-    __shared__ float coef[ML_TOKENS], part[4][256];
+    __shared__ float coef[ML_TOKENS], part[8][128];
     int t0;
     size_t place;
-    const int n = ml_chunk(a, place, t0), h = blockIdx.y, i = threadIdx.x, K = a.z.K, column = i & 255, group = i >> 8;
+    const int n = ml_chunk(a, place, t0), h = blockIdx.y / ktiles, i = threadIdx.x, column = i & 127, group = i >> 7, k = (blockIdx.y - h * ktiles) * 128 + column;
     if (n <= 0) return;
     const size_t at = (size_t)(t0 + i) * a.z.H + h, head = place * a.z.H + h;
-    ct_gates(i < n ? a.log_decay[at] : 0.f, i < n ? a.write[at] : 0.f, a.gates + head, a.totals + head, coef);
+    const float log_decay = i < n ? a.log_decay[at] : 0.f, write = i < n ? a.write[at] : 0.f;
     const CtRows r = ml_rows(a, t0, n, h);
-    for (int k0 = 0; k0 < K; k0 += 256) {
-        const int k = k0 + column;
-        float sum = 0.f;
+    float key[16];
 #pragma unroll
-        for (int e = 0; e < 32; ++e) {
-            const int j = 32 * group + e;
-            if (j < n && k < K) sum += coef[j] * r.k[(size_t)j * r.ld + k];
-        }
-        __syncthreads();
-        part[group][column] = sum;
-        __syncthreads();
-        if (group == 0 && k < K) a.own_n[head * K + k] = (part[0][column] + part[1][column]) + (part[2][column] + part[3][column]);
-    }
+    for (int e = 0; e < 16; ++e) key[e] = 16 * group + e < n && k < a.z.K ? r.k[(size_t)(16 * group + e) * r.ld + k] : 0.f;
+    ct_gates(log_decay, write, a.gates + head, a.totals + head, coef);
+    float sum = 0.f;
+#pragma unroll
+    for (int e = 0; e < 16; ++e)
+        if (16 * group + e < n) sum += coef[16 * group + e] * key[e];
+    part[group][column] = sum;
+    __syncthreads();
+    if (group == 0 && k < a.z.K)
+        a.own_n[head * a.z.K + k] = ((part[0][column] + part[1][column]) + (part[2][column] + part[3][column])) + ((part[4][column] + part[5][column]) + (part[6][column] + part[7][column]));
 }
 
 // grid (chunks, 2 H + H * ptiles * ktiles, B): the scores of a head's chunk with 64 of its tokens, or 64 values x 128 key rows of its own sum
@@ -805,7 +819,7 @@ extern "C" int qwb_mlstm_tiles(const float* x, int ld, int i_col, int f_col, con
     cudaError_t e = cudaFuncSetAttribute(mlstm_tile_state_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, CT_SMEM);
     if (e == cudaSuccess) e = cudaFuncSetAttribute(mlstm_tile_out_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, CT_SMEM);
     if (e != cudaSuccess) return qwb_fail(QWB_ERR_CUDA, "mlstm_tiles: %s", cudaGetErrorString(e));
-    qwb_launch(mlstm_tile_gates_kernel, dim3(chunks, H, B), 1024, 0, stream, a);
+    qwb_launch(mlstm_tile_gates_kernel, dim3(chunks, H * ktiles, B), 1024, 0, stream, a, ktiles);
     if (int rc = qwb_check_launch("mlstm_tile_gates")) return rc;
     qwb_launch(mlstm_tile_state_kernel, dim3(chunks, 2 * H + H * ptiles * ktiles, B), CT_THREADS, CT_SMEM, stream, a, ptiles, ktiles);
     if (int rc = qwb_check_launch("mlstm_tile_state")) return rc;
