@@ -1,5 +1,6 @@
 """Rules that pick a kernel's form by sizes alone."""
 import pytest
+import torch
 
 from questwend_b200.kernels import ops
 
@@ -16,3 +17,19 @@ def test_latent_prompts_refuse_the_same_query_sizes_in_both_forms():
     """Query sizes that are no multiple of 16 are refused by the mma.sync kernel: the tcgen05 one does not take them either."""
     assert ops.latent_prefill_tc_fits(128, 64, 128) and ops.latent_prefill_tc_fits(24, 8, 40) and ops.latent_prefill_tc_fits(8, 8, 8)
     assert not ops.latent_prefill_tc_fits(24, 0, 64) and not ops.latent_prefill_tc_fits(64, 8, 64) and not ops.latent_prefill_tc_fits(128, 64, 136)
+
+
+@pytest.mark.parametrize("lens, heads, key_dim, vdim, tiles", [
+    ([4096], 4, 256, 512, True), ([64], 4, 256, 512, True), ([64] * 8, 4, 256, 512, True), ([2048] + [1] * 63, 4, 256, 512, False), ([100], 16, 128, 128, True),
+    ([130] * 16, 16, 128, 128, True), ([64] * 8, 16, 128, 128, False), ([4096], 4, 64, 64, False), ([4096], 15, 128, 128, False)])
+def test_matrix_memory_takes_long_chunks_for_large_memories(lens, heads, key_dim, vdim, tiles):
+    assert ops._mlstm_tiles(sum(lens), len(lens), heads, key_dim, vdim) is tiles
+
+
+@pytest.mark.parametrize("tokens, top, experts, shared, dtype, grouped", [
+    (128, 6, 64, 2816, torch.bfloat16, False), (129, 1, 256, 0, torch.bfloat16, True), (17, 6, 64, 2816, torch.bfloat16, False), (17, 6, 64, 2812, torch.bfloat16, True),
+    (16, 8, 8, 2812, torch.bfloat16, False), (128, 2, 16, 0, torch.bfloat16, False), (128, 2, 15, 0, torch.bfloat16, True), (64, 2, 8, 0, torch.bfloat16, False),
+    (200, 6, 64, 0, torch.float32, False)])
+def test_experts_are_sorted_only_in_long_steps(tokens, top, experts, shared, dtype, grouped):
+    x, up, down = (torch.empty(s, dtype=dtype, device="meta") for s in ((tokens, 64), (experts, 64, 64), (experts, 64, 32)))
+    assert ops.moe_grouped_fits(x, up, down, top, shared) is grouped
