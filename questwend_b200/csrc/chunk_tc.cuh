@@ -1,5 +1,5 @@
 // The matrix products of the recurrences whose state is a sum of outer products with one decay a token and head (Mamba-2, the mLSTM), in
-// chunks of 128 tokens, on tcgen05.  With k_j, v_j the keys and values of a chunk's tokens, q_i what reads, w_j the write strengths, G_i the
+// chunks of 128 tokens, on tcgen05 (the delta rule's outputs take ct_products from here too).  With k_j, v_j the keys and values of a chunk's tokens, q_i what reads, w_j the write strengths, G_i the
 // sum of the log decays up to token i and S0 the state at the chunk's start,
 //     own   = sum_j k_j (e^(G_end - G_j) w_j v_j)^T                                          ct_state
 //     out_i = (e^(G_i) q_i) S0 + sum_{j <= i} (e^(G_i - G_j) w_j (q_i . k_j)) v_j            ct_out, the products q_i . k_j from ct_pairs

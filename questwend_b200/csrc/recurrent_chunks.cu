@@ -1,6 +1,6 @@
 // Long prompts through the recurrences of recurrent.cu in chunks: inside a chunk the tokens meet in small matrix products,
-// from chunk to chunk only the state is carried.  Everything is 32-bit: Mamba-2's products on the tensor cores as sums of products of
-// bfloat16 parts (chunk_tc.cuh), the delta rule's in plain multiply-adds.  Decays enter as sums of their
+// from chunk to chunk only the state is carried.  Everything is 32-bit: Mamba-2's products and the delta rule's outputs on the tensor cores
+// as sums of products of bfloat16 parts (chunk_tc.cuh), the rest of the delta rule in plain multiply-adds.  Decays enter as sums of their
 // logarithms, always of tokens between two others, so every exponential is of a number that is at most 0: nothing overflows, and
 // what underflows is below the smallest float in truth too.
 #include "chunk_tc.cuh"
@@ -166,9 +166,9 @@ extern "C" int qwb_ssm_chunked(const float* xbc, int ldx, const float* dt_raw, i
 // its sub-block's end, what decays in the sub-blocks between, and what decays from the start of i's sub-block to i are three
 // factors of at most 1.  Sums of logarithms (base 2) span what they decay and nothing else.
 // Chunk c of the z-th sequence that these kernels take, b, is place cu_seqlens[b] / 64 + z + c of the scratch memory.
-// 16 heads of 128 x 128 with a decay per channel, the convolution before it, the scan and now: 2,048 tokens 955 -> 328 us (prep 123,
-// walk 133, out 49 in ncu), three sequences of 2,900 in all 1,194 -> 484 us; a decay per head, four of 4,096 in all, 1,198 -> 596 us.
-// Bound by what shared memory hands to registers (128 bytes a cycle), the walk more than the others.
+// 16 heads of 128 x 128 with a decay per channel, the convolution before it, three sequences of 2,900 tokens in all: 1,194 us by the scan,
+// 498 with plain multiply-adds in 8 x 8 sums a thread, 411 now (prep 157, walk 143, out 42, the convolution 35, norms 21).
+// The first two are bound by what shared memory hands to registers (128 bytes a cycle).
 // Scratch of a place and head:
 //     W [64][K] | k e_end [64][K] | q e_0 [64][K] | Q [64 (i)][64 (j)] | U, then u [64][P] | decay of the chunk [K] | S0 [K][P]
 // ---------------------------------------------------------------------------------
