@@ -277,7 +277,8 @@ rmsnorm_rows_kernel(const float* x, const float* delta, const float* planes, con
     }
 }
 
-// Many rows of up to 1,024 values: a warp a row, eight rows a block, no barrier.  A block a row is bound by its start, its two
+// Many rows of up to 1,024 values: a warp a row, eight rows a block, no barrier; the same sums in the same order, so the same bits
+// however many rows there are.  A block a row is bound by its start, its two
 // barriers and one load a thread; a warp has the whole row in flight.  us, a block a row -> a warp a row, norm alone and with
 // the residual's sum (bf16 out, rows in L2): 3,001 rows of 1,024  6.9 -> 3.7, 7.8 -> 6.2; 2,048 of 1,024  5.1 -> 3.6, 5.9 -> 5.3;
 // 1,024 of 512  3.2 -> 2.6, 3.5 -> 3.0; 512 of 256  2.3 -> 2.0, 2.4 -> 2.2.  A warp's own chain is the longer one, so a chip that
@@ -305,13 +306,29 @@ rmsnorm_warps_kernel(const float* x, const float* delta, float* sum_out, const f
                 v[k].x += delta_scale * d.x; v[k].y += delta_scale * d.y; v[k].z += delta_scale * d.z; v[k].w += delta_scale * d.w;
             }
     }
-    float ss = 0.f;
+    float part[8];
 #pragma unroll
     for (int k = 0; k < 8; ++k) {
         if (sum_out && lane + 32 * k < D / 4) reinterpret_cast<float4*>(sum_out + src)[lane + 32 * k] = v[k];
-        ss += v[k].x * v[k].x + v[k].y * v[k].y + v[k].z * v[k].z + v[k].w * v[k].w;
+        part[k] = v[k].x * v[k].x + v[k].y * v[k].y + v[k].z * v[k].z + v[k].w * v[k].w;
     }
-    const float scale = rsqrtf(warp_sum(ss) / (float)D + eps);
+    // the sums of the eight warps that a block a row has, each by the tree that warp_sum adds it up by: every step adds half of
+    // what is left across one bit of the lane, which then says which half is kept
+#pragma unroll
+    for (int bit = 16, n = 4; n > 0; bit >>= 1, n >>= 1) {
+        const bool up = lane & bit;
+#pragma unroll
+        for (int e = 0; e < n; ++e) {
+            const float keep = up ? part[n + e] : part[e], give = up ? part[e] : part[n + e];
+            part[e] = keep + __shfl_xor_sync(0xffffffffu, give, bit);
+        }
+    }
+    part[0] += __shfl_xor_sync(0xffffffffu, part[0], 2);
+    part[0] += __shfl_xor_sync(0xffffffffu, part[0], 1);        // of values 128 (lane / 4) .. + 127
+    float total = 0.f;
+#pragma unroll
+    for (int k = 0; k < 8; ++k) total += __shfl_sync(0xffffffffu, part[0], 4 * k);
+    const float scale = rsqrtf(total / (float)D + eps);
     TOut* o = out + (size_t)r * D;
 #pragma unroll
     for (int k = 0; k < 8; ++k) {

@@ -80,6 +80,20 @@ def test_rmsnorm_of_many_rows(n, D):
         close(out, pm.rms_norm((f64(x) + f64(delta))[rows.tolist()], f64(w), 1e-5), out_dtype)
 
 
+@pytest.mark.parametrize("D", [4, 100, 128, 256, 388, 512, 772, 1020, 1024])
+def test_rmsnorm_of_a_row_does_not_depend_on_how_many_there_are(D):
+    """The same bits from a block a row and from a warp a row: each adds a row's squares up in one order."""
+    g = torch.Generator().manual_seed(D)
+    n = max(512, -(-3 * D // 2)) + 5
+    x, delta = (torch.randn(n, D, generator=g) * 3).to(DEV), torch.randn(n, D, generator=g).to(DEV)
+    w = (1 + 0.1 * torch.randn(D, generator=g)).to(DEV)
+    for add in (None, delta):
+        for out_dtype in DTYPES:
+            many = ops.rmsnorm(x, w, 1e-5, out_dtype, delta=add)
+            few = torch.cat([ops.rmsnorm(x[i:i + 300], w, 1e-5, out_dtype, delta=None if add is None else add[i:i + 300]) for i in range(0, n, 300)])
+            assert torch.equal(many, few)
+
+
 def test_rmsnorm_refuses_a_row_that_does_not_fit():
     with pytest.raises(KernelError, match="shared memory"):
         ops.rmsnorm(torch.zeros(1, 60000, device=DEV), torch.ones(60000, device=DEV), 1e-6, torch.float32)
