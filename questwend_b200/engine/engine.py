@@ -200,11 +200,11 @@ class Engine:
         return logits
 
     def check_kernels(self) -> None:
-        """Raise if a kernel with bounded waits (the TMA-fed products, the tcgen05 attention) gave one up since the last
-        check: its result is then not valid.  Reads one int from the device, so it waits for the work queued so far."""
-        if self.dtype == torch.bfloat16:
-            with torch.cuda.device(self.device):
-                ops.gemm_tc_check(self.device)
+        """Raise if a kernel with bounded waits (the TMA-fed products, the tcgen05 attention, in both engines the recurrences in
+        chunks) gave one up since the last check: its result is then not valid.  Reads one int from the device, so it waits for the
+        work queued so far, if such a kernel was launched at all."""
+        with torch.cuda.device(self.device):
+            ops.gemm_tc_check(self.device)
 
     def decode_runner(self, batch: int, sampling, use_graph: bool = True):
         """The fixed buffers and CUDA graphs for decode steps of ``batch`` sequences (made once, kept).  The sampling

@@ -793,7 +793,7 @@ def gemm_ring_xielu(x: torch.Tensor, weight: torch.Tensor, params: torch.Tensor)
     return out
 
 
-_TC_ERROR: dict = {}    # device -> one int32 that a gemm_tc kernel sets when one of its waits gives up
+_TC_ERROR: dict = {}    # device -> one int32 that a kernel sets when one of its bounded waits gives up; made when the first such kernel is launched
 TC_EPILOGUES = {"store": 0, "add": 1, "swiglu": 2}
 
 
@@ -805,14 +805,16 @@ def gemm_tc_error_word(device) -> torch.Tensor:
 
 
 def gemm_tc_check(device) -> None:
-    """Raise if a tcgen05 kernel (product or attention) on this device gave up a wait since the last check (reads one
-    int: synchronises)."""
-    word = gemm_tc_error_word(device)
+    """Raise if a tcgen05 kernel (product, attention, or a recurrence in chunks) on this device gave up a wait since the last check
+    (reads one int: synchronises; where no such kernel was launched there is nothing to read)."""
+    word = _TC_ERROR.get(torch.device(device).index or 0)
+    if word is None:
+        return
     code = int(word.item())
     if code:
         word.zero_()
         where = {1: "the loader waiting for a free stage", 2: "the tensor-core issuer waiting for its operands",
-                 3: "the epilogue or softmax warps waiting for the tensor core",
+                 3: "the epilogue, softmax or collecting warps waiting for the tensor core",
                  7: "shared memory was not aligned to 1024 bytes"}.get(code, f"code {code}")
         raise KernelError(f"a bounded wait in a tcgen05 kernel ran out ({where}); that kernel's result is not valid")
 
