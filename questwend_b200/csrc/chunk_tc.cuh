@@ -7,7 +7,7 @@
 // of each `own` the state that its chunk starts from.
 //
 // Every product is 128 x R by R x 64, in stages of 32 of R.  32-bit products: a number is the sum of three bfloat16 ones (each the nearest to
-// what the ones before leave: exact), a product of two is six products of parts; the other three are below 2^-24 of it.  The tensor cores
+// what the ones before leave: exact), a product of two is six products of parts; the other three are below 2^-26 of it.  The tensor cores
 // cut what they add and do not round it, so the largest parts' product is summed over a stage at a time, from 0, and these sums are added up
 // by rounded additions; the five small ones are summed on the side, where 2^-8 of a cut is lost.  CT_CUT is what the cut additions of a
 // stage take from its sum on average (measured: errors of the outputs against 64 bits 0.95e-7 without, 0.86 with 4e-8, 0.99 with 8e-8).  Values that are not finite, or within 0.4 % of the largest float, become no numbers.
@@ -15,7 +15,7 @@
 // 256 threads, two blocks an SM.  All of them load a stage's rows (24 values a thread, on their way while the stage before is prepared),
 // weigh them, split them and store the parts into one half of the shared memory, in the swizzled rows of 128 bytes that tcgen05 reads, while
 // the other half is multiplied; one thread issues the products, and the sums of the stage before are collected behind that.  Products that
-// share the left parts are one instruction (right parts side by side), as what bounds them is the reading of shared memory: 28 KB in place
+// share the left parts are one instruction (right parts side by side), as what bounds them is the reading of shared memory: 30 KB in place
 // of 36 for 16 of R.  Tensor memory, 64 columns each: the large sums of two stages, the two small ones.  What was measured on the way, 2,048
 // tokens of 64 Mamba-2 heads of 64 x 128, us of the own sums / of the outputs: plain multiply-adds 81 / 107; mma.sync with the parts in
 // shared memory 75 / 100 (its products alone leave 63 / 80); tcgen05 in stages of 64 that wait for their products 41 / 75; as here 39 / 60.
@@ -81,6 +81,23 @@ __device__ __forceinline__ void ct_load_planes(const float* m, int rows, int row
     const float4 x = rc_load4(at, ok && col < cols), y = rc_load4(at + (size_t)rows * 4, ok && col + 4 < cols);
     v[0] = x.x; v[1] = x.y; v[2] = x.z; v[3] = x.w; v[4] = y.x; v[5] = y.y; v[6] = y.z; v[7] = y.w;
 }
+
+// What a step of 16 of R is made of: left part a by `parts` right parts from part b on, side by side, onto the sums from `column` on (the
+// large sum of odd stages 64 further).  tcgen05.mma's are ordered against each other when accumulator and shape are the same: products onto
+// shared columns must have both.  So the last one makes its second product (2^-27 of the sum) only for its shape.
+struct CtProduct { int a, b, parts, column; };
+#define CT_PRODUCTS 4
+__device__ constexpr CtProduct ct_product[CT_PRODUCTS] = {{0, 0, 1, 0}, {0, 1, 2, 128}, {1, 0, 2, 128}, {2, 0, 2, 128}};
+__host__ __device__ constexpr bool ct_ordered() {
+    for (int i = 0; i < CT_PRODUCTS; ++i)
+        for (int j = 0; j < i; ++j) {
+            const CtProduct &x = ct_product[i], &y = ct_product[j];
+            const int wide_x = i == 0 ? 128 : 64 * x.parts, wide_y = j == 0 ? 128 : 64 * y.parts;          // the first: both large sums
+            if (x.column < y.column + wide_y && y.column < x.column + wide_x && !(x.column == y.column && x.parts == y.parts)) return false;
+        }
+    return true;
+}
+static_assert(ct_ordered(), "products onto the same columns in one shape only");
 
 // The block's shared and tensor memory; the whole block calls, ct_end too
 __device__ __forceinline__ CtBlock ct_begin(int* error) {
@@ -163,10 +180,12 @@ __device__ __forceinline__ bool ct_products(const CtBlock& c, int stages, Load l
                 for (int p = 0; p < 3; ++p) a[p] = (A_ROWS ? at_desc_mnmajor(c.a + p * CT_A_PART, 8192) : at_desc_kmajor(c.a + p * CT_A_PART)) + STEP_A * k;
 #pragma unroll
                 for (int p = 0; p < 2; ++p) b[p] = (B_ROWS ? at_desc_mnmajor(c.b + p * CT_B_PART, CT_B_PART) : at_desc_kmajor(c.b + p * CT_B_PART)) + STEP_B * k;
-                at_mma(c.tmem + 64 * (s & 1), a[0], b[0], one, i);
-                at_mma(c.tmem + 128, a[0], b[1], two, s > 0 || i > 0);      // by parts 1 and 2
-                at_mma(c.tmem + 128, a[1], b[0], two, 1);                   // by parts 0 and 1
-                at_mma(c.tmem + 192, a[2], b[0], one, 1);
+#pragma unroll
+                for (int p = 0; p < CT_PRODUCTS; ++p) {
+                    const CtProduct& m = ct_product[p];
+                    const bool first = i == 0 && (p == 0 || (p == 1 && s == 0));
+                    at_mma(c.tmem + m.column + (p == 0 ? 64 * (s & 1) : 0), a[m.a], b[m.b], m.parts == 2 ? two : one, !first);
+                }
             }
             at_commit(&c.bars[s & 1]);
         }
