@@ -10,7 +10,11 @@
 // what the ones before leave: exact), a product of two is six products of parts; the other three are below 2^-26 of it.  The tensor cores
 // cut what they add and do not round it, so the largest parts' product is summed over a stage at a time, from 0, and these sums are added up
 // by rounded additions; the five small ones are summed on the side, where 2^-8 of a cut is lost.  CT_CUT is what the cut additions of a
-// stage take from its sum on average (measured: errors of the outputs against 64 bits 0.95e-7 without, 0.86 with 4e-8, 0.99 with 8e-8).  Values that are not finite, or within 0.4 % of the largest float, become no numbers.
+// stage take from its sum on average (measured: errors of the outputs against 64 bits 0.95e-7 without, 0.86 with 4e-8, 0.99 with 8e-8).
+// A value that is not finite, or within 0.4 % of the largest float, has a part that is not finite and another that is no number, and so makes
+// all sums of its row or column no numbers, also those that it enters with a weight of 0.  A thread that ends up with such a sum forms
+// its sums again by plain multiply-adds, over the terms that they have (ct_lost).  Of a value below 2^-110 the last part has fewer digits than it
+// wants: it is below bfloat16's range.
 //
 // 256 threads, two blocks an SM.  All of them load a stage's rows (24 values a thread, on their way while the stage before is prepared),
 // weigh them, split them and store the parts into one half of the shared memory, in the swizzled rows of 128 bytes that tcgen05 reads, while
@@ -261,6 +265,27 @@ __device__ __forceinline__ void ct_gates(float log_decay, float write, CtGates* 
     }
 }
 
+// Whether a sum is no number.  If so, all of them are 0, for the caller to add its terms up without the tensor cores.
+__device__ __forceinline__ bool ct_lost(float (&sum)[32]) {
+    bool lost = false;
+#pragma unroll
+    for (int i = 0; i < 32; ++i) lost |= sum[i] != sum[i];
+    if (lost) {
+#pragma unroll
+        for (int i = 0; i < 32; ++i) sum[i] = 0.f;
+    }
+    return lost;
+}
+// sum[i] += x * w * y[i / 4][i % 4], `count` (a multiple of 4) of y, four neighbours at a time, `step` floats apart
+__device__ __forceinline__ void ct_add(float (&sum)[32], float x, float w, const float* y, size_t step, int count) {
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+        if (4 * i >= count) break;
+        const float4 v = *reinterpret_cast<const float4*>(y + i * step);
+        sum[4 * i] += x * (w * v.x); sum[4 * i + 1] += x * (w * v.y); sum[4 * i + 2] += x * (w * v.z); sum[4 * i + 3] += x * (w * v.w);
+    }
+}
+
 // Which eight of a stage are a lane's.  Of rows in memory whose neighbouring values are neighbours of R: row 8 warp + ct_row(lane), the
 // (lane % 4)-th eight; a quarter of a warp then writes to all banks of shared memory.  Of rows that are indices of R: row 4 warp + lane / 8, the
 // (lane % 8)-th eight.  Of a matrix in planes: a row a lane, an eight a warp.
@@ -285,6 +310,16 @@ __device__ __forceinline__ void ct_pairs(const CtRows& r, int K, int j0, float* 
             ct_put(c.b, CT_B_PART, row, 4 * (s & 1) + eight, v[2]);
         },
         sum);
+    if (ok && ct_lost(sum)) {
+        const int token = 32 * (warp & 3) + lane, j = j0 + 32 * (warp >> 2);
+#pragma unroll 1
+        for (int k = 0; token < r.n && k < K; ++k) {
+            const float x = r.q[(size_t)token * r.ld + k];
+#pragma unroll
+            for (int i = 0; i < 32; ++i)
+                if (j + i < r.n) sum[i] += x * r.k[(size_t)(j + i) * r.ld + k];
+        }
+    }
     if (ok) {
         float4* to = reinterpret_cast<float4*>(pairs) + (size_t)(j0 / 4 + 8 * (warp >> 2)) * CT_TOKENS + 32 * (warp & 3) + lane;
 #pragma unroll
@@ -319,6 +354,10 @@ __device__ __forceinline__ void ct_state(const CtRows& r, const CtGates* gates, 
         },
         sum);
     const int k = k0 + 32 * (warp & 3) + lane, p = p0 + 32 * (warp >> 2);
+    if (ok && ct_lost(sum) && k < K) {
+#pragma unroll 1
+        for (int j = 0; j < r.n; ++j) ct_add(sum, r.k[(size_t)j * r.ld + k], coef[j], r.v + (size_t)j * r.ld + p, 4, P - p);
+    }
     if (ok && k < K) {
         float4* to = reinterpret_cast<float4*>(own) + (size_t)(p / 4) * K + k;
 #pragma unroll
@@ -425,6 +464,16 @@ __device__ __forceinline__ void ct_out(const CtRows& r, const float* starts, con
             }
         },
         sum);
+    if (ok && ct_lost(sum) && token < r.n) {
+        const int p = p0 + 32 * (warp >> 2);
+#pragma unroll 1
+        for (int k = 0; k < K; ++k) ct_add(sum, fade[token] * r.q[(size_t)token * r.ld + k], 1.f, starts + ((size_t)(p / 4) * K + k) * 4, (size_t)K * 4, P - p);
+#pragma unroll 1
+        for (int j = 0; j <= token; ++j) {
+            const float w = (token ^ j) < 8 ? near[(j >> 2) & 1][token][j & 3] : expf((float)(G[token] - G[j | 7])) * left[j];
+            ct_add(sum, w * pairs[((size_t)(j / 4) * CT_TOKENS + token) * 4 + j % 4] + (j == token ? skip : 0.f), 1.f, r.v + (size_t)j * r.ld + p, 4, P - p);
+        }
+    }
     if (ok) {                                                       // by way of shared memory, so that a row's values leave together
         float4* stage = reinterpret_cast<float4*>(c.a);
 #pragma unroll

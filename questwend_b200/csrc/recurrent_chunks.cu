@@ -625,9 +625,23 @@ delta_chunk_out_kernel(const DcArgs a, int ptiles) {
             ct_put(block.b, CT_B_PART, token, 4 * (s & 1) + eight, v[2]);
         },
         sum);
-    const int p = p0 + 32 * (warp & 3) + lane;
+    const int p = p0 + 32 * (warp & 3) + lane, first = 32 * (warp >> 2);
+    if (ok && ct_lost(sum) && p < P) {                              // token `first` + i sees the chunk's tokens up to itself
+#pragma unroll 1
+        for (int k = 0; k < K; ++k) {
+            const float x = at.start[(size_t)k * P + p];
+#pragma unroll
+            for (int i = 0; i < 32; ++i) sum[i] += x * at.q0[(first + i) * K + k];
+        }
+#pragma unroll 1
+        for (int j = 0; j < n; ++j) {
+            const float x = at.u[(size_t)j * P + p];
+#pragma unroll
+            for (int i = 0; i < 32; ++i)
+                if (j <= first + i) sum[i] += x * at.q_pairs[(first + i) * DC_TOKENS + j];
+        }
+    }
     if (ok && p < P) {
-        const int first = 32 * (warp >> 2);
         float* out = a.o + (size_t)(t0 + first) * a.H * P + h * P + p;
 #pragma unroll
         for (int i = 0; i < 32; ++i)
