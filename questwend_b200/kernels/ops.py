@@ -1862,7 +1862,7 @@ def _moe_sizes(what, x, w_up, w_down, chosen, weight, kind):
     return T, D, E, F, top
 
 
-MOE_STREAM_COPIES = 2048    # csrc/moe.cu: MS_MAX_COPIES
+MOE_STREAM_COPIES, MOE_STREAM_MAX_EXPERTS = 2048, 1024      # csrc/moe.cu: MS_MAX_COPIES, QWB_MOE_MAX_EXPERTS
 # When bfloat16 tokens' experts are read once for all the tokens that chose them: with this many choices and three for four experts, where
 # the copies' rereading begins to cost more than the lists and the merge of that form, or from this many tokens on.  us, a row of the
 # weights for each copy / once for all / the library's grouped product: 6 of 64 experts of 2,048 x 1,408 and a shared one, 4 tokens 59 / 72 / -, 8
@@ -1873,10 +1873,10 @@ MOE_STREAM_COPIES = 2048    # csrc/moe.cu: MS_MAX_COPIES
 MOE_STREAM_MIN_CHOICES, MOE_STREAM_MIN_TOKENS = 12, 17
 
 
-def moe_stream_fits(D: int, F: int, Fs: int, top: int) -> bool:
+def moe_stream_fits(D: int, F: int, Fs: int, top: int, experts: int = 1) -> bool:
     """Whether bfloat16 experts of these sizes have the form that reads an expert's weights once for all the tokens that chose it (each
     tensor at a multiple of 16 bytes)."""
-    return D % 8 == 0 and F % 8 == 0 and Fs % 8 == 0 and top <= MOE_MAX_TOP
+    return D % 8 == 0 and F % 8 == 0 and Fs % 8 == 0 and 0 < top <= MOE_MAX_TOP and 0 < experts <= MOE_STREAM_MAX_EXPERTS
 
 
 def moe_experts(x: torch.Tensor, w_up: torch.Tensor, w_down: torch.Tensor, chosen: torch.Tensor, weight: torch.Tensor,
@@ -1905,7 +1905,7 @@ def moe_experts(x: torch.Tensor, w_up: torch.Tensor, w_down: torch.Tensor, chose
         out = _empty((T, D), dtype=torch.float32, device=x.device)
     act = _empty((T * top, F), dtype=x.dtype, device=x.device)
     act_s = _empty((T, Fs), dtype=x.dtype, device=x.device) if Fs else None
-    stream = x.dtype == torch.bfloat16 and (4 * T * top >= max(3 * E, 4 * MOE_STREAM_MIN_CHOICES) or T >= MOE_STREAM_MIN_TOKENS) and moe_stream_fits(D, F, Fs, top) and not any(
+    stream = x.dtype == torch.bfloat16 and (4 * T * top >= max(3 * E, 4 * MOE_STREAM_MIN_CHOICES) or T >= MOE_STREAM_MIN_TOKENS) and moe_stream_fits(D, F, Fs, top, E) and not any(
         t.data_ptr() % 16 for t in (x, w_up, w_down, out, shared_up, shared_down) if t is not None)
     per = MOE_STREAM_COPIES // top if stream else max(1, _MOE_SLOTS_PER_LAUNCH // (top + 1))
     if stream:

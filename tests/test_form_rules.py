@@ -33,3 +33,9 @@ def test_matrix_memory_takes_long_chunks_for_large_memories(lens, heads, key_dim
 def test_experts_are_sorted_only_in_long_steps(tokens, top, experts, shared, dtype, grouped):
     x, up, down = (torch.empty(s, dtype=dtype, device="meta") for s in ((tokens, 64), (experts, 64, 64), (experts, 64, 32)))
     assert ops.moe_grouped_fits(x, up, down, top, shared) is grouped
+
+
+@pytest.mark.parametrize("sizes, fits", [((2048, 1408, 2816, 6, 64), True), ((8, 8, 0, 16, 1024), True), ((8, 8, 0, 16, 1025), False), ((8, 8, 0, 17, 64), False),
+                                         ((8, 8, 0, 0, 64), False), ((8, 8, 0, 1, 0), False), ((12, 8, 0, 1, 4), False), ((8, 12, 0, 1, 4), False), ((8, 8, 4, 1, 4), False)])
+def test_experts_are_read_once_for_all_where_the_lists_hold_them(sizes, fits):
+    assert ops.moe_stream_fits(*sizes) is fits

@@ -780,3 +780,19 @@ def test_experts_read_once_for_all_their_tokens(T, E, top, D, F, Fs, activation,
             want = ref + base.double() if out is not None else ref
             # an activation that lies at the border of two bfloat16 numbers may be rounded the other way: 2^-8 of one of F terms
             assert torch.isfinite(got).all() and (got.double() - want).norm() <= 2 ** -9 * ref.norm() and (got.double() - want).abs().max() <= 2 ** -6 * (1 + ref.abs().max())
+
+
+@pytest.mark.parametrize("T, E", [(3, 1025), (17, 1024), (17, 1025), (40, 1500)])
+def test_any_number_of_experts(T, E):
+    """More experts than the lists of the form that reads them once hold: the rows for each copy."""
+    torch.manual_seed(E + T)
+    D, F, top = 16, 8, 2
+    x, up, down = (torch.randn(*s, device=DEV).to(torch.bfloat16) for s in ((T, D), (E, F, D), (E, D, F)))
+    chosen, weight = torch.randint(0, E, (T, top), device=DEV).int(), torch.rand(T, top, device=DEV)
+    chosen[-1, 0] = E - 1
+    got = ops.moe_experts(x, up, down, chosen, weight, "relu2")
+    z = torch.relu(torch.einsum("tkfd,td->tkf", up[chosen.long()].double(), x.double())).square().to(torch.bfloat16).double()
+    want = torch.einsum("tkdf,tkf,tk->td", down[chosen.long()].double(), z, weight.double())
+    assert (got.double() - want).norm() <= 2 ** -9 * want.norm()         # an activation at the border of two bfloat16 numbers: 2^-8 of one of F terms
+    with pytest.raises(ops.KernelError):
+        ops.moe_experts(x, up, down, chosen[:, :0].contiguous(), weight[:, :0].contiguous(), "relu2")
