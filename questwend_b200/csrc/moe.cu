@@ -215,8 +215,9 @@ moe_up_kernel(const T* __restrict__ x, const T* __restrict__ wu, const int* __re
 
 // grid (ceil(D / NR), T), a warp per choice and one or more for the shared expert: NR outputs of one token; the warps' products
 // are weighted and summed in the order of the choices, the shared expert last.  out may be added onto (`onto`).  A shared expert
-// about s times as wide as the others is cut into s warps' shares for one or two tokens, where a block waits for its longest warp (6 of 64
-// experts of 2,048 x 1,408 and one of 2,816, us: 1 token 10.2 -> 8.7, 2 19.5 -> 18.1, but 4 29.3 -> 30.8, 8 50.9 -> 53.6).
+// about s times as wide as the others is cut into s warps' shares, as a block waits for its longest warp: by sizes alone, so that a token's
+// sum has one order.  Both products, 6 of 64 experts of 2,048 x 1,408 and one of 2,816, us with a warp / shares: 1 token 19.7 / 17.6, 2 36.8 / 35.1, 3
+// 48.2 / 46.4, 4 56.1 / 57.4, 7 88.4 / 91.3; experts of 2,048 x 704 7 58.6 / 57.3; 32-bit 1 38.3 / 33.7, 4 112.7 / 103.3, 16 377 / 356.
 template <typename T, int NR>
 __global__ void moe_down_kernel(const T* __restrict__ act, const T* __restrict__ wd, const int* __restrict__ chosen,
                                 const float* __restrict__ weight, const T* __restrict__ act_s, const T* __restrict__ wsd,
@@ -263,7 +264,7 @@ static void launch_moe_experts(const void* x, const void* wu, const void* wd, co
     else
         qwb_launch(moe_up_kernel<T, 2>, g1, 256, 0, stream, (const T*)x, (const T*)wu, chosen, weight_in, (T*)act, (const T*)wsu, (T*)act_s, n_tok, D, F, Fs, top, kind);
     int shared_warps = Fs > 0 ? 1 : 0;
-    if (n_tok <= 2 && Fs > F && Fs % 8 == 0) shared_warps = min((Fs + F / 2) / F, MOE_SHARED_WARPS);
+    if (Fs > F && Fs % 8 == 0) shared_warps = min((Fs + F / 2) / F, MOE_SHARED_WARPS);
     qwb_launch(moe_down_kernel<T, 4>, g2, 32 * (top + shared_warps), 0, stream, (const T*)act, (const T*)wd, chosen, weight, (const T*)act_s,
                (const T*)wsd, gate, out, D, F, Fs, top, onto);
 }

@@ -796,3 +796,20 @@ def test_any_number_of_experts(T, E):
     assert (got.double() - want).norm() <= 2 ** -9 * want.norm()         # an activation at the border of two bfloat16 numbers: 2^-8 of one of F terms
     with pytest.raises(ops.KernelError):
         ops.moe_experts(x, up, down, chosen[:, :0].contiguous(), weight[:, :0].contiguous(), "relu2")
+
+
+@pytest.mark.parametrize("dtype, classes", [(torch.float32, [(1, 2, 3, 8, 40)]), (torch.bfloat16, [(1, 2, 3, 5, 7), (8, 9, 24, 130, 500)])])
+@pytest.mark.parametrize("Fs", [0, 24, 72, 136])
+def test_a_token_s_experts_are_the_same_bits_beside_others(dtype, classes, Fs):
+    """Within a form (the rows for each copy; an expert's rows once for all of its tokens) a token's sums have one order, whatever the
+    number of tokens and whoever else chose its experts."""
+    torch.manual_seed(Fs)
+    E, top, D, F = 64, 6, 264, 40
+    x, up, down = (torch.randn(*s, device=DEV).mul(f).to(dtype) for s, f in (((500, D), 1.0), ((E, F, D), D ** -0.5), ((E, D, F), F ** -0.5)))
+    su, sd = (torch.randn(Fs, D, device=DEV).mul(D ** -0.5).to(dtype), torch.randn(D, Fs, device=DEV).mul(Fs ** -0.5).to(dtype)) if Fs else (None, None)
+    chosen, weight = ops.moe_route(torch.randn(500, E, device=DEV), top)
+    gate = torch.rand(500, device=DEV) if Fs else None
+    for sizes in classes:
+        outs = [ops.moe_experts(x[:n], up, down, chosen[:n], weight[:n], "relu2", su, sd, gate[:n] if Fs else None) for n in sizes]
+        for small, large in zip(outs, outs[1:]):
+            assert torch.equal(small, large[:len(small)])
