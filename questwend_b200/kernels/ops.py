@@ -93,8 +93,9 @@ def _lookup(module: str, fn: str):
     entry = _FUNCTIONS.get((module, fn))
     if entry is None:
         lib = load_module(module)
-        entry = _FUNCTIONS[module, fn] = (lib, getattr(lib, fn))
-        _ADDRESSES[module, fn] = ctypes.cast(entry[1], ctypes.c_void_p).value
+        function = getattr(lib, fn)
+        _ADDRESSES[module, fn] = ctypes.cast(function, ctypes.c_void_p).value       # before the entry: who finds that finds this
+        entry = _FUNCTIONS[module, fn] = (lib, function)
     return entry
 
 

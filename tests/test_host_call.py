@@ -2,11 +2,13 @@
 import ctypes
 import shutil
 import subprocess
+import threading
+from types import SimpleNamespace
 
 import pytest
 import torch
 
-from questwend_b200.kernels import build
+from questwend_b200.kernels import build, ops
 
 SOURCE = """
 #include <string.h>
@@ -88,3 +90,29 @@ def test_lists_into_arrays(host):
         assert host.fill(array, numbers) is False
     with pytest.raises((BufferError, ValueError)):
         host.fill(np.zeros(4, dtype=np.int32)[::2], [1, 2])
+
+
+def test_a_launcher_is_looked_up_by_several_threads_at_once(host, lib, monkeypatch):
+    """A thread that finds another one in the middle of the first look-up of a launcher."""
+    others, errors = [], []
+
+    def call():
+        try:
+            ops._call("module", "take", *range(16))
+        except Exception as e:          # noqa: BLE001 - reported below
+            errors.append(e)
+
+    def cast(*args):
+        if not others:
+            others.append(threading.Thread(target=call))
+            others[0].start()
+            others[0].join()
+        return ctypes.cast(*args)
+
+    monkeypatch.setattr(ops, "_HOST", SimpleNamespace(call=lambda address, *args: 0))
+    monkeypatch.setattr(ops, "load_module", lambda name: lib)
+    monkeypatch.setattr(ops, "ctypes", SimpleNamespace(cast=cast, c_void_p=ctypes.c_void_p))
+    monkeypatch.setattr(ops, "_FUNCTIONS", {})
+    monkeypatch.setattr(ops, "_ADDRESSES", {})
+    call()
+    assert others and not errors, errors
