@@ -2,7 +2,8 @@
 
 Each ``csrc/<module>.cu`` becomes one shared library ``_build/qwb_<module>.so``
 with a C ABI, compiled for sm_100a by nvcc the first time the module is asked
-for, and loaded with ctypes.  A stamp beside the library holds a hash of the
+for, and loaded with ctypes; calls go to it through a native module compiled by g++
+at the same time, or through ctypes where there is none.  A stamp beside the library holds a hash of the
 sources and flags; a library whose stamp does not match is rebuilt.  Only the
 modules that a model uses are ever compiled.  There is no fallback: a module
 that cannot be built or loaded raises ``KernelBuildError``.
@@ -138,10 +139,11 @@ def compile_module(module: str, verbose: bool = True) -> str:
 
 
 def compile_modules(modules, verbose: bool = True) -> None:
-    """Compile several modules side by side."""
+    """Compile several modules side by side, and the way from Python to their launchers (without which they go through ctypes)."""
     todo = [m for m in modules if not is_built(m)]
-    if not todo:
-        return
+    host = None if host_calls_built() else threading.Thread(target=host_calls)
+    if host is not None:
+        host.start()
     errors: list[BaseException] = []
 
     def work(m):
@@ -153,7 +155,7 @@ def compile_modules(modules, verbose: bool = True) -> None:
     threads = [threading.Thread(target=work, args=(m,)) for m in todo]
     for t in threads:
         t.start()
-    for t in threads:
+    for t in threads + ([host] if host is not None else []):
         t.join()
     if errors:
         raise errors[0]
@@ -212,7 +214,10 @@ def compile_host_calls() -> None:
     if host_calls_built():
         return
     tmp = f"{_host_path()}.{os.getpid()}.tmp"
-    proc = subprocess.run(_host_command(tmp), stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True)
+    try:
+        proc = subprocess.run(_host_command(tmp), stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True)
+    except OSError as e:
+        raise KernelBuildError(f"cannot compile csrc/host_call.cpp: {e}") from None
     if proc.returncode != 0:
         raise KernelBuildError(f"g++ failed for csrc/host_call.cpp:\n{proc.stdout}")
     os.replace(tmp, _host_path())
@@ -220,15 +225,23 @@ def compile_host_calls() -> None:
         f.write(_host_stamp())
 
 
+_host_lock = threading.Lock()
+_host_loaded: list = []         # the module, or None where it cannot be had
+
+
 def host_calls():
-    """The module of csrc/host_call.cpp, or None where it is not built for this torch and Python: calls then go through ctypes."""
-    if not host_calls_built():
-        return None
-    try:
-        spec = importlib.util.spec_from_file_location(HOST_MODULE, _host_path())
-        module = importlib.util.module_from_spec(spec)
-        spec.loader.exec_module(module)
-        return module
-    except ImportError as e:
-        _log(f"{_host_path()} cannot be loaded ({e}): calls go through ctypes")
-        return None
+    """The module of csrc/host_call.cpp, compiled first if needed, or None where it cannot be had (said once): calls then go through
+    ctypes."""
+    with _host_lock:
+        if not _host_loaded:
+            module = None
+            try:
+                compile_host_calls()
+                spec = importlib.util.spec_from_file_location(HOST_MODULE, _host_path())
+                module = importlib.util.module_from_spec(spec)
+                spec.loader.exec_module(module)
+            except (KernelBuildError, ImportError, OSError) as e:
+                module = None
+                _log(f"launches go through ctypes, which takes longer: {e}")
+            _host_loaded.append(module)
+        return _host_loaded[0]

@@ -13,7 +13,7 @@ import operator
 
 import torch
 
-from .build import host_calls, load_module
+from .build import host_calls, host_calls_built, load_module
 
 DT_F32, DT_BF16 = 0, 1
 PAGE_SIZE = 64          # tokens per cache page
@@ -43,14 +43,26 @@ def _stream():
 
 # A launcher's arguments: tensors (None: a null pointer), other addresses, whole numbers, 32-bit floats; and the outputs' memory.  Through
 # csrc/host_call.cpp, where it is built, they go as they are (20 arguments 0.8 us, an output 1.7); ctypes wants an object each (4.8 and 4.4).
-_HOST = host_calls()
-if _HOST is not None:
-    _ptr, _i, _f, _address, _empty = _HOST.same, operator.index, float, _HOST.same, _HOST.empty
-else:
-    _i, _f, _address, _empty = ctypes.c_int, ctypes.c_float, ctypes.c_void_p, torch.empty
+# Where it is not built yet, it is with the first launcher that is looked up; a call whose arguments were made before goes either way.
+_HOST, _host_wanted = None, True
 
-    def _ptr(t: torch.Tensor | None) -> ctypes.c_void_p:
-        return ctypes.c_void_p(0 if t is None else t.data_ptr())
+
+def _ptr_object(t: torch.Tensor | None) -> ctypes.c_void_p:
+    return ctypes.c_void_p(0 if t is None else t.data_ptr())
+
+
+def _bind_host(module) -> None:
+    """Let the launchers' arguments go through this module, or through ctypes (None)."""
+    global _HOST, _ptr, _i, _f, _address, _empty
+    if module is not None:
+        _HOST = module                  # first: arguments for it are made only where it is
+        _ptr, _i, _f, _address, _empty = module.same, operator.index, float, module.same, module.empty
+    else:
+        _ptr, _i, _f, _address, _empty = _ptr_object, ctypes.c_int, ctypes.c_float, ctypes.c_void_p, torch.empty
+        _HOST = None
+
+
+_bind_host(host_calls() if host_calls_built() else None)
 
 
 def fill_int32(array, numbers) -> bool:
@@ -90,8 +102,13 @@ _ADDRESSES: dict = {}    # (module, name) -> the function's address
 
 
 def _lookup(module: str, fn: str):
+    global _host_wanted
     entry = _FUNCTIONS.get((module, fn))
     if entry is None:
+        if _host_wanted:
+            _host_wanted = False
+            if _HOST is None:
+                _bind_host(host_calls())
         lib = load_module(module)
         function = getattr(lib, fn)
         _ADDRESSES[module, fn] = ctypes.cast(function, ctypes.c_void_p).value       # before the entry: who finds that finds this

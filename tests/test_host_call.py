@@ -116,3 +116,68 @@ def test_a_launcher_is_looked_up_by_several_threads_at_once(host, lib, monkeypat
     monkeypatch.setattr(ops, "_ADDRESSES", {})
     call()
     assert others and not errors, errors
+
+
+@pytest.fixture
+def unbound(monkeypatch):
+    """As in a process that has not looked a launcher up, where the native module was not there at the import."""
+    for name in ("_HOST", "_ptr", "_i", "_f", "_address", "_empty"):
+        monkeypatch.setattr(ops, name, getattr(ops, name))
+    monkeypatch.setattr(ops, "_host_wanted", True)
+    monkeypatch.setattr(build, "_host_loaded", [])
+    ops._bind_host(None)
+
+
+def test_the_native_module_is_built_on_first_use(host, lib, unbound, tmp_path, monkeypatch):
+    built = build._host_path()
+    monkeypatch.setattr(build, "_host_path", lambda: str(tmp_path / "qwb_host_call.so"))
+    monkeypatch.setattr(build, "_host_command", lambda out: ["cp", built, out])         # what g++ would write
+    monkeypatch.setattr(ops, "load_module", lambda name: lib)
+    monkeypatch.setattr(ops, "_FUNCTIONS", {})
+    monkeypatch.setattr(ops, "_ADDRESSES", {})
+    assert not build.host_calls_built()
+    args = (ops._ptr(None), ops._i(-3), ops._f(0.5), ctypes.c_double(1.5), ctypes.c_longlong(7), ops._ptr(torch.zeros(1)), *(ops._i(i) for i in range(3)), ctypes.c_uint(9),
+            ops._f(2.0), ctypes.c_ulonglong(3), ops._i(4), ops._f(1.0), ops._address(64), ops._i(5))
+    n = lib.take(*args)
+    want = ctypes.string_at(lib.what(), n)
+    with pytest.raises(AttributeError):                     # of the library, behind the look-up; made for ctypes, these go either way
+        ops._call("module", "take", *args)
+    assert build.host_calls_built() and ops._HOST is not None and ops._i(3) == 3 and ops._empty is ops._HOST.empty
+    assert ctypes.string_at(lib.what(), n) == want
+    assert ops.fill_int32(torch.zeros(2, dtype=torch.int32).numpy(), [1, 2])
+
+
+def test_without_a_compiler_calls_go_through_ctypes(unbound, tmp_path, monkeypatch, capfd):
+    monkeypatch.setattr(build, "_host_path", lambda: str(tmp_path / "qwb_host_call.so"))
+    for command in (["false"], [str(tmp_path / "no-such-compiler")]):
+        monkeypatch.setattr(build, "_host_loaded", [])
+        monkeypatch.setattr(build, "_host_command", lambda out: command)
+        build.compile_modules([])                           # says so and goes on
+        assert build.host_calls() is None and capfd.readouterr().err.count("through ctypes") == 1
+        with pytest.raises(build.KernelBuildError):
+            build.compile_host_calls()
+    ops._bind_host(build.host_calls())
+    assert ops._HOST is None and ops._empty is torch.empty and not ops.fill_int32(torch.zeros(1, dtype=torch.int32).numpy(), [1])
+
+
+@pytest.mark.gpu
+def test_kernels_through_both_ways_give_the_same_bits(host, unbound):
+    dev = torch.device("cuda:0")
+    torch.manual_seed(1)
+    x, w = torch.randn(9, 256, device=dev), 1 + torch.rand(256, device=dev)
+    xb, wb = x.bfloat16(), torch.randn(64, 256, device=dev).bfloat16()
+    positions, freq = torch.arange(9, device=dev).int(), torch.rand(32, device=dev, dtype=torch.float64)
+    chosen, weight = torch.randint(0, 8, (9, 2), device=dev).int(), torch.rand(9, 2, device=dev)
+    up, down = torch.randn(8, 16, 256, device=dev), torch.randn(8, 256, 16, device=dev)
+
+    def run():
+        return [ops.rmsnorm(x, w, 1e-6, torch.float32), ops.gemm_tc(xb, wb), *ops.rope_table(positions, freq, 0.75), *ops.moe_route(x[:, :8].contiguous(), 2, weight_scale=0.3),
+                ops.moe_experts(x, up, down, chosen, weight, "relu2"), ops.sample(x, 0.8, top_k=5, top_p=0.9, seed=3)]
+
+    results = []
+    for module in (None, host):
+        ops._bind_host(module)
+        results.append(run())
+    assert all(torch.equal(a, b) for a, b in zip(*results))
+    with pytest.raises(ops.KernelError, match="weight has"):
+        ops.rmsnorm(x, w[:8].contiguous(), 1e-6, torch.float32)
