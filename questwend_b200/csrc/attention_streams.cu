@@ -34,6 +34,8 @@
 // 8,192 tokens: 2,447 -> 583 -> 507 us (cap 50: 3,261 -> 696 -> 673), 2,048 tokens with a window of 1,024: 170 -> 51 -> 45 us.
 #include "attention_tc.cuh"
 
+#include <atomic>
+
 #define AS_THREADS(apart) ((apart) ? 512 : 384)
 // Registers a thread of the loader's and issuers' warps, of the streams' softmax warps, of the warps that move O: as many in all as the block is
 // launched with (128 a thread, all of an SM's), which is what setmaxnreg has to give.
@@ -607,21 +609,49 @@ static int as_map(const char* what, CUtensorMap* map, const void* base, int rank
     return r == CUDA_SUCCESS ? 0 : qwb_fail(QWB_ERR_CUDA, "%s: cuTensorMapEncodeTiled failed with %d", what, (int)r);
 }
 
+// Whether the uncapped kernel was built with the registers that its warps share out among themselves (else they would wait for some that
+// there are not): 1, 0, or -1 where that cannot be found out now.
+template <int KA, int VA, bool MAPS>
+static int as_built() {
+    static std::atomic<int> regs{0};
+    if (regs == 0) {
+        cudaFuncAttributes f;
+        if (cudaFuncGetAttributes(&f, attn_streams_kernel<KA, VA, MAPS, false>) != cudaSuccess) return -1;
+        regs = f.numRegs;
+    }
+    return regs == AS_LAUNCH_REGS;
+}
+
 template <int KA, int VA, bool MAPS, bool CAP>
 static int as_launch(const char* what, dim3 grid, const CUtensorMap* maps, const AsArgs& args, cudaStream_t stream) {
     constexpr size_t smem = AsSmem<KA, VA, MAPS>::BYTES;
     auto kernel = attn_streams_kernel<KA, VA, MAPS, CAP>;
     cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return qwb_fail(QWB_ERR_CUDA, "%s: %s", what, cudaGetErrorString(e));
-    static const int regs = [&] { cudaFuncAttributes f; return cudaFuncGetAttributes(&f, kernel) == cudaSuccess ? f.numRegs : 0; }();
-    if (!CAP && regs != AS_LAUNCH_REGS)                         // built otherwise: the warps would wait for registers that there are not
-        return qwb_fail(QWB_ERR_CUDA, "%s: built with %d registers a thread, not %d", what, regs, AS_LAUNCH_REGS);
+    if (!CAP && as_built<KA, VA, MAPS>() != 1) return qwb_fail(QWB_ERR_CUDA, "%s: not built with %d registers a thread", what, AS_LAUNCH_REGS);
     e = qwb_launch(kernel, grid, AS_THREADS(!CAP), smem, stream, maps[0], maps[1], maps[2], maps[3], maps[4], args);
     if (e != cudaSuccess) return qwb_fail(QWB_ERR_CUDA, "%s: launch failed: %s", what, cudaGetErrorString(e));
     return qwb_check_launch(what);
 }
 
 static int as_pieces(int n) { return (n + 63) / 64; }
+
+// Whether uncapped prompts of these sizes may take this kernel as it was built; where they may not, the caller takes another one.
+extern "C" int qwb_streams_built(int maps, int key_pieces, int value_pieces) {
+    switch ((maps ? 100 : 0) + 10 * key_pieces + value_pieces) {
+        case 11: return as_built<1, 1, false>() != 0;
+        case 12: return as_built<1, 2, false>() != 0;
+        case 21: return as_built<2, 1, false>() != 0;
+        case 22: return as_built<2, 2, false>() != 0;
+        case 31: return as_built<3, 1, false>() != 0;
+        case 32: return as_built<3, 2, false>() != 0;
+        case 111: return as_built<1, 1, true>() != 0;
+        case 112: return as_built<1, 2, true>() != 0;
+        case 121: return as_built<2, 1, true>() != 0;
+        case 122: return as_built<2, 2, true>() != 0;
+    }
+    return 0;
+}
 
 static bool as_latent_fits(int K, int R, int DV) {
     return K > 0 && R >= 0 && DV > 0 && K % 8 == 0 && R % 8 == 0 && (K + R) % 16 == 0 && DV % 8 == 0 && DV <= 128 && as_pieces(K) + as_pieces(R) <= 3;
