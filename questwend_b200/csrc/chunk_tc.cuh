@@ -391,11 +391,10 @@ __device__ __forceinline__ void ct_carry(float* own, size_t step, const float* t
     if (keep) { S[0] = s.x; S[K] = s.y; S[2 * K] = s.z; S[3 * K] = s.w; }
 }
 
-// A chunk's 128 tokens x 64 values (from p0 of P): put(token, value column, four sums).  starts: the chunk's, in planes; skip: what a token's own
-// value is multiplied by besides.  norm0 (K values) or null: divide(token, n . q) too.
-template <class Put, class Divide>
-__device__ __forceinline__ void ct_out(const CtRows& r, const float* starts, const float* pairs, const CtGates* gates, float skip, int K, int P, int p0,
-                                       const float* norm0, int* error, Put put, Divide divide) {
+// A chunk's 128 tokens x 64 values (from p0 of P): put(token, value column, four sums, what ahead(token, value column) gave).  starts: the chunk's, in planes.  norm0 (K values) or null: divide(token, n . q) too.
+template <class Ahead, class Put, class Divide>
+__device__ __forceinline__ void ct_out(const CtRows& r, const float* starts, const float* pairs, const CtGates* gates, int K, int P, int p0,
+                                       const float* norm0, int* error, Ahead ahead, Put put, Divide divide) {
     __shared__ double G[CT_TOKENS];
     __shared__ float left[CT_TOKENS], fade[CT_TOKENS], norms[3][CT_TOKENS];
     __shared__ __align__(16) float near[2][CT_TOKENS][4];
@@ -455,9 +454,6 @@ __device__ __forceinline__ void ct_out(const CtRows& r, const float* starts, con
                         for (int e = 0; e < 8; ++e) v[i][e] = token >= j + e ? v[i][e] * near[e >> 2][token][e & 3] : 0.f;
                     }
                     if (norm0) token_norm += ((v[i][0] + v[i][1]) + (v[i][2] + v[i][3])) + ((v[i][4] + v[i][5]) + (v[i][6] + v[i][7]));
-#pragma unroll
-                    for (int e = 0; e < 8; ++e)
-                        if (token == j + e) v[i][e] += skip;
                     ct_put(c.a, CT_A_PART, token, 4 * (s & 1) + (warp >> 2) + 2 * i, v[i]);
                 }
                 ct_put(c.b, CT_B_PART, CT_R * (s & 1) + index, lane & 7, v[2]);
@@ -471,7 +467,7 @@ __device__ __forceinline__ void ct_out(const CtRows& r, const float* starts, con
 #pragma unroll 1
         for (int j = 0; j <= token; ++j) {
             const float w = (token ^ j) < 8 ? near[(j >> 2) & 1][token][j & 3] : expf((float)(G[token] - G[j | 7])) * left[j];
-            ct_add(sum, w * pairs[((size_t)(j / 4) * CT_TOKENS + token) * 4 + j % 4] + (j == token ? skip : 0.f), 1.f, r.v + (size_t)j * r.ld + p, 4, P - p);
+            ct_add(sum, w * pairs[((size_t)(j / 4) * CT_TOKENS + token) * 4 + j % 4], 1.f, r.v + (size_t)j * r.ld + p, 4, P - p);
         }
     }
     if (ok) {                                                       // by way of shared memory, so that a row's values leave together
@@ -479,6 +475,12 @@ __device__ __forceinline__ void ct_out(const CtRows& r, const float* starts, con
 #pragma unroll
         for (int i = 0; i < 8; ++i)
             stage[token * 16 + ((8 * (warp >> 2) + i) ^ (token & 7))] = make_float4(sum[4 * i], sum[4 * i + 1], sum[4 * i + 2], sum[4 * i + 3]);
+        float4 own[8];                                              // asked for before the barrier
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            const int t = 16 * i + 2 * warp + (lane >> 4), p = p0 + 4 * (lane & 15);
+            if (t < r.n && p < P) own[i] = ahead(t, p);
+        }
         if (norm0) {
 #pragma unroll
             for (int i = 0; i < 2; ++i) {
@@ -493,7 +495,7 @@ __device__ __forceinline__ void ct_out(const CtRows& r, const float* starts, con
 #pragma unroll
         for (int i = 0; i < 8; ++i) {
             const int t = 16 * i + 2 * warp + (lane >> 4), p = p0 + 4 * (lane & 15);
-            if (t < r.n && p < P) put(t, p, stage[t * 16 + ((lane & 15) ^ (t & 7))]);
+            if (t < r.n && p < P) put(t, p, stage[t * 16 + ((lane & 15) ^ (t & 7))], own[i]);
         }
         if (norm0 && (int)threadIdx.x < r.n) divide(threadIdx.x, norms[2][threadIdx.x] + (norms[0][threadIdx.x] + norms[1][threadIdx.x]));
     }

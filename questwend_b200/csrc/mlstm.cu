@@ -676,9 +676,10 @@ mlstm_tile_out_kernel(const MlArgs a, int ptiles) {
     size_t place;
     const int n = ml_chunk(a, place, t0);
     if (n <= 0) return;
-    ct_out(ml_rows(a, t0, n, h), a.own + (place * H + h) * (size_t)P * K, a.scores + (place * H + h) * ML_TOKENS * ML_TOKENS, a.gates + place * H + h, 0.f, K, P, p0,
+    ct_out(ml_rows(a, t0, n, h), a.own + (place * H + h) * (size_t)P * K, a.scores + (place * H + h) * ML_TOKENS * ML_TOKENS, a.gates + place * H + h, K, P, p0,
            p0 == 0 ? a.own_n + (place * H + h) * K : nullptr, a.error,
-           [&](int i, int p, float4 v) {
+           [](int, int) { return make_float4(0.f, 0.f, 0.f, 0.f); },
+           [&](int i, int p, float4 v, float4) {
                *reinterpret_cast<float4*>(a.raw + ((size_t)(t0 + i) * H + h) * P + p) = make_float4(v.x * a.q_scale, v.y * a.q_scale, v.z * a.q_scale, v.w * a.q_scale);
            },
            [&](int i, float v) {

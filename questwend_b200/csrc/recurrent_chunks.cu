@@ -108,8 +108,14 @@ ssm_chunk_out_kernel(const ScArgs a, int ptiles) {
     if (n <= 0) return;
     const CtRows rows = sc_rows(a, t0, n, h, g);
     float* y = a.y + (size_t)t0 * a.H * a.P + h * a.P;
-    ct_out(rows, a.own + (place * a.H + h) * (size_t)a.P * a.N, a.products + (place * a.G + g) * SC_TOKENS * SC_TOKENS, a.gates + place * a.H + h, a.D[h], a.N, a.P,
-           p0, nullptr, a.error, [&](int i, int p, float4 v) { *reinterpret_cast<float4*>(y + (size_t)i * a.H * a.P + p) = v; }, [](int, float) {});
+    const float skip = a.D[h];                                      // added behind the sums: it is no product that was cut
+    ct_out(rows, a.own + (place * a.H + h) * (size_t)a.P * a.N, a.products + (place * a.G + g) * SC_TOKENS * SC_TOKENS, a.gates + place * a.H + h, a.N, a.P, p0,
+           nullptr, a.error,
+           [&](int i, int p) { return *reinterpret_cast<const float4*>(rows.v + (size_t)i * rows.ld + p); },
+           [&](int i, int p, float4 v, float4 x) {
+               *reinterpret_cast<float4*>(y + (size_t)i * a.H * a.P + p) = make_float4(v.x + skip * x.x, v.y + skip * x.y, v.z + skip * x.z, v.w + skip * x.w);
+           },
+           [](int, float) {});
 }
 
 // Floats of scratch that qwb_ssm_chunked needs; 0: these sizes are not taken (more than a grid holds, or states that the scan refuses).

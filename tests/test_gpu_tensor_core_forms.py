@@ -529,6 +529,23 @@ def test_delta_rule_in_chunks(H, Hk, K, P, per_head, pace, monkeypatch):
     assert torch.equal(state, before)
 
 
+def test_mamba2_adds_a_token_s_own_value_with_one_rounding():
+    """Outputs that are D x but for little: the sum's error is that of the multiply-add, 2^-25 to 2^-24 of it, 2.9e-8 on average (a third of
+    2^-24 squared, over the numbers between two powers of two); what is given back for the tensor cores' cuts must not reach it."""
+    torch.manual_seed(8)
+    H, P, N, G, T = 4, 64, 128, 2, 300
+    xbc, dt = torch.randn(T, H * P + 2 * G * N, device=DEV), torch.randn(T, H, device=DEV) - 12.0
+    d, zero, state = 1.0 + torch.rand(H, device=DEV), torch.zeros(H, device=DEV), torch.zeros(1, H, P, N, device=DEV)
+    step, x, S, ref = Steps([T], [0]), xbc[:, :H * P].double().view(T, H, P), torch.zeros(H, P, N, dtype=F64, device=DEV), torch.empty(T, H, P, dtype=F64, device=DEV)
+    y = ops.ssm_scan(xbc, dt, 0, zero, zero, d, state, step, H, P, N, G).view(T, H, P)
+    for i in range(T):
+        b, c = (xbc[i, H * P + k * G * N:H * P + (k + 1) * G * N].double().view(G, N).repeat_interleave(H // G, 0) for k in (0, 1))
+        s = torch.nn.functional.softplus(dt[i].double())
+        S = torch.exp(-s)[:, None, None] * S + (s[:, None] * x[i])[:, :, None] * b[:, None, :]
+        ref[i] = (S @ c[:, :, None])[..., 0] + d.double()[:, None] * x[i]
+    assert (y.double() - ref).norm() <= 2.9e-8 * ref.norm()
+
+
 @pytest.mark.parametrize("kind", ["mamba2", "mlstm", "delta", "delta_per_head"])
 @pytest.mark.parametrize("where", ["value", "key", "query"])
 @pytest.mark.parametrize("number", [math.inf, -math.inf, math.nan, 3.4e38])
