@@ -22,7 +22,8 @@
 // share the left parts are one instruction (right parts side by side), as what bounds them is the reading of shared memory: 30 KB in place
 // of 36 for 16 of R.  Tensor memory, 64 columns each: the large sums of two stages, the two small ones.  What was measured on the way, 2,048
 // tokens of 64 Mamba-2 heads of 64 x 128, us of the own sums / of the outputs: plain multiply-adds 81 / 107; mma.sync with the parts in
-// shared memory 75 / 100 (its products alone leave 63 / 80); tcgen05 in stages of 64 that wait for their products 41 / 75; as here 39 / 60.
+// shared memory 75 / 100 (its products alone leave 63 / 80); tcgen05 in stages of 64 that wait for their products 41 / 75; in stages
+// of 32 39 / 60 (the last product as wide as those before it, and a token's own value behind the sums, since: 3 and 3 more in all).
 #pragma once
 
 #include "chunks.cuh"

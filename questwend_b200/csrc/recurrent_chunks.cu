@@ -15,9 +15,10 @@
 // A step's sequences of at least `from` tokens go through these kernels, the others through the scan.  Chunk c of the z-th of them,
 // b, is place cu_seqlens[b] / 128 + z + c of the scratch memory, which T / 128 and one for each of them hold:
 //     own / starts [places, H, P / 4, N, 4], products [places, G, 32, 128 (i), 4 (j)], gates [places, H], total decays [places, H]
-// The sums of logarithms are 64-bit (only their differences are used).  64 heads of 64 x 128 in 8 groups, 2,048 tokens, us: gates 5,
-// state 39, carries 13, outputs 60; with the convolution before it 153 where 8 x 8 sums a thread in plain multiply-adds took 233 (state 81,
-// carries 10, outputs 107: bound by what shared memory hands to registers).  Error against 64 bits 1.2e-7 as before.
+// The sums of logarithms are 64-bit (only their differences are used).  64 heads of 64 x 128 in 8 groups, 2,048 tokens, us under ncu (cold
+// caches): gates 7, state 42, carries 19, outputs 68; with the convolution before it 158 in a run, where 8 x 8 sums a thread in plain
+// multiply-adds took 233 (state 85, carries 14, outputs 113: bound by what shared memory hands to registers).  Errors against 64 bits, of the
+// outputs 0.70e-7 (plain multiply-adds 0.79e-7), of the states 1.05 to 1.3e-7 (1.1 to 1.35e-7).
 // ---------------------------------------------------------------------------------
 #define SC_TOKENS CT_TOKENS
 #define SC_FORGETS -128.f               // the exponential of this is 0 in 32-bit: a log decay below (-infinity too) counts as this much,

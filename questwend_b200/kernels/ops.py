@@ -932,9 +932,10 @@ def short_conv(x: torch.Tensor, col0: int, channels: int, weight: torch.Tensor, 
 
 
 # Tokens from which a sequence goes through the recurrence in chunks (csrc/recurrent_chunks.cu), by its own length, whatever else
-# the step brings.  With its convolution, 64 heads of 64 x 128, us, scan / chunks: 64 tokens 33 / 42, 100 tokens 48 / 48, 400 tokens 179 / 74.
-# Steps with both, all by the scan / each its own way: a prompt of 200 beside 63 single tokens 151 / 154, beside 255 444 / 462, one of
-# 2,048 beside 63 952 / 335 (all of them in chunks, a whole chunk each: 861, 3,388, 1,096).
+# the step brings.  64 heads of 64 x 128, us, scan / chunks: 48 tokens 19 / 21, 64 25 / 22, 96 37 / 23, 200 74 / 28; 16 heads, 64 tokens 22 / 20.  Steps
+# with both, all by the scan / each its own way: a prompt of 64 beside 31 single tokens 62 / 73, of 96 beside 63 125 / 128 (16 heads, beside 31 34 / 35),
+# of 144 137 / 132, of 200 152 / 132, of 300 176 / 139.  Alone the chunks are ahead from about 56 tokens on, beside single tokens from about 100: the line
+# is where a step with both loses nothing.
 SSM_CHUNKED_FROM = 96
 CHUNK_SCRATCH_MAX = 1 << 30     # floats of scratch memory that a chunked form may take; a longer prompt runs without
 
@@ -996,10 +997,10 @@ def ssm_scan(xbc: torch.Tensor, dt: torch.Tensor, dt_col0: int, dt_bias, a_log, 
 
 
 # Tokens from which a sequence goes through the delta rule in chunks (csrc/recurrent_chunks.cu), by its own length.  16 heads of
-# 128 x 128, us, scan / chunks: 64 tokens 44 / 68 and 400 tokens 194 / 101 (with the convolution), 200 tokens 92 / 79, two of 150 and 160
-# 135 / 89.  Beside single tokens, whose scan then waits for the chunks' launches, all by the scan / each its own way: 200 beside 63
-# 143 / 173, beside 255 389 / 426, 2,048 beside 63 1,051 / 395 (all of them in chunks: 609, 2,210, 864).  Alone the chunks are ahead from
-# about 144 tokens on, beside many single ones from about 300: the line lies between.
+# 128 x 128, us, scan / chunks, decays per channel and per head: 96 tokens 52 / 60 and 40 / 58, 128 65 / 60 and 51 / 59, 160 78 / 64 and 61 / 62, 192 90 / 64
+# and 72 / 62, 300 134 / 71 and 108 / 69.  Beside 63 single tokens, whose scan then waits for the chunks' launches, all by the scan / each its own way: 192
+# 142 / 154 and 111 / 134, 256 161 / 161 and 126 / 140, 300 172 / 166 and 137 / 145, 400 217 / 175 and 166 / 154.  Alone the chunks are ahead from about 120
+# and 160 tokens on, beside many single ones from about 256 and 350: the line lies between.
 DELTA_CHUNKED_FROM = 192
 
 
@@ -1178,10 +1179,15 @@ def gated_part_norm(y: torch.Tensor, gate: torch.Tensor, gate_col0: int, weight:
 MLSTM_CHUNKED_FROM = 64         # steps whose longest sequence brings at least this many tokens take the chunked form
 # Its chunks of 128 tokens (csrc/mlstm.cu: mlstm_tile_*, on tcgen05), for sizes and rows in multiples of 4, against those of 64: a chunk costs
 # about the same in both however few tokens are in it, so they win wherever sequences fill more than one of 64; with small memories the
-# fifth launch costs what the products save.  us, 64 / 128 tokens a chunk: 4 heads of 256 x 512, 64 tokens 65 / 51, 500 80 / 60, 2,048 243 / 125,
-# 4,096 447 / 217, 8 x 300 (92 tokens a place that its chunks have) 307 / 170, 8 x 64 (42) 87 / 81, 2,048 beside 63 single tokens (26) 795 / 867;
-# 8 of 512 x 256, 1,000 tokens 227 / 132, 16 x 130 (65) 647 / 398; 2 of 256 x 512, 100 tokens 62 / 51; 16 of 128 x 128, 100 tokens 48 / 45, 1,000
-# 81 / 69, 4,096 298 / 220, 16 x 130 (65) 217 / 187, 8 x 64 (42) 58 / 64; 4 of 64 x 64, 100 tokens 34 / 42, 4,096 60 / 65.
+# fifth launch costs what the products save.  us, 64 / 128 tokens a chunk: 4 heads of 256 x 512, 64 tokens 56 / 36, 300 63 / 43, 1,000 113 / 62, 4,096
+# 438 / 200, 8 x 300 (92 tokens a place that its chunks have) 296 / 155, 16 x 130 (65) 338 / 196, 8 x 64 (42) 77 / 66, 2,048 beside 63 single tokens (26)
+# 795 / 867; 2 of 256 x 512, 100 tokens 54 / 36, 4,096 230 / 110; 16 of 128 x 128, 100 40 / 31, 1,000 70 / 51, 4,096 287 / 180, 16 x 130 205 / 152, 8 x 64
+# 50 / 47; 4 of 64 x 64, 100 tokens 22 / 26, 4,096 50 / 49; 16 of 64 x 64, 100 24 / 27, 16 x 130 80 / 84, 4,096 126 / 115.  By rows of the keys, long steps
+# of narrow memories: 16 of 256 x 64, 4,096 tokens 307 / 197 (mlstm_tiles_pay).
+# The lines leave sizes on the safe side of 2^14 values a memory where chunks of 128 are the faster ones too, and keep the chunks of 64 that they had:
+# 8 heads of 128 x 128, 100 tokens 39 / 29, 4,096 152 / 110, 8 x 300 101 / 74; 1 of 256 x 512, 100 53 / 35; 4 of 512 x 64, 100 60 / 51, 4,096 156 / 117; 4 of
+# 64 x 512, 100 31 / 27, 4,096 166 / 113.  From memories of 128 x 128 on, whatever the number of heads, would be the line by time alone; 128 x 64 is mixed
+# (16 heads, 100 tokens 29 / 30, 4,096 193 / 138).
 MLSTM_TILES_KEYS, MLSTM_TILES_BLOCKS, MLSTM_TILES_FILL = 256, 512, 105
 MLSTM_TILES_MEMORY, MLSTM_TILES_WIDE = 1 << 18, 1 << 16        # values of all heads' memories; of one that is worth half-filled chunks
 
@@ -1894,7 +1900,11 @@ MOE_STREAM_COPIES, MOE_STREAM_MAX_EXPERTS = 2048, 1024      # csrc/moe.cu: MS_MA
 # 103 / 92 / -, 16 178 / 122 / 206, 32 330 / 136 / 224, 128 - / 211 / 234, 160 - / 256 / 233; the same gated, no shared one, 4 72 / 81 / -, 8 122 / 114 / -,
 # 32 448 / 196 / 267, 128 - / 259 / 278, 160 - / 326 / 292; 8 of 128 gated of 2,048 x 768, 8 96 / 106 / -, 12 133 / 135 / -, 32 329 / 218 / 278, 128 - / 275 /
 # 298; 8 of 256 of these, 16 178 / 180 / 230, 24 257 / 252 / 312, 128 - / 491 / 520; 2 of 8 gated of 4,096 x 2,048, 5 69 / 74 / -, 6 92 / 76 / -, 32 366 / 87 /
-# 141, 64 - / 137 / 133; 4 of 32 and a shared one of 2,048 x 1,408, 6 57 / 53 / -, 128 - / 185 / 202.
+# 141, 64 - / 137 / 133; 4 of 32 and a shared one of 2,048 x 1,408, 6 57 / 53 / -, 128 - / 185 / 202.  Between a few tokens and these, a row for each copy / once for all: 6 of 64 and one of 2,816, 5 tokens 68 / 66, 6 79 / 75, 7 90 / 80, 8
+# 98 / 88; 4 of 32 and one of 1,408, 5 46 / 48, 6 50 / 51, 7 57 / 54; 2 of 8 of 4,096 x 2,048 and one of 2,048, 3 44 / 43, 5 57 / 50, 6 66 / 56; 8 of 128 of 2,048 x 768
+# and one as wide, 8 67 / 76, 12 93 / 98, with one of 1,536 8 72 / 75, 12 102 / 97; 2 of 16 of 2,048 x 1,024 and one as wide, 6 23 / 25, 8 27 / 28, 12 35 / 32; 4 of
+# 32 of 1,024 x 512 and one as wide, 8 15 / 18, 12 19 / 20.  A wide shared expert, whose rows go out for each token too, moves the line to half as many
+# choices as experts, small experts to as many: three for four is within an eighth of the faster form in all of these but the smallest.
 MOE_STREAM_MIN_CHOICES, MOE_STREAM_MIN_TOKENS = 12, 17
 
 
