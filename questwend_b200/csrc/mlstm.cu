@@ -572,22 +572,20 @@ struct MlArgs {
     int* error;
     MlstmSizes z;
     float q_scale, tiny;
-    int write_state;
+    int write_state, B;
 };
 
-// a chunk's place, first token and tokens (0: none)
+// a block's place, and its chunk's first token and tokens (0: none)
 __device__ __forceinline__ int ml_chunk(const MlArgs& a, size_t& place, int& t0) {
-    const int b = blockIdx.z, c = blockIdx.x;
-    t0 = a.cu_seqlens[b] + c * ML_TOKENS;
-    place = (size_t)(a.cu_seqlens[b] / ML_TOKENS + b + c);
-    return min(ML_TOKENS, a.cu_seqlens[b + 1] - t0);
+    place = blockIdx.x;
+    return rc_chunk<ML_TOKENS>(a.cu_seqlens, a.B, 0, blockIdx.x, t0);
 }
 __device__ __forceinline__ CtRows ml_rows(const MlArgs& a, int t0, int n, int h) {
     const float* x = a.rows.x + (size_t)t0 * a.rows.ld;
     return {x + h * a.z.K, x + (a.z.H + h) * a.z.K, x + 2 * a.z.H * a.z.K + h * a.z.P, a.rows.ld, n};
 }
 
-// grid (chunks, H * ktiles, B), 1,024 threads: a chunk's gates, and its own sum of the normaliser over 128 key rows, 16 tokens and a key
+// grid (places, H * ktiles), 1,024 threads: a chunk's gates, and its own sum of the normaliser over 128 key rows, 16 tokens and a key
 // row a thread.  Each block makes the gates (all write the same); the keys are asked for before that, and a thread's 16 fit its
 // registers.  A chain of waits either way: 14.0 us with a block a head, 32 tokens a thread and the keys asked for behind the
 // gates, 9.2 now (4,096 tokens of 4 heads of 256 x 512).
@@ -617,7 +615,7 @@ mlstm_tile_gates_kernel(const MlArgs a, int ktiles) {
         a.own_n[head * a.z.K + k] = ((part[0][column] + part[1][column]) + (part[2][column] + part[3][column])) + ((part[4][column] + part[5][column]) + (part[6][column] + part[7][column]));
 }
 
-// grid (chunks, 2 H + H * ptiles * ktiles, B): the scores of a head's chunk with 64 of its tokens, or 64 values x 128 key rows of its own sum
+// grid (places, 2 H + H * ptiles * ktiles): the scores of a head's chunk with 64 of its tokens, or 64 values x 128 key rows of its own sum
 __global__ void __launch_bounds__(CT_THREADS, 2)
 mlstm_tile_state_kernel(const MlArgs a, int ptiles, int ktiles) {
     pdl_wait();
@@ -666,7 +664,7 @@ mlstm_tile_carry_kernel(const MlArgs a, int matrix_blocks) {
         for (int p = threadIdx.x; p <= P; p += 256) a.m_state[head * (P + 1) + p] = a.m_run[(size_t)(t0 + n - 1) * H + h];
 }
 
-// grid (chunks, H * ptiles, B): a chunk's 128 tokens x 64 values; a head's first tile of values also makes the divisors
+// grid (places, H * ptiles): a chunk's 128 tokens x 64 values; a head's first tile of values also makes the divisors
 __global__ void __launch_bounds__(CT_THREADS, 2)
 mlstm_tile_out_kernel(const MlArgs a, int ptiles) {
     pdl_wait();
@@ -804,15 +802,15 @@ extern "C" int qwb_mlstm_tiles(const float* x, int ld, int i_col, int f_col, con
     const MlstmRows rows{x, ld, i_col, f_col};
     const MlstmGates gates{i_bias, f_bias, cap};
     if (int rc = check_mlstm("mlstm_tiles", z, rows, B)) return rc;
-    const int chunks = (max_new + ML_TOKENS - 1) / ML_TOKENS, ptiles = (P + 63) / 64, ktiles = (K + 127) / 128;
+    const int ptiles = (P + 63) / 64, ktiles = (K + 127) / 128;
     if (!(cap > 0.f) || !gate_rows || !scratch || !error || !qwb_mlstm_tiles_scratch(T, B, H, K, P) || ld % 4)
         return qwb_fail(QWB_ERR_ARG, "mlstm_tiles: cap %g, %d heads of %d x %d in rows of %d", (double)cap, H, K, P, ld);
     if (!mlstm_aligned(x) || !mlstm_aligned(scratch) || !mlstm_aligned(raw)) return qwb_fail(QWB_ERR_ARG, "mlstm_tiles: a tensor is not 16-byte aligned");
     float *log_decay = gate_rows, *write = gate_rows + (size_t)T * H, *m_run = gate_rows + 2 * (size_t)T * H;
     qwb_launch(mlstm_gates_kernel, dim3(H, B), mlstm_gate_threads(T), 0, stream, rows, gates, (const float*)m_state, cu_seqlens, slots, log_decay, write, m_run, H, P);
     if (int rc = qwb_check_launch("mlstm_gates")) return rc;
-    const size_t heads = ((size_t)T / ML_TOKENS + B) * H;
-    MlArgs a = {rows, log_decay, write, m_run, cu_seqlens, slots, state, m_state, scratch, nullptr, nullptr, nullptr, raw, divisor, nullptr, error, z, q_scale, tiny, write_state};
+    const size_t places = (size_t)T / ML_TOKENS + B, heads = places * H;
+    MlArgs a = {rows, log_decay, write, m_run, cu_seqlens, slots, state, m_state, scratch, nullptr, nullptr, nullptr, raw, divisor, nullptr, error, z, q_scale, tiny, write_state, B};
     a.scores = a.own + heads * P * K;
     a.gates = reinterpret_cast<CtGates*>(a.scores + heads * ML_TOKENS * ML_TOKENS);
     a.own_n = reinterpret_cast<float*>(a.gates + heads);
@@ -820,13 +818,13 @@ extern "C" int qwb_mlstm_tiles(const float* x, int ld, int i_col, int f_col, con
     cudaError_t e = cudaFuncSetAttribute(mlstm_tile_state_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, CT_SMEM);
     if (e == cudaSuccess) e = cudaFuncSetAttribute(mlstm_tile_out_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, CT_SMEM);
     if (e != cudaSuccess) return qwb_fail(QWB_ERR_CUDA, "mlstm_tiles: %s", cudaGetErrorString(e));
-    qwb_launch(mlstm_tile_gates_kernel, dim3(chunks, H * ktiles, B), 1024, 0, stream, a, ktiles);
+    qwb_launch(mlstm_tile_gates_kernel, dim3(rc_places(T, B, 0, ML_TOKENS), H * ktiles), 1024, 0, stream, a, ktiles);
     if (int rc = qwb_check_launch("mlstm_tile_gates")) return rc;
-    qwb_launch(mlstm_tile_state_kernel, dim3(chunks, 2 * H + H * ptiles * ktiles, B), CT_THREADS, CT_SMEM, stream, a, ptiles, ktiles);
+    qwb_launch(mlstm_tile_state_kernel, dim3(rc_places(T, B, 0, ML_TOKENS), 2 * H + H * ptiles * ktiles), CT_THREADS, CT_SMEM, stream, a, ptiles, ktiles);
     if (int rc = qwb_check_launch("mlstm_tile_state")) return rc;
     const int matrix_blocks = (K * (P / 4) + 255) / 256;
     qwb_launch(mlstm_tile_carry_kernel, dim3(matrix_blocks + (K + 255) / 256, H, B), 256, 0, stream, a, matrix_blocks);
     if (int rc = qwb_check_launch("mlstm_tile_carry")) return rc;
-    qwb_launch(mlstm_tile_out_kernel, dim3(chunks, H * ptiles, B), CT_THREADS, CT_SMEM, stream, a, ptiles);
+    qwb_launch(mlstm_tile_out_kernel, dim3(rc_places(T, B, 0, ML_TOKENS), H * ptiles), CT_THREADS, CT_SMEM, stream, a, ptiles);
     return qwb_check_launch("mlstm_tile_out");
 }

@@ -33,20 +33,17 @@ struct ScArgs {
     int ldx, ld_dt, H, P, N, G, write_state, B, from;
 };
 
-// a chunk's place, first token and tokens (0: none)
+// a block's place, and its chunk's first token and tokens (0: none)
 __device__ __forceinline__ int sc_chunk(const ScArgs& a, size_t& place, int& t0) {
-    const int b = rc_sequence(a.cu_seqlens, a.B, a.from, blockIdx.z), c = blockIdx.x;
-    if (b < 0) return 0;
-    t0 = a.cu_seqlens[b] + c * SC_TOKENS;
-    place = (size_t)(a.cu_seqlens[b] / SC_TOKENS + blockIdx.z + c);
-    return min(SC_TOKENS, a.cu_seqlens[b + 1] - t0);
+    place = blockIdx.x;
+    return rc_chunk<SC_TOKENS>(a.cu_seqlens, a.B, a.from, blockIdx.x, t0);
 }
 __device__ __forceinline__ CtRows sc_rows(const ScArgs& a, int t0, int n, int h, int g) {
     const float *x = a.xbc + (size_t)t0 * a.ldx, *bs = x + a.H * a.P + g * a.N;
     return {bs + a.G * a.N, bs, x + h * a.P, a.ldx, n};
 }
 
-// grid (chunks, H, B), 128 threads
+// grid (places, H), 128 threads
 __global__ void __launch_bounds__(SC_TOKENS)
 ssm_chunk_gates_kernel(const ScArgs a) {
     pdl_wait();
@@ -65,7 +62,7 @@ ssm_chunk_gates_kernel(const ScArgs a) {
     ct_gates(fade, dt, a.gates + place * a.H + h, a.totals + place * a.H + h, coef);
 }
 
-// grid (chunks, 2 G + H * ptiles * ntiles, B): the products of a group's chunk with 64 of its tokens, or 64 values x 128 state rows of a head's own sum
+// grid (places, 2 G + H * ptiles * ntiles): the products of a group's chunk with 64 of its tokens, or 64 values x 128 state rows of a head's own sum
 __global__ void __launch_bounds__(CT_THREADS, 2)
 ssm_chunk_state_kernel(const ScArgs a, int ptiles, int ntiles) {
     pdl_wait();
@@ -98,7 +95,7 @@ ssm_chunk_carry_kernel(const ScArgs a) {
              a.state + ((size_t)a.slots[b] * a.H + h) * size, a.N, a.P, blockIdx.x * 256 + threadIdx.x, a.write_state);
 }
 
-// grid (chunks, H * ptiles, B): a chunk's 128 tokens x 64 values
+// grid (places, H * ptiles): a chunk's 128 tokens x 64 values
 __global__ void __launch_bounds__(CT_THREADS, 2)
 ssm_chunk_out_kernel(const ScArgs a, int ptiles) {
     pdl_wait();
@@ -137,7 +134,7 @@ extern "C" int qwb_ssm_chunked(const float* xbc, int ldx, const float* dt_raw, i
         return qwb_fail(QWB_ERR_ARG, "ssm_chunked: %d heads, %d groups, state %d x %d in rows of %d", H, G, N, P, ldx);
     for (const void* p : {(const void*)xbc, (const void*)state, (const void*)y, (const void*)scratch})
         if (!p || !rc_aligned16(p)) return qwb_fail(QWB_ERR_ARG, "ssm_chunked: a tensor is not 16-byte aligned");
-    const int chunks = (max_new + SC_TOKENS - 1) / SC_TOKENS, ptiles = (P + 63) / 64, ntiles = (N + 127) / 128, planes = rc_planes(T, B, from);
+    const int ptiles = (P + 63) / 64, ntiles = (N + 127) / 128, planes = rc_planes(T, B, from);
     const size_t places = (size_t)T / SC_TOKENS + planes;
     ScArgs a = {xbc, dt_raw, dt_bias, A_log, D, cu_seqlens, slots, state, y, nullptr, nullptr, nullptr, nullptr, error, ldx, ld_dt, H, P, N, G, write_state, B, from};
     a.own = scratch;
@@ -147,13 +144,13 @@ extern "C" int qwb_ssm_chunked(const float* xbc, int ldx, const float* dt_raw, i
     cudaError_t e = cudaFuncSetAttribute(ssm_chunk_state_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, CT_SMEM);
     if (e == cudaSuccess) e = cudaFuncSetAttribute(ssm_chunk_out_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, CT_SMEM);
     if (e != cudaSuccess) return qwb_fail(QWB_ERR_CUDA, "ssm_chunked: %s", cudaGetErrorString(e));
-    qwb_launch(ssm_chunk_gates_kernel, dim3(chunks, H, planes), SC_TOKENS, 0, stream, a);
+    qwb_launch(ssm_chunk_gates_kernel, dim3(rc_places(T, B, from, SC_TOKENS), H), SC_TOKENS, 0, stream, a);
     if (int rc = qwb_check_launch("ssm_chunk_gates")) return rc;
-    qwb_launch(ssm_chunk_state_kernel, dim3(chunks, 2 * G + H * ptiles * ntiles, planes), CT_THREADS, CT_SMEM, stream, a, ptiles, ntiles);
+    qwb_launch(ssm_chunk_state_kernel, dim3(rc_places(T, B, from, SC_TOKENS), 2 * G + H * ptiles * ntiles), CT_THREADS, CT_SMEM, stream, a, ptiles, ntiles);
     if (int rc = qwb_check_launch("ssm_chunk_state")) return rc;
     qwb_launch(ssm_chunk_carry_kernel, dim3((N * (P / 4) + 255) / 256, H, planes), 256, 0, stream, a);
     if (int rc = qwb_check_launch("ssm_chunk_carry")) return rc;
-    qwb_launch(ssm_chunk_out_kernel, dim3(chunks, H * ptiles, planes), CT_THREADS, CT_SMEM, stream, a, ptiles);
+    qwb_launch(ssm_chunk_out_kernel, dim3(rc_places(T, B, from, SC_TOKENS), H * ptiles), CT_THREADS, CT_SMEM, stream, a, ptiles);
     return qwb_check_launch("ssm_chunk_out");
 }
 
@@ -195,8 +192,7 @@ struct DcPlace { float *w, *k_end, *q0, *q_pairs, *u, *decay, *start; };
 __host__ __device__ __forceinline__ size_t dc_floats(int K, int P) {      // of one place and head: a multiple of 4
     return (size_t)3 * K * DC_TOKENS + DC_TOKENS * DC_TOKENS + (size_t)DC_TOKENS * P + K + (size_t)K * P;
 }
-__device__ __forceinline__ DcPlace dc_place(const DcArgs& a, int b, int c, int h) {      // in plane blockIdx.z of the grid
-    const size_t place = (size_t)(a.cu_seqlens[b] / DC_TOKENS + blockIdx.z + c);
+__device__ __forceinline__ DcPlace dc_place(const DcArgs& a, size_t place, int h) {
     DcPlace p;
     p.w = a.scratch + (place * a.H + h) * dc_floats(a.K, a.P);
     p.k_end = p.w + a.K * DC_TOKENS;
@@ -224,7 +220,7 @@ __device__ __forceinline__ float dc_quad_sum(float v) {
     return v + __shfl_xor_sync(0xffffffffu, v, 2);
 }
 
-// grid (chunks, H, B), 256 threads; dynamic shared memory: 3 x [64][128], A, totals [4][128], beta [64] (two blocks an SM)
+// grid (places, H), 256 threads; dynamic shared memory: 3 x [64][128], A, totals [4][128], beta [64] (two blocks an SM)
 __global__ void __launch_bounds__(256, 2)
 delta_chunk_prep_kernel(const DcArgs a) {
     pdl_wait();
@@ -236,11 +232,10 @@ delta_chunk_prep_kernel(const DcArgs a) {
     float* As = gs + DC_TOKENS * DC_MAX_K;                             // beta_i A_ij
     float* totals = As + DC_A_FLOATS;                               // [4][128]
     float* beta = totals + 4 * DC_MAX_K;
-    const int c = blockIdx.x, h = blockIdx.y, b = rc_sequence(a.cu_seqlens, a.B, a.from, blockIdx.z), tid = threadIdx.x, K = a.K, P = a.P;
-    if (b < 0) return;
-    const int t0 = a.cu_seqlens[b] + c * DC_TOKENS, n = min(DC_TOKENS, a.cu_seqlens[b + 1] - t0);
+    int t0;
+    const int h = blockIdx.y, n = rc_chunk<DC_TOKENS>(a.cu_seqlens, a.B, a.from, blockIdx.x, t0), tid = threadIdx.x, K = a.K, P = a.P;
     if (n <= 0) return;
-    const DcPlace at = dc_place(a, b, c, h);
+    const DcPlace at = dc_place(a, blockIdx.x, h);
     const int kh = h / (a.H / a.Hk);
     const float rate = -expf(a.A_log[h]) * 1.4426950408889634f;
     if (tid < DC_TOKENS) beta[tid] = tid < n ? a.beta[(size_t)(t0 + tid) * a.H + h] : 0.f;
@@ -514,7 +509,7 @@ delta_chunk_walk_kernel(const DcArgs a) {
         }
         rc_commit();
     };
-    DcPlace at = dc_place(a, b, 0, h);
+    DcPlace at = dc_place(a, a.cu_seqlens[b] / DC_TOKENS + blockIdx.z, h);
     const size_t step = a.H * dc_floats(K, P);
     copy(Ws, ldw, at.w, true);
     copy(Ke, K, at.k_end, true);
@@ -599,18 +594,16 @@ delta_chunk_walk_kernel(const DcArgs a) {
     }
 }
 
-// grid (chunks, H * ptiles, B): a chunk's 64 tokens x 128 values, from S0 and then from the chunk's own u, as o^T on tcgen05 (chunk_tc.cuh: the
+// grid (places, H * ptiles): a chunk's 64 tokens x 128 values, from S0 and then from the chunk's own u, as o^T on tcgen05 (chunk_tc.cuh: the
 // values are the product's 128 rows).  65 us with 8 x 8 sums a thread, 58 on mma.sync, 42 here (three prompts of 2,900 tokens in all)
 __global__ void __launch_bounds__(CT_THREADS, 2)
 delta_chunk_out_kernel(const DcArgs a, int ptiles) {
     pdl_wait();
     pdl_launch_dependents();
-    const int c = blockIdx.x, h = blockIdx.y / ptiles, p0 = (blockIdx.y - h * ptiles) * 128, K = a.K, P = a.P;
-    const int b = rc_sequence(a.cu_seqlens, a.B, a.from, blockIdx.z);
-    if (b < 0) return;
-    const int t0 = a.cu_seqlens[b] + c * DC_TOKENS, n = min(DC_TOKENS, a.cu_seqlens[b + 1] - t0);
+    int t0;
+    const int h = blockIdx.y / ptiles, p0 = (blockIdx.y - h * ptiles) * 128, K = a.K, P = a.P, n = rc_chunk<DC_TOKENS>(a.cu_seqlens, a.B, a.from, blockIdx.x, t0);
     if (n <= 0) return;
-    const DcPlace at = dc_place(a, b, c, h);
+    const DcPlace at = dc_place(a, blockIdx.x, h);
     const CtBlock block = ct_begin(a.error);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, state_stages = (K + CT_R - 1) / CT_R;
     const int index = 4 * warp + (lane >> 3), token = 8 * warp + ct_row(lane), eight = lane & 3;
@@ -674,7 +667,8 @@ extern "C" int qwb_delta_chunked(const float* qkv, int ld, const float* beta, co
         return qwb_fail(QWB_ERR_ARG, "delta_chunked: %d heads, %d key heads, state %d x %d in rows of %d, %d decays a head", H, Hk, K, P, ld, decay_k);
     for (const void* p : {(const void*)qkv, (const void*)state, (const void*)o, (const void*)scratch})
         if (!p || !rc_aligned16(p)) return qwb_fail(QWB_ERR_ARG, "delta_chunked: a tensor is not 16-byte aligned");
-    const int chunks = (max_new + DC_TOKENS - 1) / DC_TOKENS, ptiles = (P + 127) / 128, planes = rc_planes(T, B, from);
+    const int ptiles = (P + 127) / 128, planes = rc_planes(T, B, from);
+    const unsigned places = rc_places(T, B, from, DC_TOKENS);
     const DcArgs a = {qkv, beta, a_raw, dt_bias, A_log, cu_seqlens, slots, state, o, scratch, error, ld, ld_a, H, Hk, K, P, decay_k, write_state, B, from};
     const size_t smem1 = (3 * DC_TOKENS * DC_MAX_K + DC_A_FLOATS + 4 * DC_MAX_K + DC_TOKENS) * sizeof(float);
     const size_t smem2 = ((3 * K + 4) * DC_TOKENS + DC_WALK_P * (K + 4) + DC_TOKENS * (DC_WALK_P + 4)) * sizeof(float);
@@ -682,10 +676,10 @@ extern "C" int qwb_delta_chunked(const float* qkv, int ld, const float* beta, co
     if (e == cudaSuccess) e = cudaFuncSetAttribute(delta_chunk_out_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, CT_SMEM);
     if (e == cudaSuccess) e = cudaFuncSetAttribute(delta_chunk_walk_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem2);
     if (e != cudaSuccess) return qwb_fail(QWB_ERR_CUDA, "delta_chunked: %s", cudaGetErrorString(e));
-    qwb_launch(delta_chunk_prep_kernel, dim3(chunks, H, planes), 256, smem1, stream, a);
+    qwb_launch(delta_chunk_prep_kernel, dim3(places, H), 256, smem1, stream, a);
     if (int rc = qwb_check_launch("delta_chunk_prep")) return rc;
     qwb_launch(delta_chunk_walk_kernel, dim3((P + DC_WALK_P - 1) / DC_WALK_P, H, planes), 256, smem2, stream, a);
     if (int rc = qwb_check_launch("delta_chunk_walk")) return rc;
-    qwb_launch(delta_chunk_out_kernel, dim3(chunks, H * ptiles, planes), CT_THREADS, CT_SMEM, stream, a, ptiles);
+    qwb_launch(delta_chunk_out_kernel, dim3(places, H * ptiles), CT_THREADS, CT_SMEM, stream, a, ptiles);
     return qwb_check_launch("delta_chunk_out");
 }

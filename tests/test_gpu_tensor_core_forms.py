@@ -403,6 +403,58 @@ def test_matrix_memory_in_chunks_of_128(H, K, P, forget, monkeypatch):
     assert torch.equal(st, before) and torch.equal(m, m_before)
 
 
+@pytest.mark.parametrize("lens", [[1] * 33 + [300, 1, 128, 129, 127] + [1] * 34 + [257], [400] + [1] * 70, [1] * 64 + [130], [5, 1, 700]])
+def test_matrix_memory_in_chunks_of_128_among_many_sequences(lens, monkeypatch):
+    """Chunks of sequences anywhere among more than a warp's worth of others, against the chunks of 64."""
+    torch.manual_seed(len(lens))
+    H, K, P, T = 2, 20, 36, sum(lens)
+    at, slots = H * (2 * K + P), [(7 * i + 3) % len(lens) for i in range(len(lens))] if len(lens) % 7 else list(range(len(lens)))[::-1]
+    proj, zero = torch.randn(T, at + 2 * H, device=DEV), torch.zeros(H, device=DEV)
+    start, m_start = 0.5 * torch.randn(len(lens), H, P + 1, K, device=DEV), torch.rand(len(lens), H, 1, device=DEV).repeat(1, 1, P + 1)
+    forms = []
+    for tiles in (False, True):
+        monkeypatch.setattr(ops, "mlstm_tiles_pay", lambda *sizes: tiles)
+        st, m = start.clone(), m_start.clone()
+        forms.append((*ops.mlstm_scan(proj, at, at + H, zero, zero, 15.0, st, m, Steps(lens, slots), H, K, P, K ** -0.5, 1e-6), st, m))
+    for got, want in zip(forms[1], forms[0]):
+        sums_close(got, want.double(), 2 ** -18)
+
+
+@pytest.mark.parametrize("kind", ["mamba2", "delta", "mlstm"])
+def test_a_long_prompt_beside_many_single_tokens_costs_what_it_has_to_do(kind, monkeypatch):
+    """Twice what the two cost alone at most: no grid is as long as the longest sequence and as wide as all of them (6 times, then)."""
+    H, K, P, G, prompt, others = (64, 128, 64, 8, 8192, 63) if kind == "mamba2" else (16, 128, 128, 16, 8192, 63)
+    monkeypatch.setattr(ops, "_mlstm_tiles", lambda *sizes: True)
+
+    def call(lens):
+        T, step = sum(lens), Steps(lens, list(range(len(lens))))
+        step.min_new, rows, zero = min(lens), torch.randn(T, H * (2 * K + P) + 2 * H, device=DEV), torch.zeros(H * K, device=DEV)
+        if kind == "mamba2":
+            xbc, state = rows[:, :H * P + 2 * G * K].contiguous(), torch.zeros(len(lens), H, P, K, device=DEV)
+            return lambda: ops.ssm_scan(xbc, rows, 0, zero[:H].contiguous(), zero[:H].contiguous(), zero[:H].contiguous(), state, step, H, P, K, G)
+        if kind == "delta":
+            qkv, side, state = rows[:, :H * (2 * K + P)].contiguous(), rows[:, :H].contiguous(), torch.zeros(len(lens), H, P, K, device=DEV)
+            return lambda: ops.delta_rule(qkv, side, 0, side, zero[:H].contiguous(), zero[:H].contiguous(), state, step, H, H, K, P, 1e-6, K ** -0.5, per_head=True)
+        state, m, n = torch.zeros(len(lens), H, P + 1, K, device=DEV), torch.zeros(len(lens), H, P + 1, device=DEV), H * (2 * K + P)
+        return lambda: ops.mlstm_scan(rows, n, n + H, zero[:H].contiguous(), zero[:H].contiguous(), 15.0, state, m, step, H, K, P, K ** -0.5, 1e-6)
+
+    def took(f):
+        best = math.inf
+        for _ in range(6):
+            a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            f()
+            a.record()
+            f()
+            b.record()
+            b.synchronize()
+            best = min(best, a.elapsed_time(b))
+        return best
+
+    alone, rest, both = took(call([prompt])), took(call([1] * others)), took(call([prompt] + [1] * others))
+    torch.cuda.empty_cache()                                # large blocks that a test of little memory would find room in
+    assert both <= 2.0 * (alone + rest), (alone, rest, both)
+
+
 @pytest.mark.parametrize("kind", ["mamba2", "mlstm"])
 @pytest.mark.parametrize("H, K, P", [(2, 36, 20), (4, 128, 64), (2, 260, 132)])
 def test_products_of_three_parts_keep_32_bits(kind, H, K, P, monkeypatch):
