@@ -178,6 +178,7 @@ extern "C" int qwb_ssm_chunked(const float* xbc, int ldx, const float* dt_raw, i
 // ---------------------------------------------------------------------------------
 #define DC_TOKENS 64
 #define DC_SUB 16
+#define DC_WALK_ALONE (120 * 1024)        // bytes of shared memory of which an SM has no two
 #define DC_MAX_K 128
 #define DC_WALK_P 16
 
@@ -672,13 +673,19 @@ extern "C" int qwb_delta_chunked(const float* qkv, int ld, const float* beta, co
     const DcArgs a = {qkv, beta, a_raw, dt_bias, A_log, cu_seqlens, slots, state, o, scratch, error, ld, ld_a, H, Hk, K, P, decay_k, write_state, B, from};
     const size_t smem1 = (3 * DC_TOKENS * DC_MAX_K + DC_A_FLOATS + 4 * DC_MAX_K + DC_TOKENS) * sizeof(float);
     const size_t smem2 = ((3 * K + 4) * DC_TOKENS + DC_WALK_P * (K + 4) + DC_TOKENS * (DC_WALK_P + 4)) * sizeof(float);
+    // The walk of one sequence is (P / 16) H blocks in a chain of chunks, which two on an SM slow down to 0.6.  Of a grid with room for other
+    // sequences the SMs take neighbours two at a time, so where the longest sequence stands alone, or by far the most of the others take
+    // the scan, a block asks for an SM's shared memory.  us, 16 heads of 128 x 128, two / one an SM: 2,048 tokens beside 16 single ones 371 / 293,
+    // beside 31 of 100 1,262 / 1,184, beside 3 of 300 415 / 374; 2 x 2,048 469 / 502, 16 x 300 561 / 611.
+    const bool alone = T < 2LL * max_new || T - max_new < (long long)(B - 1) * from;
+    const size_t walk_smem = alone && smem2 < DC_WALK_ALONE ? DC_WALK_ALONE : smem2;
     cudaError_t e = cudaFuncSetAttribute(delta_chunk_prep_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem1);
     if (e == cudaSuccess) e = cudaFuncSetAttribute(delta_chunk_out_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, CT_SMEM);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(delta_chunk_walk_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem2);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(delta_chunk_walk_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(smem2 < DC_WALK_ALONE ? DC_WALK_ALONE : smem2));
     if (e != cudaSuccess) return qwb_fail(QWB_ERR_CUDA, "delta_chunked: %s", cudaGetErrorString(e));
     qwb_launch(delta_chunk_prep_kernel, dim3(places, H), 256, smem1, stream, a);
     if (int rc = qwb_check_launch("delta_chunk_prep")) return rc;
-    qwb_launch(delta_chunk_walk_kernel, dim3((P + DC_WALK_P - 1) / DC_WALK_P, H, planes), 256, smem2, stream, a);
+    qwb_launch(delta_chunk_walk_kernel, dim3((P + DC_WALK_P - 1) / DC_WALK_P, H, planes), 256, walk_smem, stream, a);
     if (int rc = qwb_check_launch("delta_chunk_walk")) return rc;
     qwb_launch(delta_chunk_out_kernel, dim3(places, H * ptiles), CT_THREADS, CT_SMEM, stream, a, ptiles);
     return qwb_check_launch("delta_chunk_out");

@@ -422,7 +422,8 @@ def test_matrix_memory_in_chunks_of_128_among_many_sequences(lens, monkeypatch):
 
 @pytest.mark.parametrize("kind", ["mamba2", "delta", "mlstm"])
 def test_a_long_prompt_beside_many_single_tokens_costs_what_it_has_to_do(kind, monkeypatch):
-    """Twice what the two cost alone at most: no grid is as long as the longest sequence and as wide as all of them (6 times, then)."""
+    """Twice what the two cost alone at most: no grid is as long as the longest sequence and as wide as all of them (6 times, then).
+    The delta rule's chain through the prompt's chunks has its SMs for itself (1.28 times where it shares them, 0.98 where it does not)."""
     H, K, P, G, prompt, others = (64, 128, 64, 8, 8192, 63) if kind == "mamba2" else (16, 128, 128, 16, 8192, 63)
     monkeypatch.setattr(ops, "_mlstm_tiles", lambda *sizes: True)
 
@@ -452,7 +453,7 @@ def test_a_long_prompt_beside_many_single_tokens_costs_what_it_has_to_do(kind, m
 
     alone, rest, both = took(call([prompt])), took(call([1] * others)), took(call([prompt] + [1] * others))
     torch.cuda.empty_cache()                                # large blocks that a test of little memory would find room in
-    assert both <= 2.0 * (alone + rest), (alone, rest, both)
+    assert both <= (1.15 if kind == "delta" else 2.0) * (alone + rest), (alone, rest, both)
 
 
 @pytest.mark.parametrize("kind", ["mamba2", "mlstm"])
