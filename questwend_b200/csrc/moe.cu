@@ -332,8 +332,15 @@ __device__ __forceinline__ void ms_tile(float (&acc)[NT][4], const bf16* lo, con
     }
 }
 
-// What moe_lists leaves: the experts that are chosen, in order, where each one's copies begin (and the last one's end), the copies.
-struct MsLists { int n; int expert[QWB_MOE_MAX_EXPERTS], begin[QWB_MOE_MAX_EXPERTS + 1], copies[MS_MAX_COPIES]; };
+// What moe_lists leaves: the experts that are chosen, in order, in slots of up to MS_SLOT copies, where each slot's copies begin (and the last
+// one's end), the copies.  An expert that many tokens chose has several slots, whose blocks run side by side: with one slot an expert its blocks
+// went through its copies 32 at a time, one pass behind the other.  us,
+// tokens of which most chose the same experts, sorted through the grouped product / a slot an expert / now: 6 of 64 and a shared one, 64 tokens
+// 122 / 115 / 97, 128 140 / 212 / 180; 8 of 128, 64 86 / 114 / 102, 128 122 / 194 / 167; 2 of 8 of 4,096 x 2,048, 64 65 / 125 / 78; evenly chosen, the first
+// of these 204 / 150 / 149 and 208 / 204 / 188.
+#define MS_SLOT 32
+#define MS_MAX_SLOTS (QWB_MOE_MAX_EXPERTS + MS_MAX_COPIES / MS_SLOT)
+struct MsLists { int n; int expert[MS_MAX_SLOTS], begin[MS_MAX_SLOTS + 1], copies[MS_MAX_COPIES]; };
 
 struct MsArgs {
     const bf16 *in, *in_s, *w, *w_s;        // vectors of copies (up: of tokens) and of the shared expert's tokens; experts' and shared weights
@@ -360,17 +367,18 @@ moe_lists_kernel(const int* chosen, MsLists* lists, int S, int E) {
     }
     __syncthreads();
     const int mine = tid < E ? count[tid] : 0;
-    int copies = mine, active = mine > 0;                           // sums over the experts up to this one
+    const int own = (mine + MS_SLOT - 1) / MS_SLOT;
+    int copies = mine, slots = own;                                 // sums over the experts up to this one
     for (int o = 1; o < 32; o <<= 1) {
-        const int a = __shfl_up_sync(0xffffffffu, copies, o), b = __shfl_up_sync(0xffffffffu, active, o);
-        if (lane >= o) { copies += a; active += b; }
+        const int a = __shfl_up_sync(0xffffffffu, copies, o), b = __shfl_up_sync(0xffffffffu, slots, o);
+        if (lane >= o) { copies += a; slots += b; }
     }
-    if (lane == 31) { warps[0][warp] = copies; warps[1][warp] = active; }
+    if (lane == 31) { warps[0][warp] = copies; warps[1][warp] = slots; }
     __syncthreads();
-    for (int w = 0; w < warp; ++w) { copies += warps[0][w]; active += warps[1][w]; }
-    if (mine) { lists->expert[active - 1] = tid; lists->begin[active] = copies; }
+    for (int w = 0; w < warp; ++w) { copies += warps[0][w]; slots += warps[1][w]; }
+    for (int k = 0; k < own; ++k) { lists->expert[slots - own + k] = tid; lists->begin[slots - own + k + 1] = min(copies - mine + MS_SLOT * (k + 1), copies); }
     if (tid == 0) lists->begin[0] = 0;
-    if (tid == 1023) lists->n = active;
+    if (tid == 1023) lists->n = slots;
     if (tid < E) count[tid] = copies - mine;
     __syncthreads();
     for (int e = warp; e < E; e += 32) {
@@ -425,10 +433,9 @@ __device__ __forceinline__ void ms_rows(const MsArgs& a, bool shared, const bf16
             (shared ? a.act_s + (size_t)c * a.rows_s : a.act + (size_t)c * a.rows)[f] = from_f32<bf16>(v);
         }
     }
-    __syncthreads();
 }
 
-// Blocks: the shared expert's tiles, then (slot, tile).  A tile is 16 rows, of a gated expert 8 gate rows and their 8 up rows.
+// Blocks: the shared expert's tiles, once for every MS_SLOT tokens, then (slot, tile).  A tile is 16 rows, of a gated expert 8 gate rows and their 8 up rows.
 template <bool DOWN>
 __global__ void __launch_bounds__(32 * MS_WARPS, 7)
 moe_stream_kernel(const MsArgs a, int tiles, int tiles_s) {
@@ -436,11 +443,15 @@ moe_stream_kernel(const MsArgs a, int tiles, int tiles_s) {
     pdl_wait();
     __shared__ float part[MS_WARPS * 4 * 4 * 32];
     const int lane = threadIdx.x & 31, g = lane >> 2;
-    const bool shared = (int)blockIdx.x < tiles_s, gated = !DOWN && !shared && a.kind == QWB_MOE_GATED;
-    const int item = (int)blockIdx.x - tiles_s, slot = item / tiles, tile = shared ? blockIdx.x : item - slot * tiles;
+    const int blocks_s = tiles_s * ((a.T + MS_SLOT - 1) / MS_SLOT);
+    const bool shared = (int)blockIdx.x < blocks_s, gated = !DOWN && !shared && a.kind == QWB_MOE_GATED;
+    const int item = (int)blockIdx.x - blocks_s, slot = item / tiles, tile = shared ? (int)blockIdx.x % tiles_s : item - slot * tiles;
     const int* copies = nullptr;
-    int n = a.T, e = 0;
-    if (!shared) {
+    int first = 0, n = 0, e = 0;
+    if (shared) {
+        first = (int)blockIdx.x / tiles_s * MS_SLOT;
+        n = min(a.T, first + MS_SLOT);
+    } else {
         const int begin = __ldcg(a.lists->begin + slot), end = __ldcg(a.lists->begin + slot + 1);
         e = __ldcg(a.lists->expert + slot);
         if (slot >= __ldcg(&a.lists->n)) return;
@@ -451,11 +462,9 @@ moe_stream_kernel(const MsArgs a, int tiles, int tiles_s) {
     const bf16* w = shared ? a.w_s : a.w + (size_t)e * (gated ? 2 * rows : rows) * K;
     const int r0 = f0 + g, r1 = gated ? rows + f0 + g : f0 + g + 8;
     const bf16 *lo = r0 < rows ? w + (size_t)r0 * K : nullptr, *hi = (gated ? r0 : r1) < rows ? w + (size_t)r1 * K : nullptr;
-    for (int first = 0; first < n;) {
-        if (n - first <= 8) { ms_rows<1, DOWN>(a, shared, lo, hi, f0, copies, n, first, part); first += 8; }
-        else if (n - first <= 16) { ms_rows<2, DOWN>(a, shared, lo, hi, f0, copies, n, first, part); first += 16; }
-        else { ms_rows<4, DOWN>(a, shared, lo, hi, f0, copies, n, first, part); first += 32; }
-    }
+    if (n - first <= 8) ms_rows<1, DOWN>(a, shared, lo, hi, f0, copies, n, first, part);
+    else if (n - first <= 16) ms_rows<2, DOWN>(a, shared, lo, hi, f0, copies, n, first, part);
+    else ms_rows<4, DOWN>(a, shared, lo, hi, f0, copies, n, first, part);
 }
 
 // grid (ceil(D / 1,024), T), 256 threads: four outputs of a token a thread, from the rows of its copies
@@ -491,7 +500,8 @@ extern "C" int qwb_moe_stream(const void* x, const void* wu, const void* wd, con
     if (kind != QWB_MOE_GATED && !qwb_activation_known(kind)) return qwb_fail(QWB_ERR_ARG, "moe_stream: unknown activation %d", kind);
     for (const void* p : {x, wu, wd, wsu, wsd, (const void*)act, (const void*)act_s, (const void*)y, (const void*)out})
         if ((uintptr_t)p % 16) return qwb_fail(QWB_ERR_ARG, "moe_stream: a tensor is not 16-byte aligned");
-    const int slots = T * top < E ? T * top : E;
+    const int copies = T * top, slots = min(copies, min(copies, E) + copies / MS_SLOT);      // an expert's slots but for one are full
+    const int passes = (T + MS_SLOT - 1) / MS_SLOT;                 // of the shared expert's tokens
     const int up_tiles = kind == QWB_MOE_GATED ? F / 8 : (F + 15) / 16, up_shared = (Fs + 15) / 16, down_tiles = (D + 15) / 16, down_shared = Fs > 0 ? down_tiles : 0;
     MsLists* lists = reinterpret_cast<MsLists*>(y + (size_t)T * (top + (Fs > 0 ? 1 : 0)) * D);
     float* y_s = Fs > 0 ? y + (size_t)T * top * D : nullptr;
@@ -500,9 +510,9 @@ extern "C" int qwb_moe_stream(const void* x, const void* wu, const void* wd, con
     const MsArgs down = {(const bf16*)act, (const bf16*)act_s, (const bf16*)wd, (const bf16*)wsd, lists, nullptr, nullptr, nullptr, y, y_s, T, top, F, Fs, D, D, kind};
     qwb_launch_link(T, MS_LINK_ROWS, moe_lists_kernel, 1, 1024, 0, stream, chosen, lists, T * top, E);
     if (int rc = qwb_check_launch("moe_lists")) return rc;
-    qwb_launch_link(T, MS_LINK_ROWS, moe_stream_kernel<false>, up_shared + slots * up_tiles, 32 * MS_WARPS, 0, stream, up, up_tiles, up_shared);
+    qwb_launch_link(T, MS_LINK_ROWS, moe_stream_kernel<false>, passes * up_shared + slots * up_tiles, 32 * MS_WARPS, 0, stream, up, up_tiles, up_shared);
     if (int rc = qwb_check_launch("moe_stream up")) return rc;
-    qwb_launch_link(T, MS_LINK_ROWS, moe_stream_kernel<true>, down_shared + slots * down_tiles, 32 * MS_WARPS, 0, stream, down, down_tiles, down_shared);
+    qwb_launch_link(T, MS_LINK_ROWS, moe_stream_kernel<true>, passes * down_shared + slots * down_tiles, 32 * MS_WARPS, 0, stream, down, down_tiles, down_shared);
     if (int rc = qwb_check_launch("moe_stream down")) return rc;
     qwb_launch_link(T, MS_LINK_ROWS, moe_merge_kernel, dim3((D + 1023) / 1024, T), 256, 0, stream, (const float*)y, (const float*)y_s, on_input ? nullptr : weight, gate, out, D, top, onto);
     return qwb_check_launch("moe_merge");

@@ -851,7 +851,7 @@ def test_experts_read_once_for_all_their_tokens(T, E, top, D, F, Fs, activation,
     x, up, down = (torch.randn(*s, device=DEV).mul(f).to(torch.bfloat16) for s, f in (((T, D), 1.0), ((E, (2 if gated else 1) * F, D), D ** -0.5), ((E, D, F), F ** -0.5)))
     su, sd, gate = (None, None, None) if not Fs else (torch.randn(Fs, D, device=DEV).mul(D ** -0.5).to(torch.bfloat16), torch.randn(D, Fs, device=DEV).mul(Fs ** -0.5).to(torch.bfloat16), torch.rand(T, device=DEV))
     logits = torch.randn(T, E, device=DEV)
-    logits[:, 0] += 3.0                                     # most tokens choose the first one, few the last
+    logits[:, 0] += 3.0 if T != 140 else 1e3                # most tokens choose the first one, few the last; 140: all of them, more than four slots
     logits[:, -1] -= 3.0 * (E > top)
     chosen, weight = ops.moe_route(logits, top)
     act = {"relu2": lambda z: torch.relu(z).square(), "gelu": lambda z: torch.nn.functional.gelu(z, approximate="tanh"), "silu": torch.nn.functional.silu}
