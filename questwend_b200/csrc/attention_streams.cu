@@ -21,7 +21,9 @@
 // streams' softmax warps, 12-15 multiply O by what a row's reference has moved: in most tiles some row of a warp's 32 moves it, and a
 // softmax warp that did this itself waited for the product before, 780 to 1,830 of a tile's 3,000 cycles.  One warp for both streams'
 // products spent 3,500 cycles a tile (65 to 80 a product, about 200 a wait, passed or not).  With capped scores the softmax's multiply-adds
-// fill the schedulers and want the registers: there its warps move O themselves (8,192 tokens 673 us, with warps for it 760).
+// fill the schedulers and want the registers: there its warps move O themselves (8,192 tokens 673 us, with warps for it 760).  So they do for latent
+// prompts, whose products of 192 values hide the wait: 4,096 tokens 85.2 us, with warps for it 87.2, 2,048 36.7 and 40.1, 32 of 64 18.0 and 19.0.  Two
+// maps without a cap, the same: 4,096 154 and 140, 1,024 25.9 and 23.4, 32 of 64 12.7 and 13.1.
 //
 // Sizes that are no multiples of 64 are filled up by the TMA loads with zeros.  In the last tile, rows of V behind the last
 // key that the block sees are overwritten with zeros before the product: they can belong to another sequence, and what stands
@@ -30,12 +32,13 @@
 // one with two maps.
 //
 // Bound by the issue of products of 64 keys and the softmax's chain, near each other.  16 heads: latent 128 + 64 / 128, one prompt of 4,096, with
-// the mma.sync kernels 816 us, one issuing warp 112, now 92 (600 tokens 55 -> 19.7 -> 19.0); two maps of 64 over 4 key/value heads, values of 128,
+// the mma.sync kernels 816 us, one issuing warp 108, now 85 (600 tokens 55 -> 15.3 -> 15.2); two maps of 64 over 4 key/value heads, values of 128,
 // 8,192 tokens: 2,447 -> 583 -> 507 us (cap 50: 3,261 -> 696 -> 673), 2,048 tokens with a window of 1,024: 170 -> 51 -> 45 us.
 #include "attention_tc.cuh"
 
 #include <atomic>
 
+#define AS_APART(maps, cap) ((maps) && !(cap))      // warps of their own move O
 #define AS_THREADS(apart) ((apart) ? 512 : 384)
 // Registers a thread of the loader's and issuers' warps, of the streams' softmax warps, of the warps that move O: as many in all as the block is
 // launched with (128 a thread, all of an SM's), which is what setmaxnreg has to give.
@@ -150,12 +153,12 @@ struct AsArgs {
 };
 
 template <int KA, int VA, bool MAPS, bool CAP>
-__global__ void __launch_bounds__(AS_THREADS(!CAP), 1)
+__global__ void __launch_bounds__(AS_THREADS(AS_APART(MAPS, CAP)), 1)
 attn_streams_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_q2, const __grid_constant__ CUtensorMap map_k,
                     const __grid_constant__ CUtensorMap map_k2, const __grid_constant__ CUtensorMap map_v, const AsArgs p) {
     using Smem = AsSmem<KA, VA, MAPS>;
     constexpr int VD = 64 * VA, STAGES = Smem::STAGES;
-    constexpr bool APART = !CAP;
+    constexpr bool APART = AS_APART(MAPS, CAP);
     constexpr uint32_t K_BYTES = Smem::K_BYTES, V_BYTES = Smem::V_BYTES;
     extern __shared__ __align__(1024) unsigned char smem_raw[];
     if (at_smem(smem_raw) & 1023u) {                    // never seen; refuse rather than compute with a wrong layout
@@ -609,14 +612,14 @@ static int as_map(const char* what, CUtensorMap* map, const void* base, int rank
     return r == CUDA_SUCCESS ? 0 : qwb_fail(QWB_ERR_CUDA, "%s: cuTensorMapEncodeTiled failed with %d", what, (int)r);
 }
 
-// Whether the uncapped kernel was built with the registers that its warps share out among themselves (else they would wait for some that
+// Whether the uncapped kernel for two maps was built with the registers that its warps share out among themselves (else they would wait for some that
 // there are not): 1, 0, or -1 where that cannot be found out now.
-template <int KA, int VA, bool MAPS>
+template <int KA, int VA>
 static int as_built() {
     static std::atomic<int> regs{0};
     if (regs == 0) {
         cudaFuncAttributes f;
-        if (cudaFuncGetAttributes(&f, attn_streams_kernel<KA, VA, MAPS, false>) != cudaSuccess) return -1;
+        if (cudaFuncGetAttributes(&f, attn_streams_kernel<KA, VA, true, false>) != cudaSuccess) return -1;
         regs = f.numRegs;
     }
     return regs == AS_LAUNCH_REGS;
@@ -628,27 +631,22 @@ static int as_launch(const char* what, dim3 grid, const CUtensorMap* maps, const
     auto kernel = attn_streams_kernel<KA, VA, MAPS, CAP>;
     cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return qwb_fail(QWB_ERR_CUDA, "%s: %s", what, cudaGetErrorString(e));
-    if (!CAP && as_built<KA, VA, MAPS>() != 1) return qwb_fail(QWB_ERR_CUDA, "%s: not built with %d registers a thread", what, AS_LAUNCH_REGS);
-    e = qwb_launch(kernel, grid, AS_THREADS(!CAP), smem, stream, maps[0], maps[1], maps[2], maps[3], maps[4], args);
+    if constexpr (AS_APART(MAPS, CAP))
+        if (as_built<KA, VA>() != 1) return qwb_fail(QWB_ERR_CUDA, "%s: not built with %d registers a thread", what, AS_LAUNCH_REGS);
+    e = qwb_launch(kernel, grid, AS_THREADS(AS_APART(MAPS, CAP)), smem, stream, maps[0], maps[1], maps[2], maps[3], maps[4], args);
     if (e != cudaSuccess) return qwb_fail(QWB_ERR_CUDA, "%s: launch failed: %s", what, cudaGetErrorString(e));
     return qwb_check_launch(what);
 }
 
 static int as_pieces(int n) { return (n + 63) / 64; }
 
-// Whether uncapped prompts of these sizes may take this kernel as it was built; where they may not, the caller takes another one.
-extern "C" int qwb_streams_built(int maps, int key_pieces, int value_pieces) {
-    switch ((maps ? 100 : 0) + 10 * key_pieces + value_pieces) {
-        case 11: return as_built<1, 1, false>() != 0;
-        case 12: return as_built<1, 2, false>() != 0;
-        case 21: return as_built<2, 1, false>() != 0;
-        case 22: return as_built<2, 2, false>() != 0;
-        case 31: return as_built<3, 1, false>() != 0;
-        case 32: return as_built<3, 2, false>() != 0;
-        case 111: return as_built<1, 1, true>() != 0;
-        case 112: return as_built<1, 2, true>() != 0;
-        case 121: return as_built<2, 1, true>() != 0;
-        case 122: return as_built<2, 2, true>() != 0;
+// Whether uncapped prompts with two maps of these sizes may take this kernel as it was built; where they may not, the caller takes another one.
+extern "C" int qwb_streams_built(int key_pieces, int value_pieces) {
+    switch (10 * key_pieces + value_pieces) {
+        case 11: return as_built<1, 1>() != 0;
+        case 12: return as_built<1, 2>() != 0;
+        case 21: return as_built<2, 1>() != 0;
+        case 22: return as_built<2, 2>() != 0;
     }
     return 0;
 }

@@ -1517,7 +1517,7 @@ def maps_attention(q: torch.Tensor, k_pool, v_pool, page_table, ctx, maps: int, 
                             chunk=chunk)
     if (impl in ("auto", "tc") and scale > 0.0 and ctx.max_new * (H // G) >= 64 and ctx.max_new * (H // G) <= 65535 * 64
             and maps_prefill_tc_fits(q.dtype, maps, dim, vdim, H // G) and not any(t.data_ptr() % 16 for t in (q, k_pool, v_pool))
-            and (softcap > 0.0 or _streams_built(maps, [dim], vdim))):
+            and (softcap > 0.0 or _streams_built(dim, vdim))):
         _call("attention_streams", "qwb_maps_prefill_tc", _ptr(q), _ptr(k_pool), _ptr(v_pool), _ptr(page_table), _ptr(ctx.cu_seqlens),
               _ptr(ctx.pos0), _ptr(out), _i(ctx.n_seqs), _i(T), _i(ctx.max_new), _i(k_pool.shape[0]), _i(H), _i(G), _i(dim), _i(vdim), _i(width),
               _f(scale), _f(softcap), _i(chunk), _i(window), _f(lam), _i(1 if norm_out else 0), _f(eps), _f(out_scale), *gate_args,
@@ -1746,10 +1746,10 @@ def latent_prefill_fits(dtype: torch.dtype, dim: int, rot_dim: int, vdim: int, r
 LATENT_PREFILL_TC = True    # prompts take the tcgen05 kernel where it fits; False: always the mma.sync one
 
 
-def _streams_built(maps: int, dims: list, vdim: int) -> bool:
-    """Whether the two-stream kernel of uncapped prompts was built with the registers that it shares out among its warps; a build by
-    other tools or flags may not be, and the mma.sync kernels take the call then."""
-    return bool(_lookup("attention_streams", "qwb_streams_built")[1](ctypes.c_int(maps > 1), ctypes.c_int(sum(-(-n // 64) for n in dims)), ctypes.c_int(-(-vdim // 64))))
+def _streams_built(dim: int, vdim: int) -> bool:
+    """Whether the two-stream kernel of uncapped prompts with two maps was built with the registers that it shares out among its warps; a build by
+    other tools or flags may not be, and the mma.sync kernel takes the call then."""
+    return bool(_lookup("attention_streams", "qwb_streams_built")[1](ctypes.c_int(-(-dim // 64)), ctypes.c_int(-(-vdim // 64))))
 
 
 def latent_prefill_tc_fits(dim: int, rot_dim: int, vdim: int) -> bool:
@@ -1777,7 +1777,7 @@ def latent_prefill(q: torch.Tensor, k_plain: torch.Tensor, rows: torch.Tensor, v
         _need(sink, "sink", torch.float32, 1)
     out = _empty((T, heads * vdim), dtype=torch.bfloat16, device=q.device)
     ld = rows.shape[1]
-    if scale > 0.0 and ld % 8 == 0 and latent_prefill_tc_fits(dim, rot_dim, vdim) and _streams_built(1, [dim, rot_dim], vdim):
+    if scale > 0.0 and ld % 8 == 0 and latent_prefill_tc_fits(dim, rot_dim, vdim):
         _call("attention_streams", "qwb_latent_prefill_tc", _ptr(q), _ptr(k_plain),
               _address(rows.data_ptr() + 2 * (ld - rot_dim)), _i(ld), _ptr(v), _ptr(ctx.cu_seqlens), _ptr(sink), _ptr(out),
               _i(ctx.n_seqs), _i(T), _i(ctx.max_new), _i(heads), _i(dim), _i(rot_dim), _i(vdim), _f(scale), _i(window),
