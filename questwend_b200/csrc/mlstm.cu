@@ -558,7 +558,7 @@ mlstm_chunk_out_kernel(MlstmRows rows, const float* __restrict__ log_decay, cons
 //     own / starts [places, H, P / 4, K, 4], scores [places, H, 32, 128 (i), 4 (j)], gates [places, H], normalisers [places, H, K],
 //     total decays [places, H]
 // 4,096 tokens, 4 heads of 256 x 512, us under ncu (cold caches): gates of the tokens 17, of the chunks 11, state 76, carries 28, outputs 92; in
-// a run 210 in all, where the same chunks took 395 in plain multiply-adds and those of 64 tokens take 438.  Errors against 64 bits, of the
+// a run 213 in all, where the same chunks took 395 in plain multiply-adds and those of 64 tokens take 438.  Errors against 64 bits, of the
 // read-outs 2.0 to 2.6e-7 (plain multiply-adds 3.8 to 4.3e-7), of the memories 1.7 to 2.9e-7 (2.1 to 3.3e-7).
 // ---------------------------------------------------------------------------------
 #define ML_TOKENS CT_TOKENS

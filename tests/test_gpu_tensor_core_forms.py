@@ -844,7 +844,7 @@ def test_experts_read_once_for_all_their_tokens(T, E, top, D, F, Fs, activation,
     x, up, down = (torch.randn(*s, device=DEV).mul(f).to(torch.bfloat16) for s, f in (((T, D), 1.0), ((E, (2 if gated else 1) * F, D), D ** -0.5), ((E, D, F), F ** -0.5)))
     su, sd, gate = (None, None, None) if not Fs else (torch.randn(Fs, D, device=DEV).mul(D ** -0.5).to(torch.bfloat16), torch.randn(D, Fs, device=DEV).mul(Fs ** -0.5).to(torch.bfloat16), torch.rand(T, device=DEV))
     logits = torch.randn(T, E, device=DEV)
-    logits[:, 0] += 3.0 if T != 140 else 1e3                # most tokens choose the first one, few the last; 140: all of them, more than four slots
+    logits[:, 0] += 3.0                                     # most tokens choose the first one, few the last
     logits[:, -1] -= 3.0 * (E > top)
     chosen, weight = ops.moe_route(logits, top)
     act = {"relu2": lambda z: torch.relu(z).square(), "gelu": lambda z: torch.nn.functional.gelu(z, approximate="tanh"), "silu": torch.nn.functional.silu}
@@ -886,14 +886,17 @@ def test_any_number_of_experts(T, E):
 
 @pytest.mark.parametrize("dtype, classes", [(torch.float32, [(1, 2, 3, 8, 40)]), (torch.bfloat16, [(1, 2, 3, 5, 7), (8, 9, 24, 130, 500)])])
 @pytest.mark.parametrize("Fs", [0, 24, 72, 136])
-def test_a_token_s_experts_are_the_same_bits_beside_others(dtype, classes, Fs):
+@pytest.mark.parametrize("skew", [0.0, 3.0, 1e3])
+def test_a_token_s_experts_are_the_same_bits_beside_others(dtype, classes, Fs, skew):
     """Within a form (the rows for each copy; an expert's rows once for all of its tokens) a token's sums have one order, whatever the
-    number of tokens and whoever else chose its experts."""
+    number of tokens and whoever else chose its experts: most of them the same ones, or all, in many slots an expert."""
     torch.manual_seed(Fs)
     E, top, D, F = 64, 6, 264, 40
     x, up, down = (torch.randn(*s, device=DEV).mul(f).to(dtype) for s, f in (((500, D), 1.0), ((E, F, D), D ** -0.5), ((E, D, F), F ** -0.5)))
     su, sd = (torch.randn(Fs, D, device=DEV).mul(D ** -0.5).to(dtype), torch.randn(D, Fs, device=DEV).mul(Fs ** -0.5).to(dtype)) if Fs else (None, None)
-    chosen, weight = ops.moe_route(torch.randn(500, E, device=DEV), top)
+    logits = torch.randn(500, E, device=DEV)
+    logits[:, 5:5 + top] += skew
+    chosen, weight = ops.moe_route(logits, top)
     gate = torch.rand(500, device=DEV) if Fs else None
     for sizes in classes:
         outs = [ops.moe_experts(x[:n], up, down, chosen[:n], weight[:n], "relu2", su, sd, gate[:n] if Fs else None) for n in sizes]
